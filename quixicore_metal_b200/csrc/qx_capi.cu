@@ -189,9 +189,8 @@ qx_status qx_cuda_decode_linear_partial(void* stream, const void* x, const void*
   st = bind_scratch(op, (cudaStream_t)stream, projection_scratch_bytes(a), workspace, workspace_bytes, &hold,
                     &a.scratch, &a.scratch_bytes);
   if (st.code != QX_OK) return st;
-  if (stream_path_ok(a) && launch_gemv_stream((cudaStream_t)stream, a)) return check_launch(op);
-  if (stream_passes_ok(a) && launch_gemv_stream_passes((cudaStream_t)stream, a)) return check_launch(op);
-  if (tc_path_ok(a) && launch_gemm_tc((cudaStream_t)stream, a)) return check_launch(op);
+  bool fused = false;
+  if (launch_tensor_core((cudaStream_t)stream, a, &fused)) return check_launch(op);
   return fail(QX_UNSUPPORTED_LAYOUT, op,
               "fp32 partial projections need bf16/f16 activations, 16-byte aligned bases and K a "
               "multiple of 512 columns");

@@ -7,22 +7,33 @@ namespace qx {
 size_t projection_scratch_bytes(const GemvArgs& a) {
   if (options().force_generic) return 0;
   const size_t s = stream_scratch_bytes(a);
-  const size_t t = tc_scratch_bytes(a);
-  return s > t ? s : t;
+  size_t t = tc_scratch_bytes(a);
+  if (t < s) t = s;
+  const size_t u = ts_scratch_bytes(a);
+  return t > u ? t : u;
+}
+
+// The tensor-core kernels, in order of preference; false when none serves the call.  *fused: the kernel
+// also wrote the requested MXFP8 output rows.
+bool launch_tensor_core(cudaStream_t st, const GemvArgs& a, bool* fused) {
+  const bool fusable = a.out_quant == OQ_MXFP8 && !a.out_f32 && a.N % 32 == 0 && a.q_codes;
+  *fused = false;
+  if (options().force_generic) return false;
+  const bool passes_first = options().stream_passes == 2 && stream_passes_ok(a);
+  if (!passes_first && launch_ts(st, a, fused)) return true;
+  *fused = fusable;
+  if (stream_path_ok(a) && launch_gemv_stream(st, a)) return true;
+  if (stream_passes_ok(a) && launch_gemv_stream_passes(st, a)) return true;
+  if (tc_path_ok(a) && launch_gemm_tc(st, a, fused)) { *fused = fusable && *fused; return true; }
+  *fused = false;
+  return false;
 }
 
 // Returns true when the kernel that ran also wrote the requested MXFP8 output rows; every other
 // output quantisation is a second launch by the caller.
 bool launch_projection(cudaStream_t st, const GemvArgs& a) {
-  const bool fusable = a.out_quant == OQ_MXFP8 && !a.out_f32 && a.N % 32 == 0 && a.q_codes;
-  if (!options().force_generic) {
-    if (stream_path_ok(a) && launch_gemv_stream(st, a)) return fusable;
-    if (stream_passes_ok(a) && launch_gemv_stream_passes(st, a)) return fusable;
-    if (tc_path_ok(a)) {
-      bool fused = false;
-      if (launch_gemm_tc(st, a, &fused)) return fusable && fused;
-    }
-  }
+  bool fused = false;
+  if (launch_tensor_core(st, a, &fused)) return fused;
   launch_gemv_generic(st, a);
   return false;
 }

@@ -38,6 +38,7 @@ struct Options {
   int stream_passes = 1;        // 17 - 64 rows as passes of the streaming kernel: 0 never, 1 when faster, 2 whenever possible
   bool force_generic = false;   // keep every call on the shape-generic kernels
   bool tc_pipeline = true;      // batch > 16 on the tcgen05 pipeline
+  int ts_min_rows = 0;          // batch from which the tensor-memory-operand kernel serves a call; 0: by rows and bytes
   bool lm_head_ksplit = true;   // share the items of a partial round over K between CTAs
 };
 const Options& options();
@@ -58,6 +59,9 @@ bool launch_gemv_stream_passes(cudaStream_t st, const GemvArgs& a);
 bool tc_path_ok(const GemvArgs& a);
 // *fused_quant (optional): set when the kernel that ran packed the requested MXFP8 output rows itself
 bool launch_gemm_tc(cudaStream_t st, const GemvArgs& a, bool* fused_quant = nullptr);
+// Tensor-memory-operand kernel (16-bit activations, K % 256 == 0): see qx_ts.cuh.
+size_t ts_scratch_bytes(const GemvArgs& a);
+bool launch_ts(cudaStream_t st, const GemvArgs& a, bool* fused_quant);
 // Value of the device-side error flag that bounded waits raise (synchronises the device).
 int read_device_error_flag();
 // Device address of that flag on the current device (nullptr if it cannot be resolved).
@@ -75,6 +79,7 @@ void launch_prep_activations(cudaStream_t st, const void* x, qx_dtype dtype, __h
 // Picks the kernel family for one projection call (format, dtype, batch, alignment); true when the
 // kernel that ran also wrote the requested MXFP8 output rows.
 bool launch_projection(cudaStream_t st, const GemvArgs& a);
+bool launch_tensor_core(cudaStream_t st, const GemvArgs& a, bool* fused_quant);
 
 // Per-row allow mask of lm_head_masked: bit (v & 31) of word bits[t * words + (v >> 5)] admits global
 // vocabulary id v for hidden row t; norm_allowed: the log-sum-exp runs over admitted ids only.

@@ -1,0 +1,338 @@
+// Host side and projection epilogue of the tensor-memory-operand kernel (qx_ts.cuh): plans, tensor maps,
+// activation preparation, and the launches behind decode_linear_epilogue / decode_swiglu.
+#include "qx_kernels.h"
+#include "qx_tmap.h"
+#include "qx_ts.cuh"
+
+namespace qx {
+
+static size_t round256(size_t n) { return (n + 255) & ~(size_t)255; }
+
+struct TsGeom { int bytes, pitch, terms; };
+static TsGeom ts_geom(int f) {
+  switch (f) {
+    case F_Q4_0: return {TsFmt<F_Q4_0>::BYTES, TsFmt<F_Q4_0>::PITCH, TsFmt<F_Q4_0>::TERMS};
+    case F_Q8_0: return {TsFmt<F_Q8_0>::BYTES, TsFmt<F_Q8_0>::PITCH, TsFmt<F_Q8_0>::TERMS};
+    case F_Q6_K: return {TsFmt<F_Q6_K>::BYTES, TsFmt<F_Q6_K>::PITCH, TsFmt<F_Q6_K>::TERMS};
+    case F_MXFP8: return {TsFmt<F_MXFP8>::BYTES, TsFmt<F_MXFP8>::PITCH, TsFmt<F_MXFP8>::TERMS};
+    case F_NVFP4: return {TsFmt<F_NVFP4>::BYTES, TsFmt<F_NVFP4>::PITCH, TsFmt<F_NVFP4>::TERMS};
+    default: return {TsFmt<F_MXFP4>::BYTES, TsFmt<F_MXFP4>::PITCH, TsFmt<F_MXFP4>::TERMS};
+  }
+}
+
+// K in whole raw stages (so every row is a multiple of 8 bytes; q6_K of 2), 16-byte aligned matrices.
+bool ts_shape_ok(int format, int64_t K, int64_t N, const void* w0, const void* w1) {
+  return K % TS_KC == 0 && N >= 16 && (((uintptr_t)w0 | (uintptr_t)w1) & 15) == 0;
+}
+
+bool ts_plan(TsPlan* p, int format, int64_t M, int64_t K, int64_t N, int rb, int dual, int max_group, size_t aux, bool may_cut) {
+  const TsGeom g = ts_geom(format);
+  const int64_t row_bytes = K / TS_KC * g.bytes;
+  p->dual = dual; p->rb = dual ? 2 : rb;
+  p->P = 1;
+  while ((row_bytes * p->P) % 16 != 0) p->P *= 2;
+  p->groups = (int)((M + max_group - 1) / max_group);
+  p->mg = (int)((M + p->groups - 1) / p->groups);
+  p->nb = (p->mg + 15) / 16 * 16;
+  p->mp = p->mg <= 1 ? 1 : (p->mg <= 2 ? 2 : (p->mg <= 4 ? 4 : (p->mg <= 8 ? 8 : p->nb)));
+  p->tile_rows = dual ? 128 : 128 * rb;
+  p->tiles = (int)((N + p->tile_rows - 1) / p->tile_rows);
+  p->nks = (int)(K / TS_KC);
+  p->items = p->tiles * p->groups;
+  // TMEM (512 columns): running sums and two chunk buffers of rb * nb columns, the rest operand slots, at least
+  // one per worker group (so that a group's waits are never two ring rounds apart).  With two row blocks one chunk
+  // buffer is enough: the blocks take turns.  Without room for the sums (128 rows and two blocks) an
+  // item is one chunk - a format whose terms are short enough for that only (max_group).
+  const int slot = 32 * g.terms, acc = p->rb * p->nb, least = 4 * slot;
+  p->sums = 1;
+  if (3 * acc + 2 * least <= 512) p->nd = 2;
+  else if (p->rb == 2 && 2 * acc + 2 * least <= 512) p->nd = 1;      // eight slots (two issuers) before a second buffer
+  else if (3 * acc + least <= 512) p->nd = 2;
+  else if (2 * acc + least <= 512) p->nd = 1;
+  else if (acc + least <= 512) { p->sums = 0; p->nd = 1; }
+  else return false;
+  p->na = (512 - (p->sums + p->nd) * acc) / slot;
+  p->na = p->na >= 16 && format != F_Q6_K ? 16 : (p->na >= 8 && format != F_Q6_K ? 8 : 4);
+  p->issuers = p->rb == 2 && p->na >= 8 ? 2 : 1;
+  // activation stages of 256 columns; from 48 rows on they are handed over by quarters, so that a ring of two
+  // (or one) keeps flowing
+  p->actq = p->mp <= 32 ? 1 : 4;
+  const size_t act_stage = (size_t)TS_KC * p->mp * 2;
+  p->nact = p->mp <= 16 ? 4 : (p->mp <= 32 ? 3 : (p->mp <= 80 ? 2 : 1));
+  const size_t stage = (size_t)128 * g.pitch;
+  const size_t bar_bytes = 8 * (2 * TS_MAX_RAW + 2 * TS_MAX_ACT + 2 * TS_MAX_SLOTS + 12) + 4 * (4 + TS_MARK_RING * 8 + 128);
+  const size_t act = (act_stage * p->nact + 256 + 127) & ~(size_t)127;   // + what overlapping core matrices read past the end
+  const size_t fixed = act + ((aux + 127) & ~(size_t)127) + bar_bytes + 128;
+  if (fixed + 2 * stage > 227 * 1024) return false;
+  p->nraw = (int)((227 * 1024 - fixed) / stage);
+  if (p->nraw > TS_MAX_RAW) p->nraw = TS_MAX_RAW;
+  if (format == F_Q6_K) p->nraw &= ~1;               // its worker groups alternate stages: a slot always has the same readers
+  p->off_act = stage * p->nraw;
+  p->off_aux = p->off_act + act;
+  p->off_bar = p->off_aux + ((aux + 127) & ~(size_t)127);
+  p->smem = p->off_bar + bar_bytes + 128;
+  // grid: every SM, a multiple of the groups, no CTA without a unit
+  const int sms = sm_count();
+  if (p->groups > sms || (int64_t)p->tiles * p->nks >= (1 << 30)) return false;
+  p->whole = may_cut ? 0 : 1;
+  const int64_t units = may_cut ? (int64_t)p->tiles * p->nks : p->tiles;
+  const int64_t per = sms / p->groups;
+  p->grid = (unsigned)((per < units ? per : units) * p->groups);
+  p->img_bytes = round256((size_t)p->groups * p->mp * K * 2);
+  p->scale_bytes = round256((size_t)M * 4);
+  p->count_bytes = may_cut ? round256((size_t)p->items * 4) : 0;
+  p->part_bytes = (size_t)p->grid * 4 * p->rb * p->nb * 128 * 4;
+  return true;
+}
+
+TsScratch ts_carve(const TsPlan& p, void* scratch) {
+  char* c = (char*)scratch;
+  TsScratch s;
+  s.img = (uint8_t*)c;
+  s.rowscale = (float*)(c + p.img_bytes);
+  s.count = (unsigned*)(c + p.img_bytes + p.scale_bytes);
+  s.part = (float*)(c + p.img_bytes + p.scale_bytes + p.count_bytes);
+  return s;
+}
+
+bool ts_maps(const TsPlan& p, int format, const void* w, int64_t K, int64_t N, CUtensorMap* m) {
+  const TsGeom g = ts_geom(format);
+  const int64_t row_bytes = K / TS_KC * g.bytes;
+  if (p.P == 1) {
+    if (!cached_box_map(&m[0], w, 4, row_bytes / 4, N, (size_t)row_bytes, g.pitch / 4, 128)) return false;
+    m[1] = m[0];
+    return true;
+  }
+  const int64_t full = N / p.P, rest = N % p.P;
+  const size_t pitch = (size_t)(row_bytes * p.P);
+  if (!cached_box_map(&m[1], w, 2, row_bytes * p.P / 2, full, pitch, g.pitch / 2, 128 / p.P)) return false;
+  m[0] = m[1];
+  // the last, partial super-row holds `rest` rows: nothing past the matrix may be touched
+  return rest == 0 || cached_box_map(&m[0], w, 2, row_bytes * rest / 2, full + 1, pitch, g.pitch / 2, 128 / p.P);
+}
+
+// ---- activation preparation ------------------------------------------------------------------------
+// One CTA per row: largest finite magnitude -> power-of-two scale 2^-S that puts it in [2^14, 2^15), then
+// f16(x * 2^-S) into the image [group][K / 8][mp][8] (16-byte chunks of one row, mp rows side by side: the
+// unswizzled operand layout), 32-column units in the decoder's order.  Latency-bound: a row is one pass
+// over 2 K bytes, the second read hits L1.  Rows past the group's end are never read back.
+template <typename T>
+__global__ void __launch_bounds__(256)
+ts_prep_kernel(const T* __restrict__ x, uint4* __restrict__ img, float* __restrict__ rowscale, unsigned* __restrict__ count,
+               int ncount, int K, int mg, int mp, int fmt) {
+  __shared__ float red[8];
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int m = blockIdx.x;
+  if (m == 0)
+    for (int i = threadIdx.x; i < ncount; i += blockDim.x) count[i] = 0u;
+  const uint4* xv = reinterpret_cast<const uint4*>(x + (size_t)m * K);
+  float amax = 0.f;
+  for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
+    const uint4 v = __ldg(xv + i);
+    const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const float a = fabsf(to_f32<T>(e[j]));
+      if (a < 3.0e38f) amax = fmaxf(amax, a);                        // inf / nan do not choose the scale
+    }
+  }
+  amax = warp_max(amax);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
+  __syncthreads();
+  amax = red[0];
+#pragma unroll
+  for (int i = 1; i < 8; ++i) amax = fmaxf(amax, red[i]);
+  int S = 0;
+  if (amax > 0.f) {
+    S = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 - 14;
+    S = max(-110, min(110, S));
+  }
+  const float down = __uint_as_float((uint32_t)(127 - S) << 23);
+  const int grp = m / mg, ml = m - grp * mg;
+  uint4* out = img + ((size_t)grp * (K / 8)) * mp + ml;
+  // a thread makes one 16-byte chunk (8 positions) of a unit; its source columns lie in the unit's 64 bytes
+  for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
+    const int u = i >> 2, c4 = i & 3;
+    __half h[8];
+    if (fmt == F_Q4_0 || fmt == F_MXFP4 || fmt == F_NVFP4) {
+      const T* xu = x + (size_t)m * K + (size_t)u * 32;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int pos = 8 * c4 + j;                                  // inverse of ts_position
+        int c;
+        if (fmt == F_NVFP4) c = (pos & 16) | ((pos & 15) >> 1) | ((pos & 1) << 3);
+        else if (fmt == F_MXFP4) c = (pos >> 1) | ((pos & 1) << 4);
+        else c = ((pos >> 1) & 1) * 16 + (pos >> 3) * 4 + (((pos >> 2) & 1) | ((pos & 1) << 1));
+        h[j] = __float2half_rn(to_f32<T>(xu[c]) * down);
+      }
+    } else {
+      const uint4 v = __ldg(xv + i);
+      const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) h[j] = __float2half_rn(to_f32<T>(e[j]) * down);
+    }
+    out[(size_t)i * mp] = *reinterpret_cast<const uint4*>(h);
+  }
+  if (threadIdx.x == 0) rowscale[m] = __uint_as_float((uint32_t)(127 + S) << 23);
+}
+
+void ts_launch_prep(cudaStream_t st, const TsPlan& p, int format, const void* x, qx_dtype dtype, const TsScratch& s, int M, int K) {
+  const int ncount = p.whole ? 0 : p.items;
+  if (dtype == QX_DTYPE_F16)
+    ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__half>, (const __half*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
+  else
+    ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
+}
+
+// ---- projection epilogue ------------------------------------------------------------------------------
+struct TsProj {
+  struct Args {
+    const void* bias0; const void* bias1; const void* residual; void* y;
+    int half;                 // I/O type: 1 f16, 0 bf16 (bias, residual, output)
+    int raw;                  // output fp32 dots, nothing else applied
+    int activation, use_bias, use_residual;
+    uint8_t* mx;              // MXFP8 rows of the rounded output (N % 32 == 0)
+  };
+  __device__ __forceinline__ static float load(const void* p, size_t i, int half) {
+    const uint16_t b = reinterpret_cast<const uint16_t*>(p)[i];
+    return half ? __half2float(__ushort_as_half(b)) : __uint_as_float((uint32_t)b << 16);
+  }
+  // Four columns at a time; warps 0..3 take the even groups of four, warps 4..7 the odd ones, a lane one weight row.
+  // The MXFP8 rows are packed from the stored outputs of the same warp.
+  __device__ __forceinline__ static void sum4(const TsItem& it, size_t at, float (&v)[4]) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = __ldcg(it.first + at + i * 128);
+#pragma unroll 2
+    for (int k = 1; k < it.parts; ++k) {
+      const float* s = it.part(k) + at;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] += __ldcg(s + i * 128);
+    }
+  }
+  __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, uint8_t*, int warp,
+                                             int lane) {
+    const TsPlan& p = q.p;
+    const int blocks = p.dual ? 1 : p.rb;
+    const int row = (warp & 3) * 32 + lane;
+#pragma unroll 1
+    for (int rb = 0; rb < blocks; ++rb) {
+      const int n = it.tile * p.tile_rows + rb * 128 + row;
+      if (n >= q.N) continue;
+      const float b0 = a.use_bias ? load(a.bias0, n, a.half) : 0.f;
+      const float b1 = p.dual && a.use_bias ? load(a.bias1, n, a.half) : 0.f;
+#pragma unroll 1
+      for (int c = (warp >> 2) * 4; c < it.m_count; c += 8) {
+        float v[4], w[4] = {0.f, 0.f, 0.f, 0.f};
+        const size_t o0 = (size_t)(it.m_base + c) * q.N + n;
+        if (a.use_residual) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) if (c + i < it.m_count) w[i] = load(a.residual, o0 + (size_t)i * q.N, a.half);
+        }
+        sum4(it, ((size_t)rb * p.nb + c) * 128 + row, v);
+        if (p.dual) sum4(it, ((size_t)p.nb + c) * 128 + row, w);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          if (c + i >= it.m_count) break;
+          const size_t o = o0 + (size_t)i * q.N;
+          float d = v[i] * scale[c + i];
+          if (a.raw) { reinterpret_cast<float*>(a.y)[o] = d; continue; }
+          if (p.dual) d = silu(d + b0) * (w[i] * scale[c + i] + b1);
+          else d = apply_act(d + b0, a.activation) + w[i];
+          reinterpret_cast<uint16_t*>(a.y)[o] = a.half ? __half_as_ushort(__float2half_rn(d)) : __bfloat16_as_ushort(__float2bfloat16_rn(d));
+        }
+      }
+      if (a.mx) {                                    // N % 32 == 0: 32 lanes = 32 consecutive channels
+#pragma unroll 1
+        for (int c = (warp >> 2) * 4; c < it.m_count; c += 8) {
+          const int e = min(c + 4, it.m_count);
+#pragma unroll 2
+          for (int m = c; m < e; ++m) {
+            const float r = load(a.y, (size_t)(it.m_base + m) * q.N + n, a.half);
+            mxfp8_block_store(r, lane, a.mx + ((size_t)(it.m_base + m) * (q.N >> 5) + (n >> 5)) * 33);
+          }
+        }
+      }
+    }
+  }
+  __device__ __forceinline__ static void tail(const Args&, const TsParams&, uint8_t*, int, int) {}
+};
+
+// Row blocks per item: two share every activation stage (half the L2 reads of the activations) while there
+// are enough of them to keep the cut items few.
+static int ts_blocks(const GemvArgs& a) { return a.N >= 128 * 148 ? 2 : 1; }
+
+// Activation rows per group: 64 with running sums; nvfp4 and mxfp4, whose products have at most 14 bits, take 128 in
+// one chunk per item (error at K = 8192: 1e-6 and 4e-7), which decodes the weights half as often.
+static bool ts_projection_plan(const GemvArgs& a, TsPlan* p) {
+  if (a.dtype != QX_DTYPE_BF16 && a.dtype != QX_DTYPE_F16) return false;
+  if (a.M < 2 || a.M > 0xFFFF || ((uintptr_t)a.x & 15) != 0 || !ts_shape_ok(a.format, a.K, a.N, a.w0, a.w1)) return false;
+  const bool short_terms = a.format == F_NVFP4 || a.format == F_MXFP4;
+  const int rb = a.format == F_Q6_K && a.M > 32 && !a.w1 ? 1 : ts_blocks(a);
+  const int group = a.format == F_Q6_K ? (a.w1 ? 32 : 64) : (short_terms ? 128 : 64);
+  return ts_plan(p, a.format, a.M, a.K, a.N, rb, a.w1 != nullptr, group, 0, true);
+}
+
+// Where this kernel takes over from the 16-row streaming kernel (and its passes).  Measured, K = 8192 -> N = 28672 and
+// 4096 -> 4096, us, streaming / this kernel:  nvfp4 16 rows 52 / 40 and 11 / 17; 32 rows (one pass) 102 / 45 and
+// 15 / 20; 64 rows 117 / 59 and 28 / 24.  Its time hardly depends on the rows, but a call pays about 10 us for
+// preparation, start-up and the sum over cut items, so small matrices stay where they are up to 32 rows.
+bool ts_preferred(const GemvArgs& a) {
+  const int first = options().ts_min_rows;
+  if (first > 0) return a.M >= first;
+  const int64_t bytes = a.N * (a.K / block_k_of(a.format)) * block_bytes_of(a.format) * (a.w1 ? 2 : 1);
+  if (a.M > 32) return true;
+  if (a.M > 16) return bytes >= (a.w1 ? (16 << 20) : (28 << 20));
+  if (a.M > 8) return bytes >= (a.format == F_MXFP4 || a.format == F_MXFP8 ? (56 << 20) : (100 << 20)) && a.format != F_Q6_K;
+  return false;
+}
+
+size_t ts_scratch_bytes(const GemvArgs& a) {
+  TsPlan p;
+  return ts_preferred(a) && ts_projection_plan(a, &p) ? p.scratch() : 0;
+}
+
+template <int FMT>
+static bool launch_ts_fmt(cudaStream_t st, const GemvArgs& a, const TsPlan& p, int* err, bool* fused) {
+  static bool attr_set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (dev < 0 || dev >= 64) return false;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(ts_kernel<FMT, TsProj>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    attr_set[dev] = true;
+  }
+  CUtensorMap m[4];
+  if (!ts_maps(p, FMT, a.w0, a.K, a.N, m)) return false;
+  if (a.w1) { if (!ts_maps(p, FMT, a.w1, a.K, a.N, m + 2)) return false; }
+  else { m[2] = m[0]; m[3] = m[1]; }
+  const TsScratch s = ts_carve(p, a.scratch);
+  TsParams q{p, {(const uint8_t*)a.w0, (const uint8_t*)a.w1}, a.x, a.dtype == QX_DTYPE_BF16, s.img, s.rowscale, s.part, s.count,
+             (int)a.M, (int)a.K, (int)a.N, err};
+  *fused = a.out_quant == OQ_MXFP8 && !a.out_f32 && a.N % 32 == 0 && a.q_codes;
+  const TsProj::Args ea{a.bias0, a.bias1, a.residual, a.y, a.dtype == QX_DTYPE_F16, a.out_f32, a.activation, a.use_bias,
+                        a.use_residual, *fused ? (uint8_t*)a.q_codes : nullptr};
+  ts_launch_prep(st, p, FMT, a.x, a.dtype, s, (int)a.M, (int)a.K);
+  return ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsProj>, m[0], m[1], m[2], m[3], q, ea);
+}
+
+bool launch_ts(cudaStream_t st, const GemvArgs& a, bool* fused) {
+  *fused = false;
+  TsPlan p;
+  if (!ts_preferred(a) || !ts_projection_plan(a, &p) || !a.scratch || a.scratch_bytes < p.scratch()) return false;
+  int* err = device_error_flag();
+  if (!err) return false;
+  switch (a.format) {
+    case F_Q4_0: return launch_ts_fmt<F_Q4_0>(st, a, p, err, fused);
+    case F_Q8_0: return launch_ts_fmt<F_Q8_0>(st, a, p, err, fused);
+    case F_Q6_K: return launch_ts_fmt<F_Q6_K>(st, a, p, err, fused);
+    case F_MXFP8: return launch_ts_fmt<F_MXFP8>(st, a, p, err, fused);
+    case F_NVFP4: return launch_ts_fmt<F_NVFP4>(st, a, p, err, fused);
+    default: return launch_ts_fmt<F_MXFP4>(st, a, p, err, fused);
+  }
+}
+
+}  // namespace qx

@@ -287,7 +287,7 @@ static size_t partial_bytes(int64_t T, int64_t V, int mode, int topk) {
 
 size_t qx_cuda_lm_head_workspace_bytes(int64_t T, int64_t V, int64_t K, int mode, int topk) {
   if (T <= 0 || V <= 0 || K <= 0) return 0;
-  return partial_bytes(T, V, mode, topk) + lm_head_scratch_full_bytes(T, K);
+  return partial_bytes(T, V, mode, topk) + lm_head_scratch_full_bytes(T, V, K);
 }
 
 }  // extern "C"
@@ -308,7 +308,7 @@ qx_status lm_head_sample_on(const char* op, void* stream, const void* h, const v
   if (mode == 3 && !(top_p > 0.0 && top_p <= 1.0))
     return fail(QX_INVALID_ARGUMENT, op, "topp requires top_p in (0, 1]");
   const size_t pbytes = partial_bytes(T, V, mode, topk);
-  const size_t need = pbytes + (min_only ? lm_head_scratch_min_bytes(T, K) : lm_head_scratch_full_bytes(T, K));
+  const size_t need = pbytes + (min_only ? lm_head_scratch_min_bytes(T, K) : lm_head_scratch_full_bytes(T, V, K));
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255) != 0)
     return fail(QX_INSUFFICIENT_WORKSPACE, op, "workspace must be 256-byte aligned and at least qx_cuda_lm_head_workspace_bytes");
   if (!device_ready(op, &st)) return st;
@@ -513,7 +513,7 @@ static qx_status check_head_weight(const char* op, const void* h, const void* w,
 
 size_t qx_cuda_lm_head_masked_workspace_bytes(int64_t T, int64_t V, int64_t K, int topk) {
   if (T <= 0 || V <= 0 || K <= 0 || topk <= 0) return 0;
-  return partial_bytes(T, V, 3, topk) + lm_head_scratch_full_bytes(T, K);
+  return partial_bytes(T, V, 3, topk) + lm_head_scratch_full_bytes(T, V, K);
 }
 
 qx_status qx_cuda_lm_head_masked(void* stream, const void* h, const void* w, const float* bias,
@@ -577,7 +577,7 @@ qx_status qx_cuda_lm_head_candidates(void* stream, const void* h, const void* w,
 size_t qx_cuda_lm_head_beam_workspace_bytes(int64_t rows, int64_t V, int64_t K, int beam_width) {
   if (rows <= 0 || V <= 0 || K <= 0 || beam_width <= 0) return 0;
   return partial_bytes(rows, V, 3, 2 * beam_width) + 2 * align256((size_t)rows * 2 * beam_width * 4) +
-         lm_head_scratch_full_bytes(rows, K);
+         lm_head_scratch_full_bytes(rows, V, K);
 }
 
 qx_status qx_cuda_lm_head_beam_advance(void* stream, const void* h, const void* wq, const float* bias,
@@ -628,7 +628,7 @@ int64_t qx_cuda_lm_head_shard_candidates(int mode, int topk, int64_t max_tiles) 
 
 size_t qx_cuda_lm_head_shard_workspace_bytes(int64_t T, int64_t V_local, int64_t K, int mode, int topk) {
   if (T <= 0 || V_local <= 0 || K <= 0) return 0;
-  size_t n = lm_head_scratch_full_bytes(T, K);
+  size_t n = lm_head_scratch_full_bytes(T, V_local, K);
   if (mode != 3) {
     const size_t kk = mode == 2 ? (size_t)(topk > 0 ? topk : 1) : 1;
     n += 2 * align256((size_t)T * (size_t)tiles_of(V_local) * kk * 4);

@@ -102,7 +102,7 @@ struct LmHeadArgs {
 // Minimum scratch of stage 1 (without exchange slots: items are then not shared) and the size
 // with which every sharing choice fits.
 size_t lm_head_scratch_min_bytes(int64_t T, int64_t K);
-size_t lm_head_scratch_full_bytes(int64_t T, int64_t K);
+size_t lm_head_scratch_full_bytes(int64_t T, int64_t V, int64_t K);
 // part_val/part_id: (T, tiles_stride, kk) with kk = 1 (modes 0/1) or topk; part_lse: (T, tiles_stride)
 void launch_lm_head_partials(cudaStream_t st, const LmHeadArgs& a, float* part_val,
                              int32_t* part_id, float* part_lse, int64_t tiles_stride);

@@ -19,6 +19,7 @@
 #include "qx_kernels.h"
 #include "qx_stream.cuh"
 #include "qx_tmap.h"
+#include "qx_ts.cuh"
 
 namespace qx {
 
@@ -453,6 +454,7 @@ template <> struct LmhCfg<F_MXFP8> { static constexpr int KC = 128, STAGES = 2; 
 #endif
 constexpr int LMH_LOGIT_PITCH = 257;
 constexpr int LMH_TOK_CHUNK = 16;
+constexpr int LMH_STREAM_ROWS = 16;      // hidden rows up to which the streaming kernel is the faster form
 
 // WROWS = vocabulary rows per warp: 32 (8 warps, two m-tiles share every activation fragment) or
 // 16 (16 warps: more loads in flight; used from 9 hidden rows per pass).
@@ -628,111 +630,55 @@ lmh_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __half* __rest
   }
 }
 
-}  // namespace qx
-#include "qx_tc_pipeline.cuh"
-namespace qx {
-
-// Epilogue of the tensor-core pipeline for LM-head stage 1: the worker warps move the logits of the
-// item's 256 vocabulary rows to shared memory ([hidden row][256]), then every warp reduces hidden
-// rows to their tile partials.
-template <int BN>
-struct LmhEpi {
+// Output policy of the tensor-memory-operand kernel (qx_ts.cuh) for LM-head stage 1: each of the 8 output warps
+// brings the 256 logits of two hidden rows at a time to shared memory and reduces them to their tile
+// partials, while the other roles work on the next tile.
+constexpr size_t LMH_TS_AUX = (size_t)TS_OUT * 2 * LMH_TILE * 4;
+struct TsLmHead {
   struct Args {
     const float* bias;
     float* part_val; int32_t* part_id; float* part_lse;
-    int T_total, V;
     long long vocab_offset, tiles_stride;
     int mode, topk;
     float invtemp;
     uint32_t seed;
-    // items shared by several CTAs (each took a slice of K): where the other CTAs leave their partial
-    // logits ([shared item][part - 1][BN * 256] floats), the flags that say so, and the value that
-    // means "written during this launch"
-    float* xchg; unsigned* flags; unsigned epoch;
-    int* err_flag;
     LmhMask mask;
   };
-  static constexpr bool DUAL = false;
-  __device__ __forceinline__ static void run(const Args& a, const TcItem& it) {
-    constexpr int CW = BN / 4;
-    if (it.warp < LTC_DQW) {
-      const uint32_t lane_sel = (uint32_t)((it.warp & 3) * 32) << 16;
-      const int RS = (it.warp & 3) * 32 + it.lane;
-      const int cg = it.warp >> 2;
+  __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, uint8_t* aux,
+                                             int warp, int lane) {
+    float* logit = reinterpret_cast<float*>(aux) + warp * 2 * LMH_TILE;
+    const int v0 = it.tile * LMH_TILE, nvalid = min(LMH_TILE, q.N - v0);
+#pragma unroll 1
+    for (int m0 = warp; m0 < it.m_count; m0 += 2 * TS_OUT) {
+      const float* rows[2] = {logit, logit + LMH_TILE};
+      const int trow[2] = {it.m_base + m0, m0 + TS_OUT < it.m_count ? it.m_base + m0 + TS_OUT : -1};
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        uint32_t v[CW];
-        tmem_ld_nowait<CW>(it.tmem_base + lane_sel + (uint32_t)(h * BN + cg * CW), v);
-        tmem_wait_ld();
+      for (int r = 0; r < 2; ++r) {
+        const int m = m0 + r * TS_OUT;
+        if (m >= it.m_count) break;
+        float v[8];
 #pragma unroll
-        for (int i = 0; i < CW; ++i) {
-          const int m = cg * CW + i;
-          const float rs = m < it.m_count ? it.rowscale[it.m_base + m] : 0.f;
-          it.smem_f32[m * LMH_TILE + h * 128 + RS] = __uint_as_float(v[i]) * rs;
-        }
-      }
-    }
-    tc_fence_before();
-    __syncthreads();
-    if (it.kparts > 1) {
-      // the logits above are this CTA's slice of K; part 0 collects the others and selects
-      constexpr int N4 = BN * LMH_TILE / 4;
-      const int tid = it.warp * 32 + it.lane;
-      float4* mine = reinterpret_cast<float4*>(it.smem_f32);
-      float* slots = a.xchg + (size_t)it.split_index * (it.kparts - 1) * (BN * LMH_TILE);
-      unsigned* fl = a.flags + it.split_index * (it.kparts - 1);
-      if (it.kpart != 0) {
-        float4* dst = reinterpret_cast<float4*>(slots + (size_t)(it.kpart - 1) * (BN * LMH_TILE));
-        for (int i = tid; i < N4; i += LTC_WARPS * 32) dst[i] = mine[i];
-        __threadfence();
-        __syncthreads();
-        if (tid == 0) asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(fl + it.kpart - 1), "r"(a.epoch) : "memory");
-        return;
-      }
-      if (tid == 0) {
-        for (int p = 1; p < it.kparts; ++p) {
-          bool seen = false;
-          for (int k = 0; k < (1 << 22) && !seen; ++k) {      // bounded: about a second
-            unsigned v;
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(fl + p - 1) : "memory");
-            seen = v == a.epoch;
-            if (!seen) __nanosleep(200);
-          }
-          if (!seen) atomicExch(a.err_flag, 4);
-        }
-      }
-      __syncthreads();
-      for (int p = 1; p < it.kparts; ++p) {
-        const float4* src = reinterpret_cast<const float4*>(slots + (size_t)(p - 1) * (BN * LMH_TILE));
-        for (int i = tid; i < N4; i += LTC_WARPS * 32) {
-          const float4 o = __ldcg(src + i);
-          float4 v = mine[i];
-          v.x += o.x; v.y += o.y; v.z += o.z; v.w += o.w;
-          mine[i] = v;
-        }
-      }
-      __syncthreads();
-    }
-    const int v0 = it.tile * LMH_TILE;
-    const int nvalid = min(LMH_TILE, a.V - v0);
-    // every warp takes up to four hidden rows (warp, warp + 18, ...) and reduces them together
-    constexpr int RPW = (BN + LTC_WARPS - 1) / LTC_WARPS;
-    const float* rows[RPW];
-    int trow[RPW];
+        for (int j = 0; j < 8; ++j) v[j] = __ldcg(it.first + ((size_t)(j >> 2) * q.p.nb + m) * 128 + (j & 3) * 32 + lane);
+#pragma unroll 1
+        for (int k = 1; k < it.parts; ++k) {
+          const float* s = it.part(k) + (size_t)m * 128 + lane;
 #pragma unroll
-    for (int r = 0; r < RPW; ++r) {
-      const int m = it.warp + r * LTC_WARPS;
-      rows[r] = it.smem_f32 + (m < it.m_count ? m : 0) * LMH_TILE;
-      trow[r] = m < it.m_count ? it.m_base + m : -1;
+          for (int j = 0; j < 8; ++j) v[j] += __ldcg(s + (size_t)(j >> 2) * q.p.nb * 128 + (j & 3) * 32);
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) logit[r * LMH_TILE + j * 32 + lane] = v[j] * scale[m];
+      }
+      __syncwarp();
+      lmh_select_rows<2>(rows, trow, nvalid, v0, a.vocab_offset, a.bias, it.tile, a.tiles_stride, a.mode, a.topk, a.invtemp,
+                         a.seed, a.part_val, a.part_id, a.part_lse, lane, a.mask);
+      __syncwarp();
     }
-    lmh_select_rows<RPW>(rows, trow, nvalid, v0, a.vocab_offset, a.bias, it.tile, a.tiles_stride, a.mode, a.topk,
-                         a.invtemp, a.seed, a.part_val, a.part_id, a.part_lse, it.lane, a.mask);
   }
   // padding tiles of a short shard carry absent partials
-  __device__ __forceinline__ static void tail(const Args& a, const float* scratch, int real_tiles, int warp, int lane) {
-    for (long long tile = real_tiles + blockIdx.x; tile < a.tiles_stride; tile += gridDim.x)
-      for (int m = warp; m < a.T_total; m += LTC_WARPS)
-        lmh_select_token(scratch, 0, 0, a.vocab_offset, nullptr, m, (int)tile, a.tiles_stride, a.mode,
+  __device__ __forceinline__ static void tail(const Args& a, const TsParams& q, uint8_t* aux, int warp, int lane) {
+    for (long long tile = q.p.tiles + blockIdx.x; tile < a.tiles_stride; tile += gridDim.x)
+      for (int m = warp; m < q.M; m += TS_OUT)
+        lmh_select_token(reinterpret_cast<const float*>(aux), 0, 0, a.vocab_offset, nullptr, m, (int)tile, a.tiles_stride, a.mode,
                          a.topk, a.invtemp, a.seed, a.part_val, a.part_id, a.part_lse, lane);
   }
 };
@@ -791,125 +737,59 @@ static void launch_lmh_stream_nt(cudaStream_t st, const LmHeadArgs& a, const __h
 }
 
 // ---- stage-1 scratch ----------------------------------------------------------------------------
-// [0, 1 KB)  release flags of K-split items (cleared before every launch that shares items)
-// [1 KB, ..) prepared activations (row-major, or the operand-tile image in groups of 32 / 64 rows)
-// then       one fp32 row scale per hidden row
-// then       exchange slots of K-split items, as far as the scratch reaches
-constexpr size_t LMH_FLAG_BYTES = 1024;
+// Streaming kernel: prepared activations (row-major), one fp32 row scale per hidden row.  Tensor-memory-operand
+// kernel: what its plan asks for (operand image, row scales, tickets, accumulators on their way to the output
+// warps).
 static size_t lmh_round256(size_t n) { return (n + 255) & ~(size_t)255; }
 static size_t lmh_act_bytes(int64_t T, int64_t K) { return lmh_round256((size_t)((T + 63) / 64 * 64) * K * 2); }
 size_t lm_head_scratch_min_bytes(int64_t T, int64_t K) {
-  return LMH_FLAG_BYTES + lmh_act_bytes(T, K) + lmh_round256((size_t)T * 4);
+  return lmh_act_bytes(T, K) + lmh_round256((size_t)T * 4);
 }
-size_t lm_head_scratch_full_bytes(int64_t T, int64_t K) {
-  // at most 3/4 of the SMs hold a partner slot of 64 x 256 floats
-  return lm_head_scratch_min_bytes(T, K) + (T > 16 ? (size_t)(3 * sm_count() / 4) * 64 * LMH_TILE * 4 : 0);
+size_t lm_head_scratch_full_bytes(int64_t T, int64_t V, int64_t K) {
+  const int64_t groups = (T + 63) / 64, nb = ((T + groups - 1) / groups + 15) / 16 * 16;
+  return lm_head_scratch_min_bytes(T, K) + lmh_round256((size_t)((V + LMH_TILE - 1) / LMH_TILE) * groups * 4) +
+         (size_t)sm_count() * 4 * 2 * nb * 128 * 4;
 }
-struct LmhScratch {
-  unsigned* flags; __half* act; float* rowscale; float* xchg; size_t xchg_bytes;
-};
+struct LmhScratch { __half* act; float* rowscale; };
 static bool lmh_carve(const LmHeadArgs& a, LmhScratch* out) {
   const size_t need = lm_head_scratch_min_bytes(a.T, a.K);
   if (!a.scratch || a.scratch_bytes < need) return false;
-  char* p = (char*)a.scratch;
-  out->flags = (unsigned*)p;
-  out->act = (__half*)(p + LMH_FLAG_BYTES);
-  out->rowscale = (float*)(p + LMH_FLAG_BYTES + lmh_act_bytes(a.T, a.K));
-  out->xchg = (float*)(p + need);
-  out->xchg_bytes = a.scratch_bytes - need;
+  out->act = (__half*)a.scratch;
+  out->rowscale = (float*)((char*)a.scratch + lmh_act_bytes(a.T, a.K));
   return true;
 }
 
-// tcgen05 form of stage 1 for more than 16 hidden rows.
-template <int FMT, int BN>
-static bool launch_lmh_tc_bn(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl,
-                             int64_t tiles_stride, int* err) {
-  using S = TcSmem<FMT, BN>;
-  using C = TcCfg<FMT>;
-  using Epi = LmhEpi<BN>;
-  static_assert(S::TOTAL <= 227 * 1024, "stage-1 tensor-core configuration exceeds shared memory");
+// Tensor-memory-operand form of stage 1.
+template <int FMT>
+static bool launch_lmh_ts(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t tiles_stride) {
+  if ((a.dtype != QX_DTYPE_BF16 && a.dtype != QX_DTYPE_F16) || ((uintptr_t)a.h & 15) != 0 || a.T > 0xFFFF ||
+      !ts_shape_ok(FMT, a.K, a.V, a.wq, nullptr))
+    return false;
+  const int group = FMT == F_Q6_K ? 32 : 64;
+  TsPlan p;
+  if (!ts_plan(&p, FMT, a.T, a.K, a.V, 2, 0, group, LMH_TS_AUX, options().lm_head_ksplit)) return false;
+  int* err = device_error_flag();
+  if (!err || !a.scratch || a.scratch_bytes < p.scratch()) return false;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    if (cudaFuncSetAttribute(tc_pipeline_kernel<FMT, BN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) {
+  if (dev < 0 || dev >= 64) return false;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(ts_kernel<FMT, TsLmHead>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
       cudaGetLastError();
       return false;
     }
     attr_set[dev] = true;
   }
-  LmhScratch sc;
-  if (!lmh_carve(a, &sc)) return false;
-  const size_t row_bytes = (size_t)(a.K / StreamFmt<FMT>::BK) * StreamFmt<FMT>::BB;
-  CUtensorMap wmap;
-  if (!cached_weight_map(&wmap, a.wq, a.V, row_bytes, C::BOX)) return false;
-  const int groups = (int)((a.T + BN - 1) / BN);
-  const int real_tiles = (int)((a.V + LMH_TILE - 1) / LMH_TILE);
-  const long long items = (long long)real_tiles * groups;
-  // The last, partial round of items (all items, when there are fewer than SMs - a small vocabulary
-  // shard): when it would leave at least half of the SMs idle, each of its items is shared by 2 or
-  // 4 CTAs that take a slice of K each, as far as the exchange slots fit the scratch.
-  const int nks = (int)(a.K / LTC_KS);
-  const long long sms = sm_count();
-  const long long leftover = items % sms;
-  int ksplit = 1;
-  // not while the stream is being captured: a cooperative launch that fails there would
-  // invalidate the capture, and there is no second attempt inside one
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  cudaStreamIsCapturing(st, &cap);
-  const size_t slot_bytes = (size_t)BN * LMH_TILE * 4;
-  auto fits = [&](int ks) {
-    return (size_t)leftover * (ks - 1) * slot_bytes <= sc.xchg_bytes && (size_t)leftover * (ks - 1) * 4 <= LMH_FLAG_BYTES;
-  };
-  if (options().lm_head_ksplit && leftover > 0 && cap == cudaStreamCaptureStatusNone) {
-    if (leftover * 4 <= sms && nks % 4 == 0 && fits(4)) ksplit = 4;
-    else if (leftover * 2 <= sms && nks % 2 == 0 && fits(2)) ksplit = 2;
-  }
-  const unsigned grid = (unsigned)(items >= sms ? sms : items * ksplit);
-  static std::atomic<unsigned> epoch_counter{1};
-  const unsigned epoch = epoch_counter.fetch_add(1) | 0x40000000u;     // never 0
-  launch_prep_activations(st, a.h, a.dtype, sc.act, sc.rowscale, (int)a.T, (int)a.K, StreamFmt<FMT>::PERM, BN);
-  note_launch();
-  const typename Epi::Args ea{a.bias, pv, pi, pl, (int)a.T, (int)a.V, (long long)a.vocab_offset,
-                              (long long)tiles_stride, a.mode, a.topk, a.invtemp, a.seed,
-                              sc.xchg, sc.flags, epoch, err, a.mask};
-  bool launched = false;
-  if (ksplit > 1) {
-    // the flags start every launch at zero, whatever an earlier user of the scratch left there
-    if (cudaMemsetAsync(sc.flags, 0, LMH_FLAG_BYTES, st) != cudaSuccess) { cudaGetLastError(); ksplit = 1; }
-  }
-  if (ksplit > 1) {
-    // CTAs of this launch wait for one another: ask for a cooperative launch, which only starts
-    // when the whole grid is resident
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(LTC_WARPS * 32);
-    cfg.dynamicSmemBytes = S::TOTAL;
-    cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeCooperative;
-    attr[0].val.cooperative = 1;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    launched = cudaLaunchKernelEx(&cfg, tc_pipeline_kernel<FMT, BN, Epi>, wmap, wmap, (const __half*)sc.act,
-                                  (const float*)sc.rowscale, (int)a.T, (int)a.V, (int)a.K, ksplit, err, ea) == cudaSuccess;
-    if (!launched) { cudaGetLastError(); ksplit = 1; }
-  }
-  if (!launched) {
-    const unsigned grid1 = (unsigned)(items >= sms ? sms : items);
-    tc_pipeline_kernel<FMT, BN, Epi><<<grid1, LTC_WARPS * 32, S::TOTAL, st>>>(
-        wmap, wmap, sc.act, sc.rowscale, (int)a.T, (int)a.V, (int)a.K, 1, err, ea);
-  }
-  note_launch();
-  return true;
-}
-
-template <int FMT>
-static bool launch_lmh_tc(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl,
-                          int64_t tiles_stride, int* err) {
-  if (a.T <= 16 || a.K % LTC_KS != 0 || a.V < 128) return false;
-  if (a.T <= 32) return launch_lmh_tc_bn<FMT, 32>(st, a, pv, pi, pl, tiles_stride, err);
-  return launch_lmh_tc_bn<FMT, 64>(st, a, pv, pi, pl, tiles_stride, err);
+  CUtensorMap m[2];
+  if (!ts_maps(p, FMT, a.wq, a.K, a.V, m)) return false;
+  const TsScratch s = ts_carve(p, a.scratch);
+  const TsParams q{p, {(const uint8_t*)a.wq, nullptr}, a.h, a.dtype == QX_DTYPE_BF16, s.img, s.rowscale, s.part, s.count,
+                   (int)a.T, (int)a.K, (int)a.V, err};
+  const TsLmHead::Args ea{a.bias, pv, pi, pl, (long long)a.vocab_offset, (long long)tiles_stride, a.mode, a.topk, a.invtemp,
+                          a.seed, a.mask};
+  ts_launch_prep(st, p, FMT, a.h, a.dtype, s, (int)a.T, (int)a.K);
+  return ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsLmHead>, m[0], m[1], m[0], m[1], q, ea);
 }
 
 template <int FMT>
@@ -918,7 +798,6 @@ static bool launch_lmh_stream(cudaStream_t st, const LmHeadArgs& a, float* pv, i
   if (!lmh_stream_ok<FMT>(a)) return false;
   int* err = device_error_flag();
   if (!err) return false;
-  if (launch_lmh_tc<FMT>(st, a, pv, pi, pl, tiles_stride, err)) return true;
   LmhScratch sc;
   if (!lmh_carve(a, &sc)) return false;
   CUtensorMap wmap;
@@ -938,29 +817,27 @@ static bool launch_lmh_stream(cudaStream_t st, const LmHeadArgs& a, float* pv, i
   }
   launch_prep_activations(st, a.h, a.dtype, x16, rowscale, (int)a.T, (int)a.K, StreamFmt<FMT>::PERM);
   note_launch();
-  // hidden rows per CTA: 64 when there are enough vocabulary tiles to fill the GPU; fewer rows
-  // per CTA (more CTAs, each re-reading the weights from L2) when the vocabulary shard is small
-  const int real_tiles = (int)((a.V + LMH_TILE - 1) / LMH_TILE);
-  int tpg = 64;
-  while (tpg > 8 && (long long)real_tiles * ((a.T + tpg - 1) / tpg) < sm_count() && a.T > tpg / 2) tpg >>= 1;
-  while (tpg > 8 && a.T <= tpg / 2) tpg >>= 1;
-  if (tpg <= 8) launch_lmh_stream_nt<FMT, 1, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
-  else if (tpg <= 16) launch_lmh_stream_nt<FMT, 2, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
-  else if (tpg <= 32) launch_lmh_stream_nt<FMT, 4, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
-  else launch_lmh_stream_nt<FMT, 8, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
+  if (a.T <= 8) launch_lmh_stream_nt<FMT, 1, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
+  else launch_lmh_stream_nt<FMT, 2, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
   return true;
 }
 
-static bool launch_lmh_stream_any(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi,
-                                  float* pl, int64_t ts) {
+template <int FMT>
+static bool launch_lmh_fast(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t ts) {
+  if constexpr (FMT != F_Q6_K)
+    if (a.T <= LMH_STREAM_ROWS && launch_lmh_stream<FMT>(st, a, pv, pi, pl, ts)) return true;
+  return launch_lmh_ts<FMT>(st, a, pv, pi, pl, ts);
+}
+
+static bool launch_lmh_fast_any(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t ts) {
   if (options().force_generic) return false;
   switch (a.format) {
-    case F_Q8_0: return launch_lmh_stream<F_Q8_0>(st, a, pv, pi, pl, ts);
-    case F_Q4_0: return launch_lmh_stream<F_Q4_0>(st, a, pv, pi, pl, ts);
-    case F_NVFP4: return launch_lmh_stream<F_NVFP4>(st, a, pv, pi, pl, ts);
-    case F_MXFP4: return launch_lmh_stream<F_MXFP4>(st, a, pv, pi, pl, ts);
-    case F_MXFP8: return launch_lmh_stream<F_MXFP8>(st, a, pv, pi, pl, ts);
-    default: return false;    // q6_K heads take the generic kernel
+    case F_Q8_0: return launch_lmh_fast<F_Q8_0>(st, a, pv, pi, pl, ts);
+    case F_Q4_0: return launch_lmh_fast<F_Q4_0>(st, a, pv, pi, pl, ts);
+    case F_NVFP4: return launch_lmh_fast<F_NVFP4>(st, a, pv, pi, pl, ts);
+    case F_MXFP4: return launch_lmh_fast<F_MXFP4>(st, a, pv, pi, pl, ts);
+    case F_MXFP8: return launch_lmh_fast<F_MXFP8>(st, a, pv, pi, pl, ts);
+    default: return launch_lmh_fast<F_Q6_K>(st, a, pv, pi, pl, ts);
   }
 }
 
@@ -1279,7 +1156,7 @@ static void launch_partials_f(cudaStream_t st, const LmHeadArgs& a, float* pv, i
 
 void launch_lm_head_partials(cudaStream_t st, const LmHeadArgs& a, float* part_val,
                              int32_t* part_id, float* part_lse, int64_t tiles_stride) {
-  if (launch_lmh_stream_any(st, a, part_val, part_id, part_lse, tiles_stride)) return;
+  if (launch_lmh_fast_any(st, a, part_val, part_id, part_lse, tiles_stride)) return;
   if (a.dtype == QX_DTYPE_F32) launch_partials_f<float>(st, a, part_val, part_id, part_lse, tiles_stride);
   else if (a.dtype == QX_DTYPE_F16) launch_partials_f<__half>(st, a, part_val, part_id, part_lse, tiles_stride);
   else launch_partials_f<__nv_bfloat16>(st, a, part_val, part_id, part_lse, tiles_stride);

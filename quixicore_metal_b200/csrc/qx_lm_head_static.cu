@@ -51,7 +51,7 @@ extern "C" qx_status qx_cuda_lm_head_sample_q_noalloc(void* stream, const void* 
   // (with none left, tiles are simply not shared).  The K-dependent part makes the limit depend
   // on T * K as well as on T * tiles * k.
   if (T > 0 && V > 0 && K > 0) {
-    const size_t need = qx_cuda_lm_head_workspace_bytes(T, V, K, mode, topk) - lm_head_scratch_full_bytes(T, K) +
+    const size_t need = qx_cuda_lm_head_workspace_bytes(T, V, K, mode, topk) - lm_head_scratch_full_bytes(T, V, K) +
                         lm_head_scratch_min_bytes(T, K);
     if (need > kStaticScratchBytes)
       return fail(QX_INSUFFICIENT_WORKSPACE, op,

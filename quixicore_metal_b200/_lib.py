@@ -171,6 +171,31 @@ def check(st: Status) -> None:
         raise QxError(st)
 
 
+_native = None
+
+
+def native():
+    """lib/_qx_native.so: the C++ side of the torch binding (argument checks, outputs, stream, C ABI call)."""
+    global _native
+    if _native is None:
+        path = os.path.join(HERE, "lib", "_qx_native.so")
+        if not os.path.exists(path):
+            raise ImportError(f"{path} is missing: build it with `python -m quixicore_metal_b200.build`. "
+                              "This backend has no fallback path.")
+        import importlib.util
+        import torch  # noqa: F401  (its libraries are the module's dependencies)
+        lib()
+        spec = importlib.util.spec_from_file_location("_qx_native", path)
+        m = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(m)
+
+        def raise_status(code, operation, detail):
+            raise QxError(Status(code, operation.encode(), detail.encode()))
+        m.set_status_handler(raise_status)
+        _native = m
+    return _native
+
+
 def set_option(name: str, value: int) -> None:
     """Chooses between equivalent device paths (see qx_cuda_set_option in the header)."""
     if not lib().qx_cuda_set_option(name.encode(), int(value)):

@@ -1,9 +1,10 @@
-"""Builds the in-tree CUDA shared library for sm_100a with nvcc (no JIT cache, no torch headers).
+"""Builds the in-tree CUDA shared library for sm_100a with nvcc (no JIT cache).
 
     python -m quixicore_metal_b200.build            # incremental
     python -m quixicore_metal_b200.build --force    # rebuild everything
 
-Objects go to quixicore_metal_b200/lib/obj, the result is quixicore_metal_b200/lib/libquixicore_cuda.so.
+Objects go to quixicore_metal_b200/lib/obj, the result is quixicore_metal_b200/lib/libquixicore_cuda.so
+(no torch headers) and, where torch is importable, lib/_qx_native.so: the C++ side of the Python binding.
 """
 from __future__ import annotations
 
@@ -18,6 +19,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIBDIR = os.path.join(HERE, "lib")
 LIB = os.path.join(LIBDIR, "libquixicore_cuda.so")
+BINDING = os.path.join(LIBDIR, "_qx_native.so")
 INCLUDE = os.path.join(os.path.dirname(HERE), "include")
 
 NVCC_FLAGS = [
@@ -74,7 +76,32 @@ def build(force: bool = False, verbose: bool = False) -> str:
         p = subprocess.run(cmd, capture_output=True, text=True)
         if p.returncode != 0:
             raise RuntimeError("link failed:\n" + p.stdout + p.stderr)
+    build_binding(force)
     return LIB
+
+
+def build_binding(force: bool = False) -> None:
+    """lib/_qx_native.so from csrc/qx_binding.cpp.  A host without torch has no use for it."""
+    src = os.path.join(CSRC, "qx_binding.cpp")
+    header = os.path.join(INCLUDE, "quixicore_cuda.h")
+    if not force and os.path.exists(BINDING) and os.path.getmtime(BINDING) >= max(os.path.getmtime(src), os.path.getmtime(header)):
+        return
+    try:
+        import torch
+    except ImportError:
+        return
+    import sysconfig
+    root = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    inc = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
+           sysconfig.get_path("include"), os.path.join(cuda, "include")]
+    cmd = [os.environ.get("CXX") or shutil.which("g++") or "c++", "-O2", "-std=c++17", "-fPIC", "-shared",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", "-o", BINDING, src,
+           *[f"-I{d}" for d in inc], f"-L{os.path.join(root, 'lib')}", f"-L{LIBDIR}", "-lquixicore_cuda", "-ltorch",
+           "-ltorch_cpu", "-ltorch_cuda", "-lc10", "-lc10_cuda", "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
+    p = subprocess.run(cmd, capture_output=True, text=True)
+    if p.returncode != 0:
+        raise RuntimeError("binding build failed:\n" + (p.stdout + p.stderr)[-4000:])
 
 
 if __name__ == "__main__":

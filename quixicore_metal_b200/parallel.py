@@ -398,8 +398,6 @@ class TPDecodeStack:
 
     def _sum_add_residual(self, part, x):
         """x + sum over the ranks of `part` (fp32 partial of this rank), in x's dtype."""
-        if self.world == 1:
-            return (part + x.float()).to(x.dtype)
         n = part.numel()
         # decode-sized partials are latency-bound: one-shot peer stores while a rank sends at most 4 MB
         # (8 bytes per float and peer); larger ones keep NCCL's bandwidth-optimal algorithms
@@ -418,6 +416,14 @@ class TPDecodeStack:
                                             st["status"].data_ptr(), _DT[x.dtype], 5000))
         return out
 
+    def _row_parallel(self, y, weight, x):
+        """x + y @ weight.T with K split over the ranks.  On one GPU the residual add and the cast are the
+        projection's own epilogue (one rounding either way), not three elementwise launches behind it."""
+        from . import tk, tk_torch
+        if self.world == 1:
+            return tk.decode_linear_epilogue(y, weight, None, x, format=self.fmt)
+        return self._sum_add_residual(tk_torch.decode_linear_partial(y, weight, self.fmt), x)
+
     def exchange_used(self) -> str:
         """How the most recent partial sum crossed the ranks: 'peer', 'nccl', or 'none' on one GPU."""
         return "none" if self.world == 1 else getattr(self, "_last", "nccl")
@@ -429,18 +435,18 @@ class TPDecodeStack:
     def layer(self, x, L, trace=None):
         """One block.  `trace`, if given, is a dict that receives the residual stream after the
         O projection ("h"), for tests that compare each half of the block on its own inputs."""
-        from . import tk, tk_torch
+        from . import tk
         qkv = tk.decode_linear_epilogue(x, L["qkv"], format=self.fmt)
         # identity on V: the G query heads of KV group g all take that group's value vector
         hd = self.head_dim
         n_kv = self.kv_local // hd
         v = qkv[:, self.q_local + self.kv_local:].reshape(-1, n_kv, 1, hd)
         attn = v.expand(-1, n_kv, self.q_local // self.kv_local, hd).reshape(-1, self.q_local).contiguous()
-        x = self._sum_add_residual(tk_torch.decode_linear_partial(attn, L["o"], self.fmt), x)
+        x = self._row_parallel(attn, L["o"], x)
         if trace is not None:
             trace["h"] = x
         mid = tk.decode_swiglu(x, L["gate"], L["up"], format=self.fmt)
-        return self._sum_add_residual(tk_torch.decode_linear_partial(mid, L["down"], self.fmt), x)
+        return self._row_parallel(mid, L["down"], x)
 
     def forward(self, x):
         for L in self.layers:

@@ -75,38 +75,7 @@ def _workspace(device, nbytes: int):
     return ws
 
 
-def _check_weight(x, weight, fmt: str, name: str) -> int:
-    """The reference's check_decode_epilogue_weight (torch_kernels.mm:6376-6405) for CUDA."""
-    _check(x.is_cuda and weight.is_cuda and x.dtype in _DT and x.dim() == 2 and x.size(0) > 0
-           and x.size(1) > 0, f"{name}: x must be non-empty (B,K) fp32/fp16/bf16")
-    _check(fmt in _BLOCK, f"{name}: format must be q4_0, q8_0, q6_K, mxfp8, nvfp4, or mxfp4 "
-           "(dense weights are routed to the framework matmul, not to this backend)")
-    bk, bb = _BLOCK[fmt]
-    K = x.size(1)
-    _check(weight.dtype == torch.uint8 and weight.dim() == 3 and weight.size(0) > 0 and K % bk == 0
-           and weight.size(1) == K // bk and weight.size(2) == bb,
-           f"{name}: packed weight must be uint8 (N,K/block_k,block_bytes)")
-    return weight.size(0)
-
-
-def _quant_outputs(x, B, N, output_quant):
-    """Buffers for a fused output quantisation: (kind, codes, scale)."""
-    kind = _lib.OUT_QUANT.get(output_quant, -1)
-    _check(kind >= 0, "output_quant must be None, 'fp8', 'int8', or 'mxfp8'")
-    if kind == 0:
-        return 0, None, None
-    if kind == 3:
-        _check(N % 32 == 0, "output_quant='mxfp8' needs N to be a multiple of 32")
-        return 3, torch.empty((B, N // 32, 33), dtype=torch.uint8, device=x.device), None
-    codes = torch.empty((B, N), dtype=torch.uint8 if kind == 1 else torch.int8, device=x.device)
-    return kind, codes, torch.empty((B,), dtype=torch.float32, device=x.device)
-
-
-def _quant_result(out, kind, codes, scale, with_output=False):
-    if kind == 0:
-        return out
-    q = codes if kind == 3 else (codes, scale)
-    return (out, q) if with_output else q
+_native = _lib.native       # the operators of a decode step run their host side in C++ (csrc/qx_binding.cpp)
 
 
 def decode_linear_epilogue(x, weight, bias, residual, format="", activation=0,
@@ -118,73 +87,22 @@ def decode_linear_epilogue(x, weight, bias, residual, format="", activation=0,
     (codes, scale) of the per-token quantizer applied to the rounded output, 'mxfp8' the packed
     MXFP8 rows, all inside the same call; with_output=True returns (output, quantised) instead, the
     x.dtype output being the one the codes were made from."""
-    fmt, activation = str(format), int(activation)
-    _check(0 <= activation <= 2, "decode_linear_epilogue: activation must be 0, 1, or 2")
-    N = _check_weight(x, weight, fmt, "decode_linear_epilogue")
-    _same_device("decode_linear_epilogue", x, weight, bias if use_bias else None,
-                 residual if use_residual else None)
-    B, K = x.shape
-    _check(not use_bias or (bias.is_cuda and bias.dim() == 1 and bias.size(0) == N
-                            and bias.dtype == x.dtype),
-           "decode_linear_epilogue: bias must be (N,) with x dtype")
-    _check(not use_residual or (residual.is_cuda and residual.dim() == 2 and residual.size(0) == B
-                                and residual.size(1) == N and residual.dtype == x.dtype),
-           "decode_linear_epilogue: residual must be (B,N) with x dtype")
-    with _guard(x.device):
-        xc, wc = x.contiguous(), weight.contiguous()
-        bc = bias.contiguous() if use_bias else None
-        rc = residual.contiguous() if use_residual else None
-        out = torch.empty((B, N), dtype=x.dtype, device=x.device)
-        kind, codes, scale = _quant_outputs(x, B, N, output_quant)
-        _lib.check(_lib.lib().qx_cuda_decode_linear_epilogue(
-            _stream(), _ptr(xc), _ptr(wc), _ptr(bc), _ptr(rc), _ptr(out), B, K, N, fmt.encode(),
-            _DT[x.dtype], activation, int(bool(use_bias)), int(bool(use_residual)),
-            kind, _ptr(codes), _ptr(scale), None, 0))
-    return _quant_result(out, kind, codes, scale, with_output)
+    return _native().decode_linear_epilogue(x, weight, bias, residual, str(format), int(activation), use_bias, use_residual,
+                                            _lib.OUT_QUANT.get(output_quant, -1), with_output)
 
 
 def decode_linear_partial(x, weight, format):
     """fp32 (B,N) raw projection x @ dequant(weight).T with no epilogue: one rank's share of a
     row-parallel (K-split) linear, summed over ranks by the caller."""
-    fmt = str(format)
-    N = _check_weight(x, weight, fmt, "decode_linear_partial")
-    _same_device("decode_linear_partial", x, weight)
-    B, K = x.shape
-    with _guard(x.device):
-        xc, wc = x.contiguous(), weight.contiguous()
-        out = torch.empty((B, N), dtype=torch.float32, device=x.device)
-        _lib.check(_lib.lib().qx_cuda_decode_linear_partial(
-            _stream(), _ptr(xc), _ptr(wc), _ptr(out), B, K, N, fmt.encode(), _DT[x.dtype], None, 0))
-    return out
+    return _native().decode_linear_partial(x, weight, str(format))
 
 
 def decode_swiglu(x, gate_weight, up_weight, gate_bias, up_bias, format="", use_bias=False, *,
                   output_quant=None, with_output=False):
     """Packed gate/up decode projections with fused SwiGLU: silu(gate.x+gb) * (up.x+ub).
     output_quant: as in decode_linear_epilogue."""
-    fmt = str(format)
-    N = _check_weight(x, gate_weight, fmt, "decode_swiglu")
-    up_N = _check_weight(x, up_weight, fmt, "decode_swiglu")
-    _check(up_N == N and up_weight.shape == gate_weight.shape,
-           "decode_swiglu: gate and up weights must have identical shapes")
-    _same_device("decode_swiglu", x, gate_weight, up_weight, gate_bias if use_bias else None,
-                 up_bias if use_bias else None)
-    _check(not use_bias or (gate_bias.is_cuda and up_bias.is_cuda and gate_bias.dtype == x.dtype
-                            and up_bias.dtype == x.dtype and gate_bias.dim() == 1
-                            and up_bias.dim() == 1 and gate_bias.size(0) == N
-                            and up_bias.size(0) == N),
-           "decode_swiglu: both biases must be (N,) with x dtype")
-    B, K = x.shape
-    with _guard(x.device):
-        xc, gc, uc = x.contiguous(), gate_weight.contiguous(), up_weight.contiguous()
-        gb = gate_bias.contiguous() if use_bias else None
-        ub = up_bias.contiguous() if use_bias else None
-        out = torch.empty((B, N), dtype=x.dtype, device=x.device)
-        kind, codes, scale = _quant_outputs(x, B, N, output_quant)
-        _lib.check(_lib.lib().qx_cuda_decode_swiglu(
-            _stream(), _ptr(xc), _ptr(gc), _ptr(uc), _ptr(gb), _ptr(ub), _ptr(out), B, K, N,
-            fmt.encode(), _DT[x.dtype], int(bool(use_bias)), kind, _ptr(codes), _ptr(scale), None, 0))
-    return _quant_result(out, kind, codes, scale, with_output)
+    return _native().decode_swiglu(x, gate_weight, up_weight, gate_bias, up_bias, str(format), use_bias,
+                                   _lib.OUT_QUANT.get(output_quant, -1), with_output)
 
 
 def _quantize_per_token(x, kind: int, name: str):
@@ -249,26 +167,8 @@ def lm_head_sample_q(h, Wq, bias, V, K, fmt, mode, topk, temperature, seed, top_
     mode 0 argmax, 1 categorical, 2 top-k, 3 top-p (nucleus over the per-256-row top-k pool with
     the exact full-vocabulary normalizer).  bias: fp32 (V,) or a 1-element placeholder.
     Returns int32 (T,).  Unlike the Metal original, q6_K takes every mode and every h dtype."""
-    V, K, fmt, mode, topk = int(V), int(K), str(fmt), int(mode), int(topk)
-    temperature, seed, top_p = float(temperature), int(seed), float(top_p)
-    _check_lm_head(h, Wq, bias, V, K, fmt, mode, topk, temperature, top_p)
-    if mode in (2, 3):
-        _check(topk <= V, "lm_head_sample_q: k must be <= vocab size V")
-    T = h.size(0)
-    use_bias = bias is not None and bias.numel() > 1
-    if use_bias:
-        _check(bias.numel() == V, "lm_head_sample_q: bias must be (V,)")
-    with _guard(h.device):
-        hc, wc = h.contiguous(), Wq.contiguous()
-        bc = bias.to(torch.float32).contiguous() if use_bias else None
-        out = torch.empty((T,), dtype=torch.int32, device=h.device)
-        L = _lib.lib()
-        nbytes = L.qx_cuda_lm_head_workspace_bytes(T, V, K, mode, topk)
-        ws = _workspace(h.device, nbytes)
-        _lib.check(L.qx_cuda_lm_head_sample_q(
-            _stream(), _ptr(hc), _ptr(wc), _ptr(bc), _ptr(out), _ptr(ws), nbytes, T, V, K,
-            fmt.encode(), _DT[h.dtype], mode, topk, temperature, seed & 0xFFFFFFFF, top_p))
-    return out
+    return _native().lm_head_sample_q(h, Wq, bias, int(V), int(K), str(fmt), int(mode), int(topk), float(temperature),
+                                      int(seed), float(top_p))
 
 
 def lm_head_sample(h, W, bias, mode, k, temperature, seed):
@@ -520,28 +420,7 @@ def dequant_gather(table, ids, format, scale=1.0):
 
 
 def _rms_norm_add(x, residual, weight, eps, quant, static_scale=0.0, group=0, ue8m0=False, name="rms_norm_add"):
-    _check(x.is_cuda and x.dtype in _DT and x.dim() >= 1 and x.numel() > 0,
-           f"{name}: x must be a non-empty CUDA fp32/fp16/bf16 tensor")
-    D = x.size(-1)
-    _check(residual.shape == x.shape and residual.dtype == x.dtype and weight.dim() == 1 and weight.size(0) == D
-           and weight.dtype == x.dtype, f"{name}: residual must match x, weight must be (D,) with x dtype")
-    _same_device(name, x, residual, weight)
-    rows = x.numel() // D
-    with _guard(x.device):
-        xc, rc, wc = x.contiguous(), residual.contiguous(), weight.contiguous()
-        added = torch.empty_like(xc)
-        y = torch.empty_like(xc) if quant == 0 else None
-        codes = scale = None
-        if quant:
-            codes = torch.empty(x.shape, dtype=torch.int8 if quant in (3, 5) else torch.uint8, device=x.device)
-        if quant in (2, 3):
-            scale = torch.empty(x.shape[:-1], dtype=torch.float32, device=x.device)
-        elif quant in (4, 5):
-            scale = torch.empty(tuple(x.shape[:-1]) + (D // group,), dtype=torch.float32, device=x.device)
-        _lib.check(_lib.lib().qx_cuda_rms_norm_add(
-            _stream(), _ptr(xc), _ptr(rc), _ptr(wc), _ptr(y), _ptr(codes), _ptr(added), _ptr(scale), rows, D,
-            _DT[x.dtype], float(eps), quant, float(static_scale), int(group), int(bool(ue8m0))))
-    return y, codes, added, scale
+    return _native().rms_norm_add(x, residual, weight, float(eps), quant, float(static_scale), int(group), bool(ue8m0), name)
 
 
 def rms_norm_add(x, residual, weight, eps=1e-5):
@@ -579,24 +458,8 @@ _ACTQ_MODES = {"swiglu": 0, "swiglu_oai": 1}
 
 
 def _silu_mul_quant(x, gate, act, alpha, limit, quant, group=0, ue8m0=False, name="silu_mul_quant_fp8"):
-    _check(act in _ACTQ_MODES, f"{name}: act must be 'swiglu' or 'swiglu_oai'")
-    _check(x.is_cuda and x.dtype in _DT and x.dim() >= 1 and x.numel() > 0 and gate.shape == x.shape
-           and gate.dtype == x.dtype, f"{name}: x and gate must be matching non-empty CUDA float tensors")
-    _same_device(name, x, gate)
-    D = x.size(-1)
-    rows = x.numel() // D
-    if quant == 4:
-        _check(group > 0 and group % 4 == 0 and D % group == 0,
-               f"{name}: group_size must be a multiple of 4 that divides D")
-    with _guard(x.device):
-        xc, gc = x.contiguous(), gate.contiguous()
-        codes = torch.empty(x.shape, dtype=torch.int8 if quant == 3 else torch.uint8, device=x.device)
-        sshape = tuple(x.shape[:-1]) + ((D // group,) if quant == 4 else ())
-        scale = torch.empty(sshape, dtype=torch.float32, device=x.device)
-        _lib.check(_lib.lib().qx_cuda_silu_mul_quant(
-            _stream(), _ptr(xc), _ptr(gc), _ptr(codes), _ptr(scale), rows, D, _DT[x.dtype], _ACTQ_MODES[act],
-            float(alpha), float(limit), quant, int(group), int(bool(ue8m0))))
-    return codes, scale
+    return _native().silu_mul_quant(x, gate, _ACTQ_MODES.get(act, -1), float(alpha), float(limit), quant, int(group),
+                                    bool(ue8m0), name)
 
 
 def silu_mul_quant_fp8(x, gate, act="swiglu", alpha=1.702, limit=7.0):
@@ -689,32 +552,16 @@ def base_qembedding(codes, scales, biases, ids, bits, group_size, scale_dtype="b
     return out
 
 
-def _bq_matmul(name, codes, scales, biases, x, desc, gemv_only):
-    planes, keep, (rows,), K = _bq_planes(name, codes, scales, biases, desc)
-    _check(x.is_cuda and x.dim() == 2 and x.size(0) == K, f"{name}: x must be (K, M) with K matching the packed weights")
-    _check(not gemv_only or x.size(1) == 1, "base_qgemv: x must be (K, 1)")
-    _check(x.dtype in _DT, "BaseQN matmul: x must be float16, bfloat16, or float32")
-    _check(x.size(1) > 0, "BaseQN matmul: M must be positive")
-    _same_device(name, codes, x)
-    M = x.size(1)
-    with _guard(x.device):
-        xc = x.contiguous()
-        out = torch.empty((rows, M), dtype=x.dtype, device=x.device)
-        L = _lib.lib()
-        ws, n = _bq_ws(L, x.device, K, M, 0, x.dtype)
-        _lib.check(L.qx_cuda_base_qgemm(_stream(), planes, desc, _ptr(xc), _ptr(out), rows, K, M, _DT[x.dtype],
-                                        _ptr(ws), n))
-    return out
-
-
 def base_qgemv(codes, scales, biases, x, bits, group_size, scale_dtype="bf16", symmetric=False, layout="metal"):
     """dequant(BaseQN weights) @ x for x (K, 1)."""
-    return _bq_matmul("base_qgemv", codes, scales, biases, x, _bq_desc(bits, group_size, scale_dtype, symmetric, layout), True)
+    return _native().base_q_matmul(codes, scales, biases, x, int(bits), int(group_size), str(scale_dtype), bool(symmetric),
+                                   str(layout), "base_qgemv", True)
 
 
 def base_qgemm(codes, scales, biases, x, bits, group_size, scale_dtype="bf16", symmetric=False, layout="metal"):
     """dequant(BaseQN weights) @ x for x (K, M)."""
-    return _bq_matmul("base_qgemm", codes, scales, biases, x, _bq_desc(bits, group_size, scale_dtype, symmetric, layout), False)
+    return _native().base_q_matmul(codes, scales, biases, x, int(bits), int(group_size), str(scale_dtype), bool(symmetric),
+                                   str(layout), "base_qgemm", False)
 
 
 def base_qgemv_qkv(q_codes, q_scales, q_biases, k_codes, k_scales, k_biases, v_codes, v_scales, v_biases, x, bits,

@@ -103,22 +103,15 @@ __device__ __forceinline__ float warp_max(float v) {
 // ---- output quantizer encoders (fp32 arithmetic on already-rounded I/O-dtype values) ---------
 // e4m3: nearest with halves rounded AWAY from zero, |x| >= 448 and NaN -> 0x7E, |x| < 2^-10 ->
 // signed zero.  int8: round half away, clamp to +-127.
+// Without a branch: adding half a step to the bits of |x| rounds the mantissa to 3 bits and carries into the
+// exponent; below 2^-6 the code is |x| * 512 rounded (the sum truncated, so that no second rounding can cross
+// a half).  33 instructions with four branches became 11.
 __device__ __forceinline__ uint32_t e4m3_encode(float x) {
   const uint32_t sign = (x < 0.0f) ? 0x80u : 0u;
   const float a = fabsf(x);
-  if (!(a < 448.0f)) return sign | 0x7Eu;                 // overflow and NaN saturate
-  const uint32_t bits = __float_as_uint(a);
-  const int E = (int)((bits >> 23) & 0xFFu) - 127;
-  if (E < -6) {                                           // e4m3 subnormal range: steps of 2^-9
-    const int m = (int)roundf(a * 512.0f);           // half away from zero, exact
-    if (m <= 0) return sign;
-    return sign | (uint32_t)(m >= 8 ? 8 : m);
-  }
-  int mant = (int)(((bits & 0x7FFFFFu) + 0x80000u) >> 20);
-  int exp = E + 7;
-  if (mant >= 8) { mant = 0; exp += 1; }
-  if (exp > 15 || (exp == 15 && mant >= 7)) return sign | 0x7Eu;
-  return sign | ((uint32_t)exp << 3) | (uint32_t)mant;
+  const uint32_t normal = ((__float_as_uint(a) + 0x80000u) >> 20) - 120u * 8u;
+  const uint32_t small = (uint32_t)__float2int_rz(__fadd_rz(a * 512.0f, 0.5f));
+  return sign | min(a < 0.015625f ? small : normal, 0x7Eu);
 }
 
 __device__ __forceinline__ int int8_encode(float x) {
@@ -138,13 +131,15 @@ __device__ __forceinline__ int ceil_log2(float q) {
 // One MXFP8 block {e8m0 exponent; 32 e4m3 codes} from the 32 values held one per lane of a full
 // warp: scale 2^ceil(log2(amax / 448)) (amax > 0), an all-zero block stores exponent 127.
 __device__ __forceinline__ void mxfp8_block_store(float v, int lane, uint8_t* __restrict__ block) {
-  const float amax = warp_max(fabsf(v));
+  // largest magnitude as bits (one warp reduction; NaN does not choose the scale); 448 = 1.75 * 2^8, so
+  // ceil(log2(amax / 448)) is the exponent of amax - 8, plus one when its mantissa is above 1.75
+  const uint32_t top = __reduce_max_sync(0xffffffffu, v == v ? __float_as_uint(v) & 0x7FFFFFFFu : 0u);
   int code = 127;
-  if (amax > 0.0f) {
-    const int e = ceil_log2(fmaxf(amax, 1e-10f) / 448.0f);
-    code = min(max(e + 127, 1), 254);
+  if (top != 0u) {
+    const uint32_t t = max(top, __float_as_uint(1e-10f));
+    code = min(max((int)(t >> 23) - 8 + ((t & 0x7FFFFFu) > 0x600000u ? 1 : 0), 1), 254);
   }
-  const float inv = 1.0f / __uint_as_float((uint32_t)code << 23);
+  const float inv = __uint_as_float(max((uint32_t)(254 - code) << 23, 0x00400000u));     // 2^(127 - code)
   block[1 + lane] = (uint8_t)e4m3_encode(v * inv);
   if (lane == 0) block[0] = (uint8_t)code;
 }

@@ -176,6 +176,19 @@ qx_status qx_cuda_decode_linear_epilogue(void* stream, const void* x, const void
                                          int use_residual, int out_quant, void* out_codes,
                                          float* out_scale, void* workspace, size_t workspace_bytes);
 
+/* The two projections with a fixed order of the K sums: the streaming kernels' up to 16 rows (and in their
+ * passes), one accumulator over the whole of K per output above - the results of releases before the
+ * faster kernel for large batches, bit for bit.  For chains of blocks, where one output that rounds the other way
+ * reaches every later value.  Arguments and workspace as the plain forms, without output quantisation. */
+qx_status qx_cuda_decode_linear_epilogue_ordered(void* stream, const void* x, const void* weight, const void* bias,
+                                                 const void* residual, void* y, int64_t M, int64_t K, int64_t N,
+                                                 const char* format, qx_dtype dtype, int activation, int use_bias,
+                                                 int use_residual, void* workspace, size_t workspace_bytes);
+qx_status qx_cuda_decode_swiglu_ordered(void* stream, const void* x, const void* gate_weight, const void* up_weight,
+                                        const void* gate_bias, const void* up_bias, void* y, int64_t M, int64_t K,
+                                        int64_t N, const char* format, qx_dtype dtype, int use_bias, void* workspace,
+                                        size_t workspace_bytes);
+
 /* y[m,n] = dot(x[m,:], deq(W[n,:])) as fp32, no epilogue: the per-rank piece of a row-parallel
  * (K-split) projection, to be summed over ranks before bias / activation / residual are applied
  * once.  No counterpart in the reference (single device).  Needs bf16 / f16 activations, 16-byte

@@ -149,7 +149,7 @@ PyObject* quant_result(const at::Tensor& out, int kind, const Quant& q, bool wit
 }
 void* ptr(const at::Tensor& t) { return t.defined() ? t.data_ptr() : nullptr; }
 
-// (x, weight, bias, residual, format, activation, use_bias, use_residual, quant_kind, with_output)
+// (x, weight, bias, residual, format, activation, use_bias, use_residual, quant_kind, with_output, ordered)
 PyObject* decode_linear_epilogue(PyObject*, PyObject* const* a, Py_ssize_t) {
   return guarded([&]() -> PyObject* {
     static const char* op = "decode_linear_epilogue";
@@ -172,6 +172,13 @@ PyObject* decode_linear_epilogue(PyObject*, PyObject* const* a, Py_ssize_t) {
     if (ur) rc = dense(*r);
     const int kind = (int)integer(a[8]);
     at::Tensor out = empty({B, N}, x.scalar_type(), x);
+    if (truth(a[10])) {
+      check(kind == 0, op, "the ordered form has no output_quant");
+      check_status(qx_cuda_decode_linear_epilogue_ordered(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), ptr(bc), ptr(rc),
+                                                          ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), (int)act, ub, ur,
+                                                          nullptr, 0));
+      return wrap(out);
+    }
     Quant q = quant_outputs(x, B, N, kind);
     check_status(qx_cuda_decode_linear_epilogue(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), ptr(bc), ptr(rc), ptr(out),
                                                 B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), (int)act, ub, ur, kind,
@@ -197,7 +204,7 @@ PyObject* decode_linear_partial(PyObject*, PyObject* const* a, Py_ssize_t) {
   });
 }
 
-// (x, gate, up, gate_bias, up_bias, format, use_bias, quant_kind, with_output)
+// (x, gate, up, gate_bias, up_bias, format, use_bias, quant_kind, with_output, ordered)
 PyObject* decode_swiglu(PyObject*, PyObject* const* a, Py_ssize_t) {
   return guarded([&]() -> PyObject* {
     static const char* op = "decode_swiglu";
@@ -216,6 +223,12 @@ PyObject* decode_swiglu(PyObject*, PyObject* const* a, Py_ssize_t) {
     if (ub) { gbc = dense(*gb); bbc = dense(*bb); }
     const int kind = (int)integer(a[7]);
     at::Tensor out = empty({B, N}, x.scalar_type(), x);
+    if (truth(a[9])) {
+      check(kind == 0, op, "the ordered form has no output_quant");
+      check_status(qx_cuda_decode_swiglu_ordered(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(uc), ptr(gbc), ptr(bbc),
+                                                 ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), ub, nullptr, 0));
+      return wrap(out);
+    }
     Quant q = quant_outputs(x, B, N, kind);
     check_status(qx_cuda_decode_swiglu(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(uc), ptr(gbc), ptr(bbc), ptr(out),
                                        B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), ub, kind, ptr(q.codes),
@@ -389,9 +402,9 @@ PyObject* counted(PyObject* m, PyObject* const* a, Py_ssize_t n) {
 }
 #define QX_METHOD(name, n) {#name, (PyCFunction)(void (*)(void))counted<name, n>, METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
-    QX_METHOD(decode_linear_epilogue, 10),
+    QX_METHOD(decode_linear_epilogue, 11),
     QX_METHOD(decode_linear_partial, 3),
-    QX_METHOD(decode_swiglu, 9),
+    QX_METHOD(decode_swiglu, 10),
     QX_METHOD(lm_head_sample_q, 11),
     QX_METHOD(rms_norm_add, 9),
     QX_METHOD(silu_mul_quant, 9),

@@ -142,15 +142,17 @@ size_t qx_cuda_projection_workspace_bytes(int64_t M, int64_t K, int64_t N, const
   size_t need = projection_scratch_bytes(a);
   a.out_f32 = 1;                                  // the fp32-partial form of the same shape
   const size_t p = swiglu ? 0 : projection_scratch_bytes(a);
-  return need > p ? need : p;
+  if (p > need) need = p;
+  a.out_f32 = 0;
+  a.ordered = 1;
+  const size_t o = projection_scratch_bytes(a);
+  return need > o ? need : o;
 }
 
-qx_status qx_cuda_decode_linear_epilogue(void* stream, const void* x, const void* weight,
-                                         const void* bias, const void* residual, void* y,
-                                         int64_t M, int64_t K, int64_t N, const char* format,
-                                         qx_dtype dtype, int activation, int use_bias,
-                                         int use_residual, int out_quant, void* out_codes,
-                                         float* out_scale, void* workspace, size_t workspace_bytes) {
+static qx_status linear_epilogue(int ordered, void* stream, const void* x, const void* weight, const void* bias,
+                                 const void* residual, void* y, int64_t M, int64_t K, int64_t N, const char* format,
+                                 qx_dtype dtype, int activation, int use_bias, int use_residual, int out_quant,
+                                 void* out_codes, float* out_scale, void* workspace, size_t workspace_bytes) {
   static const char* op = "decode_linear_epilogue";
   if (activation < 0 || activation > 2)
     return fail(QX_INVALID_ARGUMENT, op, "activation must be 0, 1, or 2");
@@ -165,6 +167,7 @@ qx_status qx_cuda_decode_linear_epilogue(void* stream, const void* x, const void
   if (!device_ready(op, &st)) return st;
   GemvArgs a{x, weight, nullptr, bias, nullptr, residual, y, M, K, N, f, dtype,
              activation, use_bias ? 1 : 0, use_residual ? 1 : 0};
+  a.ordered = ordered;
   a.out_quant = out_quant; a.q_codes = out_codes; a.q_scale = out_scale;
   ScratchHold hold;
   st = bind_scratch(op, (cudaStream_t)stream, projection_scratch_bytes(a), workspace, workspace_bytes, &hold,
@@ -173,6 +176,23 @@ qx_status qx_cuda_decode_linear_epilogue(void* stream, const void* x, const void
   const bool fused = launch_projection((cudaStream_t)stream, a);
   finish_out_quant((cudaStream_t)stream, a, fused);
   return check_launch(op);
+}
+
+qx_status qx_cuda_decode_linear_epilogue(void* stream, const void* x, const void* weight,
+                                         const void* bias, const void* residual, void* y,
+                                         int64_t M, int64_t K, int64_t N, const char* format,
+                                         qx_dtype dtype, int activation, int use_bias,
+                                         int use_residual, int out_quant, void* out_codes,
+                                         float* out_scale, void* workspace, size_t workspace_bytes) {
+  return linear_epilogue(0, stream, x, weight, bias, residual, y, M, K, N, format, dtype, activation, use_bias, use_residual,
+                         out_quant, out_codes, out_scale, workspace, workspace_bytes);
+}
+qx_status qx_cuda_decode_linear_epilogue_ordered(void* stream, const void* x, const void* weight, const void* bias,
+                                                 const void* residual, void* y, int64_t M, int64_t K, int64_t N,
+                                                 const char* format, qx_dtype dtype, int activation, int use_bias,
+                                                 int use_residual, void* workspace, size_t workspace_bytes) {
+  return linear_epilogue(1, stream, x, weight, bias, residual, y, M, K, N, format, dtype, activation, use_bias, use_residual, 0,
+                         nullptr, nullptr, workspace, workspace_bytes);
 }
 
 qx_status qx_cuda_decode_linear_partial(void* stream, const void* x, const void* weight, float* y,
@@ -196,11 +216,10 @@ qx_status qx_cuda_decode_linear_partial(void* stream, const void* x, const void*
               "multiple of 512 columns");
 }
 
-qx_status qx_cuda_decode_swiglu(void* stream, const void* x, const void* gate_weight,
-                                const void* up_weight, const void* gate_bias, const void* up_bias,
-                                void* y, int64_t M, int64_t K, int64_t N, const char* format,
-                                qx_dtype dtype, int use_bias, int out_quant, void* out_codes,
-                                float* out_scale, void* workspace, size_t workspace_bytes) {
+static qx_status swiglu_pair(int ordered, void* stream, const void* x, const void* gate_weight, const void* up_weight,
+                             const void* gate_bias, const void* up_bias, void* y, int64_t M, int64_t K, int64_t N,
+                             const char* format, qx_dtype dtype, int use_bias, int out_quant, void* out_codes,
+                             float* out_scale, void* workspace, size_t workspace_bytes) {
   static const char* op = "decode_swiglu";
   int f = -1;
   qx_status st = check_projection(op, x, gate_weight, y, M, K, N, format, dtype, &f);
@@ -214,6 +233,7 @@ qx_status qx_cuda_decode_swiglu(void* stream, const void* x, const void* gate_we
   if (!device_ready(op, &st)) return st;
   GemvArgs a{x, gate_weight, up_weight, gate_bias, up_bias, nullptr, y, M, K, N, f, dtype,
              0, use_bias ? 1 : 0, 0};
+  a.ordered = ordered;
   a.out_quant = out_quant; a.q_codes = out_codes; a.q_scale = out_scale;
   ScratchHold hold;
   st = bind_scratch(op, (cudaStream_t)stream, projection_scratch_bytes(a), workspace, workspace_bytes, &hold,
@@ -222,6 +242,22 @@ qx_status qx_cuda_decode_swiglu(void* stream, const void* x, const void* gate_we
   const bool fused = launch_projection((cudaStream_t)stream, a);
   finish_out_quant((cudaStream_t)stream, a, fused);
   return check_launch(op);
+}
+
+qx_status qx_cuda_decode_swiglu(void* stream, const void* x, const void* gate_weight,
+                                const void* up_weight, const void* gate_bias, const void* up_bias,
+                                void* y, int64_t M, int64_t K, int64_t N, const char* format,
+                                qx_dtype dtype, int use_bias, int out_quant, void* out_codes,
+                                float* out_scale, void* workspace, size_t workspace_bytes) {
+  return swiglu_pair(0, stream, x, gate_weight, up_weight, gate_bias, up_bias, y, M, K, N, format, dtype, use_bias, out_quant,
+                     out_codes, out_scale, workspace, workspace_bytes);
+}
+qx_status qx_cuda_decode_swiglu_ordered(void* stream, const void* x, const void* gate_weight, const void* up_weight,
+                                        const void* gate_bias, const void* up_bias, void* y, int64_t M, int64_t K,
+                                        int64_t N, const char* format, qx_dtype dtype, int use_bias, void* workspace,
+                                        size_t workspace_bytes) {
+  return swiglu_pair(1, stream, x, gate_weight, up_weight, gate_bias, up_bias, y, M, K, N, format, dtype, use_bias, 0, nullptr,
+                     nullptr, workspace, workspace_bytes);
 }
 
 qx_status qx_cuda_quantize_per_token(void* stream, const void* x, void* codes, float* scale,

@@ -25,6 +25,9 @@ struct GemvArgs {
   int out_quant = 0;
   void* q_codes = nullptr;
   float* q_scale = nullptr;
+  // 1: the sums of the streaming kernels and of the in-place pipeline in their order (see
+  // qx_cuda_decode_linear_epilogue_ordered), whatever other kernel would be faster.
+  int ordered = 0;
   // Device scratch of at least projection_scratch_bytes(*this) bytes, 256-byte aligned.
   void* scratch = nullptr;
   size_t scratch_bytes = 0;

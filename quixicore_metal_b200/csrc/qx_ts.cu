@@ -22,7 +22,7 @@ static TsGeom ts_geom(int f) {
 
 // K in whole raw stages (so every row is a multiple of 8 bytes; q6_K of 2), 16-byte aligned matrices.
 bool ts_shape_ok(int format, int64_t K, int64_t N, const void* w0, const void* w1) {
-  return K % TS_KC == 0 && N >= 16 && (((uintptr_t)w0 | (uintptr_t)w1) & 15) == 0;
+  return K % TS_KC == 0 && N >= 8 && (((uintptr_t)w0 | (uintptr_t)w1) & 15) == 0;
 }
 
 bool ts_plan(TsPlan* p, int format, int64_t M, int64_t K, int64_t N, int rb, int dual, int max_group, size_t aux, bool may_cut) {
@@ -198,8 +198,9 @@ struct TsProj {
     const uint16_t b = reinterpret_cast<const uint16_t*>(p)[i];
     return half ? __half2float(__ushort_as_half(b)) : __uint_as_float((uint32_t)b << 16);
   }
-  // Four columns at a time; warps 0..3 take the even groups of four, warps 4..7 the odd ones, a lane one weight row.
-  // The MXFP8 rows are packed from the stored outputs of the same warp.
+  // Four columns at a time, the next four asked for before these are finished; warps 0..3 take the even groups of
+  // four, warps 4..7 the odd ones, a lane one weight row.  MXFP8 rows are packed from the registers (a block
+  // is 32 lanes): packed in a second pass over y they cost 128 us of 272 at 256 x 28672.
   __device__ __forceinline__ static void sum4(const TsItem& it, size_t at, float (&v)[4]) {
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[i] = __ldcg(it.first + at + i * 128);
@@ -221,37 +222,41 @@ struct TsProj {
       if (n >= q.N) continue;
       const float b0 = a.use_bias ? load(a.bias0, n, a.half) : 0.f;
       const float b1 = p.dual && a.use_bias ? load(a.bias1, n, a.half) : 0.f;
-#pragma unroll 1
-      for (int c = (warp >> 2) * 4; c < it.m_count; c += 8) {
-        float v[4], w[4] = {0.f, 0.f, 0.f, 0.f};
-        const size_t o0 = (size_t)(it.m_base + c) * q.N + n;
-        if (a.use_residual) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) if (c + i < it.m_count) w[i] = load(a.residual, o0 + (size_t)i * q.N, a.half);
-        }
+      int c = (warp >> 2) * 4;
+      float v[4], w[4] = {0.f, 0.f, 0.f, 0.f};
+      auto fetch = [&](int c, float (&v)[4], float (&w)[4]) {
         sum4(it, ((size_t)rb * p.nb + c) * 128 + row, v);
-        if (p.dual) sum4(it, ((size_t)p.nb + c) * 128 + row, w);
+        if (p.dual) {
+          sum4(it, ((size_t)p.nb + c) * 128 + row, w);
+        } else if (a.use_residual) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            if (c + i < it.m_count) w[i] = load(a.residual, (size_t)(it.m_base + c + i) * q.N + n, a.half);
+        }
+      };
+      if (c < it.m_count) fetch(c, v, w);
+#pragma unroll 1
+      while (c < it.m_count) {
+        float nv[4], nw[4] = {0.f, 0.f, 0.f, 0.f};
+        if (c + 8 < it.m_count) fetch(c + 8, nv, nw);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           if (c + i >= it.m_count) break;
-          const size_t o = o0 + (size_t)i * q.N;
+          const size_t m = it.m_base + c + i, o = m * q.N + n;
           float d = v[i] * scale[c + i];
           if (a.raw) { reinterpret_cast<float*>(a.y)[o] = d; continue; }
           if (p.dual) d = silu(d + b0) * (w[i] * scale[c + i] + b1);
           else d = apply_act(d + b0, a.activation) + w[i];
-          reinterpret_cast<uint16_t*>(a.y)[o] = a.half ? __half_as_ushort(__float2half_rn(d)) : __bfloat16_as_ushort(__float2bfloat16_rn(d));
-        }
-      }
-      if (a.mx) {                                    // N % 32 == 0: 32 lanes = 32 consecutive channels
-#pragma unroll 1
-        for (int c = (warp >> 2) * 4; c < it.m_count; c += 8) {
-          const int e = min(c + 4, it.m_count);
-#pragma unroll 2
-          for (int m = c; m < e; ++m) {
-            const float r = load(a.y, (size_t)(it.m_base + m) * q.N + n, a.half);
-            mxfp8_block_store(r, lane, a.mx + ((size_t)(it.m_base + m) * (q.N >> 5) + (n >> 5)) * 33);
+          const uint16_t h = a.half ? __half_as_ushort(__float2half_rn(d)) : __bfloat16_as_ushort(__float2bfloat16_rn(d));
+          reinterpret_cast<uint16_t*>(a.y)[o] = h;
+          if (a.mx) {                                // N % 32 == 0: 32 lanes = 32 consecutive channels
+            const float r = a.half ? __half2float(__ushort_as_half(h)) : __uint_as_float((uint32_t)h << 16);
+            mxfp8_block_store(r, lane, a.mx + (m * (q.N >> 5) + (n >> 5)) * 33);
           }
         }
+        c += 8;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) { v[i] = nv[i]; w[i] = nw[i]; }
       }
     }
   }
@@ -262,26 +267,38 @@ struct TsProj {
 // are enough of them to keep the cut items few.
 static int ts_blocks(const GemvArgs& a) { return a.N >= 128 * 148 ? 2 : 1; }
 
+// Row groups of one launch (4 CTAs each on 148 SMs); more rows take several launches.
+constexpr int64_t TS_PASS_GROUPS = 37;
+
 // Activation rows per group: 64 with running sums; nvfp4 and mxfp4, whose products have at most 14 bits, take 128 in
 // one chunk per item (error at K = 8192: 1e-6 and 4e-7), which decodes the weights half as often.
 static bool ts_projection_plan(const GemvArgs& a, TsPlan* p) {
   if (a.dtype != QX_DTYPE_BF16 && a.dtype != QX_DTYPE_F16) return false;
-  if (a.M < 2 || a.M > 0xFFFF || ((uintptr_t)a.x & 15) != 0 || !ts_shape_ok(a.format, a.K, a.N, a.w0, a.w1)) return false;
+  if (((uintptr_t)a.x & 15) != 0 || !ts_shape_ok(a.format, a.K, a.N, a.w0, a.w1)) return false;
   const bool short_terms = a.format == F_NVFP4 || a.format == F_MXFP4;
   const int rb = a.format == F_Q6_K && a.M > 32 && !a.w1 ? 1 : ts_blocks(a);
   const int group = a.format == F_Q6_K ? (a.w1 ? 32 : 64) : (short_terms ? 128 : 64);
-  return ts_plan(p, a.format, a.M, a.K, a.N, rb, a.w1 != nullptr, group, 0, true);
+  const int64_t M = a.M < TS_PASS_GROUPS * group ? a.M : TS_PASS_GROUPS * group;
+  if (!a.ordered) return ts_plan(p, a.format, M, a.K, a.N, rb, a.w1 != nullptr, group, 0, true);
+  // the caller wants the sums of the in-place pipeline (one accumulator over the whole of K per output)
+  if (!ts_plan(p, a.format, M, a.K, a.N, rb, a.w1 != nullptr, group, 0, false)) return false;
+  p->sums = 0;
+  return true;
 }
 
 // Where this kernel takes over from the 16-row streaming kernel (and its passes).  Measured, K = 8192 -> N = 28672 and
 // 4096 -> 4096, us, streaming / this kernel:  nvfp4 16 rows 52 / 40 and 11 / 17; 32 rows (one pass) 102 / 45 and
 // 15 / 20; 64 rows 117 / 59 and 28 / 24.  Its time hardly depends on the rows, but a call pays about 10 us for
-// preparation, start-up and the sum over cut items, so small matrices stay where they are up to 32 rows.
+// preparation, start-up and the sum over cut items, so small matrices stay where they are up to 32 rows.  Rows
+// whose byte pitch the streaming kernel cannot take come here at every batch (the alternative is the scalar kernel:
+// mxfp8 K = 1280, 15 rows, gate / up / down of 5888: 512 us).
 bool ts_preferred(const GemvArgs& a) {
   const int first = options().ts_min_rows;
   if (first > 0) return a.M >= first;
   const int64_t bytes = a.N * (a.K / block_k_of(a.format)) * block_bytes_of(a.format) * (a.w1 ? 2 : 1);
+  if (a.ordered) return a.format == F_NVFP4 && a.M > 16 && !stream_passes_ok(a);   // same sums, bit for bit, as the pipeline
   if (a.M > 32) return true;
+  if (!stream_path_ok(a) && !stream_passes_ok(a)) return true;
   if (a.M > 16) return bytes >= (a.w1 ? (16 << 20) : (28 << 20));
   if (a.M > 8) return bytes >= (a.format == F_MXFP4 || a.format == F_MXFP8 ? (56 << 20) : (100 << 20)) && a.format != F_Q6_K;
   return false;
@@ -319,12 +336,7 @@ static bool launch_ts_fmt(cudaStream_t st, const GemvArgs& a, const TsPlan& p, i
   return ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsProj>, m[0], m[1], m[2], m[3], q, ea);
 }
 
-bool launch_ts(cudaStream_t st, const GemvArgs& a, bool* fused) {
-  *fused = false;
-  TsPlan p;
-  if (!ts_preferred(a) || !ts_projection_plan(a, &p) || !a.scratch || a.scratch_bytes < p.scratch()) return false;
-  int* err = device_error_flag();
-  if (!err) return false;
+static bool launch_ts_pass(cudaStream_t st, const GemvArgs& a, const TsPlan& p, int* err, bool* fused) {
   switch (a.format) {
     case F_Q4_0: return launch_ts_fmt<F_Q4_0>(st, a, p, err, fused);
     case F_Q8_0: return launch_ts_fmt<F_Q8_0>(st, a, p, err, fused);
@@ -333,6 +345,27 @@ bool launch_ts(cudaStream_t st, const GemvArgs& a, bool* fused) {
     case F_NVFP4: return launch_ts_fmt<F_NVFP4>(st, a, p, err, fused);
     default: return launch_ts_fmt<F_MXFP4>(st, a, p, err, fused);
   }
+}
+
+bool launch_ts(cudaStream_t st, const GemvArgs& a, bool* fused) {
+  *fused = false;
+  TsPlan p;
+  if (!ts_preferred(a) || !ts_projection_plan(a, &p) || !a.scratch || a.scratch_bytes < p.scratch()) return false;
+  int* err = device_error_flag();
+  if (!err) return false;
+  const int64_t per = (int64_t)p.mg * p.groups;
+  for (int64_t m0 = 0; m0 < a.M; m0 += per) {
+    GemvArgs b = a;
+    b.M = a.M - m0 < per ? a.M - m0 : per;
+    b.x = (const char*)a.x + (size_t)m0 * a.K * 2;
+    b.y = (char*)a.y + (size_t)m0 * a.N * (a.out_f32 ? 4 : 2);
+    if (a.residual) b.residual = (const char*)a.residual + (size_t)m0 * a.N * 2;
+    if (a.q_codes && a.out_quant == OQ_MXFP8) b.q_codes = (char*)a.q_codes + (size_t)m0 * (a.N / 32) * 33;
+    TsPlan pb = p;
+    if (m0 + per > a.M && m0 > 0 && (!ts_projection_plan(b, &pb) || pb.scratch() > a.scratch_bytes)) return false;
+    if (!launch_ts_pass(st, b, pb, err, fused)) return false;
+  }
+  return true;
 }
 
 }  // namespace qx

@@ -419,9 +419,9 @@ class TPDecodeStack:
     def _row_parallel(self, y, weight, x):
         """x + y @ weight.T with K split over the ranks.  On one GPU the residual add and the cast are the
         projection's own epilogue (one rounding either way), not three elementwise launches behind it."""
-        from . import tk, tk_torch
+        from . import tk_torch
         if self.world == 1:
-            return tk.decode_linear_epilogue(y, weight, None, x, format=self.fmt)
+            return tk_torch.decode_linear_epilogue(y, weight, None, x, self.fmt, 0, False, True, ordered=True)
         return self._sum_add_residual(tk_torch.decode_linear_partial(y, weight, self.fmt), x)
 
     def exchange_used(self) -> str:
@@ -435,8 +435,10 @@ class TPDecodeStack:
     def layer(self, x, L, trace=None):
         """One block.  `trace`, if given, is a dict that receives the residual stream after the
         O projection ("h"), for tests that compare each half of the block on its own inputs."""
-        from . import tk
-        qkv = tk.decode_linear_epilogue(x, L["qkv"], format=self.fmt)
+        from . import tk_torch
+        # one order of the K sums in every projection: through a stack of blocks a single output that rounds the
+        # other way reaches every later value (four blocks without norms: 1 % of the result)
+        qkv = tk_torch.decode_linear_epilogue(x, L["qkv"], None, None, self.fmt, ordered=True)
         # identity on V: the G query heads of KV group g all take that group's value vector
         hd = self.head_dim
         n_kv = self.kv_local // hd
@@ -445,7 +447,7 @@ class TPDecodeStack:
         x = self._row_parallel(attn, L["o"], x)
         if trace is not None:
             trace["h"] = x
-        mid = tk.decode_swiglu(x, L["gate"], L["up"], format=self.fmt)
+        mid = tk_torch.decode_swiglu(x, L["gate"], L["up"], None, None, self.fmt, ordered=True)
         return self._row_parallel(mid, L["down"], x)
 
     def forward(self, x):

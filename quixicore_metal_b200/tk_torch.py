@@ -80,15 +80,16 @@ _native = _lib.native       # the operators of a decode step run their host side
 
 def decode_linear_epilogue(x, weight, bias, residual, format="", activation=0,
                            use_bias=False, use_residual=False, *, output_quant=None,
-                           with_output=False):
+                           with_output=False, ordered=False):
     """Packed decode linear with fused bias, activation and residual; returns (B,N) in x.dtype.
     Absent bias / residual are passed as placeholders and ignored when their flag is false.
     output_quant (keyword only, not in the reference's positional signature): 'fp8' / 'int8' return
     (codes, scale) of the per-token quantizer applied to the rounded output, 'mxfp8' the packed
     MXFP8 rows, all inside the same call; with_output=True returns (output, quantised) instead, the
-    x.dtype output being the one the codes were made from."""
+    x.dtype output being the one the codes were made from.  ordered=True keeps one order of the K sums
+    (qx_cuda_decode_linear_epilogue_ordered)."""
     return _native().decode_linear_epilogue(x, weight, bias, residual, str(format), int(activation), use_bias, use_residual,
-                                            _lib.OUT_QUANT.get(output_quant, -1), with_output)
+                                            _lib.OUT_QUANT.get(output_quant, -1), with_output, ordered)
 
 
 def decode_linear_partial(x, weight, format):
@@ -98,11 +99,11 @@ def decode_linear_partial(x, weight, format):
 
 
 def decode_swiglu(x, gate_weight, up_weight, gate_bias, up_bias, format="", use_bias=False, *,
-                  output_quant=None, with_output=False):
+                  output_quant=None, with_output=False, ordered=False):
     """Packed gate/up decode projections with fused SwiGLU: silu(gate.x+gb) * (up.x+ub).
-    output_quant: as in decode_linear_epilogue."""
+    output_quant, ordered: as in decode_linear_epilogue."""
     return _native().decode_swiglu(x, gate_weight, up_weight, gate_bias, up_bias, str(format), use_bias,
-                                   _lib.OUT_QUANT.get(output_quant, -1), with_output)
+                                   _lib.OUT_QUANT.get(output_quant, -1), with_output, ordered)
 
 
 def _quantize_per_token(x, kind: int, name: str):

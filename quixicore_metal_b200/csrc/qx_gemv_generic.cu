@@ -1,135 +1,251 @@
-// Shape-generic decode projections: one warp per weight row, lanes stride over 32-column spans,
-// fp32 FMA accumulation, up to 8 activation rows share one pass over the weights.
+// Shape-generic decode projections in fp32 arithmetic: the path of fp32 activations and of every 16-bit call
+// whose shape or alignment the tensor-core kernels do not take.  Correct for any K % block_k == 0.
 //
-// This is the path for every (dtype, shape, alignment) the streaming tensor-core kernels do not
-// take: fp32 / fp16 activations, rows whose byte pitch is not a multiple of 16, tiny problems.
-// It reads each weight byte exactly once per pass and is correct for any K % block_k == 0.
+// What bounds it: latency (a 4096 x 1536 q4_0 matrix is 3.5 MB, 0.5 us of HBM time) and, for larger ones, the
+// issue slots of decode + FMA.  So everything a lane needs for a step is asked for at once and coalesced:
+// four lanes share a 32-column unit - a lane holds 8 weights of it, two groups of four consecutive columns, so
+// that the activations are two vector loads - a warp covers 256 columns of R rows per step, and the warps of a
+// CTA share the steps of a row when there are too few rows to fill the GPU.  A scale multiplies the partial sum
+// of its 8 weights.  One warp per row with a 32-column span per lane (scalar, strided activation loads): 30.7 us for
+// that matrix at one row with the full epilogue, now 4.5 to 5.
 #include "qx_formats.cuh"
 #include "qx_kernels.h"
+#include "qx_stream.cuh"
 
 namespace qx {
 
-template <typename T>
-__device__ __forceinline__ void load_x32(const T* __restrict__ p, float (&x)[32]) {
-#pragma unroll
-  for (int i = 0; i < 32; ++i) x[i] = to_f32<T>(p[i]);
+namespace {
+
+// 4 / 8 bytes at any address, from the aligned words that hold them (no word without a wanted byte is read)
+__device__ __forceinline__ uint32_t ldg4(const uint8_t* p) {
+  const uint32_t* b = reinterpret_cast<const uint32_t*>((uintptr_t)p & ~(uintptr_t)3);
+  const uint32_t sh = (uint32_t)((uintptr_t)p & 3) * 8u;
+  const uint32_t lo = __ldg(b), hi = sh ? __ldg(b + 1) : 0u;
+  return __funnelshift_r(lo, hi, sh);
+}
+__device__ __forceinline__ uint2 ldg8(const uint8_t* p) {
+  const uint32_t* b = reinterpret_cast<const uint32_t*>((uintptr_t)p & ~(uintptr_t)3);
+  const uint32_t sh = (uint32_t)((uintptr_t)p & 3) * 8u;
+  const uint32_t w0 = __ldg(b), w1 = __ldg(b + 1), w2 = sh ? __ldg(b + 2) : 0u;
+  return make_uint2(__funnelshift_r(w0, w1, sh), __funnelshift_r(w1, w2, sh));
+}
+__device__ __forceinline__ float ldg_f16(const uint8_t* p) {          // 2-byte aligned
+  return __half2float(__ushort_as_half(__ldg(reinterpret_cast<const uint16_t*>(p))));
+}
+__device__ __forceinline__ uint32_t e4m3_pair_bits(uint32_t v) {      // codes at [15:8], [31:24] -> f16 pair of value * 2^-8
+  return ((v >> 1) & 0x3F803F80u) | (v & 0x80008000u);
 }
 
-// MB activation rows per pass; DUAL = gate/up pair (SwiGLU) sharing the activation reads.
-template <int FMT, typename T, int MB, bool DUAL>
-__global__ void __launch_bounds__(256)
-gemv_generic_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w0,
-                    const uint8_t* __restrict__ w1, const T* __restrict__ bias0,
-                    const T* __restrict__ bias1, const T* __restrict__ residual,
-                    T* __restrict__ y, int M, int K, int N, int activation, int use_bias,
-                    int use_residual) {
-  constexpr int BK = block_k_of(FMT), BB = block_bytes_of(FMT);
-  const int lane = threadIdx.x & 31;
-  const int warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int warps_total = (gridDim.x * blockDim.x) >> 5;
-  const int m0 = blockIdx.y * MB;
-  const int mcount = min(MB, M - m0);
-  const size_t row_bytes = (size_t)(K / BK) * BB;
-  const int spans = K / 32 + ((K % 32) ? 1 : 0);  // nvfp4 allows K % 32 == 16
+// The 8 weights of lane quarter t of 32-column unit u: raw() loads, weights() gives them without their scale.
+// cols(): first columns (inside the unit) of weights 0..3 and 4..7.
+template <int FMT> struct Lane8 {
+  uint32_t a, b, c, d;                             // code words (q6_K: low nibbles a, b and high bits c, d)
+  float scale;
+  __device__ __forceinline__ static int first(int t) {
+    return FMT == F_Q4_0 || FMT == F_MXFP4 ? 4 * t : (FMT == F_NVFP4 ? 16 * (t >> 1) + 4 * (t & 1) : 8 * t);
+  }
+  static constexpr int GAP = FMT == F_Q4_0 || FMT == F_MXFP4 ? 16 : (FMT == F_NVFP4 ? 8 : 4);
 
-  for (int n = warp_global; n < N; n += warps_total) {
-    float acc0[MB], acc1[MB];
-#pragma unroll
-    for (int m = 0; m < MB; ++m) { acc0[m] = 0.f; acc1[m] = 0.f; }
-    const uint8_t* r0 = w0 + (size_t)n * row_bytes;
-    const uint8_t* r1 = DUAL ? w1 + (size_t)n * row_bytes : nullptr;
-    for (int s = lane; s < spans; s += 32) {
-      float wv0[32], wv1[32];
-      const bool half_span = (FMT == F_NVFP4) && (s * 32 + 16 >= K);
-      if (half_span) {
-        // last 16 columns of an nvfp4 row whose K is 16 mod 32: decode one block by hand
-        const uint8_t* b = r0 + (size_t)s * 18;
-        const float sc = e4m3_to_f32(b[0]);
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          wv0[i] = sc * e2m1_to_f32(b[1 + i] & 15u);
-          wv0[i + 8] = sc * e2m1_to_f32(b[1 + i] >> 4);
-          wv0[i + 16] = 0.f; wv0[i + 24] = 0.f;
-        }
-        if (DUAL) {
-          const uint8_t* c = r1 + (size_t)s * 18;
-          const float sd = e4m3_to_f32(c[0]);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            wv1[i] = sd * e2m1_to_f32(c[1 + i] & 15u);
-            wv1[i + 8] = sd * e2m1_to_f32(c[1 + i] >> 4);
-            wv1[i + 16] = 0.f; wv1[i + 24] = 0.f;
-          }
-        }
-      } else {
-        decode_span32<FMT>(r0, s, wv0);
-        if (DUAL) decode_span32<FMT>(r1, s, wv1);
-      }
-      const int ncol = half_span ? 16 : 32;
-#pragma unroll
-      for (int m = 0; m < MB; ++m) {
-        if (m < mcount) {
-          const T* xp = x + (size_t)(m0 + m) * K + (size_t)s * 32;
-          float a0 = 0.f, a1 = 0.f;
-#pragma unroll
-          for (int i = 0; i < 32; ++i) {
-            if (i < ncol) {
-              const float xv = to_f32<T>(xp[i]);
-              a0 = fmaf(xv, wv0[i], a0);
-              if (DUAL) a1 = fmaf(xv, wv1[i], a1);
-            }
-          }
-          acc0[m] += a0;
-          if (DUAL) acc1[m] += a1;
-        }
-      }
+  __device__ __forceinline__ void raw(const uint8_t* __restrict__ row, int u, int t) {
+    if constexpr (FMT == F_Q4_0) {
+      const uint8_t* p = row + (size_t)u * 18;
+      a = ldg4(p + 2 + 4 * t); scale = ldg_f16(p);
+    } else if constexpr (FMT == F_MXFP4) {
+      const uint8_t* p = row + (size_t)u * 17;
+      a = ldg4(p + 1 + 4 * t); scale = e8m0_to_f32(__ldg(p));
+    } else if constexpr (FMT == F_NVFP4) {
+      const uint8_t* p = row + (size_t)(2 * u + (t >> 1)) * 9;
+      a = ldg4(p + 1 + 4 * (t & 1)); scale = e4m3_to_f32(__ldg(p));
+    } else if constexpr (FMT == F_Q8_0) {
+      const uint8_t* p = row + (size_t)u * 34;
+      const uint2 v = ldg8(p + 2 + 8 * t);
+      a = v.x; b = v.y; scale = ldg_f16(p);
+    } else if constexpr (FMT == F_MXFP8) {
+      const uint8_t* p = row + (size_t)u * 33;
+      const uint2 v = ldg8(p + 1 + 8 * t);
+      a = v.x; b = v.y; scale = e8m0_to_f32(__ldg(p)) * 256.f;
+    } else {
+      const uint8_t* p = row + (size_t)(u >> 3) * 210;
+      const int ch = (u >> 2) & 1, g = u & 3;      // 128-column half, 32-column quarter of it
+      const uint2 q = ldg8(p + 64 * ch + 32 * (g & 1) + 8 * t), h = ldg8(p + 128 + 32 * ch + 8 * t);
+      const int qs = 4 * (g >> 1), hs = 2 * g;
+      a = q.x >> qs; b = q.y >> qs; c = h.x >> hs; d = h.y >> hs;
+      scale = ldg_f16(p + 208) * (float)(int)(int8_t)__ldg(p + 192 + 8 * ch + 2 * g + (t >> 1));
     }
+  }
+  __device__ __forceinline__ static void pair(uint32_t h, float& x, float& y) {
+    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&h));
+    x = f.x; y = f.y;
+  }
+  // bytes of c4 (each a small integer) minus `off`, in order
+  __device__ __forceinline__ static void ints(uint32_t c4, uint32_t off2, float* w) {
+    pair(h2sub(__byte_perm(c4, 0x64646464u, 0x4140), off2), w[0], w[1]);
+    pair(h2sub(__byte_perm(c4, 0x64646464u, 0x4342), off2), w[2], w[3]);
+  }
+  __device__ __forceinline__ void weights(float (&w)[8]) const {
+    if constexpr (FMT == F_Q4_0) {
+      ints(a & 0x0F0F0F0Fu, 0x64086408u, w);
+      ints((a >> 4) & 0x0F0F0F0Fu, 0x64086408u, w + 4);
+    } else if constexpr (FMT == F_MXFP4 || FMT == F_NVFP4) {
+      pair(cvt_e2m1x2<0>(a), w[0], w[4]); pair(cvt_e2m1x2<1>(a), w[1], w[5]);
+      pair(cvt_e2m1x2<2>(a), w[2], w[6]); pair(cvt_e2m1x2<3>(a), w[3], w[7]);
+    } else if constexpr (FMT == F_Q8_0) {
+      ints(a ^ 0x80808080u, 0x64806480u, w);
+      ints(b ^ 0x80808080u, 0x64806480u, w + 4);
+    } else if constexpr (FMT == F_MXFP8) {
+      pair(e4m3_pair_bits(__byte_perm(a, 0u, 0x1404)), w[0], w[1]); pair(e4m3_pair_bits(__byte_perm(a, 0u, 0x3424)), w[2], w[3]);
+      pair(e4m3_pair_bits(__byte_perm(b, 0u, 0x1404)), w[4], w[5]); pair(e4m3_pair_bits(__byte_perm(b, 0u, 0x3424)), w[6], w[7]);
+    } else {
+      ints((a & 0x0F0F0F0Fu) | ((c << 4) & 0x30303030u), 0x64206420u, w);
+      ints((b & 0x0F0F0F0Fu) | ((d << 4) & 0x30303030u), 0x64206420u, w + 4);
+    }
+  }
+};
+
+// four consecutive activations; vec: the address is aligned for one vector load
+template <typename T>
+__device__ __forceinline__ void load_x4(const T* __restrict__ p, bool vec, float* o) {
+  if (vec) {
+    if constexpr (sizeof(T) == 4) {
+      const float4 v = __ldg(reinterpret_cast<const float4*>(p));
+      o[0] = v.x; o[1] = v.y; o[2] = v.z; o[3] = v.w;
+    } else {
+      const uint2 v = __ldg(reinterpret_cast<const uint2*>(p));
+      const T* e = reinterpret_cast<const T*>(&v);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) o[i] = to_f32<T>(e[i]);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o[i] = to_f32<T>(p[i]);
+  }
+}
+
+constexpr int GEN_WARPS = 8;
+
+}  // namespace
+
+// MB activation rows per pass (blockIdx.y); a warp owns R output rows (of both matrices when DUAL) and takes every
+// S-th step of 256 columns, S = 1 << slog warps sharing the rows.
+template <int FMT, typename T, int MB, int R, bool DUAL>
+__global__ void __launch_bounds__(GEN_WARPS * 32)
+gemv_generic_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w0, const uint8_t* __restrict__ w1,
+                    const T* __restrict__ bias0, const T* __restrict__ bias1, const T* __restrict__ residual,
+                    T* __restrict__ y, int M, int K, int N, int activation, int use_bias, int use_residual, int slog,
+                    int vec) {
+  constexpr int BK = block_k_of(FMT), BB = block_bytes_of(FMT), NR = R * (DUAL ? 2 : 1);
+  __shared__ float red[GEN_WARPS][NR * MB];
+  asm volatile("griddepcontrol.launch_dependents;");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = lane & 3;
+  const int S = 1 << slog, slice = warp & (S - 1), grp = warp >> slog;
+  const int n0 = (blockIdx.x * (GEN_WARPS >> slog) + grp) * R;
+  const int m0 = blockIdx.y * MB, mcount = min(MB, M - m0);
+  const size_t row_bytes = (size_t)(K / BK) * BB;
+  const uint8_t* rows[NR];
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const size_t at = (size_t)min(n0 + r, N - 1) * row_bytes;
+    rows[r] = w0 + at;
+    if constexpr (DUAL) rows[R + r] = w1 + at;
+  }
+  float acc[NR][MB];
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+#pragma unroll
+    for (int m = 0; m < MB; ++m) acc[r][m] = 0.f;
+
+  const int first = Lane8<FMT>::first(t);
+  constexpr int GAP = Lane8<FMT>::GAP;
+#pragma unroll 2
+  for (int k0 = slice * 256; k0 < K; k0 += S * 256) {
+    const int u = (k0 >> 5) + (lane >> 2), col = 32 * u + first;
+    if (col >= K) continue;                        // the lanes past the end of the last step
+    Lane8<FMT> q[NR];
+#pragma unroll
+    for (int r = 0; r < NR; ++r) q[r].raw(rows[r], u, t);
+    float xv[MB][8];
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
-      acc0[m] = warp_sum(acc0[m]);
-      if (DUAL) acc1[m] = warp_sum(acc1[m]);
+      const T* xp = x + (size_t)(m0 + min(m, mcount - 1)) * K + col;
+      load_x4<T>(xp, vec, xv[m]);
+      load_x4<T>(xp + GAP, vec, xv[m] + 4);
     }
-    if (lane == 0) {
+#pragma unroll
+    for (int r = 0; r < NR; ++r) {
+      float w[8];
+      q[r].weights(w);
 #pragma unroll
       for (int m = 0; m < MB; ++m) {
-        if (m < mcount) {
-          const size_t o = (size_t)(m0 + m) * N + n;
-          float v = acc0[m];
-          if (DUAL) {
-            float u = acc1[m];
-            if (use_bias) { v += to_f32<T>(bias0[n]); u += to_f32<T>(bias1[n]); }
-            y[o] = from_f32<T>(silu(v) * u);
-          } else {
-            if (use_bias) v += to_f32<T>(bias0[n]);
-            v = apply_act(v, activation);
-            if (use_residual) v += to_f32<T>(residual[o]);
-            y[o] = from_f32<T>(v);
-          }
-        }
+        float s = w[0] * xv[m][0];
+#pragma unroll
+        for (int i = 1; i < 8; ++i) s = fmaf(w[i], xv[m][i], s);
+        acc[r][m] = fmaf(q[r].scale, s, acc[r][m]);
       }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < NR; ++r)
+#pragma unroll
+    for (int m = 0; m < MB; ++m) {
+      const float s = warp_sum(acc[r][m]);
+      if (lane == 0) red[warp][r * MB + m] = s;
+    }
+  __syncthreads();
+  // outputs of the CTA's row groups
+  for (int i = threadIdx.x; i < (GEN_WARPS >> slog) * R * MB; i += GEN_WARPS * 32) {
+    const int g = i / (R * MB), r = (i / MB) % R, m = i % MB;
+    const int n = (blockIdx.x * (GEN_WARPS >> slog) + g) * R + r;
+    if (n >= N || m >= mcount) continue;
+    float v = 0.f, up = 0.f;
+    for (int k = 0; k < S; ++k) {
+      v += red[(g << slog) + k][r * MB + m];
+      if constexpr (DUAL) up += red[(g << slog) + k][(R + r) * MB + m];
+    }
+    const size_t o = (size_t)(m0 + m) * N + n;
+    if constexpr (DUAL) {
+      if (use_bias) { v += to_f32<T>(bias0[n]); up += to_f32<T>(bias1[n]); }
+      y[o] = from_f32<T>(silu(v) * up);
+    } else {
+      if (use_bias) v += to_f32<T>(bias0[n]);
+      v = apply_act(v, activation);
+      if (use_residual) v += to_f32<T>(residual[o]);
+      y[o] = from_f32<T>(v);
     }
   }
 }
 
+template <int FMT, typename T, int MB, int R, bool DUAL>
+static void launch_mb(cudaStream_t st, const GemvArgs& a) {
+  const int steps = (int)((a.K + 255) / 256);
+  const int64_t groups = (a.N + R - 1) / R;
+  // warps share a row's steps until there are 24 warps per SM
+  int slog = 0;
+  while (slog < 3 && (groups << slog) < 24ll * sm_count() && (2 << slog) <= steps) ++slog;
+  const int per_block = GEN_WARPS >> slog;
+  const int vec = ((uintptr_t)a.x & (4 * sizeof(T) - 1)) == 0 && a.K % 4 == 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((groups + per_block - 1) / per_block), (unsigned)((a.M + MB - 1) / MB));
+  cfg.blockDim = dim3(GEN_WARPS * 32);
+  cfg.stream = st;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, gemv_generic_kernel<FMT, T, MB, R, DUAL>, (const T*)a.x, (const uint8_t*)a.w0, (const uint8_t*)a.w1,
+                     (const T*)a.bias0, (const T*)a.bias1, (const T*)a.residual, (T*)a.y, (int)a.M, (int)a.K, (int)a.N,
+                     a.activation, a.use_bias, a.use_residual, slog, vec);
+  note_launch();
+}
+
 template <int FMT, typename T, bool DUAL>
 static void launch_fmt(cudaStream_t st, const GemvArgs& a) {
-  const int warps_per_block = 8;
-  int blocks = (int)((a.N + warps_per_block - 1) / warps_per_block);
-  const int cap = sm_count() * 8;
-  if (blocks > cap) blocks = cap;
-  if (blocks < 1) blocks = 1;
-#define QX_LAUNCH(MBV)                                                                         \
-  gemv_generic_kernel<FMT, T, MBV, DUAL><<<dim3(blocks, (unsigned)((a.M + MBV - 1) / MBV)),   \
-                                           warps_per_block * 32, 0, st>>>(                     \
-      (const T*)a.x, (const uint8_t*)a.w0, (const uint8_t*)a.w1, (const T*)a.bias0,            \
-      (const T*)a.bias1, (const T*)a.residual, (T*)a.y, (int)a.M, (int)a.K, (int)a.N,          \
-      a.activation, a.use_bias, a.use_residual)
-  if (a.M == 1) QX_LAUNCH(1);
-  else if (a.M == 2) QX_LAUNCH(2);
-  else if (a.M <= 4) QX_LAUNCH(4);
-  else QX_LAUNCH(8);
-#undef QX_LAUNCH
-  note_launch();
+  constexpr int R = DUAL ? 2 : 4;                  // few activation rows: more weight rows in flight per lane
+  if (a.M == 1) launch_mb<FMT, T, 1, R, DUAL>(st, a);
+  else if (a.M == 2) launch_mb<FMT, T, 2, R, DUAL>(st, a);
+  else if (a.M <= 4) launch_mb<FMT, T, 4, R / 2, DUAL>(st, a);
+  else launch_mb<FMT, T, 8, R / 2, DUAL>(st, a);
 }
 
 template <typename T, bool DUAL>

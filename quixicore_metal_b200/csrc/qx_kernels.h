@@ -58,10 +58,10 @@ bool launch_gemv_stream(cudaStream_t st, const GemvArgs& a);
 // The same kernel in passes of 32 / 16 rows for batches of 17 - 64 rows, when that beats the tcgen05 path.
 bool stream_passes_ok(const GemvArgs& a);
 bool launch_gemv_stream_passes(cudaStream_t st, const GemvArgs& a);
-// tcgen05 path (bf16 activations, batch > 16, K % 256 == 0, single weight matrix).
+// tcgen05 pipeline (16-bit activations, batch > 16, K % 128 == 0; not q6_K).
 bool tc_path_ok(const GemvArgs& a);
-// *fused_quant (optional): set when the kernel that ran packed the requested MXFP8 output rows itself
-bool launch_gemm_tc(cudaStream_t st, const GemvArgs& a, bool* fused_quant = nullptr);
+// *fused_quant: set when the kernel that ran packed the requested MXFP8 output rows itself
+bool launch_gemm_tc(cudaStream_t st, const GemvArgs& a, bool* fused_quant);
 // Tensor-memory-operand kernel (16-bit activations, K % 256 == 0): see qx_ts.cuh.
 size_t ts_scratch_bytes(const GemvArgs& a);
 bool launch_ts(cudaStream_t st, const GemvArgs& a, bool* fused_quant);
@@ -74,9 +74,6 @@ size_t stream_scratch_bytes(const GemvArgs& a);
 size_t tc_scratch_bytes(const GemvArgs& a);
 size_t projection_scratch_bytes(const GemvArgs& a);
 // Row-scaled f16 copy of (M,K) bf16 / f16 activations in the column order `perm` of the decoders.
-// silu(gate + gb) * (up + ub) over fp32 (M,N) projections -> T (M,N)
-void launch_swiglu_combine(cudaStream_t st, const float* gate, const float* up, const void* gb,
-                           const void* ub, void* y, int64_t M, int64_t N, qx_dtype dtype, int use_bias);
 void launch_prep_activations(cudaStream_t st, const void* x, qx_dtype dtype, __half* x16,
                              float* rowscale, int M, int K, int perm, int img_rows = 0);
 // Picks the kernel family for one projection call (format, dtype, batch, alignment); true when the

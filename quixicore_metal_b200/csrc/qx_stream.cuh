@@ -79,14 +79,6 @@ __device__ __forceinline__ void tma_box_2d(uint32_t dst, const void* tmap, int x
       ::"r"(dst), "l"(tmap), "r"(x), "r"(y), "r"(bar)
       : "memory");
 }
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2,
-                                         uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
-      "{%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 // Shared-memory loads by 32-bit shared-window address.  Deliberately not volatile: the compiler
 // may hoist and interleave them; the mbarrier wait / __syncwarp carry the memory clobbers that
 // keep them inside their pipeline stage.

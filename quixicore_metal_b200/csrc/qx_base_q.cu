@@ -189,6 +189,11 @@ struct BQStreamParams {
   unsigned xs_off;
 };
 
+__device__ __forceinline__ uint4 bq_lds128(uint32_t addr) {
+  uint4 v;
+  asm("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr) : "memory");
+  return v;
+}
 __device__ __forceinline__ uint2 lds64(uint32_t addr) {
   uint2 v;
   asm("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(addr) : "memory");
@@ -198,45 +203,47 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
 // The 8 codes of one lane (bits [0, 8 * BITS) of the string that starts at shared byte address a)
 // as four f16 pairs: pair j = (code j, code j + 4).  A code sits in the low mantissa bits of its
 // half, i.e. it is the f16 subnormal code * 2^-24: exact, and no conversion instruction is needed.
+// Up to 5 bits the odd pairs stay where they lie, BITS higher (codes * 2^(BITS - 24), still subnormal):
+// half the shifts; their products are summed apart and scaled back by bq_odd_scale at the end.
+template <int BITS> constexpr float bq_odd_scale() { return BITS <= 5 ? 1.f / (float)(1 << BITS) : 1.f; }
 template <int BITS>
 __device__ __forceinline__ void bq_pairs(uint32_t a, uint32_t (&pr)[4]) {
   constexpr uint32_t M2 = ((1u << BITS) - 1u) * 0x00010001u;
-  uint32_t u[4];
-  if constexpr (BITS == 2) {
-    const uint32_t lo = lds16(a);
-    const uint32_t w = __byte_perm(lo, 0u, 0x1110);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) u[j] = w >> (2 * j);
-  } else if constexpr (BITS == 4) {
-    const uint32_t lo = lds32(a);
-#pragma unroll
-    for (int j = 0; j < 4; ++j) u[j] = lo >> (4 * j);
+  if constexpr (BITS <= 5) {
+    uint32_t e, h;                                 // codes 0, 1 (4, 5) and 2, 3 (6, 7) of each half, from its bit 0
+    if constexpr (BITS == 2) {
+      e = __byte_perm(lds16(a), 0u, 0x1110);
+      h = e >> 4;
+    } else if constexpr (BITS == 4) {
+      e = lds32(a);
+      h = e >> 8;
+    } else {
+      const uint32_t a0 = a & ~3u, sh = (a & 3u) * 8u;
+      const uint32_t w0 = lds32(a0), w1 = lds32(a0 + 4);
+      const uint32_t lo = __funnelshift_r(w0, w1, sh), hi = w1 >> sh;
+      if constexpr (BITS == 3) {
+        e = __byte_perm(lo, lo >> 12, 0x5410);
+        h = e >> 6;
+      } else {
+        const uint32_t f = __funnelshift_r(lo, hi, 20);
+        e = __byte_perm(lo, f, 0x5410);
+        h = __byte_perm(lo >> 10, f >> 10, 0x5410);
+      }
+    }
+    pr[0] = e & M2; pr[1] = e & (M2 << BITS);
+    pr[2] = h & M2; pr[3] = h & (M2 << BITS);
   } else if constexpr (BITS == 8) {
     const uint2 v = lds64(a);
-    u[0] = __byte_perm(v.x, v.y, 0x4400); u[1] = __byte_perm(v.x, v.y, 0x5511);
-    u[2] = __byte_perm(v.x, v.y, 0x6622); u[3] = __byte_perm(v.x, v.y, 0x7733);
-  } else {
+    pr[0] = __byte_perm(v.x, v.y, 0x4400) & M2; pr[1] = __byte_perm(v.x, v.y, 0x5511) & M2;
+    pr[2] = __byte_perm(v.x, v.y, 0x6622) & M2; pr[3] = __byte_perm(v.x, v.y, 0x7733) & M2;
+  } else {   // 6
     const uint32_t a0 = a & ~3u, sh = (a & 3u) * 8u;
     const uint32_t w0 = lds32(a0), w1 = lds32(a0 + 4);
     const uint32_t lo = __funnelshift_r(w0, w1, sh), hi = w1 >> sh;
-    if constexpr (BITS == 3) {
-      const uint32_t w = __byte_perm(lo, lo >> 12, 0x5410);
-#pragma unroll
-      for (int j = 0; j < 4; ++j) u[j] = w >> (3 * j);
-    } else if constexpr (BITS == 5) {
-      const uint32_t f = __funnelshift_r(lo, hi, 20);
-      const uint32_t w = __byte_perm(lo, f, 0x5410);
-      u[0] = w; u[1] = w >> 5; u[2] = w >> 10;
-      u[3] = __byte_perm(lo >> 15, f >> 15, 0x5410);
-    } else {   // 6
-      const uint32_t f = __funnelshift_r(lo, hi, 24);
-      const uint32_t w = __byte_perm(lo, f, 0x5410);
-      const uint32_t w2 = __byte_perm(lo >> 12, f >> 12, 0x5410);
-      u[0] = w; u[1] = w >> 6; u[2] = w2; u[3] = w2 >> 6;
-    }
+    const uint32_t f = __funnelshift_r(lo, hi, 24);
+    const uint32_t w = __byte_perm(lo, f, 0x5410), w2 = __byte_perm(lo >> 12, f >> 12, 0x5410);
+    pr[0] = w & M2; pr[1] = (w >> 6) & M2; pr[2] = w2 & M2; pr[3] = (w2 >> 6) & M2;
   }
-#pragma unroll
-  for (int j = 0; j < 4; ++j) pr[j] = u[j] & M2;
 }
 
 // A lane's scale vector (the scales of 128 columns of one row: 8, 4, 2 or 1 bytes at p) on its way to shared
@@ -294,7 +301,7 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   }
 
   // shared memory: chunk sums | partial-sum slots | counters | epochs | mbarriers | rings
-  float* S = reinterpret_cast<float*>(bq_smem);                       // [nchunks + 16][8], the tail zero
+  float* S = reinterpret_cast<float*>(bq_smem);                       // [nchunks + 16][NC], the tail zero
   float* red = S + (size_t)(nchunks + 16) * 8;                        // [SLOTS][2][128]
   int* cnt = reinterpret_cast<int*>(red + BQ_SLOTS * 256);
   int* epoch = cnt + BQ_SLOTS;
@@ -340,12 +347,13 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   // One stage: the box of codes by lane 0, and by every lane the scale and bias vectors of its 128 columns of rows
   // g and g + 8, all counted by the slot's barrier.  Loaded into registers at the item's start, as before, the
   // vectors cost every item a DRAM latency (8192 -> 28672, 4 bits, groups of 32, 1 column: 53 us; 49.7 now).
-  auto issue = [&](int i) {
+  int islot = 0;
+  auto issue = [&]() {
     int mat, stage, sidx, trow0;
     locate(icur, mat, stage, sidx, trow0);
     const BQSeg& sg = p.seg[sidx];
-    const int slot = i % nst;
-    const uint32_t bar = mybars + 8 * slot, box = myring + slot * SLOT_BYTES;
+    const uint32_t bar = mybars + 8 * islot, box = myring + islot * SLOT_BYTES;
+    islot = islot + 1 == nst ? 0 : islot + 1;
     const long long prow = rowoff + (mat == 1 ? p.expert_up_off : 0) + trow0;
     if (lane == 0) {
       const CUtensorMap* m = sg.map == 0 ? &map0 : (sg.map == 1 ? &map1 : &map2);
@@ -367,7 +375,7 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
 
   int issued = 0;
   auto fill = [&]() {
-    for (; issued < n_items && issued < nst; ++issued) issue(issued);
+    for (; issued < n_items && issued < nst; ++issued) issue();
   };
   // A programmatic dependent of the kernel before it.  With XS that may be any kernel and nothing is touched before
   // the wait; then the activation column is requested first, and the stages behind it before it is prepared.
@@ -385,9 +393,10 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     x16 = reinterpret_cast<const __half*>(bq_smem + p.xs_off);
     rowscale = reinterpret_cast<const float*>(bq_smem + p.xs_off + (size_t)K * 2);
   }
+  const uint32_t xs_s = XS ? smem_u32(bq_smem + p.xs_off) : 0u;
   auto ldx = [](const uint4* q) { if constexpr (XS) return *q; else return __ldg(q); };
-  for (int i = threadIdx.x; i < (nchunks + 16) * 8; i += blockDim.x) {
-    const int c = i >> 3, n = i & 7;
+  for (int i = threadIdx.x; i < (nchunks + 16) * NC; i += blockDim.x) {
+    const int c = i / NC, n = i % NC;
     float s = 0.f;
     if (n < ncol && c < nchunks) {
       const uint4* xp = reinterpret_cast<const uint4*>(x16 + (size_t)(col0 + n) * K + (size_t)c * 32);
@@ -404,7 +413,8 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   if (threadIdx.x < BQ_SLOTS) { cnt[threadIdx.x] = 0; epoch[threadIdx.x] = threadIdx.x; }
   __syncthreads();
 
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};        // scale path, D-fragment layout: rows g / g+8, columns 2t / 2t+1
+  // scale path, even and odd pairs, D-fragment layout: rows g / g+8, columns 2t / 2t+1
+  float acc[4] = {0.f, 0.f, 0.f, 0.f}, odd[4] = {0.f, 0.f, 0.f, 0.f};
   float bacc[2][NC];                          // bias path: rows g / g+8, this lane's chunks, every column
 #pragma unroll
   for (int rr = 0; rr < 2; ++rr)
@@ -415,17 +425,19 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   // where the scales of chunks 4t .. 4t + 3 lie in a vector: byte selectors that spread it to one scale per chunk
   const uint32_t sel_x = sb == 2 ? (gshift == 0 ? 0x3210u : 0x1010u) : (gshift == 0 ? 0x3210u : gshift == 1 ? 0x1100u : 0x0000u);
   const uint32_t sel_y = gshift == 0 ? 0x7654u : (gshift == 1 ? 0x3232u : 0x1010u);
+  int slot = 0;
+  uint32_t parity = 0;
   for (int i = 0; i < n_items && !dead; ++i) {
     int mat, stage, sidx, trow0;
     locate(cur, mat, stage, sidx, trow0);
     const int tl = cur.tl;
-    const int slot = i % nst;
-    if (!mbar_wait(mybars + 8 * slot, (uint32_t)((i / nst) & 1), p.err)) { dead = true; break; }
+    if (!mbar_wait(mybars + 8 * slot, parity, p.err)) { dead = true; break; }
     consumed = i + 1;
     const uint32_t base = myring + slot * SLOT_BYTES;
+    if (++slot == nst) { slot = 0; parity ^= 1u; }
     float sfc[2][4];
     {
-      const float* Sq = S + (size_t)(stage * 16 + 4 * t) * 8;          // rows past nchunks are zero
+      const float* Sq = S + (size_t)(stage * 16 + 4 * t) * NC;          // rows past nchunks are zero
       // a vector shorter than a word starts at byte `lead` of its word, the same for rows g and g + 8
       const int prow = (int)(rowoff + (mat == 1 ? p.expert_up_off : 0)) + trow0 + g;
       const uint32_t lead = (uint32_t)((prow * groups_per_row + ((stage * BQ_KC + t * 128) >> (5 + gshift))) * sb) & 3u;
@@ -451,50 +463,72 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
         else if (p.stype == 1) convert([&](uint2 r, int q) { return __half2float(__ushort_as_half(half(r, q))); });
         else if (p.stype == 2) convert([](uint2 r, int q) { return e8m0_to_f32((r.x >> (8 * q)) & 0xFFu); });
         else convert([](uint2 r, int q) { return e4m3_to_f32((r.x >> (8 * q)) & 0xFFu); });
-        const bool ok = stage * BQ_KC + t * 128 < K && trow0 + g + 8 * rr < p.seg[sidx].rows;
+        // rows and columns past the matrix: such rows are not written, such columns have zero sums and no chunk
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          sfc[rr][q] = ok ? sfc[rr][q] : 0.f;                          // (an e8m0 zero byte is not zero)
-          const float beta = ok ? bev[q] : 0.f;
+        for (int q = 0; q < 4; ++q)
 #pragma unroll
-          for (int n = 0; n < NC; ++n) bacc[rr][n] = fmaf(beta, Sq[q * 8 + n], bacc[rr][n]);
-        }
+          for (int n = 0; n < NC; ++n) bacc[rr][n] = fmaf(bev[q], Sq[q * NC + n], bacc[rr][n]);
       }
     }
     const uint32_t rowA = base + g * G::PITCH + t * BITS, rowB = rowA + 8 * G::PITCH;
     // lanes whose column does not exist read column 0: their D columns are never written out
     const __half* xr = x16 + (size_t)(col0 + (g < ncol ? g : 0)) * K + (size_t)stage * BQ_KC + 8 * t;
+    const uint32_t xs = XS ? xs_s + (uint32_t)(stage * BQ_KC + 8 * t) * 2u : 0u;
+    auto ldb = [&](int c) {
+      if constexpr (XS) return bq_lds128(xs + c * 64);
+      else return __ldg(reinterpret_cast<const uint4*>(xr + c * 32));
+    };
     const int nch = min(16, nchunks - stage * 16);
-    auto chunk = [&](int c, const uint4& bv) {
+    auto chunk = [&](int j, int q, const uint4& bv) {               // chunk 4j + q, its scales in lane j of the quad
+      const int c = 4 * j + q;
       uint32_t pa[4], pb[4];
       bq_pairs<BITS>(rowA + c * 4 * BITS, pa);
       bq_pairs<BITS>(rowB + c * 4 * BITS, pb);
-      float d[4];
-      mma_f16_zero(d, pa[0], pb[0], pa[1], pb[1], bv.x, bv.y);
-      mma_f16(d, pa[2], pb[2], pa[3], pb[3], bv.z, bv.w);
-      const int src = (lane & ~3) | (c >> 2);
-      const float sA = __shfl_sync(0xffffffffu, sfc[0][c & 3], src);
-      const float sB = __shfl_sync(0xffffffffu, sfc[1][c & 3], src);
-      acc[0] = fmaf(sA, d[0], acc[0]); acc[2] = fmaf(sB, d[2], acc[2]);
-      if constexpr (NC > 1) { acc[1] = fmaf(sA, d[1], acc[1]); acc[3] = fmaf(sB, d[3], acc[3]); }
+      float d[4], o[4];
+      mma_f16_zero(d, pa[0], pb[0], pa[2], pb[2], bv.x, bv.z);
+      mma_f16_zero(o, pa[1], pb[1], pa[3], pb[3], bv.y, bv.w);
+      if constexpr (NC == 1) {
+        // every D column holds the one product: the lane that holds the chunk's scales adds it
+        asm("{ .reg .pred own;\n setp.eq.s32 own, %6, %7;\n"
+            "@own fma.rn.f32 %0, %4, %8, %0;\n @own fma.rn.f32 %1, %4, %9, %1;\n"
+            "@own fma.rn.f32 %2, %5, %10, %2;\n @own fma.rn.f32 %3, %5, %11, %3;\n}"
+            : "+f"(acc[0]), "+f"(odd[0]), "+f"(acc[2]), "+f"(odd[2])
+            : "f"(sfc[0][q]), "f"(sfc[1][q]), "r"(t), "r"(j), "f"(d[0]), "f"(o[0]), "f"(d[2]), "f"(o[2]));
+      } else {
+        const int src = (lane & ~3) | j;
+        const float sA = __shfl_sync(0xffffffffu, sfc[0][q], src);
+        const float sB = __shfl_sync(0xffffffffu, sfc[1][q], src);
+        acc[0] = fmaf(sA, d[0], acc[0]); acc[1] = fmaf(sA, d[1], acc[1]);
+        acc[2] = fmaf(sB, d[2], acc[2]); acc[3] = fmaf(sB, d[3], acc[3]);
+        odd[0] = fmaf(sA, o[0], odd[0]); odd[1] = fmaf(sA, o[1], odd[1]);
+        odd[2] = fmaf(sB, o[2], odd[2]); odd[3] = fmaf(sB, o[3], odd[3]);
+      }
     };
-    if (nch == 16) {                               // a whole stage: no branches, the activation loads 4 chunks ahead
+    // a whole stage: no branches, the activation loads 4 chunks ahead; rolled where the registers are few (128), as
+    // the compiler hoists the code loads of all 16 chunks otherwise and spills (4 bits, one column: 61 us for 44)
+    constexpr int UNROLL = BITS <= 4 && NC == 1 ? 1 : 4;
+    if (nch == 16) {
       uint4 bq[4];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) bq[c] = ldx(reinterpret_cast<const uint4*>(xr + c * 32));
+      for (int q = 0; q < 4; ++q) bq[q] = ldb(q);
+#pragma unroll UNROLL
+      for (int j = 0; j < 4; ++j) {
 #pragma unroll
-      for (int c = 0; c < 16; ++c) {
-        const uint4 bv = bq[c & 3];
-        if (c + 4 < 16) bq[c & 3] = ldx(reinterpret_cast<const uint4*>(xr + (c + 4) * 32));
-        chunk(c, bv);
+        for (int q = 0; q < 4; ++q) {
+          const uint4 bv = bq[q];
+          if (j < 3) bq[q] = ldb(4 * j + 4 + q);
+          chunk(j, q, bv);
+        }
       }
     } else {
+#pragma unroll UNROLL
+      for (int j = 0; j < 4; ++j)
 #pragma unroll
-      for (int c = 0; c < 16; ++c)
-        if (c < nch) chunk(c, ldx(reinterpret_cast<const uint4*>(xr + c * 32)));
+        for (int q = 0; q < 4; ++q)
+          if (4 * j + q < nch) chunk(j, q, ldb(4 * j + q));
     }
     __syncwarp();
-    if (issued < n_items) { issue(issued); ++issued; }
+    if (issued < n_items) { issue(); ++issued; }
 
     // last item of this warp for (tile, matrix): add the partial sums to the tile's slot
     cur.advance(1, spt);
@@ -509,13 +543,23 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
       if (dead) break;
     }
     float* slotp = red + rs * 256 + mat * 128;
-    if (2 * t < ncol) {
-      atomicAdd(slotp + g * 8 + 2 * t, acc[0] * 16777216.f);
-      atomicAdd(slotp + (g + 8) * 8 + 2 * t, acc[2] * 16777216.f);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      acc[j] = (acc[j] + odd[j] * bq_odd_scale<BITS>()) * 16777216.f;
+      odd[j] = 0.f;
     }
-    if (2 * t + 1 < ncol) {
-      atomicAdd(slotp + g * 8 + 2 * t + 1, acc[1] * 16777216.f);
-      atomicAdd(slotp + (g + 8) * 8 + 2 * t + 1, acc[3] * 16777216.f);
+    if constexpr (NC == 1) {                       // scale path and bias path over the quad's chunks in one reduction
+      bacc[0][0] += acc[0];
+      bacc[1][0] += acc[2];
+    } else {
+      if (2 * t < ncol) {
+        atomicAdd(slotp + g * 8 + 2 * t, acc[0]);
+        atomicAdd(slotp + (g + 8) * 8 + 2 * t, acc[2]);
+      }
+      if (2 * t + 1 < ncol) {
+        atomicAdd(slotp + g * 8 + 2 * t + 1, acc[1]);
+        atomicAdd(slotp + (g + 8) * 8 + 2 * t + 1, acc[3]);
+      }
     }
     acc[0] = acc[1] = acc[2] = acc[3] = 0.f;
 #pragma unroll
@@ -541,10 +585,10 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     // every contribution is in: epilogue of the tile by this warp
     __threadfence_block();
     const BQSeg& so = p.seg[mats == 2 ? 0 : sidx];
-    for (int idx = lane; idx < 128; idx += 32) {
-      const int r = idx >> 3, n = idx & 7;
-      const float gsum = atomicExch(red + rs * 256 + idx, 0.f);
-      const float usum = mats == 2 ? atomicExch(red + rs * 256 + 128 + idx, 0.f) : 0.f;
+    for (int idx = lane; idx < 16 * NC; idx += 32) {
+      const int r = idx / NC, n = idx % NC;
+      const float gsum = atomicExch(red + rs * 256 + r * 8 + n, 0.f);
+      const float usum = mats == 2 ? atomicExch(red + rs * 256 + 128 + r * 8 + n, 0.f) : 0.f;
       if (n < ncol && trow0 + r < so.rows) {
         const float sc = rowscale[col0 + n];
         const float v = mats == 2 ? silu(gsum * sc) * (usum * sc) : gsum * sc;

@@ -114,6 +114,24 @@ __device__ __forceinline__ uint32_t e4m3_encode(float x) {
   return sign | min(a < 0.015625f ? small : normal, 0x7Eu);
 }
 
+// ---- codes of pairs of finite values ----
+// Both conversions below round ties to even where e4m3_encode and int8_encode go away from zero: with the last
+// mantissa bit set a tie is none any more, and no other value is moved past a rounding boundary.
+// e4m3_encode(v.x) | e4m3_encode(v.y) << 8; the sum with 0 drops the sign of -0
+__device__ __forceinline__ uint32_t e4m3_encode2(float2 v) {
+  const float2 u = __fadd2_rn(v, make_float2(0.f, 0.f));
+  const float a = __uint_as_float(__float_as_uint(u.x) | 1u), b = __uint_as_float(__float_as_uint(u.y) | 1u);
+  uint16_t r;
+  asm("cvt.rn.satfinite.e4m3x2.f32 %0, %1, %2;" : "=h"(r) : "f"(b), "f"(a));
+  return r;
+}
+// int8_encode of both, |v| < 127.5, as the low bytes of the two words: 1.5 * 2^23 + v holds v's integer there
+__device__ __forceinline__ uint2 int8_encode2(float2 v) {
+  const float2 m = __fadd2_rn(make_float2(__uint_as_float(__float_as_uint(v.x) | 1u), __uint_as_float(__float_as_uint(v.y) | 1u)),
+                          make_float2(12582912.f, 12582912.f));
+  return make_uint2(__float_as_uint(m.x), __float_as_uint(m.y));
+}
+
 __device__ __forceinline__ int int8_encode(float x) {
   float r = roundf(x);                                    // half away from zero
   r = fminf(fmaxf(r, -127.0f), 127.0f);

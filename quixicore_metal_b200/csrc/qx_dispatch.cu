@@ -19,6 +19,8 @@ bool launch_tensor_core(cudaStream_t st, const GemvArgs& a, bool* fused) {
   const bool fusable = a.out_quant == OQ_MXFP8 && !a.out_f32 && a.N % 32 == 0 && a.q_codes;
   *fused = false;
   if (options().force_generic) return false;
+  // all of them read the activations in 16-byte vectors; ones that start elsewhere take the generic kernel
+  if (((uintptr_t)a.x & 15) != 0) return false;
   const bool passes_first = options().stream_passes == 2 && stream_passes_ok(a);
   if (!passes_first && launch_ts(st, a, fused)) return true;
   *fused = fusable;

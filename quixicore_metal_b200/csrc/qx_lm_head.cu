@@ -688,7 +688,7 @@ static bool lmh_stream_ok(const LmHeadArgs& a) {
   using F = StreamFmt<FMT>;
   const size_t row_bytes = (size_t)(a.K / F::BK) * F::BB;
   return (a.dtype == QX_DTYPE_BF16 || a.dtype == QX_DTYPE_F16) && a.K % LmhCfg<FMT>::KC == 0 &&
-         row_bytes % 16 == 0 && ((uintptr_t)a.wq & 15) == 0 && a.V >= 32;
+         row_bytes % 16 == 0 && (((uintptr_t)a.wq | (uintptr_t)a.h) & 15) == 0 && a.V >= 32;
 }
 
 template <int FMT, int NT, bool XS>

@@ -1,0 +1,134 @@
+"""Sizes at which the kernels chosen by row count, alignment and type can go wrong: tile and stage remainders, the
+smallest and the largest of a range, cut work items, row pitches that no 16-byte copy can start at."""
+import numpy as np
+import pytest
+import torch
+
+from oracle import qx_oracle as O
+from tests._util import FMTS, assert_close_dtype, check_ids, dev, host, rounded
+
+pytestmark = pytest.mark.gpu
+
+tk = pytest.importorskip("quixicore_metal_b200.tk")
+tk_torch = pytest.importorskip("quixicore_metal_b200.tk_torch")
+
+
+def _linear(fmt, M, K, N, dtype, seed, pack="synth"):
+    rng = np.random.default_rng(seed)
+    x = rounded(rng.standard_normal((M, K)), dtype)
+    W = O.synth_pack(fmt, (0.02 * rng.standard_normal((N, K))).astype(np.float32)) if pack == "synth" else O.random_packed(fmt, N, K, seed)
+    return x, W, rounded(0.01 * rng.standard_normal(N), dtype), rounded(rng.standard_normal((M, N)), dtype)
+
+
+# rows around the chunks of 16 / 32 / 64 / 128 activation rows; 1031 = 8 * 128 + 7 weight rows; K = 1056 and 4640: row
+# pitches that are no multiple of 16 bytes and a last stage that is not full; 8192: items cut between CTAs
+@pytest.mark.parametrize("M,K,N", [(17, 256, 8), (32, 1056, 129), (33, 8192, 1031), (64, 4640, 35), (65, 512, 257), (128, 2048, 128),
+                                   (129, 1056, 1), (256, 768, 300)])
+@pytest.mark.parametrize("fmt", FMTS)
+def test_linear_above_16_rows(fmt, M, K, N):
+    K = K - K % O.FORMATS[fmt][0] if K % O.FORMATS[fmt][0] else K
+    dtype = "f16" if M == 65 else "bf16"
+    x, W, bias, res = _linear(fmt, M, K, N, dtype, M + K)
+    got = tk.decode_linear_epilogue(dev(x, dtype), dev(W), dev(bias, dtype), dev(res, dtype), activation="silu", format=fmt)
+    assert_close_dtype(host(got), O.decode_linear_epilogue(x, W, fmt, bias, res, 2, dtype), dtype)
+
+
+# random bytes: scales outside the range that the decoded operand holds exactly, whose rows are computed apart
+@pytest.mark.parametrize("fmt,K", [("q4_0", 1024), ("q8_0", 1056), ("q6_K", 512), ("mxfp8", 4096), ("mxfp4", 1056)])
+def test_rows_with_extreme_scales(fmt, K):
+    x, W, _, _ = _linear(fmt, 40, K, 136, "bf16", 5, pack="random")
+    ref = O.decode_linear_epilogue(x, W, fmt, None, None, 0, "bf16")
+    got = host(tk.decode_linear_epilogue(dev(x, "bf16"), dev(W), None, None, format=fmt))
+    ok = np.isfinite(ref).all(0)
+    assert ok.any()
+    for n in np.nonzero(ok)[0]:                              # every row of weights at its own scale
+        assert_close_dtype(got[:, n], ref[:, n], "bf16", scale=float(np.abs(O.dequantize(fmt, W[n:n + 1])).max()) * 30)
+
+
+@pytest.mark.parametrize("M,K,N", [(17, 1056, 96), (64, 2048, 1056), (130, 768, 160)])
+@pytest.mark.parametrize("fmt", ["q4_0", "nvfp4", "mxfp8"])
+def test_swiglu_and_mxfp8_rows_above_16(fmt, M, K, N):
+    x, g, gb, _ = _linear(fmt, M, K, N, "bf16", M)
+    _, u, ub, _ = _linear(fmt, M, K, N, "bf16", M + 1)
+    y, blocks = tk_torch.decode_swiglu(dev(x, "bf16"), dev(g), dev(u), dev(gb, "bf16"), dev(ub, "bf16"), fmt, True,
+                                       output_quant="mxfp8", with_output=True)
+    assert_close_dtype(host(y), O.decode_swiglu(x, g, u, fmt, gb, ub, "bf16"), "bf16")
+    np.testing.assert_array_equal(host(blocks), O.quantize_mxfp8_rows(host(y)))
+
+
+# the fixed summation order of the decoder stack: one row, passes of 16 and 32 rows, the uncut form above
+@pytest.mark.parametrize("M,K,N", [(1, 1024, 48), (5, 512, 257), (17, 2048, 129), (32, 1024, 256), (33, 512, 40)])
+@pytest.mark.parametrize("fmt", ["nvfp4", "q4_0", "q6_K"])
+def test_ordered_entries(fmt, M, K, N):
+    x, W, bias, res = _linear(fmt, M, K, N, "bf16", M)
+    _, u, _, _ = _linear(fmt, M, K, N, "bf16", M + 1)
+    lin = lambda: tk_torch.decode_linear_epilogue(dev(x, "bf16"), dev(W), dev(bias, "bf16"), dev(res, "bf16"), fmt, 0, True, True, ordered=True)
+    got = lin()
+    assert_close_dtype(host(got), O.decode_linear_epilogue(x, W, fmt, bias, res, 0, "bf16"), "bf16")
+    assert torch.equal(got, lin())
+    got = tk_torch.decode_swiglu(dev(x, "bf16"), dev(W), dev(u), dev(x, "bf16"), dev(x, "bf16"), fmt, False, ordered=True)
+    assert_close_dtype(host(got), O.decode_swiglu(x, W, u, fmt, None, None, "bf16"), "bf16")
+
+
+# fp32 (and 16-bit activations that start between 16-byte boundaries): K shorter than a warp's step and with a
+# remainder, row groups of every size, K slices
+@pytest.mark.parametrize("M,K,N", [(1, 256, 1), (2, 512, 35), (3, 1280, 129), (4, 8192, 64), (8, 4352, 33), (9, 768, 17)])
+@pytest.mark.parametrize("fmt", FMTS)
+def test_fp32_and_unaligned_activations(fmt, M, K, N):
+    x, W, bias, res = _linear(fmt, M, K, N, "f32", M + K)
+    _, u, _, _ = _linear(fmt, M, K, N, "f32", M + 1)
+    got = tk.decode_linear_epilogue(dev(x), dev(W), dev(bias), dev(res), activation="gelu", format=fmt)
+    assert_close_dtype(host(got), O.decode_linear_epilogue(x, W, fmt, bias, res, 1, "f32"), "f32")
+    got = tk.decode_swiglu(dev(x), dev(W), dev(u), format=fmt)
+    assert_close_dtype(host(got), O.decode_swiglu(x, W, u, fmt, None, None, "f32"), "f32")
+    xb = rounded(x, "bf16")
+    shifted = torch.zeros(M * K + 1, dtype=torch.bfloat16, device="cuda")[1:].view(M, K).copy_(dev(xb, "bf16"))
+    assert shifted.data_ptr() % 16 == 2
+    got = tk.decode_linear_epilogue(shifted, dev(W), None, None, format=fmt)
+    assert_close_dtype(host(got), O.decode_linear_epilogue(xb, W, fmt, None, None, 0, "bf16"), "bf16")
+
+
+# q6_K gate and up rows in paired warps: fewer tiles than pairs, a tile remainder, ranges that end inside a tile
+@pytest.mark.parametrize("M,K,N", [(1, 256, 16), (4, 2048, 33), (8, 512, 4099), (16, 4096, 200)])
+def test_q6k_swiglu_pairs(M, K, N):
+    x, g, gb, _ = _linear("q6_K", M, K, N, "bf16", N)
+    _, u, ub, _ = _linear("q6_K", M, K, N, "bf16", N + 1)
+    got = tk.decode_swiglu(dev(x, "bf16"), dev(g), dev(u), dev(gb, "bf16"), dev(ub, "bf16"), format="q6_K")
+    assert_close_dtype(host(got), O.decode_swiglu(x, g, u, "q6_K", gb, ub, "bf16"), "bf16")
+
+
+@pytest.mark.parametrize("T", [17, 64])
+@pytest.mark.parametrize("fmt,K", [("q6_K", 512), ("q4_0", 1056), ("mxfp8", 1056)])
+def test_lm_head_above_16_rows(fmt, K, T):
+    rng = np.random.default_rng(T)
+    W = O.synth_pack(fmt, (0.3 * rng.standard_normal((4003, K))).astype(np.float32))
+    h = rounded(0.5 * rng.standard_normal((T, K)), "bf16")
+    for mode, code, kw in (("argmax", 0, {}), ("topk", 2, dict(k=64)), ("topp", 3, dict(k=32, top_p=0.9))):
+        tok = host(tk.lm_head_sample(dev(h, "bf16"), dev(W), mode=mode, format=fmt, temperature=0.8, seed=3, **kw))
+        want, margin = O.lm_head_sample(h, W, fmt, code, temperature=0.8, seed=3, return_detail=True, **kw)
+        check_ids(tok, want, margin, 1e-4, f"{fmt}/{mode}")
+
+
+# rows in registers: one vector, a partial last warp, two and four vectors per thread, one row past what is resident
+# (the ring), a row too long for registers
+@pytest.mark.parametrize("rows,D", [(1, 8), (4800, 264), (299, 8192), (600, 4088), (3, 8200), (151, 16384), (2, 16392)])
+def test_seam_rows(rows, D):
+    rng = np.random.default_rng(D)
+    x, r = (rounded(rng.standard_normal((rows, D)), "bf16") for _ in range(2))
+    x[0, :] = -0.0
+    x[-1, : D // 2] *= 100.0                                  # exponents beyond the paired form's range
+    x = rounded(x, "bf16")
+    w = rounded(1 + 0.1 * rng.standard_normal(D), "bf16")
+    n, added_ref = O.rms_norm_add(x, r, w, 1e-5, "bf16")
+    act = O.gated_act("swiglu", x, r)
+    pick = np.unique(np.r_[0, rows // 2, rows - 1])
+    for kind in ("fp8", "int8"):
+        norm = tk.rms_norm_add_fp8 if kind == "fp8" else tk_torch.rms_norm_add_int8_dyn
+        silu = tk.silu_mul_quant_fp8 if kind == "fp8" else tk.silu_mul_quant_int8
+        codes, added, scale = norm(dev(x, "bf16"), dev(r, "bf16"), dev(w, "bf16"))
+        np.testing.assert_array_equal(host(added), added_ref)
+        for ref, (c, s) in ((n, (codes, scale)), (act, silu(dev(x, "bf16"), dev(r, "bf16")))):
+            rc, rs = O.quantize_groups(ref[pick], D, kind)
+            np.testing.assert_allclose(host(s).reshape(-1)[pick], rs.reshape(-1), rtol=1e-5)
+            same = (host(c)[pick].astype(np.int32) & 0xFF) == (rc.astype(np.int32) & 0xFF)
+            assert same.mean() >= 0.99, (kind, float(same.mean()))

@@ -551,8 +551,9 @@ uint64_t qx_cuda_launch_count(void);
 int qx_cuda_device_error(void);
 /* Chooses between device paths that compute the same result (identical up to fp32 summation
  * order); meant for tests and A/B timing.  Names: "stream_passes" (0 never / 1 when faster / 2
- * whenever possible: 17 - 64 rows as passes (32 rows; 16 for a SwiGLU pair) of the streaming kernel instead of the tcgen05
- * pipeline), "force_generic", "tc_pipeline", "lm_head_ksplit" (0 / 1).  Returns
+ * whenever possible: 17 - 64 rows as passes (32 rows; 16 for a SwiGLU pair) of the streaming kernel instead of a tcgen05
+ * kernel), "ts_min_rows" (rows from which projections run on the tensor-memory-operand kernel, 0: by rows and bytes),
+ * "force_generic", "tc_pipeline" (fixed-order calls above 16 rows), "lm_head_ksplit" (0 / 1: LM-head items cut over K).  Returns
  * 1 if the option exists and took the value.  Process-wide, not synchronised with running calls. */
 int qx_cuda_set_option(const char* name, int value);
 /* Number of device allocations the library has made for scratch of its own (calls that passed

@@ -445,10 +445,6 @@ template <> struct LmhCfg<F_MXFP4> { static constexpr int KC = 512, STAGES = 2; 
 template <> struct LmhCfg<F_MXFP8> { static constexpr int KC = 128, STAGES = 2; };
 
 // QX_LMH_UNROLL: whole stages run fully unrolled for up to this many 8-row n-tiles.
-// QX_LMH_WROWS16_MIN_NT: n-tiles from which a CTA is 16 warps of 16 rows instead of 8 warps of 32.
-#ifndef QX_LMH_WROWS16_MIN_NT
-#define QX_LMH_WROWS16_MIN_NT 2
-#endif
 #ifndef QX_LMH_UNROLL
 #define QX_LMH_UNROLL 2
 #endif
@@ -456,8 +452,12 @@ constexpr int LMH_LOGIT_PITCH = 257;
 constexpr int LMH_TOK_CHUNK = 16;
 constexpr int LMH_STREAM_ROWS = 16;      // hidden rows up to which the streaming kernel is the faster form
 
-// WROWS = vocabulary rows per warp: 32 (8 warps, two m-tiles share every activation fragment) or
-// 16 (16 warps: more loads in flight; used from 9 hidden rows per pass).
+// WROWS = vocabulary rows per warp: 32 (8 warps, two m-tiles share every activation fragment) or 16 (16 warps: four
+// per scheduler to hide the decoder's latency).  16 from 9 hidden rows, and from 2 for the formats whose codes need
+// more instructions (q4_0, 7 rows, 4096 -> 32000: 42.0 -> 34.4 us; 3 rows, 128256: 154.8 -> 141.6; q8_0 99.4 -> 98.6);
+// with one row, and for the 4-bit floats (1.3% slower with 16), the memory bounds the 8 warps already.
+template <int FMT, int NT, bool XS>
+constexpr int lmh_wrows() { return NT >= 2 || (!XS && FMT != F_NVFP4 && FMT != F_MXFP4) ? 16 : 32; }
 // XS: a single hidden row, prepared by every CTA itself into shared memory (xsrc = the raw 16-bit row,
 // bf16 if x_bf16 else f16; x16 / rowscale unused) instead of by the preparation kernel.
 template <int FMT, int NT, int WROWS, bool XS>
@@ -696,7 +696,7 @@ static void launch_lmh_stream_nt(cudaStream_t st, const LmHeadArgs& a, const __h
                                  const float* rowscale, float* pv, int32_t* pi, float* pl,
                                  int64_t tiles_stride, int* err, const CUtensorMap& wmap) {
   using C = LmhCfg<FMT>;
-  constexpr int WROWS = NT >= QX_LMH_WROWS16_MIN_NT ? 16 : 32;
+  constexpr int WROWS = lmh_wrows<FMT, NT, XS>();
   constexpr int NW = 256 / WROWS;
   using WS = WarpStream<FMT, C::KC, WROWS, C::STAGES>;
   const size_t smem = (size_t)NW * WS::WARP_BYTES + (size_t)NW * C::STAGES * 8 +
@@ -979,14 +979,24 @@ lmh_reduce_kernel(const float* __restrict__ cand_val, const int32_t* __restrict_
       int* l_id = reinterpret_cast<int*>(l_val + LMH_RED_COMPACT);
       const int lane = tid & 31, warp = tid >> 5, nwarps = nth >> 5;
       unsigned present_l = 0;
-      for (int grp = warp; grp < ngroups; grp += nwarps) {
-        uint32_t best = 0u;
+      constexpr int GU = 4;                          // groups per warp and step: their loads are in flight together
+      for (int g0 = warp; g0 < ngroups; g0 += GU * nwarps) {
+        uint32_t best[GU] = {};
         for (int e = lane; e < topk; e += 32) {
-          const long long j = (long long)grp * topk + e;
-          if (ci(j) >= 0) best = max(best, max(float_key(cv(j)), 1u));
+#pragma unroll
+          for (int u = 0; u < GU; ++u) {
+            const int grp = min(g0 + u * nwarps, ngroups - 1);
+            const long long j = (long long)grp * topk + e;
+            const int id = ci(j);
+            const float v = cv(j);
+            if (id >= 0) best[u] = max(best[u], max(float_key(v), 1u));
+          }
         }
-        best = __reduce_max_sync(0xffffffffu, best);
-        if (lane == 0) { g_key[grp] = best; present_l += best != 0u ? 1u : 0u; }
+#pragma unroll
+        for (int u = 0; u < GU; ++u) {
+          const uint32_t top = __reduce_max_sync(0xffffffffu, best[u]);
+          if (lane == 0 && g0 + u * nwarps < ngroups) { g_key[g0 + u * nwarps] = top; present_l += top != 0u ? 1u : 0u; }
+        }
       }
       __syncthreads();
       const unsigned present = block_sum_u(present_l, S);

@@ -346,28 +346,43 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   BQCursor icur{first / spt, first % spt};                            // next item to fetch
   // One stage: the box of codes by lane 0, and by every lane the scale and bias vectors of its 128 columns of rows
   // g and g + 8, all counted by the slot's barrier.  Loaded into registers at the item's start, as before, the
-  // vectors cost every item a DRAM latency (8192 -> 28672, 4 bits, groups of 32, 1 column: 53 us; 49.7 now).
-  int islot = 0;
+  // vectors cost every item a DRAM latency (8192 -> 28672, 4 bits, groups of 32, 1 column: 53 us; 49.7 with this).
+  // What only a new tile (or matrix of the pair) changes is computed there: most items advance a column offset.
+  int islot = 0, istage = -1, iy = 0;
+  bool iok0 = false, iok1 = false;
+  const CUtensorMap* imap = &map0;
+  const uint8_t* iscale = nullptr;
+  const uint8_t* ibias = nullptr;
+  const int stage_step = (BQ_KC >> (5 + gshift)) * sb, row8_step = 8 * groups_per_row * sb;   // bytes of a scale plane
   auto issue = [&]() {
-    int mat, stage, sidx, trow0;
-    locate(icur, mat, stage, sidx, trow0);
-    const BQSeg& sg = p.seg[sidx];
+    if (istage < 0 || ++istage == spt1) {
+      int mat, sidx, trow0;
+      locate(icur, mat, istage, sidx, trow0);
+      const BQSeg& sg = p.seg[sidx];
+      const long long prow = rowoff + (mat == 1 ? p.expert_up_off : 0) + trow0;
+      const size_t off = ((size_t)(prow + g) * groups_per_row + ((t * 128) >> (5 + gshift))) * sb;
+      imap = sg.map == 0 ? &map0 : (sg.map == 1 ? &map1 : &map2);
+      iy = (int)prow;
+      iok0 = trow0 + g < sg.rows; iok1 = trow0 + g + 8 < sg.rows;
+      iscale = sg.scales + off;
+      ibias = p.symmetric ? iscale : sg.biases + off;
+    }
     const uint32_t bar = mybars + 8 * islot, box = myring + islot * SLOT_BYTES;
     islot = islot + 1 == nst ? 0 : islot + 1;
-    const long long prow = rowoff + (mat == 1 ? p.expert_up_off : 0) + trow0;
     if (lane == 0) {
-      const CUtensorMap* m = sg.map == 0 ? &map0 : (sg.map == 1 ? &map1 : &map2);
       mbar_arrive_expect_tx(bar, (uint32_t)G::BOX_BYTES);
-      tma_box_2d(box, m, stage * (G::STAGE_BYTES / 4), (int)prow, bar);
+      tma_box_2d(box, imap, istage * (G::STAGE_BYTES / 4), iy, bar);
     }
-    const int colb = stage * BQ_KC + t * 128;
+    const bool in = istage * BQ_KC + t * 128 < K;                      // past the matrix: zeros, no access
+    const int at = istage * stage_step;
     const uint32_t vec = box + G::BOX_BYTES + lane * 8;
-#pragma unroll
-    for (int rr = 0; rr < 2; ++rr) {
-      const bool ok = colb < K && trow0 + g + 8 * rr < sg.rows;        // past the matrix: zeros, no access
-      const size_t off = ok ? ((size_t)(prow + g + 8 * rr) * groups_per_row + (colb >> (5 + gshift))) * sb : 0;
-      bq_copy_vec(vec + rr * 256, sg.scales + off, vec_bytes, ok);
-      if (!p.symmetric) bq_copy_vec(vec + 512 + rr * 256, sg.biases + off, vec_bytes, ok);
+    const bool ok0 = in && iok0, ok1 = in && iok1;
+    const uint8_t* s0 = p.seg[0].scales;
+    bq_copy_vec(vec, ok0 ? iscale + at : s0, vec_bytes, ok0);
+    bq_copy_vec(vec + 256, ok1 ? iscale + at + row8_step : s0, vec_bytes, ok1);
+    if (!p.symmetric) {
+      bq_copy_vec(vec + 512, ok0 ? ibias + at : s0, vec_bytes, ok0);
+      bq_copy_vec(vec + 768, ok1 ? ibias + at + row8_step : s0, vec_bytes, ok1);
     }
     asm volatile("cp.async.mbarrier.arrive.noinc.shared.b64 [%0];" :: "r"(bar) : "memory");
     icur.advance(1, spt);
@@ -425,11 +440,10 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   // where the scales of chunks 4t .. 4t + 3 lie in a vector: byte selectors that spread it to one scale per chunk
   const uint32_t sel_x = sb == 2 ? (gshift == 0 ? 0x3210u : 0x1010u) : (gshift == 0 ? 0x3210u : gshift == 1 ? 0x1100u : 0x0000u);
   const uint32_t sel_y = gshift == 0 ? 0x7654u : (gshift == 1 ? 0x3232u : 0x1010u);
-  int slot = 0;
+  int slot = 0, mat = 0, stage = -1, sidx = 0, trow0 = 0;
   uint32_t parity = 0;
   for (int i = 0; i < n_items && !dead; ++i) {
-    int mat, stage, sidx, trow0;
-    locate(cur, mat, stage, sidx, trow0);
+    if (stage < 0 || ++stage == spt1) locate(cur, mat, stage, sidx, trow0);
     const int tl = cur.tl;
     if (!mbar_wait(mybars + 8 * slot, parity, p.err)) { dead = true; break; }
     consumed = i + 1;
@@ -439,8 +453,11 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
     {
       const float* Sq = S + (size_t)(stage * 16 + 4 * t) * NC;          // rows past nchunks are zero
       // a vector shorter than a word starts at byte `lead` of its word, the same for rows g and g + 8
-      const int prow = (int)(rowoff + (mat == 1 ? p.expert_up_off : 0)) + trow0 + g;
-      const uint32_t lead = (uint32_t)((prow * groups_per_row + ((stage * BQ_KC + t * 128) >> (5 + gshift))) * sb) & 3u;
+      uint32_t lead = 0;
+      if (vec_bytes < 4) {
+        const int prow = (int)(rowoff + (mat == 1 ? p.expert_up_off : 0)) + trow0 + g;
+        lead = (uint32_t)((prow * groups_per_row + ((stage * BQ_KC + t * 128) >> (5 + gshift))) * sb) & 3u;
+      }
       const uint32_t sx = sel_x + 0x1111u * lead, sy = sel_y + 0x1111u * lead;
       const uint32_t vec = base + G::BOX_BYTES + lane * 8;
 #pragma unroll

@@ -767,7 +767,12 @@ static bool launch_lmh_ts(cudaStream_t st, const LmHeadArgs& a, float* pv, int32
     return false;
   const int group = FMT == F_Q6_K ? 32 : 64;
   TsPlan p;
-  if (!ts_plan(&p, FMT, a.T, a.K, a.V, 2, 0, group, LMH_TS_AUX, options().lm_head_ksplit)) return false;
+  // Items of one round stay whole when they fill most SMs or are short: a cut saves less than handing the parts over
+  // and selecting late costs (q4_0, 40 rows, 118 items: K = 1024 71.4 -> 54.0 us, K = 4096 98.2 -> 84.0; 63 items,
+  // K = 1024 35.2 -> 33.0).  Several rounds are cut evenly (q8_0, 64 rows, 501 items: 275.6 us, 280.6 whole).
+  const int64_t items = (a.V + 255) / 256 * ((a.T + group - 1) / group);
+  const bool whole = items <= sm_count() && (2 * items > sm_count() || a.K < 2048);
+  if (!ts_plan(&p, FMT, a.T, a.K, a.V, 2, 0, group, LMH_TS_AUX, options().lm_head_ksplit && !whole)) return false;
   int* err = device_error_flag();
   if (!err || !a.scratch || a.scratch_bytes < p.scratch()) return false;
   static bool attr_set[64] = {};

@@ -5,8 +5,9 @@
 // issue slots of decode + FMA.  So everything a lane needs for a step is asked for at once and coalesced:
 // four lanes share a 32-column unit - a lane holds 8 weights of it, two groups of four consecutive columns, so
 // that the activations are two vector loads - a warp covers 256 columns of R rows per step, and the warps of a
-// CTA share the steps of a row when there are too few rows to fill the GPU.  A scale multiplies the partial sum
-// of its 8 weights.  One warp per row with a 32-column span per lane (scalar, strided activation loads): 30.7 us for
+// CTA share the steps of a row when there are too few rows to fill the GPU.  The scale goes into the weights
+// (exact products, four packed multiplications per 8 weights): a code times a large activation, or a large scale times
+// the sum of eight products, can leave fp32 where the weight times the activation does not.  One warp per row with a 32-column span per lane (scalar, strided activation loads): 30.7 us for
 // that matrix at one row with the full epilogue, now 4.5 to 5.
 #include "qx_formats.cuh"
 #include "qx_kernels.h"
@@ -36,7 +37,7 @@ __device__ __forceinline__ uint32_t e4m3_pair_bits(uint32_t v) {      // codes a
   return ((v >> 1) & 0x3F803F80u) | (v & 0x80008000u);
 }
 
-// The 8 weights of lane quarter t of 32-column unit u: raw() loads, weights() gives them without their scale.
+// The 8 weights of lane quarter t of 32-column unit u: raw() loads, weights() gives them, scaled.
 // cols(): first columns (inside the unit) of weights 0..3 and 4..7.
 template <int FMT> struct Lane8 {
   uint32_t a, b, c, d;                             // code words (q6_K: low nibbles a, b and high bits c, d)
@@ -63,7 +64,7 @@ template <int FMT> struct Lane8 {
     } else if constexpr (FMT == F_MXFP8) {
       const uint8_t* p = row + (size_t)u * 33;
       const uint2 v = ldg8(p + 1 + 8 * t);
-      a = v.x; b = v.y; scale = e8m0_to_f32(__ldg(p)) * 256.f;
+      a = v.x; b = v.y; scale = e8m0_to_f32(__ldg(p));
     } else {
       const uint8_t* p = row + (size_t)(u >> 3) * 210;
       const int ch = (u >> 2) & 1, g = u & 3;      // 128-column half, 32-column quarter of it
@@ -93,11 +94,19 @@ template <int FMT> struct Lane8 {
       ints(a ^ 0x80808080u, 0x64806480u, w);
       ints(b ^ 0x80808080u, 0x64806480u, w + 4);
     } else if constexpr (FMT == F_MXFP8) {
-      pair(e4m3_pair_bits(__byte_perm(a, 0u, 0x1404)), w[0], w[1]); pair(e4m3_pair_bits(__byte_perm(a, 0u, 0x3424)), w[2], w[3]);
-      pair(e4m3_pair_bits(__byte_perm(b, 0u, 0x1404)), w[4], w[5]); pair(e4m3_pair_bits(__byte_perm(b, 0u, 0x3424)), w[6], w[7]);
+      // * 256 in f16 (at most 480): a scale of 2^120 and more times 256 is none in fp32
+      pair(h2mul(e4m3_pair_bits(__byte_perm(a, 0u, 0x1404)), 0x5C005C00u), w[0], w[1]);
+      pair(h2mul(e4m3_pair_bits(__byte_perm(a, 0u, 0x3424)), 0x5C005C00u), w[2], w[3]);
+      pair(h2mul(e4m3_pair_bits(__byte_perm(b, 0u, 0x1404)), 0x5C005C00u), w[4], w[5]);
+      pair(h2mul(e4m3_pair_bits(__byte_perm(b, 0u, 0x3424)), 0x5C005C00u), w[6], w[7]);
     } else {
       ints((a & 0x0F0F0F0Fu) | ((c << 4) & 0x30303030u), 0x64206420u, w);
       ints((b & 0x0F0F0F0Fu) | ((d << 4) & 0x30303030u), 0x64206420u, w + 4);
+    }
+#pragma unroll
+    for (int i = 0; i < 8; i += 2) {
+      const float2 v = __fmul2_rn(make_float2(w[i], w[i + 1]), make_float2(scale, scale));
+      w[i] = v.x; w[i + 1] = v.y;
     }
   }
 };
@@ -180,7 +189,7 @@ gemv_generic_kernel(const T* __restrict__ x, const uint8_t* __restrict__ w0, con
         float s = w[0] * xv[m][0];
 #pragma unroll
         for (int i = 1; i < 8; ++i) s = fmaf(w[i], xv[m][i], s);
-        acc[r][m] = fmaf(q[r].scale, s, acc[r][m]);
+        acc[r][m] += s;
       }
     }
   }

@@ -132,3 +132,36 @@ def test_seam_rows(rows, D):
             np.testing.assert_allclose(host(s).reshape(-1)[pick], rs.reshape(-1), rtol=1e-5)
             same = (host(c)[pick].astype(np.int32) & 0xFF) == (rc.astype(np.int32) & 0xFF)
             assert same.mean() >= 0.99, (kind, float(same.mean()))
+
+
+# ---- block scales at the ends of their range ------------------------------------------------------------------
+# e8m0 scales of 2^120 and more against small codes and codes of zero, on the generic kernel (fp32 activations, and
+# 16-bit ones that start between 16-byte boundaries): products that fp32 holds stay finite
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4"])
+@pytest.mark.parametrize("e", [0, 1, 246, 247, 254])
+def test_generic_kernel_block_scales(fmt, e):
+    K, N = 96, 35
+    x, W, _, _ = _linear(fmt, 3, K, N, "bf16", e, pack="random")
+    x = x * np.float32(2.0 ** -8)                        # 32 products of up to 2^126 stay below 2^128
+    W[:, 1, 0] = e
+    W[:, 1, 1:] &= 0x88 if fmt == "mxfp8" else 0x11      # 0, 2^-6 and their negatives; 0 and 0.5
+    W[0, 1, 1:] = 0                                      # a block of zeros
+    shifted = torch.zeros(3 * K + 1, dtype=torch.bfloat16, device="cuda")[1:].view(3, K).copy_(dev(x, "bf16"))
+    ref = x.astype(np.float64) @ O.dequantize(fmt, W).astype(np.float64).T
+    size = np.abs(x).astype(np.float64) @ np.abs(O.dequantize(fmt, W)).astype(np.float64).T
+    for xs, ulp in ((dev(x), 2.0 ** -22), (shifted, 2.0 ** -8)):
+        got = host(tk.decode_linear_epilogue(xs, dev(W), None, None, format=fmt)).astype(np.float64)
+        assert np.isfinite(got).all()
+        # one rounding of the output and, below, at most K + 8 of the sum's (2^-24 of the terms each)
+        assert (np.abs(got - ref) <= ulp * np.abs(ref) + (K + 8) * 2.0 ** -24 * size).all()
+
+
+# activations near the end of fp32: a weight times an activation is in range, its code times the activation is not
+@pytest.mark.parametrize("fmt", FMTS)
+def test_generic_kernel_large_activations(fmt):
+    x, W, _, _ = _linear(fmt, 2, 512, 19, "f32", 1)
+    x = (x * 2.0 ** 125).astype(np.float32)              # |x| up to 2^127; sums below 2^127 * 0.02 * 2 * 23
+    w = O.dequantize(fmt, W).astype(np.float64)
+    ref, size = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+    got = host(tk.decode_linear_epilogue(dev(x), dev(W), None, None, format=fmt)).astype(np.float64)
+    assert (np.abs(got - ref) <= 520 * 2.0 ** -24 * size).all()

@@ -150,12 +150,13 @@ __device__ __forceinline__ int ceil_log2(float q) {
 // warp: scale 2^ceil(log2(amax / 448)) (amax > 0), an all-zero block stores exponent 127.
 __device__ __forceinline__ void mxfp8_block_store(float v, int lane, uint8_t* __restrict__ block) {
   // largest magnitude as bits (one warp reduction; NaN does not choose the scale); 448 = 1.75 * 2^8, so
-  // ceil(log2(amax / 448)) is the exponent of amax - 8, plus one when its mantissa is above 1.75
+  // ceil(log2(amax / 448)) is the exponent of amax - 8, plus one when its mantissa is above 1.75 (the sum below
+  // carries then); an infinity takes the largest scale
   const uint32_t top = __reduce_max_sync(0xffffffffu, v == v ? __float_as_uint(v) & 0x7FFFFFFFu : 0u);
   int code = 127;
   if (top != 0u) {
     const uint32_t t = max(top, __float_as_uint(1e-10f));
-    code = min(max((int)(t >> 23) - 8 + ((t & 0x7FFFFFu) > 0x600000u ? 1 : 0), 1), 254);
+    code = t == 0x7F800000u ? 254 : (int)((t + 0x1FFFFFu) >> 23) - 8;
   }
   const float inv = __uint_as_float(max((uint32_t)(254 - code) << 23, 0x00400000u));     // 2^(127 - code)
   block[1 + lane] = (uint8_t)e4m3_encode(v * inv);

@@ -165,3 +165,11 @@ def test_generic_kernel_large_activations(fmt):
     ref, size = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
     got = host(tk.decode_linear_epilogue(dev(x), dev(W), None, None, format=fmt)).astype(np.float64)
     assert (np.abs(got - ref) <= 520 * 2.0 ** -24 * size).all()
+
+
+def test_mxfp8_rows_of_infinities():
+    x = rounded(np.random.default_rng(2).standard_normal((4, 96)), "bf16")
+    x[0, 5], x[1, 40], x[2, :32], x[3, 64:] = np.inf, -np.inf, np.inf, 3.3e38
+    x = rounded(x, "bf16")
+    for dtype in ("bf16", "f32"):
+        np.testing.assert_array_equal(host(tk_torch.quantize_mxfp8_rows(dev(x, dtype))), O.quantize_mxfp8_rows(x))

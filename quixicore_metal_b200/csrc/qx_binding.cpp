@@ -56,7 +56,7 @@ const at::Tensor& tensor(PyObject* o, const char* op) {
   if (!THPVariable_Check(o)) fail(std::string(op) + ": a tensor was expected");
   return THPVariable_Unpack(o);
 }
-const at::Tensor* tensor_or_null(PyObject* o) { return THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr; }
+const at::Tensor* tensor_or_null(PyObject* o, const char* op) { return o == Py_None ? nullptr : &tensor(o, op); }   // only None is absent
 int64_t integer(PyObject* o) {
   const int64_t v = PyLong_AsLongLong(o);
   if (v == -1 && PyErr_Occurred()) { PyErr_Clear(); fail("an integer was expected"); }
@@ -242,7 +242,7 @@ PyObject* lm_head_sample_q(PyObject*, PyObject* const* a, Py_ssize_t) {
   return guarded([&]() -> PyObject* {
     static const char* op = "lm_head_sample_q";
     const at::Tensor &h = tensor(a[0], op), &w = tensor(a[1], op);
-    const at::Tensor* b = tensor_or_null(a[2]);
+    const at::Tensor* b = tensor_or_null(a[2], op);
     const int64_t V = integer(a[3]), K = integer(a[4]), mode = integer(a[6]), topk = integer(a[7]);
     const Format* f = format_of(text(a[5]));
     const double temperature = real(a[8]), top_p = real(a[10]);
@@ -357,7 +357,7 @@ PyObject* base_q_matmul(PyObject*, PyObject* const* a, Py_ssize_t) {
     if (std::strcmp(layout, "metal") && std::strcmp(layout, "metal_lane_strided") && lane != layout)
       fail("BaseQN: layout must be metal or metal_lane_strided_q" + std::to_string(bits));
     const at::Tensor &c = tensor(a[0], op), &s = tensor(a[1], op), &x = tensor(a[3], op);
-    const at::Tensor* b = tensor_or_null(a[2]);
+    const at::Tensor* b = tensor_or_null(a[2], op);
     const at::ScalarType st = bf ? at::kBFloat16 : hf ? at::kHalf : at::kByte;
     check(c.is_cuda() && c.scalar_type() == at::kByte && c.dim() == 2, op, "codes must be uint8 (rows, packed_bytes)");
     check(s.is_cuda() && s.scalar_type() == st && s.dim() == 2, op, "scales must be a rank-2 tensor with the declared scale_dtype");

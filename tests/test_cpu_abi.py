@@ -396,3 +396,15 @@ def test_missing_library_fails_loudly(monkeypatch, tmp_path):
     monkeypatch.setattr(_lib, "LIB_PATH", str(tmp_path / "nope.so"))
     with pytest.raises(ImportError, match="no fallback"):
         _lib.lib()
+
+
+def test_only_none_is_an_absent_operand():
+    """Anything else that is no tensor is an error, not a missing bias."""
+    import torch
+    from quixicore_metal_b200 import tk_torch
+    h, w = torch.zeros(1, 64), torch.zeros(8, 2, 34, dtype=torch.uint8)
+    with pytest.raises(RuntimeError, match="a tensor was expected"):
+        tk_torch.lm_head_sample_q(h, w, [0.0] * 8, 8, 64, "q8_0", 0, 0, 1.0, 1)
+    codes, scales = torch.zeros(4, 64, dtype=torch.uint8), torch.zeros(4, 2, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="a tensor was expected"):
+        tk_torch.base_qgemm(codes, scales, [0.0], torch.zeros(64, 2), 8, 32, "bf16", True)

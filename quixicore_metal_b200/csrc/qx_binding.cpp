@@ -51,6 +51,14 @@ PyObject* guarded(F&& f) {
   return nullptr;
 }
 
+// The interpreter is released while a call copies operands, allocates and enqueues: a launch blocks when the queue
+// is full, and other threads (and host functions on the stream) go on meanwhile.  No Python object is touched inside;
+// the caller's argument tuple keeps the operands alive.
+struct Released {
+  PyThreadState* state = PyEval_SaveThread();
+  ~Released() { PyEval_RestoreThread(state); }
+};
+
 // ---- arguments -----------------------------------------------------------------------------------------
 const at::Tensor& tensor(PyObject* o, const char* op) {
   if (!THPVariable_Check(o)) fail(std::string(op) + ": a tensor was expected");
@@ -165,25 +173,31 @@ PyObject* decode_linear_epilogue(PyObject*, PyObject* const* a, Py_ssize_t) {
           "bias must be (N,) with x dtype");
     check(!ur || (r->is_cuda() && r->dim() == 2 && r->size(0) == B && r->size(1) == N && r->scalar_type() == x.scalar_type()), op,
           "residual must be (B,N) with x dtype");
-    const c10::cuda::OptionalCUDAGuard guard(x.device());
-    const at::Tensor xc = dense(x), wc = dense(w);
-    at::Tensor bc, rc;
-    if (ub) bc = dense(*b);
-    if (ur) rc = dense(*r);
     const int kind = (int)integer(a[8]);
-    at::Tensor out = empty({B, N}, x.scalar_type(), x);
-    if (truth(a[10])) {
-      check(kind == 0, op, "the ordered form has no output_quant");
-      check_status(qx_cuda_decode_linear_epilogue_ordered(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), ptr(bc), ptr(rc),
-                                                          ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), (int)act, ub, ur,
-                                                          nullptr, 0));
-      return wrap(out);
+    const bool with_output = truth(a[9]), ordered = truth(a[10]);
+    at::Tensor out;
+    Quant q;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(x.device());
+      const at::Tensor xc = dense(x), wc = dense(w);
+      at::Tensor bc, rc;
+      if (ub) bc = dense(*b);
+      if (ur) rc = dense(*r);
+      out = empty({B, N}, x.scalar_type(), x);
+      if (ordered) {
+        check(kind == 0, op, "the ordered form has no output_quant");
+        check_status(qx_cuda_decode_linear_epilogue_ordered(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), ptr(bc), ptr(rc),
+                                                            ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), (int)act, ub,
+                                                            ur, nullptr, 0));
+      } else {
+        q = quant_outputs(x, B, N, kind);
+        check_status(qx_cuda_decode_linear_epilogue(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), ptr(bc), ptr(rc),
+                                                    ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), (int)act, ub, ur,
+                                                    kind, ptr(q.codes), (float*)ptr(q.scale), nullptr, 0));
+      }
     }
-    Quant q = quant_outputs(x, B, N, kind);
-    check_status(qx_cuda_decode_linear_epilogue(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), ptr(bc), ptr(rc), ptr(out),
-                                                B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), (int)act, ub, ur, kind,
-                                                ptr(q.codes), (float*)ptr(q.scale), nullptr, 0));
-    return quant_result(out, kind, q, truth(a[9]));
+    return quant_result(out, kind, q, with_output);
   });
 }
 
@@ -195,11 +209,15 @@ PyObject* decode_linear_partial(PyObject*, PyObject* const* a, Py_ssize_t) {
     const Format* f = format_of(text(a[2]));
     const int64_t N = check_weight(x, w, f, op);
     same_device(op, x, &w);
-    const c10::cuda::OptionalCUDAGuard guard(x.device());
-    const at::Tensor xc = dense(x), wc = dense(w);
-    at::Tensor out = empty({x.size(0), N}, at::kFloat, x);
-    check_status(qx_cuda_decode_linear_partial(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), (float*)ptr(out), x.size(0),
-                                               x.size(1), N, f->name, (qx_dtype)dtype_of(x.scalar_type()), nullptr, 0));
+    at::Tensor out;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(x.device());
+      const at::Tensor xc = dense(x), wc = dense(w);
+      out = empty({x.size(0), N}, at::kFloat, x);
+      check_status(qx_cuda_decode_linear_partial(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(wc), (float*)ptr(out), x.size(0),
+                                                 x.size(1), N, f->name, (qx_dtype)dtype_of(x.scalar_type()), nullptr, 0));
+    }
     return wrap(out);
   });
 }
@@ -217,23 +235,29 @@ PyObject* decode_swiglu(PyObject*, PyObject* const* a, Py_ssize_t) {
     same_device(op, x, &g); same_device(op, x, &u); same_device(op, x, gb); same_device(op, x, bb);
     check(!ub || (gb->is_cuda() && bb->is_cuda() && gb->scalar_type() == x.scalar_type() && bb->scalar_type() == x.scalar_type() &&
                   gb->dim() == 1 && bb->dim() == 1 && gb->size(0) == N && bb->size(0) == N), op, "both biases must be (N,) with x dtype");
-    const c10::cuda::OptionalCUDAGuard guard(x.device());
-    const at::Tensor xc = dense(x), gc = dense(g), uc = dense(u);
-    at::Tensor gbc, bbc;
-    if (ub) { gbc = dense(*gb); bbc = dense(*bb); }
     const int kind = (int)integer(a[7]);
-    at::Tensor out = empty({B, N}, x.scalar_type(), x);
-    if (truth(a[9])) {
-      check(kind == 0, op, "the ordered form has no output_quant");
-      check_status(qx_cuda_decode_swiglu_ordered(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(uc), ptr(gbc), ptr(bbc),
-                                                 ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), ub, nullptr, 0));
-      return wrap(out);
+    const bool with_output = truth(a[8]), ordered = truth(a[9]);
+    at::Tensor out;
+    Quant q;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(x.device());
+      const at::Tensor xc = dense(x), gc = dense(g), uc = dense(u);
+      at::Tensor gbc, bbc;
+      if (ub) { gbc = dense(*gb); bbc = dense(*bb); }
+      out = empty({B, N}, x.scalar_type(), x);
+      if (ordered) {
+        check(kind == 0, op, "the ordered form has no output_quant");
+        check_status(qx_cuda_decode_swiglu_ordered(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(uc), ptr(gbc), ptr(bbc),
+                                                   ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), ub, nullptr, 0));
+      } else {
+        q = quant_outputs(x, B, N, kind);
+        check_status(qx_cuda_decode_swiglu(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(uc), ptr(gbc), ptr(bbc),
+                                           ptr(out), B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), ub, kind, ptr(q.codes),
+                                           (float*)ptr(q.scale), nullptr, 0));
+      }
     }
-    Quant q = quant_outputs(x, B, N, kind);
-    check_status(qx_cuda_decode_swiglu(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(uc), ptr(gbc), ptr(bbc), ptr(out),
-                                       B, K, N, f->name, (qx_dtype)dtype_of(x.scalar_type()), ub, kind, ptr(q.codes),
-                                       (float*)ptr(q.scale), nullptr, 0));
-    return quant_result(out, kind, q, truth(a[8]));
+    return quant_result(out, kind, q, with_output);
   });
 }
 
@@ -264,18 +288,22 @@ PyObject* lm_head_sample_q(PyObject*, PyObject* const* a, Py_ssize_t) {
       check(topk <= V, op, "k must be <= vocab size V");
     }
     if (ub) check(b->numel() == V, op, "bias must be (V,)");
-    const c10::cuda::OptionalCUDAGuard guard(h.device());
-    const at::Tensor hc = dense(h), wc = dense(w);
-    at::Tensor bc;
-    if (ub) bc = b->to(at::kFloat).contiguous();
-    const int64_t T = h.size(0);
-    const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
-    at::Tensor ids = empty({T}, at::kInt, h);
-    const size_t bytes = qx_cuda_lm_head_workspace_bytes(T, V, K, (int)mode, (int)topk);
-    const at::Tensor ws = workspace(h, st, bytes);
-    check_status(qx_cuda_lm_head_sample_q(st, ptr(hc), ptr(wc), (const float*)ptr(bc), (int32_t*)ptr(ids), ptr(ws), bytes, T, V, K, f->name,
-                                          (qx_dtype)dtype_of(h.scalar_type()), (int)mode, (int)topk, temperature,
-                                          (uint32_t)PyLong_AsUnsignedLongLongMask(a[9]), top_p));
+    const uint32_t seed = (uint32_t)PyLong_AsUnsignedLongLongMask(a[9]);
+    at::Tensor ids;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(h.device());
+      const at::Tensor hc = dense(h), wc = dense(w);
+      at::Tensor bc;
+      if (ub) bc = b->to(at::kFloat).contiguous();
+      const int64_t T = h.size(0);
+      const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
+      ids = empty({T}, at::kInt, h);
+      const size_t bytes = qx_cuda_lm_head_workspace_bytes(T, V, K, (int)mode, (int)topk);
+      const at::Tensor ws = workspace(h, st, bytes);
+      check_status(qx_cuda_lm_head_sample_q(st, ptr(hc), ptr(wc), (const float*)ptr(bc), (int32_t*)ptr(ids), ptr(ws), bytes, T, V, K,
+                                            f->name, (qx_dtype)dtype_of(h.scalar_type()), (int)mode, (int)topk, temperature, seed, top_p));
+    }
     return wrap(ids);
   });
 }
@@ -290,22 +318,28 @@ PyObject* rms_norm_add(PyObject*, PyObject* const* a, Py_ssize_t) {
     check(r.sizes() == x.sizes() && r.scalar_type() == x.scalar_type() && w.dim() == 1 && w.size(0) == D && w.scalar_type() == x.scalar_type(),
           op, "residual must match x, weight must be (D,) with x dtype");
     same_device(op, x, &r); same_device(op, x, &w);
-    const c10::cuda::OptionalCUDAGuard guard(x.device());
-    const at::Tensor xc = dense(x), rc = dense(r), wc = dense(w);
     const int quant = (int)integer(a[4]), group = (int)integer(a[6]);
-    at::Tensor added = at::empty_like(xc), y, codes, scale;
-    if (quant == 0) y = at::empty_like(xc);
-    else codes = empty(x.sizes(), quant == 3 || quant == 5 ? at::kChar : at::kByte, x);
-    if (quant == 2 || quant == 3) {
-      scale = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
-    } else if (quant >= 4) {
-      std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
-      shape.back() = D / group;
-      scale = empty(shape, at::kFloat, x);
+    const double eps = real(a[3]), static_scale = real(a[5]);
+    const bool ue8m0 = truth(a[7]);
+    at::Tensor added, y, codes, scale;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(x.device());
+      const at::Tensor xc = dense(x), rc = dense(r), wc = dense(w);
+      added = at::empty_like(xc);
+      if (quant == 0) y = at::empty_like(xc);
+      else codes = empty(x.sizes(), quant == 3 || quant == 5 ? at::kChar : at::kByte, x);
+      if (quant == 2 || quant == 3) {
+        scale = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
+      } else if (quant >= 4) {
+        std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+        shape.back() = D / group;
+        scale = empty(shape, at::kFloat, x);
+      }
+      check_status(qx_cuda_rms_norm_add(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(rc), ptr(wc), ptr(y), ptr(codes),
+                                        ptr(added), (float*)ptr(scale), rows, D, (qx_dtype)dtype_of(x.scalar_type()), eps, quant,
+                                        static_scale, group, ue8m0));
     }
-    check_status(qx_cuda_rms_norm_add(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(rc), ptr(wc), ptr(y), ptr(codes), ptr(added),
-                                      (float*)ptr(scale), rows, D, (qx_dtype)dtype_of(x.scalar_type()), real(a[3]), quant, real(a[5]), group,
-                                      truth(a[7])));
     return Py_BuildValue("(NNNN)", wrap_or_none(y), wrap_or_none(codes), wrap(added), wrap_or_none(scale));
   });
 }
@@ -323,18 +357,24 @@ PyObject* silu_mul_quant(PyObject*, PyObject* const* a, Py_ssize_t) {
     const int64_t D = x.size(-1), rows = x.numel() / D;
     const int quant = (int)integer(a[5]), group = (int)integer(a[6]);
     if (quant == 4) check(group > 0 && group % 4 == 0 && D % group == 0, op, "group_size must be a multiple of 4 that divides D");
-    const c10::cuda::OptionalCUDAGuard guard(x.device());
-    const at::Tensor xc = dense(x), gc = dense(g);
-    at::Tensor codes = empty(x.sizes(), quant == 3 ? at::kChar : at::kByte, x), scale;
-    if (quant == 4) {
-      std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
-      shape.back() = D / group;
-      scale = empty(shape, at::kFloat, x);
-    } else {
-      scale = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
+    const double alpha = real(a[3]), limit = real(a[4]);
+    const bool ue8m0 = truth(a[7]);
+    at::Tensor codes, scale;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(x.device());
+      const at::Tensor xc = dense(x), gc = dense(g);
+      codes = empty(x.sizes(), quant == 3 ? at::kChar : at::kByte, x);
+      if (quant == 4) {
+        std::vector<int64_t> shape(x.sizes().begin(), x.sizes().end());
+        shape.back() = D / group;
+        scale = empty(shape, at::kFloat, x);
+      } else {
+        scale = empty(x.sizes().slice(0, x.dim() - 1), at::kFloat, x);
+      }
+      check_status(qx_cuda_silu_mul_quant(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(codes), (float*)ptr(scale),
+                                          rows, D, (qx_dtype)dtype_of(x.scalar_type()), (int)act, alpha, limit, quant, group, ue8m0));
     }
-    check_status(qx_cuda_silu_mul_quant(at::cuda::getCurrentCUDAStream().stream(), ptr(xc), ptr(gc), ptr(codes), (float*)ptr(scale), rows, D,
-                                        (qx_dtype)dtype_of(x.scalar_type()), (int)act, real(a[3]), real(a[4]), quant, group, truth(a[7])));
     return Py_BuildValue("(NN)", wrap(codes), wrap(scale));
   });
 }
@@ -373,18 +413,22 @@ PyObject* base_q_matmul(PyObject*, PyObject* const* a, Py_ssize_t) {
     if (x.size(1) <= 0) fail("BaseQN matmul: M must be positive");
     same_device(op, c, &x);
     const int64_t M = x.size(1);
-    const c10::cuda::OptionalCUDAGuard guard(x.device());
-    const at::Tensor cc = dense(c), sc = dense(s), xc = dense(x);
-    at::Tensor bc, ws;
-    if (b) bc = dense(*b);
-    at::Tensor out = empty({rows, M}, x.scalar_type(), x);
-    const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
-    const qx_dtype dt = (qx_dtype)dtype_of(x.scalar_type());
-    const size_t bytes = qx_cuda_base_q_workspace_bytes(K, M, 0, dt);
-    if (bytes) ws = workspace(x, stream, bytes);
-    const qx_base_q_planes planes{ptr(cc), ptr(sc), ptr(bc)};
-    const qx_base_q_desc desc{(int32_t)bits, (int32_t)group, sd, sym, layout};
-    check_status(qx_cuda_base_qgemm(stream, &planes, &desc, ptr(xc), ptr(out), rows, K, M, dt, ptr(ws), bytes));
+    at::Tensor out;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(x.device());
+      const at::Tensor cc = dense(c), sc = dense(s), xc = dense(x);
+      at::Tensor bc, ws;
+      if (b) bc = dense(*b);
+      out = empty({rows, M}, x.scalar_type(), x);
+      const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
+      const qx_dtype dt = (qx_dtype)dtype_of(x.scalar_type());
+      const size_t bytes = qx_cuda_base_q_workspace_bytes(K, M, 0, dt);
+      if (bytes) ws = workspace(x, stream, bytes);
+      const qx_base_q_planes planes{ptr(cc), ptr(sc), ptr(bc)};
+      const qx_base_q_desc desc{(int32_t)bits, (int32_t)group, sd, sym, layout};
+      check_status(qx_cuda_base_qgemm(stream, &planes, &desc, ptr(xc), ptr(out), rows, K, M, dt, ptr(ws), bytes));
+    }
     return wrap(out);
   });
 }

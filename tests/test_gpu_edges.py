@@ -173,3 +173,30 @@ def test_mxfp8_rows_of_infinities():
     x = rounded(x, "bf16")
     for dtype in ("bf16", "f32"):
         np.testing.assert_array_equal(host(tk_torch.quantize_mxfp8_rows(dev(x, dtype))), O.quantize_mxfp8_rows(x))
+
+
+# ---- host side -------------------------------------------------------------------------------------------------
+def test_other_threads_run_while_a_launch_blocks():
+    """The launch queue behind a long kernel fills up; the thread that blocks on it must not hold the interpreter."""
+    import threading
+    import time
+    x, W, _, _ = _linear("q4_0", 1, 512, 64, "bf16", 1)
+    x, W = dev(x, "bf16"), dev(W)
+    run = lambda: tk.decode_linear_epilogue(x, W, None, None, format="q4_0")
+    run(); torch.cuda.synchronize()
+    done = threading.Event()
+
+    def work():
+        torch.cuda._sleep(int(1.5e9))                    # below a second
+        for _ in range(3000):
+            run()
+        done.set()
+    t = threading.Thread(target=work)
+    gap, last = 0.0, time.perf_counter()
+    t.start()
+    while not done.is_set():
+        now = time.perf_counter()
+        gap, last = max(gap, now - last), now
+        time.sleep(0)
+    t.join(); torch.cuda.synchronize()
+    assert gap < 0.25, gap

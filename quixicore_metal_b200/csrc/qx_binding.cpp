@@ -100,22 +100,32 @@ at::Tensor empty(at::IntArrayRef shape, at::ScalarType t, const at::Tensor& like
 }
 inline at::Tensor dense(const at::Tensor& t) { return t.is_contiguous() ? t : t.contiguous(); }
 
-// ---- workspace: one growing scratch tensor per stream, as the Python layer keeps them --------------------
-// Calls on one stream are ordered, so they share it; a replaced tensor's block goes back to the caching
-// allocator, which reuses it on this stream only.  At most 64 streams are remembered.
+// ---- workspace: one growing scratch tensor per stream ----------------------------------------------------
+// Calls on one stream are ordered, so they share it.  A captured graph keeps the addresses that its calls used for
+// as long as it lives, so memory once handed out is never given to anyone else: a tensor that became too small stays
+// (each is at least twice as large as the one before, the total below twice the largest), and streams past
+// the 64th get a tensor for the one call - a capture keeps what it allocated itself.
 struct Key { int dev; cudaStream_t st; bool operator==(const Key& o) const { return dev == o.dev && st == o.st; } };
 struct KeyHash { size_t operator()(const Key& k) const { return std::hash<void*>()((void*)k.st) * 31u + (size_t)k.dev; } };
 std::mutex g_ws_mu;
-std::unordered_map<Key, at::Tensor, KeyHash>& ws_map() { static auto* m = new std::unordered_map<Key, at::Tensor, KeyHash>(); return *m; }
-at::Tensor workspace(const at::Tensor& like, cudaStream_t st, size_t bytes) {
-  std::lock_guard<std::mutex> lock(g_ws_mu);
-  auto& m = ws_map();
-  if (m.size() >= 64 && !m.count(Key{like.get_device(), st})) m.clear();
-  at::Tensor& t = m[Key{(int)like.get_device(), st}];
-  if (!t.defined() || (size_t)t.numel() < bytes) {
-    int64_t size = std::max<int64_t>((int64_t)bytes, 1 << 20);
-    if (t.defined()) size = std::max<int64_t>(size, 2 * t.numel());
-    t = empty({size}, at::kByte, like);
+using Sizes = std::vector<at::Tensor>;             // ascending; the last one serves the calls
+std::unordered_map<Key, Sizes, KeyHash>& ws_map() { static auto* m = new std::unordered_map<Key, Sizes, KeyHash>(); return *m; }
+at::Tensor workspace(at::Device device, cudaStream_t st, size_t bytes) {      // `device` is current, the interpreter released
+  const Key key{(int)device.index(), st};
+  int64_t size = std::max<int64_t>((int64_t)bytes, 1 << 20);
+  {
+    const std::lock_guard<std::mutex> lock(g_ws_mu);
+    const auto it = ws_map().find(key);
+    if (it != ws_map().end()) {
+      if ((size_t)it->second.back().numel() >= bytes) return it->second.back();
+      size = std::max<int64_t>(size, 2 * it->second.back().numel());
+    }
+  }
+  const at::Tensor t = at::empty({size}, at::TensorOptions().dtype(at::kByte).device(device));
+  const std::lock_guard<std::mutex> lock(g_ws_mu);
+  if (ws_map().size() < 64 || ws_map().count(key)) {
+    Sizes& s = ws_map()[key];
+    if (s.empty() || s.back().numel() < size) s.push_back(t);
   }
   return t;
 }
@@ -300,7 +310,7 @@ PyObject* lm_head_sample_q(PyObject*, PyObject* const* a, Py_ssize_t) {
       const cudaStream_t st = at::cuda::getCurrentCUDAStream().stream();
       ids = empty({T}, at::kInt, h);
       const size_t bytes = qx_cuda_lm_head_workspace_bytes(T, V, K, (int)mode, (int)topk);
-      const at::Tensor ws = workspace(h, st, bytes);
+      const at::Tensor ws = workspace(h.device(), st, bytes);
       check_status(qx_cuda_lm_head_sample_q(st, ptr(hc), ptr(wc), (const float*)ptr(bc), (int32_t*)ptr(ids), ptr(ws), bytes, T, V, K,
                                             f->name, (qx_dtype)dtype_of(h.scalar_type()), (int)mode, (int)topk, temperature, seed, top_p));
     }
@@ -424,12 +434,27 @@ PyObject* base_q_matmul(PyObject*, PyObject* const* a, Py_ssize_t) {
       const cudaStream_t stream = at::cuda::getCurrentCUDAStream().stream();
       const qx_dtype dt = (qx_dtype)dtype_of(x.scalar_type());
       const size_t bytes = qx_cuda_base_q_workspace_bytes(K, M, 0, dt);
-      if (bytes) ws = workspace(x, stream, bytes);
+      if (bytes) ws = workspace(x.device(), stream, bytes);
       const qx_base_q_planes planes{ptr(cc), ptr(sc), ptr(bc)};
       const qx_base_q_desc desc{(int32_t)bits, (int32_t)group, sd, sym, layout};
       check_status(qx_cuda_base_qgemm(stream, &planes, &desc, ptr(xc), ptr(out), rows, K, M, dt, ptr(ws), bytes));
     }
     return wrap(out);
+  });
+}
+
+// (device index, bytes) -> uint8 tensor of at least that size for calls on the current stream
+PyObject* stream_workspace(PyObject*, PyObject* const* a, Py_ssize_t) {
+  return guarded([&]() -> PyObject* {
+    const at::Device device(at::kCUDA, (c10::DeviceIndex)integer(a[0]));
+    const int64_t bytes = integer(a[1]);
+    at::Tensor ws;
+    {
+      const Released released;
+      const c10::cuda::OptionalCUDAGuard guard(device);
+      ws = workspace(device, at::cuda::getCurrentCUDAStream(device.index()).stream(), (size_t)bytes);
+    }
+    return wrap(ws);
   });
 }
 
@@ -453,6 +478,7 @@ PyMethodDef methods[] = {
     QX_METHOD(rms_norm_add, 9),
     QX_METHOD(silu_mul_quant, 9),
     QX_METHOD(base_q_matmul, 11),
+    QX_METHOD(stream_workspace, 2),
     {"set_status_handler", set_status_handler, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_qx_native", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

@@ -58,21 +58,10 @@ def _same_device(name: str, first, *others) -> None:
                                f"(got {first.device} and {t.device})")
 
 
-_WS = {}
-
-
 def _workspace(device, nbytes: int):
-    """Scratch tensor for calls on the current stream of `device`, reused by later calls on the same
-    stream (they are ordered, so sharing it is safe) and grown geometrically."""
-    key = (device.index, _raw_stream(device.index) if _raw_stream is not None
-           else torch.cuda.current_stream(device).cuda_stream)
-    ws = _WS.get(key)
-    if ws is None or ws.numel() < nbytes:
-        size = max(int(nbytes), 1 << 20, 0 if ws is None else 2 * ws.numel())
-        ws = torch.empty((size,), dtype=torch.uint8, device=device)
-        _WS[key] = ws       # a smaller predecessor stays alive while enqueued work may read it:
-        #                     the caching allocator only reuses its block for this same stream
-    return ws
+    """Scratch tensor for calls on the current stream of `device`, shared by all calls on that stream
+    (they are ordered) and with the operators whose host side is native."""
+    return _native().stream_workspace(device.index, nbytes)
 
 
 _native = _lib.native       # the operators of a decode step run their host side in C++ (csrc/qx_binding.cpp)

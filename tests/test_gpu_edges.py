@@ -200,3 +200,26 @@ def test_other_threads_run_while_a_launch_blocks():
         time.sleep(0)
     t.join(); torch.cuda.synchronize()
     assert gap < 0.25, gap
+
+
+def test_workspace_of_a_captured_graph_survives_larger_calls():
+    """A graph keeps the addresses of the workspace that its calls used; later calls may not give that memory away."""
+    rng = np.random.default_rng(2)
+    V, K = 6000, 512
+    W = dev(O.synth_pack("q4_0", (0.3 * rng.standard_normal((V, K))).astype(np.float32)))
+    h = dev(rounded(rng.standard_normal((64, K)), "bf16"), "bf16")
+    call = lambda T: tk.lm_head_sample(h[:T], W, mode="topk", k=8, temperature=0.8, seed=3, format="q4_0")
+    s = torch.cuda.Stream()
+    s.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(s):
+        want = call(2)
+        g = torch.cuda.CUDAGraph()
+        s.synchronize()
+        with torch.cuda.graph(g, stream=s):
+            got = call(2)
+        call(64)                                         # a larger workspace on the same stream
+        keep = [torch.full((4 << 20,), 90, dtype=torch.uint8, device="cuda") for _ in range(32)]
+        g.replay()
+        s.synchronize()
+        assert torch.equal(got, want)
+        assert all(bool((t == 90).all()) for t in keep)

@@ -793,8 +793,8 @@ static bool launch_lmh_ts(cudaStream_t st, const LmHeadArgs& a, float* pv, int32
                    (int)a.T, (int)a.K, (int)a.V, err};
   const TsLmHead::Args ea{a.bias, pv, pi, pl, (long long)a.vocab_offset, (long long)tiles_stride, a.mode, a.topk, a.invtemp,
                           a.seed, a.mask};
-  ts_launch_prep(st, p, FMT, a.h, a.dtype, s, (int)a.T, (int)a.K);
-  return ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsLmHead>, m[0], m[1], m[0], m[1], q, ea);
+  return ts_launch_prep(st, p, FMT, a.h, a.dtype, s, (int)a.T, (int)a.K) &&
+         ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsLmHead>, m[0], m[1], m[0], m[1], q, ea);
 }
 
 template <int FMT>

@@ -121,8 +121,11 @@ __global__ void __launch_bounds__(256)
 ts_prep_kernel(const T* __restrict__ x, uint4* __restrict__ img, float* __restrict__ rowscale, unsigned* __restrict__ count,
                int ncount, int K, int mg, int mp, int fmt) {
   __shared__ float red[8];
-  asm volatile("griddepcontrol.launch_dependents;");
+  // First the wait: the contraction may be scheduled once every CTA is past it, so all that ran before this kernel is
+  // complete then - its weight loads need no wait of their own (an earlier kernel of the stream may have written
+  // them), and its bounded waits do not count while a long predecessor runs.
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;");
   const int m = blockIdx.x;
   if (m == 0)
     for (int i = threadIdx.x; i < ncount; i += blockDim.x) count[i] = 0u;
@@ -177,12 +180,11 @@ ts_prep_kernel(const T* __restrict__ x, uint4* __restrict__ img, float* __restri
   if (threadIdx.x == 0) rowscale[m] = __uint_as_float((uint32_t)(127 + S) << 23);
 }
 
-void ts_launch_prep(cudaStream_t st, const TsPlan& p, int format, const void* x, qx_dtype dtype, const TsScratch& s, int M, int K) {
+bool ts_launch_prep(cudaStream_t st, const TsPlan& p, int format, const void* x, qx_dtype dtype, const TsScratch& s, int M, int K) {
   const int ncount = p.whole ? 0 : p.items;
   if (dtype == QX_DTYPE_F16)
-    ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__half>, (const __half*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
-  else
-    ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
+    return ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__half>, (const __half*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
+  return ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
 }
 
 // ---- projection epilogue ------------------------------------------------------------------------------
@@ -333,8 +335,8 @@ static bool launch_ts_fmt(cudaStream_t st, const GemvArgs& a, const TsPlan& p, i
   *fused = a.out_quant == OQ_MXFP8 && !a.out_f32 && a.N % 32 == 0 && a.q_codes;
   const TsProj::Args ea{a.bias0, a.bias1, a.residual, a.y, a.dtype == QX_DTYPE_F16, a.out_f32, a.activation, a.use_bias,
                         a.use_residual, *fused ? (uint8_t*)a.q_codes : nullptr};
-  ts_launch_prep(st, p, FMT, a.x, a.dtype, s, (int)a.M, (int)a.K);
-  return ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsProj>, m[0], m[1], m[2], m[3], q, ea);
+  return ts_launch_prep(st, p, FMT, a.x, a.dtype, s, (int)a.M, (int)a.K) &&
+         ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsProj>, m[0], m[1], m[2], m[3], q, ea);
 }
 
 static bool launch_ts_pass(cudaStream_t st, const GemvArgs& a, const TsPlan& p, int* err, bool* fused) {

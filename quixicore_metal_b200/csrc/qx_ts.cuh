@@ -120,13 +120,15 @@ bool ts_plan(TsPlan* p, int format, int64_t M, int64_t K, int64_t N, int rb, int
 bool ts_shape_ok(int format, int64_t K, int64_t N, const void* w0, const void* w1);
 // Tensor maps of one weight matrix: [0] the residues whose last super-row exists, [1] the others.
 bool ts_maps(const TsPlan& p, int format, const void* w, int64_t K, int64_t N, CUtensorMap* m);
-// Prepared activations of a call into scratch (carved by the plan's byte counts); zeroes the tickets.
+// Prepared activations of a call into scratch (carved by the plan's byte counts); zeroes the tickets.  False: not
+// launched, and the contraction must not be.
 struct TsScratch { uint8_t* img; float* rowscale; unsigned* count; float* part; };
 TsScratch ts_carve(const TsPlan& p, void* scratch);
-void ts_launch_prep(cudaStream_t st, const TsPlan& p, int format, const void* x, qx_dtype dtype, const TsScratch& s, int M, int K);
+bool ts_launch_prep(cudaStream_t st, const TsPlan& p, int format, const void* x, qx_dtype dtype, const TsScratch& s, int M, int K);
 
 // A launch that may start before its predecessor in the stream has finished (the kernels here call
-// griddepcontrol.wait before they touch what it produces).
+// griddepcontrol.wait before they touch what it produces; the contraction's weights are complete when it starts, see
+// ts_prep_kernel).
 template <typename... P, typename... A>
 bool ts_launch_dependent(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kernel)(P...), A&&... args) {
   cudaLaunchConfig_t cfg = {};

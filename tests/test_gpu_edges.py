@@ -223,3 +223,27 @@ def test_workspace_of_a_captured_graph_survives_larger_calls():
         s.synchronize()
         assert torch.equal(got, want)
         assert all(bool((t == 90).all()) for t in keep)
+
+
+# MXFP8 rows of one projection as the packed weight of the next, nothing in between: the second kernel may start before
+# the first has finished, its weight loads may not
+def _rows_as_weight(producer_rows, consumer_rows, K=2048, N=4096, reps=12):
+    gen = torch.Generator("cuda").manual_seed(producer_rows)
+    W = dev(O.synth_pack("q8_0", (0.02 * np.random.default_rng(1).standard_normal((N, K))).astype(np.float32)))
+    x = torch.randn(reps, producer_rows, K, generator=gen, device="cuda").bfloat16()
+    z = torch.randn(consumer_rows, N, generator=gen, device="cuda").bfloat16()
+    tk.decode_linear_epilogue(z, tk.decode_linear_epilogue(x[0], W, output_quant="mxfp8", format="q8_0"), format="mxfp8")
+    torch.cuda.synchronize()
+    rows, got = [], []
+    for r in range(reps):
+        rows.append(tk.decode_linear_epilogue(x[r], W, output_quant="mxfp8", format="q8_0"))
+        got.append(tk.decode_linear_epilogue(z, rows[-1], format="mxfp8"))
+    torch.cuda.synchronize()
+    for w, y in zip(rows, got):
+        assert torch.equal(y, tk.decode_linear_epilogue(z, w, format="mxfp8"))
+        torch.cuda.synchronize()
+
+
+@pytest.mark.parametrize("producer_rows", [16, 64, 256])
+def test_fresh_rows_as_weight_above_16_rows(producer_rows):
+    _rows_as_weight(producer_rows, 40)

@@ -644,6 +644,7 @@ struct TsLmHead {
     uint32_t seed;
     LmhMask mask;
   };
+  __device__ __forceinline__ static bool packs_rows(const Args&) { return false; }
   __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, uint8_t* aux,
                                              int warp, int lane) {
     float* logit = reinterpret_cast<float*>(aux) + warp * 2 * LMH_TILE;

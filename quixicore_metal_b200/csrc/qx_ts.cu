@@ -196,6 +196,7 @@ struct TsProj {
     int activation, use_bias, use_residual;
     uint8_t* mx;              // MXFP8 rows of the rounded output (N % 32 == 0)
   };
+  __device__ __forceinline__ static bool packs_rows(const Args& a) { return a.mx != nullptr; }
   __device__ __forceinline__ static float load(const void* p, size_t i, int half) {
     const uint16_t b = reinterpret_cast<const uint16_t*>(p)[i];
     return half ? __half2float(__ushort_as_half(b)) : __uint_as_float((uint32_t)b << 16);

@@ -433,7 +433,7 @@ __device__ __forceinline__ int ts_owner(const TsPlan& p, int ctas, long long u) 
   return (int)(((u + 1) * ctas - 1) / ((long long)p.tiles * p.nks));
 }
 
-// Epi: struct Args;
+// Epi: struct Args; packs_rows(args): writes MXFP8 rows, which a later call may take as its weights;
 //      run(args, params, item, scale, aux, warp, lane), called by the 8 output warps together: the dot product of
 //        column c is the sum of the parts times scale[c]; `aux`: shared memory of the policy; barrier 1 (256
 //        threads) is free;
@@ -449,7 +449,8 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
   constexpr int TERMS = F::TERMS, SLOT_COLS = 32 * TERMS, STAGE = 128 * F::PITCH, GPS = F::GPS;
   const TsPlan& p = q.p;
   extern __shared__ uint8_t ts_smem[];
-  asm volatile("griddepcontrol.launch_dependents;");
+  // a programmatic dependent may be scheduled; it waits for this grid's end, but not with its weight loads
+  if (!Epi::packs_rows(ea)) asm volatile("griddepcontrol.launch_dependents;");
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)ts_smem + 127) & ~(uintptr_t)127);
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31;

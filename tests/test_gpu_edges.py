@@ -247,3 +247,10 @@ def _rows_as_weight(producer_rows, consumer_rows, K=2048, N=4096, reps=12):
 @pytest.mark.parametrize("producer_rows", [16, 64, 256])
 def test_fresh_rows_as_weight_above_16_rows(producer_rows):
     _rows_as_weight(producer_rows, 40)
+
+
+# one row: its kernel follows the producer directly; the producers are the streaming kernel and its passes, the
+# tensor-memory form and (few bytes, many weight rows) the in-place pipeline
+@pytest.mark.parametrize("producer_rows,K,N", [(1, 2048, 4096), (16, 2048, 4096), (32, 2048, 4096), (64, 2048, 4096), (32, 512, 28672)])
+def test_fresh_rows_as_weight_of_one_row(producer_rows, K, N):
+    _rows_as_weight(producer_rows, 1, K, N)

@@ -645,8 +645,9 @@ struct TsLmHead {
     LmhMask mask;
   };
   __device__ __forceinline__ static bool packs_rows(const Args&) { return false; }
-  __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, uint8_t* aux,
-                                             int warp, int lane) {
+  template <bool SHIFT>
+  __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, const float* back,
+                                             uint8_t* aux, int warp, int lane) {
     float* logit = reinterpret_cast<float*>(aux) + warp * 2 * LMH_TILE;
     const int v0 = it.tile * LMH_TILE, nvalid = min(LMH_TILE, q.N - v0);
 #pragma unroll 1
@@ -667,7 +668,7 @@ struct TsLmHead {
           for (int j = 0; j < 8; ++j) v[j] += __ldcg(s + (size_t)(j >> 2) * q.p.nb * 128 + (j & 3) * 32);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) logit[r * LMH_TILE + j * 32 + lane] = v[j] * scale[m];
+        for (int j = 0; j < 8; ++j) logit[r * LMH_TILE + j * 32 + lane] = SHIFT ? v[j] * scale[m] * back[j * 32 + lane] : v[j] * scale[m];
       }
       __syncwarp();
       lmh_select_rows<2>(rows, trow, nvalid, v0, a.vocab_offset, a.bias, it.tile, a.tiles_stride, a.mode, a.topk, a.invtemp,

@@ -60,7 +60,7 @@ bool ts_plan(TsPlan* p, int format, int64_t M, int64_t K, int64_t N, int rb, int
   const size_t act_stage = (size_t)TS_KC * p->mp * 2;
   p->nact = p->mp <= 16 ? 4 : (p->mp <= 32 ? 3 : (p->mp <= 80 ? 2 : 1));
   const size_t stage = (size_t)128 * g.pitch;
-  const size_t bar_bytes = 8 * (2 * TS_MAX_RAW + 2 * TS_MAX_ACT + 2 * TS_MAX_SLOTS + 12) + 4 * (4 + TS_MARK_RING * 8 + 128);
+  const size_t bar_bytes = 8 * (2 * TS_MAX_RAW + 2 * TS_MAX_ACT + 2 * TS_MAX_SLOTS + 12) + 4 * (4 + TS_MARK_RING * 8 + 128 + 256);
   const size_t act = (act_stage * p->nact + 256 + 127) & ~(size_t)127;   // + what overlapping core matrices read past the end
   const size_t fixed = act + ((aux + 127) & ~(size_t)127) + bar_bytes + 128;
   if (fixed + 2 * stage > 227 * 1024) return false;
@@ -214,8 +214,9 @@ struct TsProj {
       for (int i = 0; i < 4; ++i) v[i] += __ldcg(s + i * 128);
     }
   }
-  __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, uint8_t*, int warp,
-                                             int lane) {
+  template <bool SHIFT>
+  __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, const float* back,
+                                             uint8_t*, int warp, int lane) {
     const TsPlan& p = q.p;
     const int blocks = p.dual ? 1 : p.rb;
     const int row = (warp & 3) * 32 + lane;
@@ -225,6 +226,7 @@ struct TsProj {
       if (n >= q.N) continue;
       const float b0 = a.use_bias ? load(a.bias0, n, a.half) : 0.f;
       const float b1 = p.dual && a.use_bias ? load(a.bias1, n, a.half) : 0.f;
+      const float f0 = SHIFT ? back[rb * 128 + row] : 1.f, f1 = SHIFT ? back[128 + row] : 1.f;
       int c = (warp >> 2) * 4;
       float v[4], w[4] = {0.f, 0.f, 0.f, 0.f};
       auto fetch = [&](int c, float (&v)[4], float (&w)[4]) {
@@ -246,9 +248,9 @@ struct TsProj {
         for (int i = 0; i < 4; ++i) {
           if (c + i >= it.m_count) break;
           const size_t m = it.m_base + c + i, o = m * q.N + n;
-          float d = v[i] * scale[c + i];
+          float d = SHIFT ? v[i] * scale[c + i] * f0 : v[i] * scale[c + i];
           if (a.raw) { reinterpret_cast<float*>(a.y)[o] = d; continue; }
-          if (p.dual) d = silu(d + b0) * (w[i] * scale[c + i] + b1);
+          if (p.dual) d = silu(d + b0) * ((SHIFT ? w[i] * scale[c + i] * f1 : w[i] * scale[c + i]) + b1);
           else d = apply_act(d + b0, a.activation) + w[i];
           const uint16_t h = a.half ? __half_as_ushort(__float2half_rn(d)) : __bfloat16_as_ushort(__float2bfloat16_rn(d));
           reinterpret_cast<uint16_t*>(a.y)[o] = h;

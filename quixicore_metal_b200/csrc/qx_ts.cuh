@@ -21,9 +21,12 @@
 //   * q8_0: hi = f16(q * d), lo = fma(q, d, -hi): q * d has 19 bits and is a multiple of 2^-24 (the
 //     spacing of f16 subnormals, which the tensor core keeps), so lo is exact;
 //   * q6_K: w = q * (sc * d), at most 24 bits, in three terms the same way.
-// The accumulator is the fp32 dequantise-then-dot up to summation order.  Blocks whose scale leaves the
-// range in which this holds (|d| >= 512, or an e8m0 exponent that no trained tensor has) mark their row,
-// and the accumulator warps recompute marked rows with fp32 arithmetic (ts_slow_dot).
+// The accumulator is the fp32 dequantise-then-dot up to summation order.  The e8m0 formats hold 22 (mxfp8) and 28
+// (mxfp4) exponents that way, around the exponent of ordinary weights; a row whose first block lies away from it
+// (the rows of tokens that no training step has touched) is shifted by a power of two of its own, which the output
+// warps take back (ts_row_shift).  Blocks whose scale still leaves the range - more than three decimal orders between the
+// blocks of one row, or |d| >= 512, q6_K 16 - count as zeros and mark their row, and the accumulator warps add their share
+// to marked rows with fp32 arithmetic (ts_add_left_out).
 //
 // Accumulation.  The tensor core truncates the fp32 accumulator after every MMA; over the K / 16 * TERMS
 // MMAs of a row that is a bias towards zero of about 3e-8 per MMA (q8_0, K = 8192, one accumulator: 1.9e-5).
@@ -222,6 +225,8 @@ template <int FMT> struct TsDec {
   static constexpr int NW = (LEN + 3) / 4;
   static constexpr int REL = 0;
   uint32_t w[NW];
+  uint32_t base;                                                   // e8m0 formats: the block exponent that makes an f16 exponent of 0
+  static constexpr uint32_t BASE = FMT == F_MXFP8 ? 95u : 100u;    // ... of a row that is not shifted
 
   template <int J> __device__ __forceinline__ void load(uint32_t addr) {
     constexpr int START = J * LEN, BASE = START / UNIT * UNIT, OFF = START - BASE;
@@ -271,10 +276,10 @@ template <int FMT> struct TsDec {
       if constexpr (FMT == F_MXFP4) {
         const uint32_t e = byte<BLK>();
         const uint32_t c[2] = {get32<BLK + 1 + 8 * HALF>(), get32<BLK + 5 + 8 * HALF>()};
-        // 2^(e - 127 + 12) as f16: exact products for 101 <= e <= 128
-        uint32_t s2 = ((e - 100u) << 10) * 0x00010001u;
+        // 2^(e - 127 + 12) as f16: exact products for 101 <= e <= 128 (less the shift of the row)
+        uint32_t s2 = ((e - base) << 10) * 0x00010001u;
         bool ok = true;
-        if (e - 101u > 27u) {
+        if (e - base - 1u > 27u) {
           ok = ((c[0] | c[1]) & 0x77777777u) == 0u;
           s2 = 0u;
         }
@@ -286,10 +291,10 @@ template <int FMT> struct TsDec {
         const uint32_t c[4] = {get32<BLK + 1 + 16 * HALF>(), get32<BLK + 5 + 16 * HALF>(), get32<BLK + 9 + 16 * HALF>(),
                                get32<BLK + 13 + 16 * HALF>()};
         // code bits moved under the f16 exponent are value * 2^-8 for every code (subnormals and 0x7F = 480, which
-        // the hardware converter reads as NaN, included); times 2^(e - 127 + 17): exact for 104 <= e <= 125
-        uint32_t s2 = ((e - 95u) << 10) * 0x00010001u;
+        // the hardware converter reads as NaN, included); times 2^(e - 127 + 17): exact for 104 <= e <= 125 (less the shift)
+        uint32_t s2 = ((e - base) << 10) * 0x00010001u;
         bool ok = true;
-        if (e - 104u > 21u) {
+        if (e - base - 9u > 21u) {
           ok = ((c[0] | c[1] | c[2] | c[3]) & 0x7F7F7F7Fu) == 0u;
           s2 = 0u;
         }
@@ -392,22 +397,105 @@ struct TsDecQ6 {
   }
 };
 
-// fp32 dot of one row over columns [k0, k1) by a whole warp (marked rows only)
+// slot row L of a raw stage -> row inside its 128-row block (P > 1: box r holds the rows r, r + P, ...)
+__device__ __forceinline__ int ts_row_of(int P, int L) { return P == 1 ? L : (L % (128 / P)) * P + L / (128 / P); }
+
+// ---- rows away from the ordinary exponents (e8m0 formats) ---------------------------------------------------
+// A row's weights are decoded times 2^shift: 0 while the exponent e of its first block is that of ordinary weights
+// (largest of a block 0.003 to 1.7, mxfp4 6e-6 to 0.7) or the block holds nothing, else what moves e to 114, the middle
+// of the range; no further than TsDec::base stays positive and an exponent of 255 (infinity) out of every range.
+template <int FMT> constexpr bool ts_shifts() { return FMT == F_MXFP8 || FMT == F_MXFP4; }
 template <int FMT>
-__device__ __noinline__ float ts_slow_dot(const uint8_t* row, const void* x, int x_bf16, size_t xoff, int k0, int k1, int lane) {
-  float a = 0.f;
-  for (int s = k0 / 32 + lane; s < k1 / 32; s += 32) {
-    float w[32];
-    decode_span32<FMT>(row, s, w);
-    const uint16_t* xp = reinterpret_cast<const uint16_t*>(x) + xoff + (size_t)s * 32;
-    for (int i = 0; i < 32; ++i) {
-      const float xv = x_bf16 ? __uint_as_float((uint32_t)xp[i] << 16) : __half2float(__ushort_as_half(xp[i]));
-      a = fmaf(xv, w[i], a);
+__device__ __forceinline__ int ts_row_shift(uint32_t e, const uint8_t* row) {
+  if (FMT == F_MXFP8 ? e - 110u <= 9u : e - 107u <= 17u) return 0;
+  uint32_t any = 0u;
+#pragma unroll 8
+  for (int i = 1; i < TsFmt<FMT>::BB; ++i) any |= __ldg(row + i);
+  if ((any & (FMT == F_MXFP8 ? 0x7Fu : 0x77u)) == 0u || e == 255u) return 0;
+  return min(max(114 - (int)e, (FMT == F_MXFP8 ? 125 : 128) - 254), 95);
+}
+__device__ __forceinline__ float ts_pow2(int n) { return __uint_as_float(n < -126 ? 0x00400000u : (uint32_t)(n + 127) << 23); }   // -127 <= n
+
+// ---- blocks outside the exact range ------------------------------------------------------------------------
+// The decoders put zeros in their place and mark the row; their share of the dot is added to the finished segment.
+// Whether 32-column block b of a row is one of them (shift: ts_row_shift of the row).
+template <int FMT>
+__device__ __forceinline__ bool ts_block_left_out(const uint8_t* row, int b, int shift) {
+  if constexpr (FMT == F_Q6_K) {
+    const uint8_t* d = row + (size_t)(b >> 3) * 210 + 208;
+    return (__ldg(d + 1) & 0x7Cu) >= 0x4Cu;
+  } else if constexpr (FMT == F_Q4_0 || FMT == F_Q8_0) {
+    return (__ldg(row + (size_t)b * TsFmt<FMT>::BB + 1) & 0x7Cu) >= 0x60u;
+  } else {
+    const uint8_t* blk = row + (size_t)b * TsFmt<FMT>::BB;
+    const uint32_t x = __ldg(blk) - (TsDec<FMT>::BASE - (uint32_t)shift);
+    if (FMT == F_MXFP8 ? x - 9u <= 21u : x - 1u <= 27u) return false;
+    uint32_t any = 0u;
+#pragma unroll 1
+    for (int i = 1; i < TsFmt<FMT>::BB; ++i) any |= __ldg(blk + i);
+    return (any & (FMT == F_MXFP8 ? 0x7Fu : 0x77u)) != 0u;
+  }
+}
+// weight i of 32-column block b
+template <int FMT>
+__device__ __forceinline__ float ts_weight(const uint8_t* row, int b, int i) {
+  if constexpr (FMT == F_Q6_K) {
+    const uint8_t* s = row + (size_t)(b >> 3) * 210;
+    const int half = (b >> 2) & 1, g = b & 3;
+    const uint32_t l = (uint32_t)__ldg(s + 64 * half + 32 * (g & 1) + i) >> (4 * (g >> 1)), h = (uint32_t)__ldg(s + 128 + 32 * half + i) >> (2 * g);
+    const float d = f16_bits_to_f32(__ldg(s + 208), __ldg(s + 209)) * (float)(int)(int8_t)__ldg(s + 192 + 8 * half + 2 * g + (i >> 4));
+    return d * (float)((int)((l & 15u) | (h & 3u) << 4) - 32);
+  } else {
+    const uint8_t* s = row + (size_t)b * TsFmt<FMT>::BB;
+    if constexpr (FMT == F_Q8_0) return f16_bits_to_f32(__ldg(s), __ldg(s + 1)) * (float)(int)(int8_t)__ldg(s + 2 + i);
+    else if constexpr (FMT == F_MXFP8) return e8m0_to_f32(__ldg(s)) * e4m3_to_f32(__ldg(s + 1 + i));
+    else {
+      const uint32_t n = ((uint32_t)__ldg(s + (FMT == F_Q4_0 ? 2 : 1) + (i & 15)) >> (4 * (i >> 4))) & 15u;
+      return FMT == F_Q4_0 ? f16_bits_to_f32(__ldg(s), __ldg(s + 1)) * (float)((int)n - 8) : e8m0_to_f32(__ldg(s)) * e2m1_to_f32(n);
     }
   }
-  return warp_sum(a);
 }
-
+// The marked rows of a quadrant (mk: 4 words from one row block to the next) of a segment, over its stored accumulators
+// (`out`: [row block][column][128 rows]), by one warp; a lane takes a column.  Rolled and inline: a call here costs every
+// launch registers (64-row LM heads 5 %), and so much as a look at the marks in the output warps' loop 12 to 20 %.
+// 64 rows, mxfp8, 4096 -> 14336, 39.8 us: one block left out of one row 46.8, of 32 rows 241, of 256 rows 325; 256 rows
+// shifted 59.6.  Making whole rows again in fp32 took 244 us for one and 4.2 ms for 32 of them, and an LM head of
+// 128256 with 250 untouched rows 24 ms; now 177 us (166 with ordinary rows).
+template <int FMT>
+__device__ __forceinline__ void ts_add_left_out(const TsParams& q, float* out, const uint32_t* mk, int quad, int tile, int m_base, int m_count,
+                                                int ks0, int ks1, int lane) {
+  const TsPlan& p = q.p;
+#pragma unroll 1
+  for (int rb = 0; rb < p.rb; ++rb)
+#pragma unroll 1
+    for (uint32_t bits = mk[rb * 4]; bits; bits &= bits - 1u) {
+      const int row = ts_row_of(p.P, quad * 32 + __ffs(bits) - 1), n = tile * p.tile_rows + (p.dual ? 0 : rb * 128) + row;
+      if (n >= q.N) continue;
+      const uint8_t* w = q.w[p.dual ? rb : 0] + (size_t)n * ((size_t)(q.K / TsFmt<FMT>::BK) * TsFmt<FMT>::BB);
+      int shift = 0;
+      if constexpr (ts_shifts<FMT>()) shift = ts_row_shift<FMT>(__ldg(w), w);
+#pragma unroll 1
+      for (int b0 = ks0 * 8; b0 < ks1 * 8; b0 += 32) {
+        uint32_t left = __ballot_sync(0xffffffffu, b0 + lane < ks1 * 8 && ts_block_left_out<FMT>(w, b0 + lane, shift));
+#pragma unroll 1
+        for (; left; left &= left - 1u) {
+          const int b = b0 + __ffs(left) - 1;
+#pragma unroll 1
+          for (int c = lane; c < m_count; c += 32) {
+            const uint16_t* x = reinterpret_cast<const uint16_t*>(q.x) + (size_t)(m_base + c) * q.K + b * 32;
+            float a = 0.f;
+#pragma unroll 1
+            for (int i = 0; i < 32; ++i)
+              a = fmaf(q.x_bf16 ? __uint_as_float((uint32_t)__ldg(x + i) << 16) : __half2float(__ushort_as_half(__ldg(x + i))),
+                       ts_weight<FMT>(w, b, i), a);
+            float* o = out + ((size_t)rb * p.nb + c) * 128 + row;
+            const float unit = ts_shifts<FMT>() ? TsFmt<FMT>::ACC_SCALE * ts_pow2(-shift) : TsFmt<FMT>::ACC_SCALE;
+            __stcg(o, __ldcg(o) + a / (q.rowscale[m_base + c] * unit));
+          }
+        }
+      }
+    }
+}
 
 // Position in a ring of n slots: index and phase parity.
 struct TsRing {
@@ -434,8 +522,8 @@ __device__ __forceinline__ int ts_owner(const TsPlan& p, int ctas, long long u) 
 }
 
 // Epi: struct Args; packs_rows(args): writes MXFP8 rows, which a later call may take as its weights;
-//      run(args, params, item, scale, aux, warp, lane), called by the 8 output warps together: the dot product of
-//        column c is the sum of the parts times scale[c]; `aux`: shared memory of the policy; barrier 1 (256
+//      run<SHIFT>(args, params, item, scale, back, aux, warp, lane), called by the 8 output warps together: the dot product
+//        of column c is the sum of the parts times scale[c], with SHIFT also times back[128 * block + row]; `aux`: shared memory of the policy; barrier 1 (256
 //        threads) is free;
 //      tail(...) by the output warps after the last item.
 // Code that a launch runs once or twice is kept rolled: it is fetched cold, at about 70 clocks per 8
@@ -474,6 +562,7 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
   volatile uint32_t* ticket = words + 1;
   uint32_t* marks = words + 4;                      // [segment ring][2 row blocks][4 quadrants] marked rows
   float* scale = reinterpret_cast<float*>(words + 4 + TS_MARK_RING * 8);   // per activation row of the group
+  float* back = scale + 128;                        // e8m0 formats: 2^-shift of the item's weight rows
 
   {
     for (int i = tid; i < NB; i += TS_WARPS * 32) {
@@ -520,9 +609,12 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
     ks1 = min(nks, ks0 + (rg.u1 - u));
     u += ks1 - ks0;
   };
-  // slot row L of a raw stage -> row inside its 128-row block (P > 1: box r holds the rows r, r + P, ...)
   const int seg_rows = 128 / p.P;
-  auto row_of = [&](int L) { return p.P == 1 ? L : (L % seg_rows) * p.P + L / seg_rows; };
+  // first byte of this CTA's weight row n of row block rb (rows past the matrix: the last one)
+  auto row_start = [&](int rb, int n) {
+    const size_t row_bytes = (size_t)(q.K / F::BK) * F::BB;
+    return q.w[p.dual ? rb : 0] + (size_t)min(n + (p.dual ? 0 : rb * 128), q.N - 1) * row_bytes;
+  };
 
   if (warp < TS_WORKERS) {
     // ============================ workers ============================
@@ -535,6 +627,17 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
     TsRing raw{0, 0};
     int opb = 0; uint32_t opar = 1u;                                  // first operand slot of the stage, parity of its "empty"
     int stage_no = 0, nseg = 0;
+    // e8m0 formats: TsDec::base of this thread's rows (low half: row block 0), made of the exponents of their first
+    // blocks: from the raw stage that holds them, or from memory where the CTA starts inside an item
+    uint32_t bases = 0u;
+    const int wrow = ts_row_of(p.P, L);
+    auto set_base = [&](int tile, int rb, uint32_t e) {
+      const uint32_t b = TsDec<FMT>::BASE - (uint32_t)ts_row_shift<FMT>(e, row_start(rb, tile * p.tile_rows + wrow));
+      bases = rb ? (bases & 0xFFFFu) | b << 16 : (bases & 0xFFFF0000u) | b;
+    };
+    if constexpr (ts_shifts<FMT>())
+      if (rg.u0 < rg.u1 && rg.u0 % nks != 0)
+        for (int rb = 0; rb < rbn; ++rb) set_base(rg.u0 / nks, rb, __ldg(row_start(rb, rg.u0 / nks * p.tile_rows + wrow)));
     for (int u = rg.u0; u < rg.u1; ++nseg) {
       int tile, ks0, ks1;
       segment(u, tile, ks0, ks1);
@@ -582,6 +685,10 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
             wait(RAW_FULL(raw.slot), raw.par);
             TsDec<FMT> dec;
             const uint32_t at = slot_at0 + (uint32_t)(raw.slot * STAGE) + off;
+            if constexpr (ts_shifts<FMT>()) {
+              if (ks == 0) set_base(tile, rb, lds8(at));
+              dec.base = (bases >> (16 * rb)) & 0xFFFFu;
+            }
             if (grp == 0) dec.template load<0>(at);
             else if (grp == 1) dec.template load<1>(at);
             else if (grp == 2) dec.template load<2>(at);
@@ -618,10 +725,9 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
     // ============================ accumulators ============================
     asm volatile("griddepcontrol.wait;" ::: "memory");                // the scratch may still be read by the kernel before
     const int quad = warp & 3;
-    const int L = quad * 32 + lane, row = row_of(L);
+    const int row = ts_row_of(p.P, quad * 32 + lane);
     const uint32_t lane_sel = (uint32_t)(quad * 32) << 16;
-    const size_t row_bytes = (size_t)(q.K / F::BK) * F::BB;
-    const int m_base = rg.grp * p.mg, m_count = min(p.mg, q.M - m_base);
+    const int m_count = min(p.mg, q.M - rg.grp * p.mg);
     TsRing acc{0, 0};
     int nseg = 0;
     for (int u = rg.u0; u < rg.u1; ++nseg) {
@@ -661,50 +767,32 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
         acc.advance1(p.nd);
       }
       const uint32_t acc_at = lane_sel + (summed ? 0u : acc_base + (uint32_t)(last_buf * acc_cols));
-      uint32_t* mk = marks + (nseg & (TS_MARK_RING - 1)) * 8 + quad;
-      if ((mk[0] | mk[4]) != 0u) {                                    // cold: rows marked by the decoders, recomputed in fp32
-        for (int rb = 0; rb < rbn; ++rb)
-          for (int c = 0; c < m_count; c += 8) {
-            uint32_t r[8];
-            tmem_ld8_nowait(acc_at + (uint32_t)(rb * p.nb + c), r);
-            tmem_wait_ld();
-            for (uint32_t bal = mk[rb * 4]; bal; bal &= bal - 1u) {
-              const int src = __ffs(bal) - 1;
-              const int nrow = tile * p.tile_rows + (p.dual ? 0 : rb * 128) + __shfl_sync(0xffffffffu, row, src);
-              if (nrow >= q.N) continue;
-#pragma unroll 1
-              for (int i = 0; i < 8 && c + i < m_count; ++i) {
-                const float s = ts_slow_dot<FMT>(q.w[p.dual ? rb : 0] + (size_t)nrow * row_bytes, q.x, q.x_bf16,
-                                                 (size_t)(m_base + c + i) * q.K, ks0 * TS_KC, ks1 * TS_KC, lane) /
-                                (q.rowscale[m_base + c + i] * F::ACC_SCALE);
-#pragma unroll
-                for (int k = 0; k < 8; ++k) if (k == i && lane == src) r[k] = __float_as_uint(s);
-              }
-            }
-            tmem_st8(acc_at + (uint32_t)(rb * p.nb + c), r);
-          }
-        tmem_wait_st();
-        __syncwarp();
-        if (lane == 0) { mk[0] = 0u; mk[4] = 0u; }
-      }
       // the finished segment -> scratch: slots 0 / 1 of the CTA for the head / tail part of a cut item, else 2 / 3 in turn
       const int sb = nseg & 1;
       wait(SEG_EMPTY(sb), ((uint32_t)(nseg >> 1) & 1u) ^ 1u);
       __syncwarp();
       const int kind = ks0 > 0 ? 0 : (ks1 < nks ? 1 : 2 + sb);
-      float* out = q.part + ((size_t)(blockIdx.x * 4 + kind) * rbn) * p.nb * 128 + row;
+      float* out = q.part + ((size_t)(blockIdx.x * 4 + kind) * rbn) * p.nb * 128;
       for (int rb = 0; rb < rbn; ++rb)
 #pragma unroll 1
         for (int c = 0; c < m_count; c += 8) {
           uint32_t r[8];
           tmem_ld8_nowait(acc_at + (uint32_t)(rb * p.nb + c), r);
           tmem_wait_ld();
-          float* o = out + ((size_t)rb * p.nb + c) * 128;
+          float* o = out + ((size_t)rb * p.nb + c) * 128 + row;
 #pragma unroll
           for (int i = 0; i < 8; ++i) __stcg(o + i * 128, __uint_as_float(r[i]));
         }
       if (!summed) tc_fence_before();
       __syncwarp();
+      if constexpr (FMT != F_NVFP4) {                                 // whose scales are never out of range
+        uint32_t* mk = marks + (nseg & (TS_MARK_RING - 1)) * 8 + quad;
+        if ((mk[0] | mk[4]) != 0u) {
+          ts_add_left_out<FMT>(q, out, mk, quad, tile, rg.grp * p.mg, m_count, ks0, ks1, lane);
+          __syncwarp();
+          if (lane == 0) { mk[0] = 0u; mk[4] = 0u; }
+        }
+      }
       if (lane == 0) {
         mbar_arrive(SEG_FULL(sb));
         if (!summed)
@@ -725,8 +813,18 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
       int tile, ks0, ks1;
       segment(u, tile, ks0, ks1);
       const int sb = nseg & 1;
+      const uint8_t* wrow = nullptr;
+      uint32_t e = 0u;
+      if constexpr (ts_shifts<FMT>()) {
+        wrow = row_start(ot >> 7, tile * p.tile_rows + (ot & 127));     // (of the only block, where there is one)
+        e = __ldg(wrow);
+      }
       wait(SEG_FULL(sb), (uint32_t)(nseg >> 1) & 1u);
       __syncwarp();
+      if constexpr (ts_shifts<FMT>()) {
+        back[ot] = ts_pow2(-ts_row_shift<FMT>(e, wrow));
+        if (ks0 == 0 && ks1 == nks) sync_out();                       // a cut item has a barrier of its own below
+      }
       TsItem item{tile, m_base, m_count, q.part + (size_t)(blockIdx.x * 4 + 2 + sb) * slot, nullptr, 0, 1};
       bool mine = true;
       if (ks0 > 0 || ks1 < nks) {
@@ -746,7 +844,7 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
         item.step = (size_t)p.groups * 4 * slot;
         item.parts = last - first + 1;
       }
-      if (mine) Epi::run(ea, q, item, scale, smem + p.off_aux, ow, lane);
+      if (mine) Epi::template run<ts_shifts<FMT>()>(ea, q, item, scale, back, smem + p.off_aux, ow, lane);
       sync_out();                                                     // the ticket and the policy's buffer are free again
       if (lane == 0) mbar_arrive(SEG_EMPTY(sb));
     }

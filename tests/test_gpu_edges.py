@@ -254,3 +254,90 @@ def test_fresh_rows_as_weight_above_16_rows(producer_rows):
 @pytest.mark.parametrize("producer_rows,K,N", [(1, 2048, 4096), (16, 2048, 4096), (32, 2048, 4096), (64, 2048, 4096), (32, 512, 28672)])
 def test_fresh_rows_as_weight_of_one_row(producer_rows, K, N):
     _rows_as_weight(producer_rows, 1, K, N)
+
+
+# Rows that hold a block whose scale leaves the range in which the decoded f16 operand is exact are made again in fp32, rows
+# that lie outside it as a whole are shifted.  Such blocks in the first and the last stage, in neighbouring rows and in a
+# whole group of 32, above and below the range; K = 256 leaves items whole, the others are cut between CTAs; K = 256
+# and 768 of the mx formats have pitches that are no multiple of 16 bytes (rows interleaved in 2, 4 or 8 boxes).
+def _wild(fmt, W, n, big):
+    last = W.shape[1] - 1
+    rows = [r for r in (0, 1, 33, *range(64, 96), 127, 130, n - 1) if r < n]
+    for i, r in enumerate(rows):
+        for b in ((0,), (last,), (0, last))[i % 3]:
+            if fmt in ("q4_0", "q8_0"):
+                W[r, b, :2] = np.array([600.0 + i if big else 65504.0], np.float16).view(np.uint8)
+            elif fmt == "q6_K":
+                W[r, b, 208:210] = np.array([16.0 + i if big else 3000.0], np.float16).view(np.uint8)
+            else:
+                W[r, b, 0] = 127 + i % 12 if big else 60 + i % 40
+    return rows
+
+
+@pytest.mark.parametrize("big", [False, True])
+@pytest.mark.parametrize("M,K,N", [(17, 256, 131), (40, 768, 300), (64, 4096, 136), (129, 2048, 40)])
+@pytest.mark.parametrize("fmt", ["q4_0", "q8_0", "q6_K", "mxfp8", "mxfp4"])
+def test_rows_with_scales_outside_the_exact_range(fmt, M, K, N, big):
+    from quixicore_metal_b200 import _lib
+    x, W, _, _ = _linear(fmt, M, K, N, "bf16", 5, pack="random")
+    rows = _wild(fmt, W, N, big)
+    for r in rows[3:8]:                                  # whole rows out of range, nothing larger beside it
+        W[r, :, :] = W[r, :1, :]
+        if fmt in ("mxfp8", "mxfp4"):
+            W[r, :, 0] = 40 + r % 50
+    if fmt in ("mxfp8", "mxfp4"):
+        W[rows[-1], 0, 1:] = 0                           # a first block that holds nothing
+    w = O.dequantize(fmt, W).astype(np.float64)
+    ref = x.astype(np.float64) @ w.T
+    size = np.abs(x).astype(np.float64) @ np.abs(w).T
+    _, U, _, _ = _linear(fmt, M, K, N, "bf16", 6)
+    _lib.set_option("ts_min_rows", 1)                    # the kernel with that operand at every row count
+    try:
+        got = host(tk.decode_linear_epilogue(dev(x, "bf16"), dev(W), None, None, format=fmt)).astype(np.float64)
+        # half an ulp of bf16 and the noise of the sums: at most 2^-24 of the terms for each of the K / 16 x 3
+        # products of a chunk and the K / 256 sums over chunks
+        assert (np.abs(got - ref) <= 2.0 ** -8 * np.abs(ref) + 2e-5 * size).all()
+        part = host(tk_torch.decode_linear_partial(dev(x, "bf16"), dev(W), fmt)).astype(np.float64)
+        assert (np.abs(part - ref) <= 2e-5 * size).all()
+        for gate, up in ((W, U), (U, W)):                # marked rows in either matrix of a pair
+            want = O.decode_swiglu(x, gate, up, fmt, None, None, "f32")
+            y = host(tk.decode_swiglu(dev(x, "bf16"), dev(gate), dev(up), format=fmt))
+            dots = [x.astype(np.float64) @ O.dequantize(fmt, v).astype(np.float64).T for v in (gate, up)]
+            sums = [np.abs(x).astype(np.float64) @ np.abs(O.dequantize(fmt, v)).astype(np.float64).T for v in (gate, up)]
+            tol = 2.0 ** -8 * np.abs(want) + 2e-5 * 1.1 * (sums[0] * np.abs(dots[1]) + sums[1] * np.abs(dots[0]))  # |silu'| < 1.1, |silu(g)| <= |g|
+            ok = np.isfinite(want) & (np.abs(want) < 1e38)
+            assert (np.abs(y - want)[ok] <= tol[ok] + 1e-30).all()
+    finally:
+        _lib.set_option("ts_min_rows", 0)
+
+
+# results that fp32 does not hold in units of the scaled activations and weights (2^26 and 2^23 of them, unit
+# activations) from blocks with large e8m0 scales: whole items and cut ones
+@pytest.mark.parametrize("K", [256, 4096])
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4"])
+def test_large_results_of_shifted_rows(fmt, K):
+    x, W, _, _ = _linear(fmt, 40, K, 136, "bf16", 8, pack="random")
+    W[:100, :, 0] = 127 + (100 if fmt == "mxfp8" else 108)
+    w = O.dequantize(fmt, W).astype(np.float64)
+    ref, size = x.astype(np.float64) @ w.T, np.abs(x).astype(np.float64) @ np.abs(w).T
+    assert np.abs(ref).max() > 2.0 ** 110 and size.max() < 2.0 ** 127
+    got = host(tk.decode_linear_epilogue(dev(x, "bf16"), dev(W), None, None, format=fmt)).astype(np.float64)
+    assert (np.abs(got - ref) <= 2.0 ** -8 * np.abs(ref) + 2e-5 * size).all()
+
+
+# an LM head with rows far below the others (tokens that no training step has touched) and a few far above
+@pytest.mark.parametrize("fmt", ["mxfp8", "mxfp4", "q8_0"])
+@pytest.mark.parametrize("T,V,K", [(17, 4003, 512), (64, 700, 4096)])
+def test_lm_head_rows_outside_the_exact_range(fmt, T, V, K):
+    rng = np.random.default_rng(T)
+    W = O.synth_pack(fmt, (0.3 * rng.standard_normal((V, K))).astype(np.float32))
+    h = rounded(0.5 * rng.standard_normal((T, K)), "bf16")
+    if fmt == "q8_0":
+        W[300:310, 1, :2] = np.array([600.0], np.float16).view(np.uint8)
+    else:
+        W[256:512, :, 0] = 60
+        W[600, 1, 0] = 140
+    for mode, code, kw in (("argmax", 0, {}), ("topk", 2, dict(k=64)), ("topp", 3, dict(k=32, top_p=0.9))):
+        tok = host(tk.lm_head_sample(dev(h, "bf16"), dev(W), mode=mode, format=fmt, temperature=0.8, seed=3, **kw))
+        want, margin = O.lm_head_sample(h, W, fmt, code, temperature=0.8, seed=3, return_detail=True, **kw)
+        check_ids(tok, want, margin, 1e-4 if fmt != "q8_0" else 0.5, f"{fmt}/{mode}")

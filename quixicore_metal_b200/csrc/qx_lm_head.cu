@@ -630,6 +630,69 @@ lmh_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __half* __rest
   }
 }
 
+}  // namespace qx
+#include "qx_tc_pipeline.cuh"
+namespace qx {
+
+// Epilogue of the in-place pipeline for LM-head stage 1: the worker warps move the logits of the item's 256 vocabulary
+// rows to shared memory ([hidden row][256]), then every warp reduces hidden rows to their tile partials.
+template <int BN>
+struct LmhEpi {
+  struct Args {
+    const float* bias;
+    float* part_val; int32_t* part_id; float* part_lse;
+    int T_total, V;
+    long long vocab_offset, tiles_stride;
+    int mode, topk;
+    float invtemp;
+    uint32_t seed;
+    LmhMask mask;
+  };
+  static constexpr bool DUAL = false;
+  __device__ __forceinline__ static bool packs_rows(const Args&) { return false; }
+  __device__ __forceinline__ static void run(const Args& a, const TcItem& it) {
+    constexpr int CW = BN / 4;
+    if (it.warp < LTC_DQW) {
+      const uint32_t lane_sel = (uint32_t)((it.warp & 3) * 32) << 16;
+      const int RS = (it.warp & 3) * 32 + it.lane;
+      const int cg = it.warp >> 2;
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        uint32_t v[CW];
+        tmem_ld_nowait<CW>(it.tmem_base + lane_sel + (uint32_t)(h * BN + cg * CW), v);
+        tmem_wait_ld();
+#pragma unroll
+        for (int i = 0; i < CW; ++i) {
+          const int m = cg * CW + i;
+          it.smem_f32[m * LMH_TILE + h * 128 + RS] = m < it.m_count ? __uint_as_float(v[i]) * it.rowscale[it.m_base + m] : 0.f;
+        }
+      }
+    }
+    tc_fence_before();
+    __syncthreads();
+    const int v0 = it.tile * LMH_TILE, nvalid = min(LMH_TILE, a.V - v0);
+    // every warp takes up to four hidden rows (warp, warp + 18, ...) and reduces them together
+    constexpr int RPW = (BN + LTC_WARPS - 1) / LTC_WARPS;
+    const float* rows[RPW];
+    int trow[RPW];
+#pragma unroll
+    for (int r = 0; r < RPW; ++r) {
+      const int m = it.warp + r * LTC_WARPS;
+      rows[r] = it.smem_f32 + (m < it.m_count ? m : 0) * LMH_TILE;
+      trow[r] = m < it.m_count ? it.m_base + m : -1;
+    }
+    lmh_select_rows<RPW>(rows, trow, nvalid, v0, a.vocab_offset, a.bias, it.tile, a.tiles_stride, a.mode, a.topk, a.invtemp,
+                         a.seed, a.part_val, a.part_id, a.part_lse, it.lane, a.mask);
+  }
+  // padding tiles of a short shard carry absent partials
+  __device__ __forceinline__ static void tail(const Args& a, const float* scratch, int real_tiles, int warp, int lane) {
+    for (long long tile = real_tiles + blockIdx.x; tile < a.tiles_stride; tile += gridDim.x)
+      for (int m = warp; m < a.T_total; m += LTC_WARPS)
+        lmh_select_token(scratch, 0, 0, a.vocab_offset, nullptr, m, (int)tile, a.tiles_stride, a.mode,
+                         a.topk, a.invtemp, a.seed, a.part_val, a.part_id, a.part_lse, lane);
+  }
+};
+
 // Output policy of the tensor-memory-operand kernel (qx_ts.cuh) for LM-head stage 1: each of the 8 output warps
 // brings the 256 logits of two hidden rows at a time to shared memory and reduces them to their tile
 // partials, while the other roles work on the next tile.
@@ -643,6 +706,7 @@ struct TsLmHead {
     float invtemp;
     uint32_t seed;
     LmhMask mask;
+    int row0;                 // hidden row of the call that is row 0 of this launch
   };
   __device__ __forceinline__ static bool packs_rows(const Args&) { return false; }
   template <bool SHIFT>
@@ -653,7 +717,7 @@ struct TsLmHead {
 #pragma unroll 1
     for (int m0 = warp; m0 < it.m_count; m0 += 2 * TS_OUT) {
       const float* rows[2] = {logit, logit + LMH_TILE};
-      const int trow[2] = {it.m_base + m0, m0 + TS_OUT < it.m_count ? it.m_base + m0 + TS_OUT : -1};
+      const int t0 = a.row0 + it.m_base + m0, trow[2] = {t0, m0 + TS_OUT < it.m_count ? t0 + TS_OUT : -1};
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
         const int m = m0 + r * TS_OUT;
@@ -680,7 +744,7 @@ struct TsLmHead {
   __device__ __forceinline__ static void tail(const Args& a, const TsParams& q, uint8_t* aux, int warp, int lane) {
     for (long long tile = q.p.tiles + blockIdx.x; tile < a.tiles_stride; tile += gridDim.x)
       for (int m = warp; m < q.M; m += TS_OUT)
-        lmh_select_token(reinterpret_cast<const float*>(aux), 0, 0, a.vocab_offset, nullptr, m, (int)tile, a.tiles_stride, a.mode,
+        lmh_select_token(reinterpret_cast<const float*>(aux), 0, 0, a.vocab_offset, nullptr, a.row0 + m, (int)tile, a.tiles_stride, a.mode,
                          a.topk, a.invtemp, a.seed, a.part_val, a.part_id, a.part_lse, lane);
   }
 };
@@ -761,26 +825,17 @@ static bool lmh_carve(const LmHeadArgs& a, LmhScratch* out) {
   return true;
 }
 
-// Tensor-memory-operand form of stage 1.
+// Tensor-memory-operand form of stage 1: at most a group of rows per SM in a launch, more rows in several.
 template <int FMT>
 static bool launch_lmh_ts(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t tiles_stride) {
-  if ((a.dtype != QX_DTYPE_BF16 && a.dtype != QX_DTYPE_F16) || ((uintptr_t)a.h & 15) != 0 || a.T > 0xFFFF ||
-      !ts_shape_ok(FMT, a.K, a.V, a.wq, nullptr))
+  if ((a.dtype != QX_DTYPE_BF16 && a.dtype != QX_DTYPE_F16) || ((uintptr_t)a.h & 15) != 0 || !ts_shape_ok(FMT, a.K, a.V, a.wq, nullptr))
     return false;
-  const int group = FMT == F_Q6_K ? 32 : 64;
-  TsPlan p;
-  // Items of one round stay whole when they fill most SMs or are short: a cut saves less than handing the parts over
-  // and selecting late costs (q4_0, 40 rows, 118 items: K = 1024 71.4 -> 54.0 us, K = 4096 98.2 -> 84.0; 63 items,
-  // K = 1024 35.2 -> 33.0).  Several rounds are cut evenly (q8_0, 64 rows, 501 items: 275.6 us, 280.6 whole).
-  const int64_t items = (a.V + 255) / 256 * ((a.T + group - 1) / group);
-  const bool whole = items <= sm_count() && (2 * items > sm_count() || a.K < 2048);
-  if (!ts_plan(&p, FMT, a.T, a.K, a.V, 2, 0, group, LMH_TS_AUX, options().lm_head_ksplit && !whole)) return false;
+  constexpr int group = FMT == F_Q6_K ? 32 : 64;
   int* err = device_error_flag();
-  if (!err || !a.scratch || a.scratch_bytes < p.scratch()) return false;
   static bool attr_set[64] = {};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev < 0 || dev >= 64) return false;
+  if (!err || dev < 0 || dev >= 64) return false;
   if (!attr_set[dev]) {
     if (cudaFuncSetAttribute(ts_kernel<FMT, TsLmHead>, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024) != cudaSuccess) {
       cudaGetLastError();
@@ -788,15 +843,71 @@ static bool launch_lmh_ts(cudaStream_t st, const LmHeadArgs& a, float* pv, int32
     }
     attr_set[dev] = true;
   }
-  CUtensorMap m[2];
-  if (!ts_maps(p, FMT, a.wq, a.K, a.V, m)) return false;
-  const TsScratch s = ts_carve(p, a.scratch);
-  const TsParams q{p, {(const uint8_t*)a.wq, nullptr}, a.h, a.dtype == QX_DTYPE_BF16, s.img, s.rowscale, s.part, s.count,
-                   (int)a.T, (int)a.K, (int)a.V, err};
-  const TsLmHead::Args ea{a.bias, pv, pi, pl, (long long)a.vocab_offset, (long long)tiles_stride, a.mode, a.topk, a.invtemp,
-                          a.seed, a.mask};
-  return ts_launch_prep(st, p, FMT, a.h, a.dtype, s, (int)a.T, (int)a.K) &&
-         ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsLmHead>, m[0], m[1], m[0], m[1], q, ea);
+  const int64_t passes = (a.T + (int64_t)sm_count() * group - 1) / ((int64_t)sm_count() * group);
+  const int64_t per = (a.T + passes - 1) / passes;
+  for (int64_t m0 = 0; m0 < a.T; m0 += per) {
+    const int64_t T = a.T - m0 < per ? a.T - m0 : per;
+    TsPlan p;
+    // Items of one round stay whole when they fill most SMs or are short: a cut saves less than handing the parts over
+    // and selecting late costs (q4_0, 40 rows, 118 items: K = 1024 71.4 -> 54.0 us, K = 4096 98.2 -> 84.0; 63 items,
+    // K = 1024 35.2 -> 33.0).  Several rounds are cut evenly (q8_0, 64 rows, 501 items: 275.6 us, 280.6 whole).
+    const int64_t items = (a.V + 255) / 256 * ((T + group - 1) / group);
+    const bool whole = items <= sm_count() && (2 * items > sm_count() || a.K < 2048);
+    if (!ts_plan(&p, FMT, T, a.K, a.V, 2, 0, group, LMH_TS_AUX, options().lm_head_ksplit && !whole)) return false;
+    if (!a.scratch || a.scratch_bytes < p.scratch()) return false;
+    CUtensorMap m[2];
+    if (!ts_maps(p, FMT, a.wq, a.K, a.V, m)) return false;
+    const void* h = (const char*)a.h + (size_t)m0 * a.K * 2;
+    const TsScratch s = ts_carve(p, a.scratch);
+    const TsParams q{p, {(const uint8_t*)a.wq, nullptr}, h, a.dtype == QX_DTYPE_BF16, s.img, s.rowscale, s.part, s.count,
+                     (int)T, (int)a.K, (int)a.V, err};
+    const TsLmHead::Args ea{a.bias, pv, pi, pl, (long long)a.vocab_offset, (long long)tiles_stride, a.mode, a.topk, a.invtemp,
+                            a.seed, a.mask, (int)m0};
+    if (!ts_launch_prep(st, p, FMT, h, a.dtype, s, (int)T, (int)a.K) ||
+        !ts_launch_dependent(st, dim3(p.grid), dim3(TS_WARPS * 32), p.smem, ts_kernel<FMT, TsLmHead>, m[0], m[1], m[0], m[1], q, ea))
+      return false;
+  }
+  return true;
+}
+
+// In-place pipeline (qx_tc_pipeline.cuh) form of stage 1, in the smallest scratch.
+template <int FMT, int BN>
+static bool launch_lmh_pipeline_bn(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t tiles_stride) {
+  using S = TcSmem<FMT, BN>;
+  using Epi = LmhEpi<BN>;
+  static_assert(S::TOTAL <= 227 * 1024, "stage-1 pipeline configuration exceeds shared memory");
+  int* err = device_error_flag();
+  static bool attr_set[64] = {};
+  int dev = 0;
+  cudaGetDevice(&dev);
+  if (!err || dev < 0 || dev >= 64) return false;
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(tc_pipeline_kernel<FMT, BN, Epi>, cudaFuncAttributeMaxDynamicSharedMemorySize, S::TOTAL) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    attr_set[dev] = true;
+  }
+  LmhScratch sc;
+  if (!lmh_carve(a, &sc)) return false;
+  const size_t row_bytes = (size_t)(a.K / StreamFmt<FMT>::BK) * StreamFmt<FMT>::BB;
+  CUtensorMap wmap;
+  if (!cached_weight_map(&wmap, a.wq, a.V, row_bytes, TcCfg<FMT>::BOX)) return false;
+  const int64_t items = (a.V + LMH_TILE - 1) / LMH_TILE * ((a.T + BN - 1) / BN);
+  if (items > 0x7fffffff) return false;
+  launch_prep_activations(st, a.h, a.dtype, sc.act, sc.rowscale, (int)a.T, (int)a.K, StreamFmt<FMT>::PERM, BN);
+  const typename Epi::Args ea{a.bias, pv, pi, pl, (int)a.T, (int)a.V, (long long)a.vocab_offset, (long long)tiles_stride,
+                              a.mode, a.topk, a.invtemp, a.seed, a.mask};
+  tc_pipeline_kernel<FMT, BN, Epi><<<(unsigned)(items < sm_count() ? items : sm_count()), LTC_WARPS * 32, S::TOTAL, st>>>(
+      wmap, wmap, sc.act, sc.rowscale, (int)a.T, (int)a.V, (int)a.K, 1, err, ea);
+  note_launch(2);
+  return true;
+}
+template <int FMT>
+static bool launch_lmh_pipeline(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t tiles_stride) {
+  if (!lmh_stream_ok<FMT>(a) || a.K % LTC_KS != 0 || a.V < 128) return false;
+  return a.T <= 32 ? launch_lmh_pipeline_bn<FMT, 32>(st, a, pv, pi, pl, tiles_stride)
+                   : launch_lmh_pipeline_bn<FMT, 64>(st, a, pv, pi, pl, tiles_stride);
 }
 
 template <int FMT>
@@ -833,7 +944,13 @@ template <int FMT>
 static bool launch_lmh_fast(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t ts) {
   if constexpr (FMT != F_Q6_K)
     if (a.T <= LMH_STREAM_ROWS && launch_lmh_stream<FMT>(st, a, pv, pi, pl, ts)) return true;
-  return launch_lmh_ts<FMT>(st, a, pv, pi, pl, ts);
+  if (launch_lmh_ts<FMT>(st, a, pv, pi, pl, ts)) return true;
+  // The tensor-memory form hands its accumulators over through scratch, up to 39 MB; where there is less, the in-place
+  // pipeline needs the prepared rows only (q8_0, 4096 -> 128256 in 4 MB, 17 / 64 rows: 284 / 310 us; groups of 32 and 64
+  // rows on the streaming kernel 305 / 525).
+  if constexpr (FMT != F_Q6_K)
+    if (a.T > LMH_STREAM_ROWS) return launch_lmh_pipeline<FMT>(st, a, pv, pi, pl, ts) || launch_lmh_stream<FMT>(st, a, pv, pi, pl, ts);
+  return false;
 }
 
 static bool launch_lmh_fast_any(cudaStream_t st, const LmHeadArgs& a, float* pv, int32_t* pi, float* pl, int64_t ts) {

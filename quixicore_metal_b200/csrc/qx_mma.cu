@@ -26,6 +26,7 @@ struct ProjEpi {
     uint8_t* mx_blocks;     // fused MXFP8 output rows (N % 32 == 0): a warp holds one 32-channel block per row
   };
   static constexpr bool DUAL = DUAL_;
+  __device__ __forceinline__ static bool packs_rows(const Args& a) { return a.mx_blocks != nullptr; }
   __device__ __forceinline__ static void run(const Args& a, const TcItem& it) {
     constexpr int CW = BN / 4;
     if (it.warp >= LTC_DQW) return;

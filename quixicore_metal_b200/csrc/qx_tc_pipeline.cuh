@@ -119,6 +119,7 @@ struct TcItem {
 };
 
 // Epi: struct Args (by-value kernel argument);
+//      static bool packs_rows(args)     writes MXFP8 rows, which a later call may take as its weights
 //      static constexpr bool DUAL       half 1 reads the second weight matrix at the same rows
 //      static void run(args, item)      all warps call it after a CTA barrier; it may use CTA barriers
 //      static void tail(args, ...)      after the last item (LM head: absent partials of padding tiles)
@@ -135,7 +136,7 @@ tc_pipeline_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
   constexpr int RST = C::RST;
   extern __shared__ uint8_t smem_dyn[];
   // a programmatic dependent may be scheduled; it waits for this grid's end, but not with its weight loads
-  if (!ea.mx_blocks) asm volatile("griddepcontrol.launch_dependents;");
+  if (!Epi::packs_rows(ea)) asm volatile("griddepcontrol.launch_dependents;");
   uint8_t* smem = reinterpret_cast<uint8_t*>(((uintptr_t)smem_dyn + 1023) & ~(uintptr_t)1023);
   const uint32_t sbase = smem_u32(smem);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;

@@ -341,3 +341,29 @@ def test_lm_head_rows_outside_the_exact_range(fmt, T, V, K):
         tok = host(tk.lm_head_sample(dev(h, "bf16"), dev(W), mode=mode, format=fmt, temperature=0.8, seed=3, **kw))
         want, margin = O.lm_head_sample(h, W, fmt, code, temperature=0.8, seed=3, return_detail=True, **kw)
         check_ids(tok, want, margin, 1e-4 if fmt != "q8_0" else 0.5, f"{fmt}/{mode}")
+
+
+def _elapsed(fn, n=3):
+    fn(); fn()
+    a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+    a.record()
+    for _ in range(n):
+        fn()
+    b.record(); b.synchronize()
+    return a.elapsed_time(b) / n
+
+
+# 148 groups of 64 rows fill one launch of the LM head's tensor-memory form; one row more is a second launch (the
+# scalar kernel took 40 times as long)
+def test_lm_head_rows_past_one_launch():
+    rng = np.random.default_rng(1)
+    V, K = 3000, 1024
+    W = dev(O.synth_pack("q8_0", (0.3 * rng.standard_normal((V, K))).astype(np.float32)))
+    h = torch.randn(148 * 64 + 1, K, generator=torch.Generator("cuda").manual_seed(1), device="cuda").bfloat16()
+    call = lambda rows, mode="categorical": tk.lm_head_sample(h[rows], W, mode=mode, k=0, temperature=0.8, seed=3, format="q8_0")
+    got, first = call(slice(None)), call(slice(0, 9472))
+    assert (got[:9472] != first).float().mean() < 1e-3            # the noise of a row goes by its index in the call; near-ties
+    want, margin = O.lm_head_sample(host(h[-8:]), host(W), "q8_0", 0, temperature=0.8, seed=3, return_detail=True)
+    check_ids(host(call(slice(None), "argmax"))[-8:], want, margin, 1e-4, "last rows")
+    assert _elapsed(lambda: call(slice(None))) < 5 * _elapsed(lambda: call(slice(0, 9472)))
+

@@ -114,3 +114,30 @@ def test_noalloc_entry_rejects_oversized_requests():
                                             None, ids.data_ptr(), T, V, K, b"q8_0", _lib.DTYPE_BF16, 3, 32, 0.8, 1, 0.9)
     assert _lib.STATUS_NAMES[st.code] == "insufficient_workspace"
     assert b"scratch" in st.detail
+
+
+@pytest.mark.parametrize("T", [17, 40, 64])
+def test_noalloc_entry_above_16_rows_is_no_scalar_kernel(T):
+    """The built-in array does not hold what the tensor-memory form of stage 1 wants at a real vocabulary; the
+    entry then streams the weights (the scalar kernel takes 70 to 200 times as long as the workspace entry)."""
+    from quixicore_metal_b200 import _lib
+    g = torch.Generator("cuda").manual_seed(T)
+    V, K = 32000, 4096
+    wq = torch.randint(0, 256, (V, K // 32, 34), dtype=torch.uint8, device="cuda", generator=g)
+    wq[..., :2] = torch.tensor([0.01], dtype=torch.float16).view(torch.uint8).cuda()
+    h = torch.randn((T, K), generator=g, device="cuda").bfloat16()
+    L = _lib.lib()
+    ws = torch.empty(L.qx_cuda_lm_head_workspace_bytes(T, V, K, 0, 0), dtype=torch.uint8, device="cuda")
+    ms = {}
+    for entry in ("workspace", "noalloc"):
+        for _ in range(2):
+            r, ids = _call(entry, h, wq, "bf16", 0, 0, 1, ws)
+        assert r.code == 0, r.detail
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        for _ in range(4):
+            _call(entry, h, wq, "bf16", 0, 0, 1, ws)
+        b.record(); b.synchronize()
+        ms[entry] = (a.elapsed_time(b), ids)
+    assert torch.equal(ms["noalloc"][1], ms["workspace"][1])
+    assert ms["noalloc"][0] < 10 * ms["workspace"][0], (ms["noalloc"][0], ms["workspace"][0])

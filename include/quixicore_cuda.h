@@ -176,9 +176,12 @@ qx_status qx_cuda_decode_linear_epilogue(void* stream, const void* x, const void
                                          int use_residual, int out_quant, void* out_codes,
                                          float* out_scale, void* workspace, size_t workspace_bytes);
 
-/* The two projections with a fixed order of the K sums: the streaming kernels' up to 16 rows (and in their
- * passes), one accumulator over the whole of K per output above - the results of releases before the
- * faster kernel for large batches, bit for bit.  For chains of blocks, where one output that rounds the other way
+/* The two projections with an order of the K sums that depends on format, K and the rows only, not on how work is cut
+ * between thread blocks: the streaming kernels' up to 16 rows (and in their passes), one accumulator over the whole of K
+ * per output above, where a format has such a kernel (q4_0, q8_0, mxfp8, mxfp4 with rows of a multiple of 16 bytes;
+ * nvfp4) - there the results of releases before the faster kernel for large batches, bit for bit.  What had no tensor
+ * kernel then (q6_K above 16 rows and row pitches that are no multiple of 16 bytes) takes rounded sums over chunks of
+ * 256 columns and more.  For chains of blocks, where one output that rounds the other way
  * reaches every later value.  Arguments and workspace as the plain forms, without output quantisation. */
 qx_status qx_cuda_decode_linear_epilogue_ordered(void* stream, const void* x, const void* weight, const void* bias,
                                                  const void* residual, void* y, int64_t M, int64_t K, int64_t N,

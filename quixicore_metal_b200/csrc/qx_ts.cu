@@ -285,9 +285,11 @@ static bool ts_projection_plan(const GemvArgs& a, TsPlan* p) {
   const int group = a.format == F_Q6_K ? (a.w1 ? 32 : 64) : (short_terms ? 128 : 64);
   const int64_t M = a.M < TS_PASS_GROUPS * group ? a.M : TS_PASS_GROUPS * group;
   if (!a.ordered) return ts_plan(p, a.format, M, a.K, a.N, rb, a.w1 != nullptr, group, 0, true);
-  // the caller wants the sums of the in-place pipeline (one accumulator over the whole of K per output)
+  // A fixed order: items whole.  nvfp4 in the one accumulator over the whole of K of the in-place pipeline, whose
+  // sums it continues; the other formats, which have no such form here, keep rounded sums over chunks (q6_K, K = 27648: one
+  // accumulator over 5184 truncating steps is 1e-4 too small).
   if (!ts_plan(p, a.format, M, a.K, a.N, rb, a.w1 != nullptr, group, 0, false)) return false;
-  p->sums = 0;
+  if (a.format == F_NVFP4) p->sums = 0;
   return true;
 }
 

@@ -367,3 +367,31 @@ def test_lm_head_rows_past_one_launch():
     check_ids(host(call(slice(None), "argmax"))[-8:], want, margin, 1e-4, "last rows")
     assert _elapsed(lambda: call(slice(None))) < 5 * _elapsed(lambda: call(slice(0, 9472)))
 
+
+# The one-accumulator form of the ordered entries is for nvfp4; other formats keep rounded chunk sums.  Mean signed error
+# of 32 x 136 f16 outputs in units of the output: rounding to f16 averages to below 1e-5 (2^-11 / sqrt(12 * 4352)), a
+# truncating accumulator over the 5184 steps of this K leaves 1e-4 towards zero.
+def test_ordered_sums_are_not_biased():
+    x, W, _, _ = _linear("q6_K", 32, 27648, 136, "f16", 3)
+    ref = x.astype(np.float64) @ O.dequantize("q6_K", W).astype(np.float64).T
+    got = host(tk_torch.decode_linear_epilogue(dev(x, "f16"), dev(W), None, None, "q6_K", ordered=True)).astype(np.float64)
+    big = np.abs(ref) > 0.5
+    assert abs(np.mean(((got - ref) / ref)[big])) < 3e-5
+
+
+# nvfp4 above the passes: the uncut form against the in-place pipeline whose sums it continues, bit for bit
+@pytest.mark.parametrize("M,K,N", [(70, 2048, 300), (128, 4096, 257), (32, 512, 24640)])
+def test_ordered_nvfp4_equals_the_pipeline(M, K, N):
+    from quixicore_metal_b200 import _lib
+    x, W, _, _ = _linear("nvfp4", M, K, N, "bf16", M)
+    _, U, _, _ = _linear("nvfp4", M, K, N, "bf16", M + 1)
+    x, W, U = dev(x, "bf16"), dev(W), dev(U)
+    run = lambda: (tk_torch.decode_linear_epilogue(x, W, None, None, "nvfp4", ordered=True),
+                   tk_torch.decode_swiglu(x, W, U, None, None, "nvfp4", ordered=True))
+    got = run()
+    _lib.set_option("ts_min_rows", 1 << 20)
+    try:
+        want = run()
+    finally:
+        _lib.set_option("ts_min_rows", 0)
+    assert all(torch.equal(a, b) for a, b in zip(got, want))

@@ -722,8 +722,7 @@ bool launch_base_q_matmul(cudaStream_t st, const BaseQDesc& d, const BaseQMat* m
       p.xs_off = (unsigned)xs_off;
       smem = xs_off + cta_prepared_row_bytes((size_t)K);
     } else {
-      launch_prep_activations(st, xr, dtype, x16, rowscale, (int)M, (int)K, 5);
-      note_launch();
+      fast = launch_prep_activations(st, xr, dtype, x16, rowscale, (int)M, (int)K, 5);
     }
     CUtensorMap maps[3];
     const int pitch = BQ_KC * d.bits / 8 + 16;

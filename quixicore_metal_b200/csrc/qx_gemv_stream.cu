@@ -1,7 +1,7 @@
 // decode_linear_epilogue / decode_swiglu for bf16 / f16 activations, batch <= 16: the streaming
 // tensor-core path (see qx_stream.cuh for the design).
 //
-// Two launches per call: prep_activations_kernel turns the activations into row-scaled f16 in the
+// Two launches per call: prep_rows_kernel (qx_prep.cu) turns the activations into row-scaled f16 in the
 // decoder's column order (stream-ordered scratch of M*K*2 + M*4 bytes), then gemv_stream_kernel
 // streams the weights.  Work split of the main kernel: an m-tile is 16 weight rows (16 gate + 16 up
 // rows for SwiGLU); a step is one pipeline stage (KC columns) of one m-tile.  One CTA per SM takes a
@@ -37,113 +37,6 @@ int read_device_error_flag() {
   int v = -1;
   if (cudaMemcpyFromSymbol(&v, g_qx_device_error, sizeof(int)) != cudaSuccess) return -1;
   return v;
-}
-
-// ---- activation preparation ----------------------------------------------------------------------
-// Grid (slices, rows).  Every CTA first finds the row's largest finite magnitude by reading the
-// whole row (a few KB from L2; cheaper than a second launch or a grid-wide reduction), derives the
-// power-of-two scale 2^-S that puts it in [2^14, 2^15), then converts its slice:
-// x16[m][perm(c)] = f16(x[m][c] * 2^-S); rowscale[m] = 2^S.
-// img_rows > 0 selects the operand-tile image the tcgen05 kernels copy in bulk instead of the plain
-// row-major layout: rows are taken in groups of img_rows; a group is stored k-stage by k-stage
-// (64 columns = 128 bytes per row), each stage as img_rows consecutive 128-byte rows whose 16-byte
-// chunks are XOR-swizzled with the row index (the 128-byte swizzle of a K-major operand tile);
-// rows past M are zero.
-template <typename T>
-__global__ void __launch_bounds__(256)
-prep_activations_kernel(const T* __restrict__ x, __half* __restrict__ x16,
-                        float* __restrict__ rowscale, int M, int K, int perm, int img_rows) {
-  __shared__ float red[8];
-  asm volatile("griddepcontrol.launch_dependents;");   // a dependent grid may be scheduled from now on
-  const int m = blockIdx.y;
-  if (m >= M) {                                     // zero padding row of the last image group
-    const int per = (((K + gridDim.x - 1) / gridDim.x) + 31) & ~31;
-    const int c0 = blockIdx.x * per, c1 = min(K, c0 + per);
-    const int grp = m / img_rows, ml = m % img_rows;
-    __half* out = x16 + (size_t)grp * img_rows * K;
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x)
-      out[((size_t)(c >> 6) * img_rows + ml) * 64 + ((((c >> 3) & 7) ^ (ml & 7)) << 3) + (c & 7)] = __float2half_rn(0.f);
-    return;
-  }
-  const T* xr = x + (size_t)m * K;
-  float amax = 0.f;
-  if constexpr (sizeof(T) == 2) {
-    const uint4* xv = reinterpret_cast<const uint4*>(xr);          // 8 elements per load (K % 8 == 0)
-    const int nv = K / 8;
-    auto fold = [&](const uint4& v) {
-      const T* e = reinterpret_cast<const T*>(&v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const float a = fabsf(to_f32<T>(e[j]));
-        if (a < 3.0e38f) amax = fmaxf(amax, a);                    // inf / nan do not choose the scale
-      }
-    };
-    int i = threadIdx.x;
-    for (; i + 3 * (int)blockDim.x < nv; i += 4 * blockDim.x) {    // four loads in flight per thread
-      const uint4 v0 = __ldg(xv + i), v1 = __ldg(xv + i + blockDim.x), v2 = __ldg(xv + i + 2 * blockDim.x),
-                  v3 = __ldg(xv + i + 3 * blockDim.x);
-      fold(v0); fold(v1); fold(v2); fold(v3);
-    }
-    for (; i < nv; i += blockDim.x) fold(__ldg(xv + i));
-  } else {
-    for (int c = threadIdx.x; c < K; c += blockDim.x) {
-      const float a = fabsf(to_f32<T>(xr[c]));
-      if (a < 3.0e38f) amax = fmaxf(amax, a);
-    }
-  }
-  amax = warp_max(amax);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-  __syncthreads();
-  amax = red[0];
-#pragma unroll
-  for (int i = 1; i < 8; ++i) amax = fmaxf(amax, red[i]);
-  int S = 0;
-  if (amax > 0.f) {
-    S = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 - 14;
-    S = max(-110, min(110, S));
-  }
-  const float down = __uint_as_float((uint32_t)(127 - S) << 23);   // 2^-S
-  const int per = (((K + gridDim.x - 1) / gridDim.x) + 31) & ~31;  // slice: whole 32-column groups
-  const int c0 = blockIdx.x * per, c1 = min(K, c0 + per);
-  if (img_rows > 0) {
-    const int grp = m / img_rows, ml = m % img_rows;
-    __half* out = x16 + (size_t)grp * img_rows * K;
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-      const int pos = (c & ~31) + perm_position(perm, c & 31);
-      out[((size_t)(pos >> 6) * img_rows + ml) * 64 + ((((pos >> 3) & 7) ^ (ml & 7)) << 3) + (pos & 7)] =
-          __float2half_rn(to_f32<T>(xr[c]) * down);
-    }
-  } else if (sizeof(T) == 2) {
-    __half* out = x16 + (size_t)m * K;                             // slices are whole 32-column groups: 8 per load
-    const uint4* xv = reinterpret_cast<const uint4*>(xr);
-    for (int i = c0 / 8 + threadIdx.x; i < c1 / 8; i += blockDim.x) {
-      const uint4 v = __ldg(xv + i);
-      const T* e = reinterpret_cast<const T*>(&v);
-      const int c = 8 * i;
-#pragma unroll
-      for (int j = 0; j < 8; ++j)
-        out[(c & ~31) + perm_position(perm, (c & 31) + j)] = __float2half_rn(to_f32<T>(e[j]) * down);
-    }
-  } else {
-    __half* out = x16 + (size_t)m * K;
-    for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) {
-      const int pos = (c & ~31) + perm_position(perm, c & 31);
-      out[pos] = __float2half_rn(to_f32<T>(xr[c]) * down);
-    }
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) rowscale[m] = __uint_as_float((uint32_t)(127 + S) << 23);
-}
-
-void launch_prep_activations(cudaStream_t st, const void* x, qx_dtype dtype, __half* x16,
-                             float* rowscale, int M, int K, int perm, int img_rows) {
-  int slices = (K + 1023) / 1024;
-  if (slices > 32) slices = 32;
-  const int rows = img_rows > 0 ? (M + img_rows - 1) / img_rows * img_rows : M;
-  dim3 grid(slices, rows);
-  if (dtype == QX_DTYPE_F16)
-    prep_activations_kernel<__half><<<grid, 256, 0, st>>>((const __half*)x, x16, rowscale, M, K, perm, img_rows);
-  else
-    prep_activations_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, x16, rowscale, M, K, perm, img_rows);
 }
 
 // Whole stages run fully unrolled in the instantiations with up to this many 8-row n-tiles (0 = never).
@@ -521,9 +414,9 @@ static bool launch_stream_t(cudaStream_t st, const GemvArgs& a) {
   __half* x16 = (__half*)a.scratch;
   float* rowscale = (float*)((char*)a.scratch + x16_bytes);
   const size_t smem = (size_t)nwarps * Cfg::warp_smem(NT);
-  launch_prep_activations(st, a.x, a.dtype, x16, rowscale, (int)a.M, (int)a.K, StreamFmt<FMT>::PERM);
+  if (!launch_prep_activations(st, a.x, a.dtype, x16, rowscale, (int)a.M, (int)a.K, StreamFmt<FMT>::PERM)) return false;
   if (!launch_stream_x<FMT, NT, DUAL, HALF, T, false>(st, a, nwarps, smem, blocks, x16, rowscale, err)) return false;
-  note_launch(2);
+  note_launch();
   return true;
 }
 

@@ -73,8 +73,9 @@ int* device_error_flag();
 size_t stream_scratch_bytes(const GemvArgs& a);
 size_t tc_scratch_bytes(const GemvArgs& a);
 size_t projection_scratch_bytes(const GemvArgs& a);
-// Row-scaled f16 copy of (M,K) bf16 / f16 activations in the column order `perm` of the decoders.
-void launch_prep_activations(cudaStream_t st, const void* x, qx_dtype dtype, __half* x16,
+// Row-scaled f16 copy of (M,K) bf16 / f16 activations in the column order `perm` of the decoders (qx_prep.cu); false: not
+// launched.
+bool launch_prep_activations(cudaStream_t st, const void* x, qx_dtype dtype, __half* x16,
                              float* rowscale, int M, int K, int perm, int img_rows = 0);
 // Picks the kernel family for one projection call (format, dtype, batch, alignment); true when the
 // kernel that ran also wrote the requested MXFP8 output rows.

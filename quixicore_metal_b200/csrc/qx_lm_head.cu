@@ -895,12 +895,12 @@ static bool launch_lmh_pipeline_bn(cudaStream_t st, const LmHeadArgs& a, float* 
   if (!cached_weight_map(&wmap, a.wq, a.V, row_bytes, TcCfg<FMT>::BOX)) return false;
   const int64_t items = (a.V + LMH_TILE - 1) / LMH_TILE * ((a.T + BN - 1) / BN);
   if (items > 0x7fffffff) return false;
-  launch_prep_activations(st, a.h, a.dtype, sc.act, sc.rowscale, (int)a.T, (int)a.K, StreamFmt<FMT>::PERM, BN);
+  if (!launch_prep_activations(st, a.h, a.dtype, sc.act, sc.rowscale, (int)a.T, (int)a.K, StreamFmt<FMT>::PERM, BN)) return false;
   const typename Epi::Args ea{a.bias, pv, pi, pl, (int)a.T, (int)a.V, (long long)a.vocab_offset, (long long)tiles_stride,
                               a.mode, a.topk, a.invtemp, a.seed, a.mask};
   tc_pipeline_kernel<FMT, BN, Epi><<<(unsigned)(items < sm_count() ? items : sm_count()), LTC_WARPS * 32, S::TOTAL, st>>>(
       wmap, wmap, sc.act, sc.rowscale, (int)a.T, (int)a.V, (int)a.K, 1, err, ea);
-  note_launch(2);
+  note_launch();
   return true;
 }
 template <int FMT>
@@ -933,8 +933,7 @@ static bool launch_lmh_stream(cudaStream_t st, const LmHeadArgs& a, float* pv, i
     launch_lmh_stream_nt<FMT, 1, true>(st, a, nullptr, nullptr, pv, pi, pl, tiles_stride, err, wmap);
     return true;
   }
-  launch_prep_activations(st, a.h, a.dtype, x16, rowscale, (int)a.T, (int)a.K, StreamFmt<FMT>::PERM);
-  note_launch();
+  if (!launch_prep_activations(st, a.h, a.dtype, x16, rowscale, (int)a.T, (int)a.K, StreamFmt<FMT>::PERM)) return false;
   if (a.T <= 8) launch_lmh_stream_nt<FMT, 1, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
   else launch_lmh_stream_nt<FMT, 2, false>(st, a, x16, rowscale, pv, pi, pl, tiles_stride, err, wmap);
   return true;

@@ -117,8 +117,7 @@ static bool launch_pipeline_bn(cudaStream_t st, const GemvArgs& a, int* err) {
   if (!a.scratch || a.scratch_bytes < img_bytes + (((size_t)a.M * 4 + 255) & ~(size_t)255)) return false;
   __half* ximg = (__half*)a.scratch;
   float* rowscale = (float*)((char*)a.scratch + img_bytes);
-  launch_prep_activations(st, a.x, a.dtype, ximg, rowscale, (int)a.M, (int)a.K, StreamFmt<FMT>::PERM, BN);
-  note_launch();
+  if (!launch_prep_activations(st, a.x, a.dtype, ximg, rowscale, (int)a.M, (int)a.K, StreamFmt<FMT>::PERM, BN)) return false;
   const int item_rows = DUAL ? 128 : 256;
   const long long items = (long long)((a.N + item_rows - 1) / item_rows) * groups;
   const unsigned grid = (unsigned)(items < sm_count() ? items : sm_count());

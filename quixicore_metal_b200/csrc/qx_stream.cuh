@@ -171,7 +171,7 @@ __device__ __forceinline__ void scale_add(float (&acc)[4], float s0, float s1, c
 //         this period, so every shared-memory load inside a step has a static alignment);
 // KC    = columns one pipeline stage holds per row (a multiple of GROUP whose byte size is a
 //         multiple of 16, except q6_K whose 210-byte blocks are only 4-byte periodic);
-// PERM  = column order of the prepared activations (see prep_activations_kernel).
+// PERM  = column order of the prepared activations (see prep_rows_kernel).
 template <int FMT> struct StreamFmt;
 template <> struct StreamFmt<F_Q4_0>  { static constexpr int UNIT = 32, GROUP = 64,  KC = 512, BK = 32,  BB = 18,  PERM = 1; };
 template <> struct StreamFmt<F_Q8_0>  { static constexpr int UNIT = 32, GROUP = 64,  KC = 256, BK = 32,  BB = 34,  PERM = 0; };

@@ -111,82 +111,6 @@ bool ts_maps(const TsPlan& p, int format, const void* w, int64_t K, int64_t N, C
   return rest == 0 || cached_box_map(&m[0], w, 2, row_bytes * rest / 2, full + 1, pitch, g.pitch / 2, 128 / p.P);
 }
 
-// ---- activation preparation ------------------------------------------------------------------------
-// One CTA per row: largest finite magnitude -> power-of-two scale 2^-S that puts it in [2^14, 2^15), then
-// f16(x * 2^-S) into the image [group][K / 8][mp][8] (16-byte chunks of one row, mp rows side by side: the
-// unswizzled operand layout), 32-column units in the decoder's order.  Latency-bound: a row is one pass
-// over 2 K bytes, the second read hits L1.  Rows past the group's end are never read back.
-template <typename T>
-__global__ void __launch_bounds__(256)
-ts_prep_kernel(const T* __restrict__ x, uint4* __restrict__ img, float* __restrict__ rowscale, unsigned* __restrict__ count,
-               int ncount, int K, int mg, int mp, int fmt) {
-  __shared__ float red[8];
-  // First the wait: the contraction may be scheduled once every CTA is past it, so all that ran before this kernel is
-  // complete then - its weight loads need no wait of their own (an earlier kernel of the stream may have written
-  // them), and its bounded waits do not count while a long predecessor runs.
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;");
-  const int m = blockIdx.x;
-  if (m == 0)
-    for (int i = threadIdx.x; i < ncount; i += blockDim.x) count[i] = 0u;
-  const uint4* xv = reinterpret_cast<const uint4*>(x + (size_t)m * K);
-  float amax = 0.f;
-  for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-    const uint4 v = __ldg(xv + i);
-    const T* e = reinterpret_cast<const T*>(&v);
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float a = fabsf(to_f32<T>(e[j]));
-      if (a < 3.0e38f) amax = fmaxf(amax, a);                        // inf / nan do not choose the scale
-    }
-  }
-  amax = warp_max(amax);
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = amax;
-  __syncthreads();
-  amax = red[0];
-#pragma unroll
-  for (int i = 1; i < 8; ++i) amax = fmaxf(amax, red[i]);
-  int S = 0;
-  if (amax > 0.f) {
-    S = (int)((__float_as_uint(amax) >> 23) & 0xFFu) - 127 - 14;
-    S = max(-110, min(110, S));
-  }
-  const float down = __uint_as_float((uint32_t)(127 - S) << 23);
-  const int grp = m / mg, ml = m - grp * mg;
-  uint4* out = img + ((size_t)grp * (K / 8)) * mp + ml;
-  // a thread makes one 16-byte chunk (8 positions) of a unit; its source columns lie in the unit's 64 bytes
-  for (int i = threadIdx.x; i < K / 8; i += blockDim.x) {
-    const int u = i >> 2, c4 = i & 3;
-    __half h[8];
-    if (fmt == F_Q4_0 || fmt == F_MXFP4 || fmt == F_NVFP4) {
-      const T* xu = x + (size_t)m * K + (size_t)u * 32;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) {
-        const int pos = 8 * c4 + j;                                  // inverse of ts_position
-        int c;
-        if (fmt == F_NVFP4) c = (pos & 16) | ((pos & 15) >> 1) | ((pos & 1) << 3);
-        else if (fmt == F_MXFP4) c = (pos >> 1) | ((pos & 1) << 4);
-        else c = ((pos >> 1) & 1) * 16 + (pos >> 3) * 4 + (((pos >> 2) & 1) | ((pos & 1) << 1));
-        h[j] = __float2half_rn(to_f32<T>(xu[c]) * down);
-      }
-    } else {
-      const uint4 v = __ldg(xv + i);
-      const T* e = reinterpret_cast<const T*>(&v);
-#pragma unroll
-      for (int j = 0; j < 8; ++j) h[j] = __float2half_rn(to_f32<T>(e[j]) * down);
-    }
-    out[(size_t)i * mp] = *reinterpret_cast<const uint4*>(h);
-  }
-  if (threadIdx.x == 0) rowscale[m] = __uint_as_float((uint32_t)(127 + S) << 23);
-}
-
-bool ts_launch_prep(cudaStream_t st, const TsPlan& p, int format, const void* x, qx_dtype dtype, const TsScratch& s, int M, int K) {
-  const int ncount = p.whole ? 0 : p.items;
-  if (dtype == QX_DTYPE_F16)
-    return ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__half>, (const __half*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
-  return ts_launch_dependent(st, dim3(M), dim3(256), 0, ts_prep_kernel<__nv_bfloat16>, (const __nv_bfloat16*)x, (uint4*)s.img, s.rowscale, s.count, ncount, K, p.mg, p.mp, format);
-}
-
 // ---- projection epilogue ------------------------------------------------------------------------------
 struct TsProj {
   struct Args {

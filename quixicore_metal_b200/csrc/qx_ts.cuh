@@ -131,7 +131,7 @@ bool ts_launch_prep(cudaStream_t st, const TsPlan& p, int format, const void* x,
 
 // A launch that may start before its predecessor in the stream has finished (the kernels here call
 // griddepcontrol.wait before they touch what it produces; the contraction's weights are complete when it starts, see
-// ts_prep_kernel).
+// prep_rows_kernel).
 template <typename... P, typename... A>
 bool ts_launch_dependent(cudaStream_t st, dim3 grid, dim3 block, size_t smem, void (*kernel)(P...), A&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -395,3 +395,21 @@ def test_ordered_nvfp4_equals_the_pipeline(M, K, N):
     finally:
         _lib.set_option("ts_min_rows", 0)
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+# Activation preparation: an infinity, a NaN or a bf16 value past 3e38 in one row chooses no scale and reaches no other
+# row; a row of zeros; orders of magnitude between rows; rows of one and of several passes over K.
+@pytest.mark.parametrize("M,K", [(5, 512), (5, 12288), (20, 768), (20, 4352)])
+@pytest.mark.parametrize("dtype", ["bf16", "f16"])
+@pytest.mark.parametrize("fmt", FMTS)
+def test_prepared_rows_with_special_values(fmt, dtype, M, K):
+    x, W, _, _ = _linear(fmt, M, K, 80, dtype, M + K)
+    x[0, K - 1], x[1, 3], x[2, 7] = np.inf, np.nan, 3.3e38 if dtype == "bf16" else -np.inf
+    x[3] = 0.0
+    x[4] = rounded(x[4] * 2.0 ** (-60 if dtype == "bf16" else -9), dtype)
+    got = host(tk.decode_linear_epilogue(dev(x, dtype), dev(W), None, None, format=fmt))
+    ref = O.decode_linear_epilogue(x[3:], W, fmt, None, None, 0, dtype)
+    # one ulp, fp32 noise of the row's largest output, one step of f16 subnormals
+    ulp, step = (2.0 ** -7, 0.0) if dtype == "bf16" else (2.0 ** -10, 2.0 ** -24)
+    assert np.all(np.abs(got[3:] - ref) <= np.abs(ref) * ulp * 1.01 + 2e-5 * np.abs(ref).max(1, keepdims=True) + step)
+    assert not np.isfinite(got[:2]).any() and np.all(got[3] == 0)

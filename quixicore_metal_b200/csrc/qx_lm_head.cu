@@ -45,12 +45,13 @@ __device__ __forceinline__ void lmh_select_token(const float* __restrict__ logit
   if (mode <= 1) {
     float best = QX_NEG_INF;
     int bid = 0x7fffffff;
-    for (int lr = lane; lr < nvalid; lr += 32) {
+    for (int l0 = 0; l0 < nvalid; l0 += 32) {             // (the same count for every lane, see ts_kernel)
+      const int lr = min(l0 + lane, nvalid - 1);
       const int gid = (int)(vocab_offset + v0 + lr);
       float ls = logit[lr] * invtemp;
       if (bias) ls += bias[v0 + lr];
       if (mode == 1) ls += rng_gumbel(seed, (uint32_t)t, (uint32_t)gid);
-      if (better(ls, gid, best, bid)) { best = ls; bid = gid; }
+      if (l0 + lane < nvalid && better(ls, gid, best, bid)) { best = ls; bid = gid; }
     }
     warp_argmax(best, bid);
     if (lane == 0) {
@@ -148,9 +149,10 @@ __device__ __forceinline__ void lmh_select_token(const float* __restrict__ logit
       ties_before += __popc(bal_eq);
     }
   }
-  for (int kk = (int)out_pos + lane; kk < topk; kk += 32) {
-    part_val[pbase + kk] = QX_NEG_INF;
-    part_id[pbase + kk] = -1;
+  for (int k0 = (int)out_pos; k0 < topk; k0 += 32) {
+    if (k0 + lane >= topk) continue;
+    part_val[pbase + k0 + lane] = QX_NEG_INF;
+    part_id[pbase + k0 + lane] = -1;
   }
 }
 
@@ -267,9 +269,10 @@ __device__ __forceinline__ void lmh_select_rows(const float* const (&logit)[R], 
       out_pos += __popc(bal);
       ties_before += __popc(bal_eq);
     }
-    for (int kk = (int)out_pos + lane; kk < topk; kk += 32) {
-      part_val[pbase + kk] = QX_NEG_INF;
-      part_id[pbase + kk] = -1;
+    for (int k0 = (int)out_pos; k0 < topk; k0 += 32) {
+      if (k0 + lane >= topk) continue;
+      part_val[pbase + k0 + lane] = QX_NEG_INF;
+      part_id[pbase + k0 + lane] = -1;
     }
   }
 }
@@ -693,11 +696,13 @@ struct LmhEpi {
   }
 };
 
-// Output policy of the tensor-memory-operand kernel (qx_ts.cuh) for LM-head stage 1: each of the 8 output warps
+// Output policy of the tensor-memory-operand kernel (qx_ts.cuh) for LM-head stage 1: each of the output warps
 // brings the 256 logits of two hidden rows at a time to shared memory and reduces them to their tile
 // partials, while the other roles work on the next tile.
-constexpr size_t LMH_TS_AUX = (size_t)TS_OUT * 2 * LMH_TILE * 4;
 struct TsLmHead {
+  static constexpr bool HELP = true;
+  static constexpr int AUX = 2 * LMH_TILE * 4;               // per warp; the helpers' in the ring of raw stages
+  static_assert(TS_WORKERS * AUX <= 2 * 128 * 144, "two raw stages of the narrowest format hold it");
   struct Args {
     const float* bias;
     float* part_val; int32_t* part_id; float* part_lse;
@@ -711,16 +716,16 @@ struct TsLmHead {
   __device__ __forceinline__ static bool packs_rows(const Args&) { return false; }
   template <bool SHIFT>
   __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, const float* back,
-                                             uint8_t* aux, int warp, int lane) {
-    float* logit = reinterpret_cast<float*>(aux) + warp * 2 * LMH_TILE;
+                                             uint8_t* aux, int warp, int warps, int lane) {
+    float* logit = reinterpret_cast<float*>(aux);
     const int v0 = it.tile * LMH_TILE, nvalid = min(LMH_TILE, q.N - v0);
 #pragma unroll 1
-    for (int m0 = warp; m0 < it.m_count; m0 += 2 * TS_OUT) {
+    for (int m0 = warp; m0 < it.m_count; m0 += 2 * warps) {
       const float* rows[2] = {logit, logit + LMH_TILE};
-      const int t0 = a.row0 + it.m_base + m0, trow[2] = {t0, m0 + TS_OUT < it.m_count ? t0 + TS_OUT : -1};
+      const int t0 = a.row0 + it.m_base + m0, trow[2] = {t0, m0 + warps < it.m_count ? t0 + warps : -1};
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int m = m0 + r * TS_OUT;
+        const int m = m0 + r * warps;
         if (m >= it.m_count) break;
         float v[8];
 #pragma unroll
@@ -853,7 +858,7 @@ static bool launch_lmh_ts(cudaStream_t st, const LmHeadArgs& a, float* pv, int32
     // K = 1024 35.2 -> 33.0).  Several rounds are cut evenly (q8_0, 64 rows, 501 items: 275.6 us, 280.6 whole).
     const int64_t items = (a.V + 255) / 256 * ((T + group - 1) / group);
     const bool whole = items <= sm_count() && (2 * items > sm_count() || a.K < 2048);
-    if (!ts_plan(&p, FMT, T, a.K, a.V, 2, 0, group, LMH_TS_AUX, options().lm_head_ksplit && !whole)) return false;
+    if (!ts_plan(&p, FMT, T, a.K, a.V, 2, 0, group, TS_OUT * TsLmHead::AUX, options().lm_head_ksplit && !whole)) return false;
     if (!a.scratch || a.scratch_bytes < p.scratch()) return false;
     CUtensorMap m[2];
     if (!ts_maps(p, FMT, a.wq, a.K, a.V, m)) return false;

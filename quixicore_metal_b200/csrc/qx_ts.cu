@@ -54,11 +54,11 @@ bool ts_plan(TsPlan* p, int format, int64_t M, int64_t K, int64_t N, int rb, int
   p->na = (512 - (p->sums + p->nd) * acc) / slot;
   p->na = p->na >= 16 && format != F_Q6_K ? 16 : (p->na >= 8 && format != F_Q6_K ? 8 : 4);
   p->issuers = p->rb == 2 && p->na >= 8 ? 2 : 1;
-  // activation stages of 256 columns; from 48 rows on they are handed over by quarters, so that a ring of two
-  // (or one) keeps flowing
-  p->actq = p->mp <= 32 ? 1 : 4;
+  // Activation stages of 256 columns: at least two, and the raw ring takes the rest.  (One of 128 rows, handed over by
+  // quarters beside a longer raw ring, costs the issuers a wait per quarter: 8192 -> 28672, mxfp4, 256 rows, 190 us
+  // against 186; 4096 -> 14336, nvfp4, 128 rows, 53.5 against 49.5.)
   const size_t act_stage = (size_t)TS_KC * p->mp * 2;
-  p->nact = p->mp <= 16 ? 4 : (p->mp <= 32 ? 3 : (p->mp <= 80 ? 2 : 1));
+  p->nact = p->mp <= 16 ? 4 : (p->mp <= 32 ? 3 : 2);
   const size_t stage = (size_t)128 * g.pitch;
   const size_t bar_bytes = 8 * (2 * TS_MAX_RAW + 2 * TS_MAX_ACT + 2 * TS_MAX_SLOTS + 12) + 4 * (4 + TS_MARK_RING * 8 + 128 + 256);
   const size_t act = (act_stage * p->nact + 256 + 127) & ~(size_t)127;   // + what overlapping core matrices read past the end
@@ -125,22 +125,26 @@ struct TsProj {
     const uint16_t b = reinterpret_cast<const uint16_t*>(p)[i];
     return half ? __half2float(__ushort_as_half(b)) : __uint_as_float((uint32_t)b << 16);
   }
-  // Four columns at a time, the next four asked for before these are finished; warps 0..3 take the even groups of
-  // four, warps 4..7 the odd ones, a lane one weight row.  MXFP8 rows are packed from the registers (a block
-  // is 32 lanes): packed in a second pass over y they cost 128 us of 272 at 256 x 28672.
-  __device__ __forceinline__ static void sum4(const TsItem& it, size_t at, float (&v)[4]) {
+  static constexpr int AUX = 0;
+  static constexpr bool HELP = true;
+  // Eight columns at a time: warps w, w + 4, .. take the groups of eight in turn, a lane one weight row.  The reads of a
+  // group are in flight together, then every step runs over all eight (with one column after the other, four reads
+  // ahead, an item of 256 x 128 took 110,000 clocks, most of them one warp's latencies).  MXFP8 rows are packed from
+  // the registers (a block is 32 lanes): in a second pass over y they cost 128 us of 272 at 256 x 28672.
+  static constexpr int COLS = 8;
+  __device__ __forceinline__ static void sum(const TsItem& it, size_t at, float (&v)[COLS]) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) v[i] = __ldcg(it.first + at + i * 128);
-#pragma unroll 2
+    for (int i = 0; i < COLS; ++i) v[i] = __ldcg(it.first + at + i * 128);
+#pragma unroll 1
     for (int k = 1; k < it.parts; ++k) {
       const float* s = it.part(k) + at;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) v[i] += __ldcg(s + i * 128);
+      for (int i = 0; i < COLS; ++i) v[i] += __ldcg(s + i * 128);
     }
   }
   template <bool SHIFT>
   __device__ __forceinline__ static void run(const Args& a, const TsParams& q, const TsItem& it, const float* scale, const float* back,
-                                             uint8_t*, int warp, int lane) {
+                                             uint8_t*, int warp, int warps, int lane) {
     const TsPlan& p = q.p;
     const int blocks = p.dual ? 1 : p.rb;
     const int row = (warp & 3) * 32 + lane;
@@ -150,42 +154,66 @@ struct TsProj {
       if (n >= q.N) continue;
       const float b0 = a.use_bias ? load(a.bias0, n, a.half) : 0.f;
       const float b1 = p.dual && a.use_bias ? load(a.bias1, n, a.half) : 0.f;
-      const float f0 = SHIFT ? back[rb * 128 + row] : 1.f, f1 = SHIFT ? back[128 + row] : 1.f;
-      int c = (warp >> 2) * 4;
-      float v[4], w[4] = {0.f, 0.f, 0.f, 0.f};
-      auto fetch = [&](int c, float (&v)[4], float (&w)[4]) {
-        sum4(it, ((size_t)rb * p.nb + c) * 128 + row, v);
-        if (p.dual) {
-          sum4(it, ((size_t)p.nb + c) * 128 + row, w);
-        } else if (a.use_residual) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i)
-            if (c + i < it.m_count) w[i] = load(a.residual, (size_t)(it.m_base + c + i) * q.N + n, a.half);
-        }
-      };
-      if (c < it.m_count) fetch(c, v, w);
 #pragma unroll 1
-      while (c < it.m_count) {
-        float nv[4], nw[4] = {0.f, 0.f, 0.f, 0.f};
-        if (c + 8 < it.m_count) fetch(c + 8, nv, nw);
+      for (int c = (warp >> 2) * COLS; c < it.m_count; c += (warps >> 2) * COLS) {
+        const int cols = it.m_count - c;                             // (columns past the group: read, not written)
+        const size_t o = (size_t)(it.m_base + c) * q.N + n;
+        float v[COLS], w[COLS];
+        if (a.use_residual) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          if (c + i >= it.m_count) break;
-          const size_t m = it.m_base + c + i, o = m * q.N + n;
-          float d = SHIFT ? v[i] * scale[c + i] * f0 : v[i] * scale[c + i];
-          if (a.raw) { reinterpret_cast<float*>(a.y)[o] = d; continue; }
-          if (p.dual) d = silu(d + b0) * ((SHIFT ? w[i] * scale[c + i] * f1 : w[i] * scale[c + i]) + b1);
-          else d = apply_act(d + b0, a.activation) + w[i];
-          const uint16_t h = a.half ? __half_as_ushort(__float2half_rn(d)) : __bfloat16_as_ushort(__float2bfloat16_rn(d));
-          reinterpret_cast<uint16_t*>(a.y)[o] = h;
-          if (a.mx) {                                // N % 32 == 0: 32 lanes = 32 consecutive channels
-            const float r = a.half ? __half2float(__ushort_as_half(h)) : __uint_as_float((uint32_t)h << 16);
-            mxfp8_block_store(r, lane, a.mx + (m * (q.N >> 5) + (n >> 5)) * 33);
+          for (int i = 0; i < COLS; ++i) w[i] = i < cols ? load(a.residual, o + (size_t)i * q.N, a.half) : 0.f;
+        }
+        sum(it, ((size_t)rb * p.nb + c) * 128 + row, v);
+        if (p.dual) sum(it, ((size_t)p.nb + c) * 128 + row, w);
+        const float f0 = SHIFT ? back[rb * 128 + row] : 1.f;
+#pragma unroll
+        for (int i = 0; i < COLS; ++i) v[i] = SHIFT ? v[i] * scale[c + i] * f0 : v[i] * scale[c + i];
+        if (a.raw) {
+#pragma unroll
+          for (int i = 0; i < COLS; ++i)
+            if (i < cols) reinterpret_cast<float*>(a.y)[o + (size_t)i * q.N] = v[i];
+          continue;
+        }
+        if (p.dual) {
+          const float f1 = SHIFT ? back[128 + row] : 1.f;
+#pragma unroll
+          for (int i = 0; i < COLS; ++i) {
+            const float u = SHIFT ? w[i] * scale[c + i] * f1 : w[i] * scale[c + i];
+            v[i] = silu(v[i] + b0) * (u + b1);
+          }
+        } else {
+#pragma unroll
+          for (int i = 0; i < COLS; ++i) v[i] += b0;
+          if (a.activation == 2) {
+#pragma unroll
+            for (int i = 0; i < COLS; ++i) v[i] = silu(v[i]);
+          } else if (a.activation == 1) {
+#pragma unroll 1
+            for (int h = 0; h < 2; ++h) {                            // (four copies of its code, not eight)
+              float t[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i) { t[i] = gelu_erf_as(v[i]); v[i] = v[i + 4]; }
+#pragma unroll
+              for (int i = 0; i < 4; ++i) v[i + 4] = t[i];
+            }
+          }
+          if (a.use_residual) {
+#pragma unroll
+            for (int i = 0; i < COLS; ++i) v[i] += w[i];
           }
         }
-        c += 8;
 #pragma unroll
-        for (int i = 0; i < 4; ++i) { v[i] = nv[i]; w[i] = nw[i]; }
+        for (int i = 0; i < COLS; ++i) {
+          const uint16_t h = a.half ? __half_as_ushort(__float2half_rn(v[i])) : __bfloat16_as_ushort(__float2bfloat16_rn(v[i]));
+          if (i < cols) reinterpret_cast<uint16_t*>(a.y)[o + (size_t)i * q.N] = h;
+          v[i] = a.half ? __half2float(__ushort_as_half(h)) : __uint_as_float((uint32_t)h << 16);
+        }
+        if (a.mx) {                                                  // N % 32 == 0: 32 lanes = 32 consecutive channels
+          uint8_t* blk = a.mx + ((size_t)(it.m_base + c) * (q.N >> 5) + (n >> 5)) * 33;
+#pragma unroll
+          for (int i = 0; i < COLS; ++i)
+            if (i < cols) mxfp8_block_store(v[i], lane, blk + (size_t)i * (q.N >> 5) * 33);
+        }
       }
     }
   }

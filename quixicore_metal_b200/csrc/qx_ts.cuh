@@ -25,7 +25,7 @@
 // (mxfp4) exponents that way, around the exponent of ordinary weights; a row whose first block lies away from it
 // (the rows of tokens that no training step has touched) is shifted by a power of two of its own, which the output
 // warps take back (ts_row_shift).  Blocks whose scale still leaves the range - more than three decimal orders between the
-// blocks of one row, or |d| >= 512, q6_K 16 - count as zeros and mark their row, and the accumulator warps add their share
+// blocks of one row, or |d| >= 512, q6_K 16 - count as zeros and mark their row, and the output warps add their share
 // to marked rows with fp32 arithmetic (ts_add_left_out).
 //
 // Accumulation.  The tensor core truncates the fp32 accumulator after every MMA; over the K / 16 * TERMS
@@ -61,7 +61,7 @@ constexpr int TS_SUM_WARP = 16, TS_SUM = 4;      // accumulator warps, one per l
 constexpr int TS_OUT_WARP = 20, TS_OUT = 8;      // output warps
 constexpr int TS_MMA_WARP = 28;                  // two MMA issuers, then the loaders
 constexpr int TS_RAW_WARP = 30, TS_ACT_WARP = 31, TS_WARPS = 32;
-constexpr int TS_MARK_RING = 8;                  // segments the workers can be ahead of the accumulator warps: at most 6
+constexpr int TS_MARK_RING = 16;                 // segments the workers can be ahead of the output warps: at most 8
 constexpr int TS_KC = 256;                       // columns per raw stage
 constexpr int TS_MAX_RAW = 8, TS_MAX_ACT = 8, TS_MAX_SLOTS = 16;
 
@@ -98,7 +98,7 @@ struct TsPlan {
   int sums, nd, na;        // TMEM: running sums kept (else: one chunk per segment), chunk buffers, operand slots
   int issuers;             // MMA issuing warps: 2 (one per row block) when each has operand slots of its own
   int nraw;                // raw stages
-  int nact, actq;          // activation stages of 256 columns, each handed over in actq parts (1 or 4)
+  int nact;                // activation stages of 256 columns
   int whole;               // items are not cut between CTAs (no partials)
   unsigned grid;
   size_t smem, off_act, off_aux, off_bar;
@@ -405,14 +405,16 @@ __device__ __forceinline__ int ts_row_of(int P, int L) { return P == 1 ? L : (L 
 // (largest of a block 0.003 to 1.7, mxfp4 6e-6 to 0.7) or the block holds nothing, else what moves e to 114, the middle
 // of the range; no further than TsDec::base stays positive and an exponent of 255 (infinity) out of every range.
 template <int FMT> constexpr bool ts_shifts() { return FMT == F_MXFP8 || FMT == F_MXFP4; }
+// Called by whole warps.
 template <int FMT>
 __device__ __forceinline__ int ts_row_shift(uint32_t e, const uint8_t* row) {
-  if (FMT == F_MXFP8 ? e - 110u <= 9u : e - 107u <= 17u) return 0;
+  const bool far = !(FMT == F_MXFP8 ? e - 110u <= 9u : e - 107u <= 17u) & (e != 255u);
+  if (!__any_sync(0xffffffffu, far)) return 0;
   uint32_t any = 0u;
 #pragma unroll 8
   for (int i = 1; i < TsFmt<FMT>::BB; ++i) any |= __ldg(row + i);
-  if ((any & (FMT == F_MXFP8 ? 0x7Fu : 0x77u)) == 0u || e == 255u) return 0;
-  return min(max(114 - (int)e, (FMT == F_MXFP8 ? 125 : 128) - 254), 95);
+  const int shift = min(max(114 - (int)e, (FMT == F_MXFP8 ? 125 : 128) - 254), 95);
+  return far & ((any & (FMT == F_MXFP8 ? 0x7Fu : 0x77u)) != 0u) ? shift : 0;
 }
 __device__ __forceinline__ float ts_pow2(int n) { return __uint_as_float(n < -126 ? 0x00400000u : (uint32_t)(n + 127) << 23); }   // -127 <= n
 
@@ -429,11 +431,10 @@ __device__ __forceinline__ bool ts_block_left_out(const uint8_t* row, int b, int
   } else {
     const uint8_t* blk = row + (size_t)b * TsFmt<FMT>::BB;
     const uint32_t x = __ldg(blk) - (TsDec<FMT>::BASE - (uint32_t)shift);
-    if (FMT == F_MXFP8 ? x - 9u <= 21u : x - 1u <= 27u) return false;
     uint32_t any = 0u;
 #pragma unroll 1
     for (int i = 1; i < TsFmt<FMT>::BB; ++i) any |= __ldg(blk + i);
-    return (any & (FMT == F_MXFP8 ? 0x7Fu : 0x77u)) != 0u;
+    return !(FMT == F_MXFP8 ? x - 9u <= 21u : x - 1u <= 27u) & ((any & (FMT == F_MXFP8 ? 0x7Fu : 0x77u)) != 0u);
   }
 }
 // weight i of 32-column block b
@@ -457,7 +458,7 @@ __device__ __forceinline__ float ts_weight(const uint8_t* row, int b, int i) {
 }
 // The marked rows of a quadrant (mk: 4 words from one row block to the next) of a segment, over its stored accumulators
 // (`out`: [row block][column][128 rows]), by one warp; a lane takes a column.  Rolled and inline: a call here costs every
-// launch registers (64-row LM heads 5 %), and so much as a look at the marks in the output warps' loop 12 to 20 %.
+// launch registers (64-row LM heads 5 %).
 // 64 rows, mxfp8, 4096 -> 14336, 39.8 us: one block left out of one row 46.8, of 32 rows 241, of 256 rows 325; 256 rows
 // shifted 59.6.  Making whole rows again in fp32 took 244 us for one and 4.2 ms for 32 of them, and an LM head of
 // 128256 with 250 untouched rows 24 ms; now 177 us (166 with ordinary rows).
@@ -468,20 +469,23 @@ __device__ __forceinline__ void ts_add_left_out(const TsParams& q, float* out, c
 #pragma unroll 1
   for (int rb = 0; rb < p.rb; ++rb)
 #pragma unroll 1
-    for (uint32_t bits = mk[rb * 4]; bits; bits &= bits - 1u) {
+    for (uint32_t bits = __reduce_or_sync(0xffffffffu, mk[rb * 4]); bits; bits &= bits - 1u) {
       const int row = ts_row_of(p.P, quad * 32 + __ffs(bits) - 1), n = tile * p.tile_rows + (p.dual ? 0 : rb * 128) + row;
       if (n >= q.N) continue;
       const uint8_t* w = q.w[p.dual ? rb : 0] + (size_t)n * ((size_t)(q.K / TsFmt<FMT>::BK) * TsFmt<FMT>::BB);
       int shift = 0;
       if constexpr (ts_shifts<FMT>()) shift = ts_row_shift<FMT>(__ldg(w), w);
+      const float unit = ts_shifts<FMT>() ? TsFmt<FMT>::ACC_SCALE * ts_pow2(-shift) : TsFmt<FMT>::ACC_SCALE;
 #pragma unroll 1
       for (int b0 = ks0 * 8; b0 < ks1 * 8; b0 += 32) {
-        uint32_t left = __ballot_sync(0xffffffffu, b0 + lane < ks1 * 8 && ts_block_left_out<FMT>(w, b0 + lane, shift));
+        const int bl = min(b0 + lane, ks1 * 8 - 1);
+        uint32_t left = __ballot_sync(0xffffffffu, ts_block_left_out<FMT>(w, bl, shift) & (b0 + lane < ks1 * 8));
 #pragma unroll 1
         for (; left; left &= left - 1u) {
           const int b = b0 + __ffs(left) - 1;
 #pragma unroll 1
-          for (int c = lane; c < m_count; c += 32) {
+          for (int c0 = 0; c0 < m_count; c0 += 32) {
+            const int c = min(c0 + lane, m_count - 1);
             const uint16_t* x = reinterpret_cast<const uint16_t*>(q.x) + (size_t)(m_base + c) * q.K + b * 32;
             float a = 0.f;
 #pragma unroll 1
@@ -489,12 +493,19 @@ __device__ __forceinline__ void ts_add_left_out(const TsParams& q, float* out, c
               a = fmaf(q.x_bf16 ? __uint_as_float((uint32_t)__ldg(x + i) << 16) : __half2float(__ushort_as_half(__ldg(x + i))),
                        ts_weight<FMT>(w, b, i), a);
             float* o = out + ((size_t)rb * p.nb + c) * 128 + row;
-            const float unit = ts_shifts<FMT>() ? TsFmt<FMT>::ACC_SCALE * ts_pow2(-shift) : TsFmt<FMT>::ACC_SCALE;
-            __stcg(o, __ldcg(o) + a / (q.rowscale[m_base + c] * unit));
+            const float v = __ldcg(o) + a / (q.rowscale[m_base + c] * unit);
+            if (c0 + lane < m_count) __stcg(o, v);
           }
         }
       }
     }
+}
+
+// Marks the rows of a warp (bit = lane) that are not `ok`.  Without a branch, see ts_kernel.
+__device__ __forceinline__ void ts_mark(uint32_t* word, bool ok, int lane) {
+  const uint32_t bad = __ballot_sync(0xffffffffu, !ok);
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p red.shared.or.b32 [%0], %1;\n\t}" ::"r"(smem_u32(word)), "r"(bad),
+               "r"(lane == 0 ? bad : 0u) : "memory");
 }
 
 // Position in a ring of n slots: index and phase parity.
@@ -522,9 +533,9 @@ __device__ __forceinline__ int ts_owner(const TsPlan& p, int ctas, long long u) 
 }
 
 // Epi: struct Args; packs_rows(args): writes MXFP8 rows, which a later call may take as its weights;
-//      run<SHIFT>(args, params, item, scale, back, aux, warp, lane), called by the 8 output warps together: the dot product
-//        of column c is the sum of the parts times scale[c], with SHIFT also times back[128 * block + row]; `aux`: shared memory of the policy; barrier 1 (256
-//        threads) is free;
+//      run<SHIFT>(args, params, item, scale, back, aux, warp, warps, lane), called by `warps` warps together (8 or 24): the
+//        dot product of column c is the sum of the parts times scale[c], with SHIFT also times back[128 * block + row];
+//        `aux`: AUX bytes of shared memory of this warp's own;
 //      tail(...) by the output warps after the last item.
 // Code that a launch runs once or twice is kept rolled: it is fetched cold, at about 70 clocks per 8
 // instructions (an epilogue unrolled over 16 columns took 12,000 clocks for its first item).
@@ -654,7 +665,7 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
             if (lane == 0) mbar_arrive(RAW_EMPTY(raw.slot));
             const bool okrow = (dec.d & 0x7C00u) < 0x4C00u;           // |d| < 16
             const uint32_t d2 = okrow ? dec.d * 0x00010001u : 0u;
-            if (!okrow) atomicOr(mk + rb * 4, 1u << lane);
+            ts_mark(mk + rb * 4, okrow, lane);
             uint32_t hi[8], mid[8], lo[8];
             auto put = [&](int s) {
               tmem_st8(op_at0 + 8 * s, hi); tmem_st8(op_at0 + 32 + 8 * s, mid); tmem_st8(op_at0 + 64 + 8 * s, lo);
@@ -710,7 +721,7 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
             okrow = dec.template batch<1>(hi, lo) && okrow; put(1);
             okrow = dec.template batch<2>(hi, lo) && okrow; put(2);
             okrow = dec.template batch<3>(hi, lo) && okrow; put(3);
-            if (!okrow) atomicOr(mk + rb * 4, 1u << lane);
+            if constexpr (FMT != F_NVFP4) ts_mark(mk + rb * 4, okrow, lane);   // (whose scales are never out of range)
             tmem_wait_st();
             tc_fence_before();
             __syncwarp();
@@ -785,14 +796,6 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
         }
       if (!summed) tc_fence_before();
       __syncwarp();
-      if constexpr (FMT != F_NVFP4) {                                 // whose scales are never out of range
-        uint32_t* mk = marks + (nseg & (TS_MARK_RING - 1)) * 8 + quad;
-        if ((mk[0] | mk[4]) != 0u) {
-          ts_add_left_out<FMT>(q, out, mk, quad, tile, rg.grp * p.mg, m_count, ks0, ks1, lane);
-          __syncwarp();
-          if (lane == 0) { mk[0] = 0u; mk[4] = 0u; }
-        }
-      }
       if (lane == 0) {
         mbar_arrive(SEG_FULL(sb));
         if (!summed)
@@ -800,55 +803,7 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
       }
     }
   } else if (warp < TS_MMA_WARP) {
-    // ============================ outputs ============================
-    asm volatile("griddepcontrol.wait;" ::: "memory");                // all below reads or writes what the kernel before may
-    const int ow = warp - TS_OUT_WARP, ot = tid - TS_OUT_WARP * 32;
-    const int m_base = rg.grp * p.mg, m_count = min(p.mg, q.M - m_base);
-    for (int i = ot; i < m_count; i += TS_OUT * 32) scale[i] = q.rowscale[m_base + i] * F::ACC_SCALE;
-    auto sync_out = [] { asm volatile("bar.sync 1, 256;" ::: "memory"); };
-    sync_out();
-    const size_t slot = (size_t)rbn * p.nb * 128;                     // floats of one segment
-    int nseg = 0;
-    for (int u = rg.u0; u < rg.u1; ++nseg) {
-      int tile, ks0, ks1;
-      segment(u, tile, ks0, ks1);
-      const int sb = nseg & 1;
-      const uint8_t* wrow = nullptr;
-      uint32_t e = 0u;
-      if constexpr (ts_shifts<FMT>()) {
-        wrow = row_start(ot >> 7, tile * p.tile_rows + (ot & 127));     // (of the only block, where there is one)
-        e = __ldg(wrow);
-      }
-      wait(SEG_FULL(sb), (uint32_t)(nseg >> 1) & 1u);
-      __syncwarp();
-      if constexpr (ts_shifts<FMT>()) {
-        back[ot] = ts_pow2(-ts_row_shift<FMT>(e, wrow));
-        if (ks0 == 0 && ks1 == nks) sync_out();                       // a cut item has a barrier of its own below
-      }
-      TsItem item{tile, m_base, m_count, q.part + (size_t)(blockIdx.x * 4 + 2 + sb) * slot, nullptr, 0, 1};
-      bool mine = true;
-      if (ks0 > 0 || ks1 < nks) {
-        const int first = ts_owner(p, rg.ctas, (long long)tile * nks), last = ts_owner(p, rg.ctas, (long long)(tile + 1) * nks - 1);
-        unsigned* count = q.count + (size_t)tile * p.groups + rg.grp;
-        if (ot == 0) {
-          // release: the part of this CTA (its writers were waited for above); acquire: the parts of the others
-          unsigned t;
-          asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(count) : "memory");
-          if (t == (unsigned)(last - first)) *count = 0u;
-          *ticket = t;
-        }
-        sync_out();
-        mine = *ticket == (unsigned)(last - first);                   // every other part is in
-        item.first = q.part + (size_t)((first * p.groups + rg.grp) * 4 + 1) * slot;
-        item.rest = q.part + (size_t)(((first + 1) * p.groups + rg.grp) * 4) * slot;
-        item.step = (size_t)p.groups * 4 * slot;
-        item.parts = last - first + 1;
-      }
-      if (mine) Epi::template run<ts_shifts<FMT>()>(ea, q, item, scale, back, smem + p.off_aux, ow, lane);
-      sync_out();                                                     // the ticket and the policy's buffer are free again
-      if (lane == 0) mbar_arrive(SEG_EMPTY(sb));
-    }
-    Epi::tail(ea, q, smem + p.off_aux, ow, lane);
+    // outputs: below
   } else if (warp < TS_RAW_WARP) {
     // ============================ MMA issuers ============================
     const int rb0 = warp - TS_MMA_WARP, iss = p.issuers;
@@ -857,7 +812,6 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
       const uint64_t bdesc0 = umma_desc_plain(sbase + (uint32_t)p.off_act, p.mp);
       const uint32_t bhi = (uint32_t)(bdesc0 >> 32), blo0 = (uint32_t)bdesc0;
       const uint32_t bk = 2u * (uint32_t)p.mp;                        // descriptor step of 16 columns
-      const int actq = p.actq;
       int opb = 4 * rb0;                                              // first operand slot of this warp's next stage
       uint32_t opar = 0u;
       TsRing act{0, 0}, acc{0, 1};                                    // acc: chunk buffer and the parity of its "empty"
@@ -872,25 +826,23 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
           --left;
           const bool closes = left == 0 || ks + 1 == ks1;
           const uint32_t bstage = blo0 + (uint32_t)act.slot * 16u * bk;  // 256 columns = 16 descriptor steps
-          if (actq == 1) wait(ACT_FULL(act.slot), act.par);
+          wait(ACT_FULL(act.slot), act.par);
           for (int rb = rb0; rb < rbn; rb += iss, ++stage_no) {
-            const bool last_block = iss == 2 || rb == rbn - 1;
             const uint32_t d = acc_base + (uint32_t)(acc.slot * acc_cols + rb * p.nb);
             uint32_t fresh = opens ? 0u : 1u;                         // 0: the next MMA starts the accumulator
             if (opens) wait(ACC_EMPTY(acc.slot, rb), acc.par);
+            // One warp's chain of steps bounds the pipeline up to 64 rows: everything that a slot needs advances by a constant.
             const int slot0 = FMT == F_Q6_K ? 2 * (stage_no & 1) : opb;
-            uint32_t blo = bstage;
+            uint32_t bar = OP_FULL(slot0), a = op_base + (uint32_t)(slot0 * SLOT_COLS), blo = bstage;
 #pragma unroll 1
             for (int j = 0; j < 4; ++j, blo += 4 * bk) {
-              const int slot = slot0 + (FMT == F_Q6_K ? j >> 1 : j);
-              if (actq == 4) wait(ACT_FULL(act.slot * 4 + j), act.par);
-              wait(OP_FULL(slot), FMT == F_Q6_K ? (uint32_t)(j & 1) : opar);
+              wait(bar, FMT == F_Q6_K ? (uint32_t)(j & 1) : opar);
               tc_fence_after();
-              ts_mma_slot<TERMS>(d, op_base + (uint32_t)(slot * SLOT_COLS), blo, bhi, bk, idesc, fresh, OP_EMPTY(slot));
+              ts_mma_slot<TERMS>(d, a, blo, bhi, bk, idesc, fresh, bar + 8u * TS_MAX_SLOTS);
               fresh = 1u;
-              if (actq == 4 && last_block) ts_commit_elected(ACT_EMPTY(act.slot * 4 + j));
+              if (FMT != F_Q6_K || (j & 1)) { bar += 8u; a += SLOT_COLS; }
             }
-            if (actq == 1 && last_block) ts_commit_elected(ACT_EMPTY(act.slot));
+            if (iss == 2 || rb == rbn - 1) ts_commit_elected(ACT_EMPTY(act.slot));
             if (closes) ts_commit_elected(ACC_FULL(acc.slot, rb));
             opb += 4 * iss;
             if (opb >= p.na) { opb -= p.na; opar ^= 1u; }
@@ -943,15 +895,15 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
   } else {
     // ============================ activation stages ============================
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const uint32_t bytes = (uint32_t)(TS_KC * p.mp * 2 / p.actq);     // one part
+    const uint32_t bytes = (uint32_t)(TS_KC * p.mp * 2);
     const uint8_t* src = q.img + (size_t)rg.grp * q.K * p.mp * 2;
     TsRing act{0, 0};
     int issued = 0;
-    const int depth = p.nact * p.actq;
+    const int depth = p.nact;
     for (int u = rg.u0; u < rg.u1 && !dead;) {
       int tile, ks0, ks1;
       segment(u, tile, ks0, ks1);
-      for (int a = ks0 * p.actq; a < ks1 * p.actq; ++a) {
+      for (int a = ks0; a < ks1; ++a) {
         if (!wait(ACT_EMPTY(act.slot), act.par ^ 1u)) break;
         if (elect_one()) {
           mbar_arrive_expect_tx(ACT_FULL(act.slot), bytes);
@@ -971,6 +923,86 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
     }
   }
   __syncwarp();
+
+  if ((Epi::HELP && warp < TS_WORKERS) || (warp >= TS_OUT_WARP && warp < TS_MMA_WARP)) {
+    // ============================ outputs ============================
+    // Eight warps turn a segment into outputs while the others work on the next one.  With HELP the workers, which are done
+    // when the last segment is, take their share of it, as it runs with nothing beside it (mxfp4, 256 rows, 8192 -> 28672,
+    // MXFP8 rows out: 112,000 of 343,000 clocks).
+    // It stands behind the roles, and its loops (as all of this kernel's) run on values that are the same for the whole warp
+    // and that the compiler can see to be so - votes and reductions, not what a lane has loaded.  With a loop of each lane's
+    // own count anywhere, or this code among the roles, all roles get by without uniform registers and with a reconvergence
+    // point at every branch, and their chains set the pace (q8_0 and mxfp8, 200 rows, 4096 -> 14336: 103 and 97 us against
+    // 71 and 76; nvfp4, 32 rows: 30 against 21).
+    const bool helper = warp < TS_WORKERS;
+    asm volatile("griddepcontrol.wait;" ::: "memory");                // all below reads or writes what the kernel before may
+    const int ow = helper ? TS_OUT + warp : warp - TS_OUT_WARP, ot = ow * 32 + lane;
+    const int m_base = rg.grp * p.mg, m_count = min(p.mg, q.M - m_base);
+    uint8_t* aux = helper ? smem + warp * Epi::AUX : smem + p.off_aux + ow * Epi::AUX;   // helpers: the idle ring of raw stages
+    if (!helper) {
+      if (ot < m_count) scale[ot] = q.rowscale[m_base + ot] * F::ACC_SCALE;
+      asm volatile("bar.sync 1, 256;" ::: "memory");
+    }
+    const size_t slot = (size_t)rbn * p.nb * 128;                     // floats of one segment
+    int nseg = 0;
+    for (int u = rg.u0; u < rg.u1; ++nseg) {
+      int tile, ks0, ks1;
+      segment(u, tile, ks0, ks1);
+      const bool last = u >= rg.u1, whole = ks0 == 0 && ks1 == nks;
+      if (helper && !last) continue;
+      auto sync_out = [&] {
+        if (Epi::HELP && last) asm volatile("bar.sync 2, %0;" ::"n"((TS_OUT + TS_WORKERS) * 32) : "memory");
+        else asm volatile("bar.sync 1, %0;" ::"n"(TS_OUT * 32) : "memory");
+      };
+      const int sb = nseg & 1;
+      const uint8_t* wrow = nullptr;
+      uint32_t e = 0u;
+      if constexpr (ts_shifts<FMT>()) {
+        if (!helper) {
+          wrow = row_start(ot >> 7, tile * p.tile_rows + (ot & 127));   // (of the only block, where there is one)
+          e = __ldg(wrow);
+        }
+      }
+      wait(SEG_FULL(sb), (uint32_t)(nseg >> 1) & 1u);
+      __syncwarp();
+      if constexpr (ts_shifts<FMT>())
+        if (!helper) back[ot] = ts_pow2(-ts_row_shift<FMT>(e, wrow));
+      if constexpr (FMT != F_NVFP4) {
+        uint32_t* mk = marks + (nseg & (TS_MARK_RING - 1)) * 8 + ow;
+        if (ow < 4 && __any_sync(0xffffffffu, (mk[0] | mk[4]) != 0u)) {   // a warp adds the shares of a quadrant's marked rows
+          const int kind = ks0 > 0 ? 0 : (ks1 < nks ? 1 : 2 + sb);
+          ts_add_left_out<FMT>(q, q.part + (size_t)(blockIdx.x * 4 + kind) * slot, mk, ow, tile, m_base, m_count, ks0, ks1, lane);
+          __syncwarp();
+          if (lane == 0) { mk[0] = 0u; mk[4] = 0u; }
+        }
+      }
+      if ((Epi::HELP && last) || (FMT != F_NVFP4 && whole)) sync_out();   // (a cut item has a barrier of its own below)
+      TsItem item{tile, m_base, m_count, q.part + (size_t)(blockIdx.x * 4 + 2 + sb) * slot, nullptr, 0, 1};
+      bool mine = true;
+      if (!whole) {
+        const int first = ts_owner(p, rg.ctas, (long long)tile * nks), end = ts_owner(p, rg.ctas, (long long)(tile + 1) * nks - 1);
+        unsigned* count = q.count + (size_t)tile * p.groups + rg.grp;
+        if (ot == 0) {
+          // release: the part of this CTA (its writers were waited for above); acquire: the parts of the others
+          unsigned t;
+          asm volatile("atom.add.acq_rel.gpu.global.u32 %0, [%1], 1;" : "=r"(t) : "l"(count) : "memory");
+          if (t == (unsigned)(end - first)) *count = 0u;
+          *ticket = t;
+        }
+        sync_out();
+        mine = *ticket == (unsigned)(end - first);                    // every other part is in
+        item.first = q.part + (size_t)((first * p.groups + rg.grp) * 4 + 1) * slot;
+        item.rest = q.part + (size_t)(((first + 1) * p.groups + rg.grp) * 4) * slot;
+        item.step = (size_t)p.groups * 4 * slot;
+        item.parts = end - first + 1;
+      }
+      if (mine) Epi::template run<ts_shifts<FMT>()>(ea, q, item, scale, back, aux, ow, Epi::HELP && last ? TS_OUT + TS_WORKERS : TS_OUT, lane);
+      if (last) break;
+      sync_out();                                                     // the ticket and the policy's buffer are free again
+      if (lane == 0) mbar_arrive(SEG_EMPTY(sb));
+    }
+    if (!helper) Epi::tail(ea, q, smem + p.off_aux, ow, lane);
+  }
 
   tc_fence_before();
   __syncthreads();

@@ -413,3 +413,20 @@ def test_prepared_rows_with_special_values(fmt, dtype, M, K):
     ulp, step = (2.0 ** -7, 0.0) if dtype == "bf16" else (2.0 ** -10, 2.0 ** -24)
     assert np.all(np.abs(got[3:] - ref) <= np.abs(ref) * ulp * 1.01 + 2e-5 * np.abs(ref).max(1, keepdims=True) + step)
     assert not np.isfinite(got[:2]).any() and np.all(got[3] == 0)
+
+
+# Items of one stage each, several per CTA, with marked rows in all of them: the marks travel from the workers to the output
+# warps, up to eight items behind, and the last item is shared by more warps.
+@pytest.mark.parametrize("M,N", [(40, 148 * 128 * 9 + 5), (64, 4000)])
+@pytest.mark.parametrize("fmt", ["q8_0", "mxfp4"])
+def test_marked_rows_of_short_items(fmt, M, N):
+    K = 256
+    x, W, _, _ = _linear(fmt, M, K, 64, "bf16", M, pack="random")
+    W = np.tile(W, (-(-N // 64), 1, 1))[:N]                  # 64 rows over and over: the same outputs wherever a row lies
+    got = host(tk.decode_linear_epilogue(dev(x, "bf16"), dev(W), None, None, format=fmt))
+    ref = O.decode_linear_epilogue(x, W[:64], fmt, None, None, 0, "bf16")
+    ok = np.isfinite(ref).all(0)
+    assert ok.any()
+    for n in np.nonzero(ok)[0]:
+        assert_close_dtype(got[:, n], ref[:, n], "bf16", scale=float(np.abs(O.dequantize(fmt, W[n:n + 1])).max()) * 30)
+        assert np.all(got[:, n::64] == got[:, n:n + 1])

@@ -285,7 +285,7 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   using G = BQGeom<BITS>;
   constexpr int SLOT_BYTES = G::BOX_BYTES + BQ_VEC_BYTES;
   extern __shared__ __align__(128) uint8_t bq_smem[];
-  const int W = blockDim.x >> 5, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int W = blockDim.x >> 5, warp = warp_index(), lane = threadIdx.x & 31;
   const int g = lane >> 2, t = lane & 3;
   const int K = p.K, nchunks = K / 32, nst = p.nst;
   const int spt1 = (K + BQ_KC - 1) / BQ_KC;
@@ -445,7 +445,7 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   for (int i = 0; i < n_items && !dead; ++i) {
     if (stage < 0 || ++stage == spt1) locate(cur, mat, stage, sidx, trow0);
     const int tl = cur.tl;
-    if (!mbar_wait(mybars + 8 * slot, parity, p.err)) { dead = true; break; }
+    if (!mbar_wait_warp(mybars + 8 * slot, parity, p.err)) { dead = true; break; }
     consumed = i + 1;
     const uint32_t base = myring + slot * SLOT_BYTES;
     if (++slot == nst) { slot = 0; parity ^= 1u; }
@@ -617,7 +617,7 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
   }
   // a warp that gave up still owns copies in flight: wait for them (bounded) before the CTA may exit
   if (dead)
-    for (int i = consumed; i < issued; ++i) mbar_wait(mybars + 8 * (i % nst), (uint32_t)((i / nst) & 1), p.err);
+    for (int i = consumed; i < issued; ++i) mbar_wait_warp(mybars + 8 * (i % nst), (uint32_t)((i / nst) & 1), p.err);
 }
 
 }  // namespace

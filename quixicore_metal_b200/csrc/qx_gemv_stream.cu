@@ -101,7 +101,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
   // A programmatic dependent may be scheduled; it waits for this grid's end before it touches anything but its weights.
   // Packed rows can be such weights, so a launch that writes them lets its dependents start when it is over.
   if (!mx_blocks) asm volatile("griddepcontrol.launch_dependents;");
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_index(), nwarps = blockDim.x >> 5;
   const int g = lane >> 2, t = lane & 3;
   // range of the step list and which matrix of a pair
   const int lw = PAIR ? warp >> 1 : warp, nlw = PAIR ? nwarps >> 1 : nwarps, half = PAIR ? warp & 1 : 0;
@@ -135,7 +135,7 @@ gemv_stream_kernel(const __grid_constant__ CUtensorMap wmap0, const __grid_const
   const float* rs_ptr = rowscale;
   if constexpr (XS) {
     rs_ptr = reinterpret_cast<const float*>(xs_base + (size_t)K * 2);
-    xr[0] = SmemRow{g == 0 ? smem_u32(xs_base) : 0u};
+    xr[0] = SmemRow{smem_u32(xs_base)};
   } else {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {

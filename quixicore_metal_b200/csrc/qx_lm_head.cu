@@ -480,7 +480,7 @@ lmh_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __half* __rest
   using WS = WarpStream<FMT, C::KC, WROWS, C::STAGES>;
   using GP = GroupProc<FMT>;
   extern __shared__ __align__(128) uint8_t smem_raw[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_index();
   const int g = lane >> 2, t = lane & 3;
   // Work items are (vocabulary tile, group of hidden rows) pairs, the group index running fastest
   // so that the CTAs that stream the same tile for different row groups run at the same time and
@@ -525,7 +525,7 @@ lmh_stream_kernel(const __grid_constant__ CUtensorMap wmap, const __half* __rest
     const int row0 = tile * LMH_TILE + warp * WROWS;
     XP xr[NT];
     if constexpr (XS) {
-      xr[0] = SmemRow{g == 0 ? smem_u32(xs_base) : 0u};
+      xr[0] = SmemRow{smem_u32(xs_base)};
     } else {
 #pragma unroll
       for (int nt = 0; nt < NT; ++nt) {

@@ -58,6 +58,17 @@ __device__ __forceinline__ uint32_t mbar_try_wait(uint32_t bar, uint32_t parity)
       : "memory");
   return ok;
 }
+// Number of this warp, known to the compiler to be the same in all its lanes.  What is derived from threadIdx is not: loops
+// whose count hangs on it are compiled as divergent, without uniform registers and with a reconvergence point at every branch.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0); }
+// Bounded wait of a whole warp (a vote and a uniform branch): returns false (and records the failure) if the phase never
+// completes.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t bar, uint32_t parity, int* err_flag) {
+  for (int i = 0; i < (1 << 22); ++i)
+    if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  atomicExch(err_flag, 1);
+  return false;
+}
 // Bounded wait: returns false (and records the failure) if the phase never completes.
 __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* err_flag) {
   for (int i = 0; i < (1 << 22); ++i)
@@ -390,24 +401,28 @@ __device__ __forceinline__ void unit32(const uint32_t (&s)[2 * NSETS], uint32_t 
   }
 }
 
-__device__ __forceinline__ uint4 ldg_or_zero(const __half* row, int off) {
+// Prepared activations of one row in global memory; nullptr (zeros) for the columns of an MMA that have no row, whose reads
+// would cost as much as the others' (4 rows, mxfp4, 8192 -> 14336: 24.0 us, 27.0 with another row's data in their place).
+__device__ __forceinline__ uint4 load_act16(const __half* row, int off) {
   return row ? __ldg(reinterpret_cast<const uint4*>(row + off)) : make_uint4(0u, 0u, 0u, 0u);
 }
-__device__ __forceinline__ uint2 ldg2_or_zero(const __half* row, int off) {
+__device__ __forceinline__ uint2 load_act8(const __half* row, int off) {
   return row ? __ldg(reinterpret_cast<const uint2*>(row + off)) : make_uint2(0u, 0u);
 }
 // A prepared activation row that lives in shared memory (batch 1, prepared by the consuming kernel
-// itself): shared-window address of its first element, 0 = no row.  The group processors take the row
-// pointers as a template type, so the same code reads the row from global memory or from here.
+// itself): shared-window address of its first element.  The group processors take the row
+// pointers as a template type, so the same code reads the row from global memory or from here.  Every column of the MMA gets
+// the one row (only column 0 is used): a predicate and eight zeroed registers per group of columns cost more (nvfp4,
+// 8192 -> 28672: 35.6 us against 33.0).
 struct SmemRow { uint32_t addr; };
-__device__ __forceinline__ uint4 ldg_or_zero(SmemRow row, int off) {
-  uint4 v = make_uint4(0u, 0u, 0u, 0u);
-  if (row.addr) asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(row.addr + 2u * (uint32_t)off));
+__device__ __forceinline__ uint4 load_act16(SmemRow row, int off) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(row.addr + 2u * (uint32_t)off));
   return v;
 }
-__device__ __forceinline__ uint2 ldg2_or_zero(SmemRow row, int off) {
-  uint2 v = make_uint2(0u, 0u);
-  if (row.addr) asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(row.addr + 2u * (uint32_t)off));
+__device__ __forceinline__ uint2 load_act8(SmemRow row, int off) {
+  uint2 v;
+  asm volatile("ld.shared.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "r"(row.addr + 2u * (uint32_t)off));
   return v;
 }
 
@@ -424,7 +439,7 @@ __device__ __forceinline__ void cta_prepare_row(uint8_t* xs_base, const uint16_t
   __half* xs = reinterpret_cast<__half*>(xs_base);
   float* rs_s = reinterpret_cast<float*>(xs_base + (size_t)K * 2);
   float* red = rs_s + 1;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  const int lane = threadIdx.x & 31, warp = warp_index(), nwarps = blockDim.x >> 5;
   const uint4* xv = reinterpret_cast<const uint4*>(xsrc);
   const int nv = K / 8, nt = blockDim.x;
   uint4 keep[ROUNDS];
@@ -449,7 +464,8 @@ __device__ __forceinline__ void cta_prepare_row(uint8_t* xs_base, const uint16_t
 #pragma unroll
   for (int r = 0; r < ROUNDS; ++r)
     if (r * nt < nv) fold(keep[r]);
-  for (int i = threadIdx.x + ROUNDS * nt; i < nv; i += nt) fold(__ldg(xv + i));
+  for (int i = ROUNDS * nt; i < nv; i += nt)                           // (the same count for every lane)
+    if (i + (int)threadIdx.x < nv) fold(__ldg(xv + i + threadIdx.x));
   amax = warp_max(amax);
   if (lane == 0) red[warp] = amax;
   __syncthreads();
@@ -472,7 +488,8 @@ __device__ __forceinline__ void cta_prepare_row(uint8_t* xs_base, const uint16_t
     const int i = threadIdx.x + r * nt;
     if (i < nv) put(i, keep[r]);
   }
-  for (int i = threadIdx.x + ROUNDS * nt; i < nv; i += nt) put(i, __ldg(xv + i));
+  for (int i = ROUNDS * nt; i < nv; i += nt)
+    if (i + (int)threadIdx.x < nv) put(i + threadIdx.x, __ldg(xv + i + threadIdx.x));
   if (threadIdx.x == 0) *rs_s = __uint_as_float((uint32_t)(127 + S) << 23);
   __syncthreads();
 }
@@ -498,7 +515,7 @@ template <int FMT> struct GroupProc {
 #pragma unroll
     for (int u = 0; u < UNITS; ++u)
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) b.v[u][nt] = ldg_or_zero(xr[nt], col + 32 * u + 8 * t);
+      for (int nt = 0; nt < NT; ++nt) b.v[u][nt] = load_act16(xr[nt], col + 32 * u + 8 * t);
   }
   // PRE: the fragments were fetched one group ahead into `b` (small batches); otherwise they are
   // loaded unit by unit from xr / col (large batches, where a whole group would not fit registers).
@@ -511,7 +528,7 @@ template <int FMT> struct GroupProc {
     } else {
       uint4 bb[NT];
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) bb[nt] = ldg_or_zero(xr[nt], col + 32 * J + 8 * t);
+      for (int nt = 0; nt < NT; ++nt) bb[nt] = load_act16(xr[nt], col + 32 * J + 8 * t);
       unit32<FMT, J, NSETS, NT>(s, (uint32_t)(J * F::BB), t, bb, acc);
     }
   }
@@ -534,10 +551,10 @@ template <int FMT> struct GroupProc {
     uint4 nxt[NT];
     if constexpr (J + 1 < UNITS) {
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) nxt[nt] = ldg_or_zero(xr[nt], col + 32 * (J + 1) + 8 * t);
+      for (int nt = 0; nt < NT; ++nt) nxt[nt] = load_act16(xr[nt], col + 32 * (J + 1) + 8 * t);
     } else {
 #pragma unroll
-      for (int nt = 0; nt < NT; ++nt) nxt[nt] = has_next ? ldg_or_zero(xr[nt], col + F::GROUP + 8 * t) : make_uint4(0u, 0u, 0u, 0u);
+      for (int nt = 0; nt < NT; ++nt) nxt[nt] = has_next ? load_act16(xr[nt], col + F::GROUP + 8 * t) : make_uint4(0u, 0u, 0u, 0u);
     }
     unit32<FMT, J, NSETS, NT>(s, (uint32_t)(J * F::BB), t, cur, acc);
 #pragma unroll
@@ -548,7 +565,7 @@ template <int FMT> struct GroupProc {
   __device__ __forceinline__ static void load_first(const XP (&xr)[NT], int col, int t,
                                                     uint4 (&cur)[NT]) {
 #pragma unroll
-    for (int nt = 0; nt < NT; ++nt) cur[nt] = ldg_or_zero(xr[nt], col + 8 * t);
+    for (int nt = 0; nt < NT; ++nt) cur[nt] = load_act16(xr[nt], col + 8 * t);
   }
 };
 
@@ -589,8 +606,8 @@ template <> struct GroupProc<F_NVFP4> {
                                                 BFrag<NT>& b) {
 #pragma unroll
     for (int nt = 0; nt < NT; ++nt) {
-      b.v[0][nt] = ldg_or_zero(xr[nt], col + 16 * t);
-      b.v[1][nt] = ldg_or_zero(xr[nt], col + 16 * t + 8);
+      b.v[0][nt] = load_act16(xr[nt], col + 16 * t);
+      b.v[1][nt] = load_act16(xr[nt], col + 16 * t + 8);
     }
   }
   template <int NSETS, int NT, bool PRE, class XP>
@@ -604,7 +621,7 @@ template <> struct GroupProc<F_NVFP4> {
     for (int nt = 0; nt < NT; ++nt) {
       uint4 b0, b1;
       if constexpr (PRE) { b0 = b.v[0][nt]; b1 = b.v[1][nt]; }
-      else { b0 = ldg_or_zero(xr[nt], col + 16 * t); b1 = ldg_or_zero(xr[nt], col + 16 * t + 8); }
+      else { b0 = load_act16(xr[nt], col + 16 * t); b1 = load_act16(xr[nt], col + 16 * t + 8); }
 #pragma unroll
       for (int set = 0; set < NSETS; ++set) {
         mma_f16(acc[set][nt], a[2 * set][0][0], a[2 * set + 1][0][0], a[2 * set][0][1], a[2 * set + 1][0][1], b0.x, b0.y);
@@ -665,7 +682,7 @@ template <> struct GroupProc<F_Q6_K> {
         for (int g = 0; g < 4; ++g)
 #pragma unroll
           for (int nt = 0; nt < NT; ++nt)
-            bq[g][nt] = ldg2_or_zero(xr[nt], col + 128 * c + 32 * g + 16 * l + 4 * t);
+            bq[g][nt] = load_act8(xr[nt], col + 128 * c + 32 * g + 16 * l + 4 * t);
 #pragma unroll
         for (int r = 0; r < 2 * NSETS; ++r) {
           const uint32_t base = s[r] + boff;
@@ -772,7 +789,7 @@ struct WarpStream {
 
   __device__ __forceinline__ bool wait(int stage, uint32_t parity) {
     if (dead) return false;
-    if (!mbar_wait(bars + 8 * stage, parity, err_flag)) dead = true;
+    if (!mbar_wait_warp(bars + 8 * stage, parity, err_flag)) dead = true;
     return !dead;
   }
 };

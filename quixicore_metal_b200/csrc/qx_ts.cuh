@@ -990,7 +990,7 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
           *ticket = t;
         }
         sync_out();
-        mine = *ticket == (unsigned)(end - first);                    // every other part is in
+        mine = __all_sync(0xffffffffu, *ticket == (unsigned)(end - first));   // every other part is in
         item.first = q.part + (size_t)((first * p.groups + rg.grp) * 4 + 1) * slot;
         item.rest = q.part + (size_t)(((first + 1) * p.groups + rg.grp) * 4) * slot;
         item.step = (size_t)p.groups * 4 * slot;

@@ -156,51 +156,71 @@ __device__ __forceinline__ void lmh_select_token(const float* __restrict__ logit
   }
 }
 
-// The same reduction for up to R hidden rows at once, one warp.  The threshold search is a chain of
-// dependent warp-wide counts (about 25 steps of ~40 cycles each); running R rows through the chain
-// together hides that latency, which is what the per-tile selection of many hidden rows is bound
-// by.  logit[r] = the row's 256 tile logits in shared memory, trow[r] = its row index in the call
-// (< 0: slot unused).  Same results as lmh_select_token row by row.
+__device__ __forceinline__ float float_of_key(uint32_t k) { return __uint_as_float((k & 0x80000000u) ? k & 0x7FFFFFFFu : ~k); }
+
+// The same reduction of R hidden rows at once for a full tile (modes 0 .. 3), one warp: v[r][j] = the row's logit of
+// vocabulary row v0 + 32 j + lane, trow[r] = its row index in the call (< 0: slot unused).  Same results as lmh_select_token
+// row by row.  The threshold search is a chain of dependent warp-wide counts (about 10 steps of ~100 clocks each); running R
+// rows through the chain together hides part of that latency.  Values stay in registers from the accumulators to the
+// partials, maxima go by one reduction of order-preserving keys, and without ties at the threshold one vote per 32
+// elements places them (64 rows, q8_0, 4096 -> 64000, top-k: search and placement were 37 us of 133).
 template <int R>
-__device__ __forceinline__ void lmh_select_rows(const float* const (&logit)[R], const int (&trow)[R],
-                                                int nvalid, int v0, long long vocab_offset,
-                                                const float* __restrict__ bias, int tile,
-                                                long long tiles_stride, int mode, int topk, float invtemp,
-                                                uint32_t seed, float* __restrict__ part_val,
-                                                int32_t* __restrict__ part_id,
-                                                float* __restrict__ part_lse, int lane,
-                                                const LmhMask mask = LmhMask{nullptr, 0, 1}) {
-  if (mode <= 1 || mode == 4 || nvalid < LMH_TILE) {   // cheap modes, masked rows and ragged last tiles: row by row
+__device__ __forceinline__ void lmh_select_values(float (&v)[R][8], const int (&trow)[R], int v0, long long vocab_offset,
+                                                  const float* __restrict__ bias, int tile, long long tiles_stride, int mode, int topk,
+                                                  float invtemp, uint32_t seed, float* __restrict__ part_val,
+                                                  int32_t* __restrict__ part_id, float* __restrict__ part_lse, int lane) {
+  uint32_t key[R][8];
+  if (mode <= 1) {
 #pragma unroll
-    for (int r = 0; r < R; ++r)
-      if (trow[r] >= 0)
-        lmh_select_token(logit[r], nvalid, v0, vocab_offset, bias, trow[r], tile, tiles_stride, mode, topk,
-                         invtemp, seed, part_val, part_id, part_lse, lane, mask);
+    for (int r = 0; r < R; ++r) {
+      if (trow[r] < 0) continue;
+      uint32_t top = 0u;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        float ls = v[r][j] * invtemp;
+        if (bias) ls += bias[v0 + lane + 32 * j];
+        if (mode == 1) ls += rng_gumbel(seed, (uint32_t)trow[r], (uint32_t)(vocab_offset + v0 + lane + 32 * j));
+        key[r][j] = ls >= QX_NEG_INF ? float_key(ls) : 0u;             // NaN and -inf are never taken
+        top = max(top, key[r][j]);
+      }
+      top = __reduce_max_sync(0xffffffffu, top);
+      uint32_t id = 0xFFFFFFFFu;
+#pragma unroll
+      for (int j = 7; j >= 0; --j)
+        if (key[r][j] == top) id = (uint32_t)(vocab_offset + v0 + lane + 32 * j);
+      id = __reduce_min_sync(0xffffffffu, id);                         // lowest id of equals
+      if (lane == 0) {
+        part_val[(size_t)trow[r] * tiles_stride + tile] = top != 0u ? float_of_key(top) : QX_NEG_INF;
+        part_id[(size_t)trow[r] * tiles_stride + tile] = top != 0u ? (int)id : -1;
+      }
+    }
     return;
   }
-  // full tile: every lane holds 8 valid elements per row
-  uint32_t key[R][8];
   uint32_t hi[R], lo[R], ans[R];
   int nb[R];
   int maxnb = 0;
   const int k_eff = min(topk, LMH_TILE);
 #pragma unroll
   for (int r = 0; r < R; ++r) {
-    float mv[8];
+    if (trow[r] < 0) {
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      float ls = trow[r] >= 0 ? logit[r][lane + 32 * j] : 0.f;
-      if (bias) ls += bias[v0 + lane + 32 * j];
-      mv[j] = ls;
+      for (int j = 0; j < 8; ++j) key[r][j] = 0u;
+      ans[r] = 0u;
+      nb[r] = -1;
+      continue;
     }
-    if (mode == 3 && trow[r] >= 0) {
+    if (bias) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[r][j] += bias[v0 + lane + 32 * j];
+    }
+    if (mode == 3) {
       float lmax = QX_NEG_INF;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) lmax = fmaxf(lmax, mv[j] * invtemp);
+      for (int j = 0; j < 8; ++j) lmax = fmaxf(lmax, v[r][j] * invtemp);
       const float gmax = warp_max(lmax);
       float lsum = 0.f;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) lsum += expf(mv[j] * invtemp - gmax);
+      for (int j = 0; j < 8; ++j) lsum += expf(v[r][j] * invtemp - gmax);
       const float gsum = warp_sum(lsum);
       if (lane == 0)
         part_lse[(size_t)trow[r] * tiles_stride + tile] = gsum > 0.f ? gmax + logf(gsum) : QX_NEG_INF;
@@ -208,7 +228,7 @@ __device__ __forceinline__ void lmh_select_rows(const float* const (&logit)[R], 
     uint32_t kmax = 0u, kmin = 0xFFFFFFFFu;
 #pragma unroll
     for (int j = 0; j < 8; ++j) {
-      key[r][j] = float_key(mv[j]);
+      key[r][j] = float_key(v[r][j]);
       kmax = max(kmax, key[r][j]);
       kmin = min(kmin, key[r][j]);
     }
@@ -237,9 +257,9 @@ __device__ __forceinline__ void lmh_select_rows(const float* const (&logit)[R], 
     for (int r = 0; r < R; ++r) {
       if (b < nb[r] && c[r] >= (unsigned)k_eff) {
         ans[r] |= 1u << b;
-        if (c[r] == (unsigned)k_eff) nb[r] = 0;   // exactly k elements lie at or above ans: that is the set
+        if (c[r] == (unsigned)k_eff) nb[r] = -1;  // exactly k elements lie at or above ans: that is the set
       }
-      pending |= nb[r];
+      pending |= nb[r] & ~(nb[r] >> 31);
     }
     if (pending == 0) break;
   }
@@ -248,33 +268,65 @@ __device__ __forceinline__ void lmh_select_rows(const float* const (&logit)[R], 
   for (int r = 0; r < R; ++r) {
     if (trow[r] < 0) continue;
     const size_t pbase = ((size_t)trow[r] * tiles_stride + tile) * topk;
-    unsigned cg = 0;
+    float* pv = part_val + pbase;
+    int32_t* pi = part_id + pbase;
+    const int id0 = (int)(vocab_offset + v0) + lane;
+    unsigned ties_before = 0u, out_pos = 0u, need = 0u;
+    if (nb[r] >= 0) {                                   // perhaps more elements equal to the threshold than are taken
+      unsigned cg = 0;
 #pragma unroll
-    for (int j = 0; j < 8; ++j) cg += key[r][j] > ans[r] ? 1u : 0u;
-    const unsigned need = (unsigned)k_eff - __reduce_add_sync(0xffffffffu, cg);   // ties to take, >= 1
-    unsigned ties_before = 0u, out_pos = 0u;
+      for (int j = 0; j < 8; ++j) cg += key[r][j] > ans[r] ? 1u : 0u;
+      need = (unsigned)k_eff - __reduce_add_sync(0xffffffffu, cg);   // ties to take, >= 1
+    }
 #pragma unroll
     for (int j = 0; j < 8; ++j) {                       // id order = (j, lane) lexicographic
-      const bool eq = key[r][j] == ans[r];
-      const uint32_t bal_eq = __ballot_sync(0xffffffffu, eq);
-      const bool sel = key[r][j] > ans[r] || (eq && ties_before + __popc(bal_eq & lt_mask) < need);
+      bool sel = key[r][j] >= ans[r];
+      if (nb[r] >= 0) {
+        const bool eq = key[r][j] == ans[r];
+        const uint32_t bal_eq = __ballot_sync(0xffffffffu, eq);
+        sel = sel && (!eq || ties_before + __popc(bal_eq & lt_mask) < need);
+        ties_before += __popc(bal_eq);
+      }
       const uint32_t bal = __ballot_sync(0xffffffffu, sel);
       if (sel) {
         const uint32_t pos = out_pos + __popc(bal & lt_mask);
-        float ls = logit[r][lane + 32 * j];
-        if (bias) ls += bias[v0 + lane + 32 * j];
-        part_val[pbase + pos] = ls;
-        part_id[pbase + pos] = (int)(vocab_offset + v0 + lane + 32 * j);
+        pv[pos] = float_of_key(key[r][j]);
+        pi[pos] = id0 + 32 * j;
       }
       out_pos += __popc(bal);
-      ties_before += __popc(bal_eq);
     }
     for (int k0 = (int)out_pos; k0 < topk; k0 += 32) {
       if (k0 + lane >= topk) continue;
-      part_val[pbase + k0 + lane] = QX_NEG_INF;
-      part_id[pbase + k0 + lane] = -1;
+      pv[k0 + lane] = QX_NEG_INF;
+      pi[k0 + lane] = -1;
     }
   }
+}
+
+// ... with the logits in shared memory; masked rows and ragged last tiles row by row.
+template <int R>
+__device__ __forceinline__ void lmh_select_rows(const float* const (&logit)[R], const int (&trow)[R],
+                                                int nvalid, int v0, long long vocab_offset,
+                                                const float* __restrict__ bias, int tile,
+                                                long long tiles_stride, int mode, int topk, float invtemp,
+                                                uint32_t seed, float* __restrict__ part_val,
+                                                int32_t* __restrict__ part_id,
+                                                float* __restrict__ part_lse, int lane,
+                                                const LmhMask mask = LmhMask{nullptr, 0, 1}) {
+  if (mode <= 1 || mode == 4 || nvalid < LMH_TILE) {
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      if (trow[r] >= 0)
+        lmh_select_token(logit[r], nvalid, v0, vocab_offset, bias, trow[r], tile, tiles_stride, mode, topk,
+                         invtemp, seed, part_val, part_id, part_lse, lane, mask);
+    return;
+  }
+  float v[R][8];
+#pragma unroll
+  for (int r = 0; r < R; ++r)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[r][j] = trow[r] >= 0 ? logit[r][lane + 32 * j] : 0.f;
+  lmh_select_values<R>(v, trow, v0, vocab_offset, bias, tile, tiles_stride, mode, topk, invtemp, seed, part_val, part_id, part_lse, lane);
 }
 
 template <int FMT, typename T>
@@ -697,11 +749,11 @@ struct LmhEpi {
 };
 
 // Output policy of the tensor-memory-operand kernel (qx_ts.cuh) for LM-head stage 1: each of the output warps
-// brings the 256 logits of two hidden rows at a time to shared memory and reduces them to their tile
+// brings the 256 logits of two hidden rows at a time to registers and reduces them to their tile
 // partials, while the other roles work on the next tile.
 struct TsLmHead {
   static constexpr bool HELP = true;
-  static constexpr int AUX = 2 * LMH_TILE * 4;               // per warp; the helpers' in the ring of raw stages
+  static constexpr int AUX = LMH_TILE * 4;                   // per warp; the helpers' in the ring of raw stages
   static_assert(TS_WORKERS * AUX <= 2 * 128 * 144, "two raw stages of the narrowest format hold it");
   struct Args {
     const float* bias;
@@ -721,28 +773,43 @@ struct TsLmHead {
     const int v0 = it.tile * LMH_TILE, nvalid = min(LMH_TILE, q.N - v0);
 #pragma unroll 1
     for (int m0 = warp; m0 < it.m_count; m0 += 2 * warps) {
-      const float* rows[2] = {logit, logit + LMH_TILE};
       const int t0 = a.row0 + it.m_base + m0, trow[2] = {t0, m0 + warps < it.m_count ? t0 + warps : -1};
+      float v[2][8];
 #pragma unroll
       for (int r = 0; r < 2; ++r) {
-        const int m = m0 + r * warps;
-        if (m >= it.m_count) break;
-        float v[8];
+        const float* s = it.first + (size_t)(trow[r] >= 0 ? m0 + r * warps : m0) * 128 + lane;
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = __ldcg(it.first + ((size_t)(j >> 2) * q.p.nb + m) * 128 + (j & 3) * 32 + lane);
+        for (int j = 0; j < 8; ++j) v[r][j] = __ldcg(s + (size_t)(j >> 2) * q.p.nb * 128 + (j & 3) * 32);
+      }
 #pragma unroll 1
-        for (int k = 1; k < it.parts; ++k) {
-          const float* s = it.part(k) + (size_t)m * 128 + lane;
+      for (int k = 1; k < it.parts; ++k)
 #pragma unroll
-          for (int j = 0; j < 8; ++j) v[j] += __ldcg(s + (size_t)(j >> 2) * q.p.nb * 128 + (j & 3) * 32);
+        for (int r = 0; r < 2; ++r) {
+          const float* s = it.part(k) + (size_t)(trow[r] >= 0 ? m0 + r * warps : m0) * 128 + lane;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) v[r][j] += __ldcg(s + (size_t)(j >> 2) * q.p.nb * 128 + (j & 3) * 32);
         }
 #pragma unroll
-        for (int j = 0; j < 8; ++j) logit[r * LMH_TILE + j * 32 + lane] = SHIFT ? v[j] * scale[m] * back[j * 32 + lane] : v[j] * scale[m];
+      for (int r = 0; r < 2; ++r) {
+        const float sc = scale[trow[r] >= 0 ? m0 + r * warps : m0];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[r][j] = SHIFT ? v[r][j] * sc * back[j * 32 + lane] : v[r][j] * sc;
       }
-      __syncwarp();
-      lmh_select_rows<2>(rows, trow, nvalid, v0, a.vocab_offset, a.bias, it.tile, a.tiles_stride, a.mode, a.topk, a.invtemp,
-                         a.seed, a.part_val, a.part_id, a.part_lse, lane, a.mask);
-      __syncwarp();
+      if (a.mode <= 3 && nvalid == LMH_TILE) {
+        lmh_select_values<2>(v, trow, v0, a.vocab_offset, a.bias, it.tile, a.tiles_stride, a.mode, a.topk, a.invtemp, a.seed,
+                             a.part_val, a.part_id, a.part_lse, lane);
+      } else {
+#pragma unroll 1
+        for (int r = 0; r < 2; ++r) {
+          if (r == 1 && trow[1] < 0) break;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) logit[j * 32 + lane] = r ? v[1][j] : v[0][j];
+          __syncwarp();
+          lmh_select_token(logit, nvalid, v0, a.vocab_offset, a.bias, r ? trow[1] : trow[0], it.tile, a.tiles_stride, a.mode, a.topk,
+                           a.invtemp, a.seed, a.part_val, a.part_id, a.part_lse, lane, a.mask);
+          __syncwarp();
+        }
+      }
     }
   }
   // padding tiles of a short shard carry absent partials

@@ -430,3 +430,27 @@ def test_marked_rows_of_short_items(fmt, M, N):
     for n in np.nonzero(ok)[0]:
         assert_close_dtype(got[:, n], ref[:, n], "bf16", scale=float(np.abs(O.dequantize(fmt, W[n:n + 1])).max()) * 30)
         assert np.all(got[:, n::64] == got[:, n:n + 1])
+
+
+# Selection above 16 hidden rows: whole logits with many equals at every threshold (lowest ids win), fewer rows than output
+# warps, one more than a pair per warp, a ragged last tile, candidates of -inf.
+@pytest.mark.parametrize("T", [17, 25, 64])
+@pytest.mark.parametrize("mode,k", [("argmax", 0), ("categorical", 0), ("topk", 1), ("topk", 33), ("topp", 5), ("topp", 64)])
+def test_lm_head_ties_above_16_rows(T, mode, k):
+    rng = np.random.default_rng(T + k)
+    V, K = 5 * 256 + 100, 256
+    W = np.zeros((V, K // 32, 34), np.uint8)
+    W[..., 1] = 0x3C                                                          # scale 1.0
+    W[..., 2:] = rng.integers(-2, 3, (V, K // 32, 32)).astype(np.int8).view(np.uint8)
+    h = np.zeros((T, K), np.float32)
+    h[:, ::32] = rng.integers(-1, 2, (T, 8))                                  # logits are whole numbers, about -10 .. 10
+    bias = np.zeros(V, np.float32)
+    bias[rng.integers(0, V, 300)] = -np.inf
+    m = ("argmax", "categorical", "topk", "topp").index(mode)
+    kw = dict(temperature=1.0, seed=11, top_p=0.9)
+    got = host(tk.lm_head_sample(dev(h, "bf16"), dev(W), mode=mode, k=k, bias=dev(bias), format="q8_0", **kw))
+    L = O.lm_head_logits(h, W, "q8_0")
+    want, margin = O.lm_head_sample_from_logits(L, m, k=k if m >= 2 else 0, bias=bias, return_detail=True, **kw)
+    if mode == "argmax":
+        np.testing.assert_array_equal(got, want)
+    check_ids(got, want, margin, 1e-4, mode)

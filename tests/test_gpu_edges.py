@@ -454,3 +454,21 @@ def test_lm_head_ties_above_16_rows(T, mode, k):
     if mode == "argmax":
         np.testing.assert_array_equal(got, want)
     check_ids(got, want, margin, 1e-4, mode)
+
+
+# The merge of top-k candidates: one warp's search up to 512 tiles and 512 candidates, the block's above, ties at the threshold
+# (whole logits) that send it to the exact search by id.
+@pytest.mark.parametrize("V", [2 * 256 + 1, 9 * 256, 512 * 256, 513 * 256 - 5])
+@pytest.mark.parametrize("k,ties", [(1, False), (9, False), (9, True), (64, True), (64, False)])
+def test_top_k_merge(V, k, ties):
+    rng = np.random.default_rng(V + k)
+    T, K = 3, 256
+    W = np.zeros((V, K // 32, 34), np.uint8)
+    W[..., 1] = 0x3C if ties else 0x24                                        # scale 1, 2^-6
+    W[..., 2:] = rng.integers(-3, 4, (V, K // 32, 32)).astype(np.int8).view(np.uint8)
+    h = np.zeros((T, K), np.float32)
+    if ties: h[:, ::32] = rng.integers(-1, 2, (T, 8))
+    else: h = rounded(rng.standard_normal((T, K)), "bf16")
+    got = host(tk.lm_head_sample(dev(h, "bf16"), dev(W), mode="topk", k=k, format="q8_0", temperature=1.0, seed=5))
+    want, margin = O.lm_head_sample_from_logits(O.lm_head_logits(h, W, "q8_0"), 2, k=k, temperature=1.0, seed=5, return_detail=True)
+    check_ids(got, want, margin, 1e-4, "top-k")

@@ -245,12 +245,23 @@ static bool ts_projection_plan(const GemvArgs& a, TsPlan* p) {
   return true;
 }
 
-// Where this kernel takes over from the 16-row streaming kernel (and its passes).  Measured, K = 8192 -> N = 28672 and
-// 4096 -> 4096, us, streaming / this kernel:  nvfp4 16 rows 52 / 40 and 11 / 17; 32 rows (one pass) 102 / 45 and
-// 15 / 20; 64 rows 117 / 59 and 28 / 24.  Its time hardly depends on the rows, but a call pays about 10 us for
-// preparation, start-up and the sum over cut items, so small matrices stay where they are up to 32 rows.  Rows
-// whose byte pitch the streaming kernel cannot take come here at every batch (the alternative is the scalar kernel:
-// mxfp8 K = 1280, 15 rows, gate / up / down of 5888: 512 us).
+// Where this kernel takes over from the 16-row streaming kernel (and its passes).  Its time hardly depends on the rows (and
+// little on the bytes), the other's grows with them, fastest for the formats that cost most to decode.  us, streaming / this
+// kernel:          4096 -> 4096   4096 -> 14336  8192 -> 28672
+//   nvfp4  9 rows    10.3 / 14.9    19.4 / 21.5    47.6 / 40.2
+//         16         11.4 / 15.1    21.0 / 21.5    51.7 / 40.4
+//         32         15.0 / 15.8    29.8 / 22.0   100.8 / 41.5
+//   mxfp4  9         11.9 / 16.1    22.7 / 22.5    64.9 / 46.9
+//         16         13.0 / 16.3    26.7 / 22.7    72.9 / 46.9
+//   mxfp8  9         14.4 / 19.1    30.0 / 29.7    91.0 / 72.6
+//   q4_0  16         11.8 / 16.8    23.4 / 25.4    62.4 / 60.1
+//   q8_0   9         12.2 / 18.0    21.1 / 27.1    57.3 / 63.9
+//         16         13.3 / 18.0    24.5 / 27.2    73.6 / 64.0
+//   q6_K  16         15.4 / 22.8    32.7 / 42.6   102.7 / 123.8
+//         17         17.4 / 23.1    34.8 / 43.4   118.9 / 126.6
+//         32         23.7 / 23.3    54.2 / 43.7   201.3 / 127.1
+// SwiGLU pairs keep the lines that were measured for them.  Rows whose byte pitch the streaming kernel cannot take come
+// here at every batch (the alternative is the scalar kernel: mxfp8 K = 1280, 15 rows, gate / up / down of 5888: 512 us).
 bool ts_preferred(const GemvArgs& a) {
   const int first = options().ts_min_rows;
   if (first > 0) return a.M >= first;
@@ -259,9 +270,12 @@ bool ts_preferred(const GemvArgs& a) {
     return a.M > 16 && !stream_passes_ok(a) && (a.format == F_NVFP4 || !tc_path_ok(a));
   if (a.M > 32) return true;
   if (!stream_path_ok(a) && !stream_passes_ok(a)) return true;
-  if (a.M > 16) return bytes >= (a.w1 ? (16 << 20) : (28 << 20));
-  if (a.M > 8) return bytes >= (a.format == F_MXFP4 || a.format == F_MXFP8 ? (56 << 20) : (100 << 20)) && a.format != F_Q6_K;
-  return false;
+  if (a.M > 16) return bytes >= (a.w1 ? (16 << 20) : (28 << 20)) && !(a.format == F_Q6_K && !a.w1 && a.M <= 20);
+  if (a.M <= 8 || a.format == F_Q6_K) return false;
+  const bool many = a.M >= 12 && !a.w1;
+  if (a.format == F_Q8_0 && !a.w1 && !many) return false;
+  if (a.format == F_MXFP4 || a.format == F_MXFP8) return bytes >= (a.format == F_MXFP4 && many ? (28 << 20) : (56 << 20));
+  return bytes >= (a.format == F_NVFP4 && many ? (64 << 20) : (100 << 20));
 }
 
 size_t ts_scratch_bytes(const GemvArgs& a) {

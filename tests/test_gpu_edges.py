@@ -472,3 +472,14 @@ def test_top_k_merge(V, k, ties):
     got = host(tk.lm_head_sample(dev(h, "bf16"), dev(W), mode="topk", k=k, format="q8_0", temperature=1.0, seed=5))
     want, margin = O.lm_head_sample_from_logits(O.lm_head_logits(h, W, "q8_0"), 2, k=k, temperature=1.0, seed=5, return_detail=True)
     check_ids(got, want, margin, 1e-4, "top-k")
+
+
+# Both sides of the lines in bytes and rows between the streaming kernel and the tensor-memory one
+@pytest.mark.parametrize("fmt,M,K,N", [("mxfp4", 11, 8192, 6784), ("mxfp4", 12, 8192, 6784), ("q6_K", 20, 8192, 4608), ("q6_K", 21, 8192, 4608)])
+def test_lines_between_the_kernels(fmt, M, K, N):
+    x, W, _, _ = _linear(fmt, M, K, 64, "bf16", M)
+    W = np.tile(W, (N // 64, 1, 1))
+    got = host(tk.decode_linear_epilogue(dev(x, "bf16"), dev(W), None, None, format=fmt))
+    ref = O.decode_linear_epilogue(x, W[:64], fmt, None, None, 0, "bf16")
+    for n in range(0, N, 64):
+        assert_close_dtype(got[:, n:n + 64], ref, "bf16")

@@ -411,10 +411,14 @@ __device__ __forceinline__ int ts_row_shift(uint32_t e, const uint8_t* row) {
   const bool far = !(FMT == F_MXFP8 ? e - 110u <= 9u : e - 107u <= 17u) & (e != 255u);
   if (!__any_sync(0xffffffffu, far)) return 0;
   uint32_t any = 0u;
-#pragma unroll 8
-  for (int i = 1; i < TsFmt<FMT>::BB; ++i) any |= __ldg(row + i);
+#pragma unroll 1
+  for (int i = 1; i < TsFmt<FMT>::BB; i += 8) {                      // (rows that hold something show it in their first codes)
+#pragma unroll
+    for (int k = 0; k < 8; ++k) any |= __ldg(row + i + k) & (FMT == F_MXFP8 ? 0x7Fu : 0x77u);
+    if (!__any_sync(0xffffffffu, far & (any == 0u))) break;
+  }
   const int shift = min(max(114 - (int)e, (FMT == F_MXFP8 ? 125 : 128) - 254), 95);
-  return far & ((any & (FMT == F_MXFP8 ? 0x7Fu : 0x77u)) != 0u) ? shift : 0;
+  return far & (any != 0u) ? shift : 0;
 }
 __device__ __forceinline__ float ts_pow2(int n) { return __uint_as_float(n < -126 ? 0x00400000u : (uint32_t)(n + 127) << 23); }   // -127 <= n
 
@@ -459,9 +463,8 @@ __device__ __forceinline__ float ts_weight(const uint8_t* row, int b, int i) {
 // The marked rows of a quadrant (mk: 4 words from one row block to the next) of a segment, over its stored accumulators
 // (`out`: [row block][column][128 rows]), by one warp; a lane takes a column.  Rolled and inline: a call here costs every
 // launch registers (64-row LM heads 5 %).
-// 64 rows, mxfp8, 4096 -> 14336, 39.8 us: one block left out of one row 46.8, of 32 rows 241, of 256 rows 325; 256 rows
-// shifted 59.6.  Making whole rows again in fp32 took 244 us for one and 4.2 ms for 32 of them, and an LM head of
-// 128256 with 250 untouched rows 24 ms; now 177 us (166 with ordinary rows).
+// 64 rows, mxfp8, 4096 -> 14336, 31.4 us: one block left out of one row 36.5, of 32 and 256 rows all over the matrix 39.6 and
+// 40.7.  Making whole rows again in fp32 took 244 us for one and 4.2 ms for 32 of them.
 template <int FMT>
 __device__ __forceinline__ void ts_add_left_out(const TsParams& q, float* out, const uint32_t* mk, int quad, int tile, int m_base, int m_count,
                                                 int ks0, int ks1, int lane) {

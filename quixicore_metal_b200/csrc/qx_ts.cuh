@@ -979,7 +979,9 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
           if (lane == 0) { mk[0] = 0u; mk[4] = 0u; }
         }
       }
-      if ((Epi::HELP && last) || (FMT != F_NVFP4 && whole)) sync_out();   // (a cut item has a barrier of its own below)
+      // Also before the ticket of a cut item: thread 0's release covers the shares that the other warps have added by this barrier,
+      // none that they add after it.
+      if ((Epi::HELP && last) || FMT != F_NVFP4) sync_out();
       TsItem item{tile, m_base, m_count, q.part + (size_t)(blockIdx.x * 4 + 2 + sb) * slot, nullptr, 0, 1};
       bool mine = true;
       if (!whole) {

@@ -311,6 +311,75 @@ def test_rows_with_scales_outside_the_exact_range(fmt, M, K, N, big):
         _lib.set_option("ts_min_rows", 0)
 
 
+# A cut item's part is handed over only when the shares of all its marked rows are in: blocks left out only in the rows that
+# output warps 1 - 3 add (32 - 127 of every 128) and only in the last stages of K, which are the part of a CTA that starts
+# inside an item and goes on with the next one.
+def _marked_parts(fmt, K, seed):
+    x, W, _, _ = _linear(fmt, 64, K, 256, "bf16", seed)
+    nb = W.shape[1]
+    for r in (r for r in range(256) if r % 128 >= 32):
+        for j in range(6):
+            b = nb // 2 + (7 * r + 11 * j) % (nb // 2)
+            if fmt in ("q4_0", "q8_0"):
+                W[r, b, :2] = np.array([600.0 + r], np.float16).view(np.uint8)
+            elif fmt == "q6_K":
+                W[r, b, 208:210] = np.array([16.0 + r], np.float16).view(np.uint8)
+            else:
+                W[r, b, 0] = 130 + r % 8
+    return x, W, O.dequantize(fmt, W).astype(np.float64)
+
+
+def _assert_parts_handed_over(tiles, stages, groups):
+    """Some CTAs hold the end of an item and then the start of another."""
+    ctas = torch.cuda.get_device_properties(0).multi_processor_count // groups
+    first = [tiles * stages * c // ctas for c in range(ctas + 1)]
+    assert sum(a % stages != 0 and b > -(-a // stages) * stages for a, b in zip(first, first[1:])) > 30
+
+
+@pytest.mark.parametrize("fmt", ["q4_0", "q8_0", "q6_K", "mxfp8", "mxfp4"])
+def test_marked_rows_of_parts_handed_over(fmt):
+    M, K, N, reps = 64, 4096, 14336, 8
+    _assert_parts_handed_over(N // 128, K // 256, 1)
+    _assert_parts_handed_over(N // 128, K // 256, 2 if fmt == "q6_K" else 1)     # gate / up pairs
+    x, W, w = _marked_parts(fmt, K, 7)
+    _, U, _, _ = _linear(fmt, M, K, 256, "bf16", 8)
+    wide = lambda a: dev(a).repeat(N // 256, 1, 1)
+    X, Wd, Ud = dev(x, "bf16"), wide(W), wide(U)
+    x = x.astype(np.float64)
+    dots = [x @ w.T, x @ O.dequantize(fmt, U).astype(np.float64).T]
+    sums = [np.abs(x) @ np.abs(w).T, np.abs(x) @ np.abs(O.dequantize(fmt, U)).astype(np.float64).T]
+    # half an ulp of bf16 and the noise of the sums, as in the test above
+    got = [tk.decode_linear_epilogue(X, Wd, None, None, format=fmt) for _ in range(reps)]
+    err = np.abs(host(got[0]).reshape(M, -1, 256) - dots[0][:, None])
+    assert (err <= (2.0 ** -8 * np.abs(dots[0]) + 2e-5 * sums[0])[:, None]).all()
+    assert all(torch.equal(g, got[0]) for g in got)
+    for gate, up, (a, b) in ((Wd, Ud, (0, 1)), (Ud, Wd, (1, 0))):
+        want = dots[a] / (1 + np.exp(-np.clip(dots[a], -700, 700))) * dots[b]
+        tol = 2.0 ** -8 * np.abs(want) + 2e-5 * 1.1 * (sums[a] * np.abs(dots[b]) + sums[b] * np.abs(dots[a]))
+        got = [tk.decode_swiglu(X, gate, up, format=fmt) for _ in range(reps)]
+        assert (np.abs(host(got[0]).reshape(M, -1, 256) - want[:, None]) <= tol[:, None] + 1e-30).all()
+        assert all(torch.equal(g, got[0]) for g in got)
+
+
+@pytest.mark.parametrize("fmt", ["q4_0", "q8_0", "q6_K", "mxfp8", "mxfp4"])
+def test_marked_rows_of_head_parts_handed_over(fmt):
+    T, K, V, reps = 64, 4096, 64 * 256, 8
+    _assert_parts_handed_over(V // 256, K // 256, 2 if fmt == "q6_K" else 1)
+    h, W, w = _marked_parts(fmt, K, 9)
+    h = (h * 2.0 ** -16).astype(np.float32)                  # logits of up to about 100
+    pick = [32, 63, 64, 127, 160, 197, 233, 255]
+    allowed = [[256 * t + r for r in pick] for t in range(T)]                    # hidden row t looks at tile t
+    mask = dev(O.packed_allow_mask(allowed, V).view(np.int32))
+    H, Wd = dev(h, "bf16"), dev(W).repeat(V // 256, 1, 1)
+    got = [tk.lm_head_masked(H, Wd, mask, format=fmt, topk=len(pick)) for _ in range(reps)]
+    logits = h.astype(np.float64) @ w[pick].T
+    noise = 2e-5 * (np.abs(h).astype(np.float64) @ np.abs(w[pick]).T).max(1, keepdims=True)
+    top = np.sort(logits, 1)[:, ::-1]
+    want = top - top[:, :1] - np.log(np.exp(top - top[:, :1]).sum(1, keepdims=True))
+    assert (np.abs(host(got[0][1]) - want) <= 2 * noise + 1e-5 * np.abs(want) + 1e-6).all()
+    assert all(torch.equal(a, b) for g in got for a, b in zip(g, got[0]))
+
+
 # results that fp32 does not hold in units of the scaled activations and weights (2^26 and 2^23 of them, unit
 # activations) from blocks with large e8m0 scales: whole items and cut ones
 @pytest.mark.parametrize("K", [256, 4096])

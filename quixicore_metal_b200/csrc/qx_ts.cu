@@ -1,5 +1,5 @@
-// Host side and projection epilogue of the tensor-memory-operand kernel (qx_ts.cuh): plans, tensor maps,
-// activation preparation, and the launches behind decode_linear_epilogue / decode_swiglu.
+// Host side and projection epilogue of the tensor-memory-operand kernel (qx_ts.cuh): plans, tensor maps, the rule that
+// chooses it, and the launches behind decode_linear_epilogue / decode_swiglu.
 #include "qx_kernels.h"
 #include "qx_tmap.h"
 #include "qx_ts.cuh"
@@ -254,14 +254,29 @@ static bool ts_projection_plan(const GemvArgs& a, TsPlan* p) {
 //   mxfp4  9         11.9 / 16.1    22.7 / 22.5    64.9 / 46.9
 //         16         13.0 / 16.3    26.7 / 22.7    72.9 / 46.9
 //   mxfp8  9         14.4 / 19.1    30.0 / 29.7    91.0 / 72.6
-//   q4_0  16         11.8 / 16.8    23.4 / 25.4    62.4 / 60.1
+//   q4_0   9         11.4 / 16.5    21.9 / 25.3    57.7 / 60.3
+//         16         11.8 / 16.8    23.4 / 25.4    61.2 / 60.2
+//         17         14.6 / 17.1    28.8 / 26.0   137.6 / 61.8
 //   q8_0   9         12.2 / 18.0    21.1 / 27.1    57.3 / 63.9
 //         16         13.3 / 18.0    24.5 / 27.2    73.6 / 64.0
 //   q6_K  16         15.4 / 22.8    32.7 / 42.6   102.7 / 123.8
 //         17         17.4 / 23.1    34.8 / 43.4   118.9 / 126.6
 //         32         23.7 / 23.3    54.2 / 43.7   201.3 / 127.1
-// SwiGLU pairs keep the lines that were measured for them.  Rows whose byte pitch the streaming kernel cannot take come
-// here at every batch (the alternative is the scalar kernel: mxfp8 K = 1280, 15 rows, gate / up / down of 5888: 512 us).
+// At the lines: mxfp4 28 MiB, 12 / 16 rows 22.9 / 23.7 and 24.1 / 23.7, 56 MiB, 9 rows 33.2 / 31.2; nvfp4 64 MiB, 12 / 16 rows
+// 30.0 / 31.2 and 32.6 / 31.1, 100 MiB, 9 rows 38.8 / 35.8; mxfp8 56 MiB, 9 / 16 rows 28.5 / 29.8 and 31.1 / 30.1; q8_0 189 MiB,
+// 12 / 16 rows 49.5 / 56.3 and 54.4 / 56.3, 238 MiB, 12 rows 64.3 / 64.0; from 17 rows 28 MiB nvfp4 23.1 / 21.9, mxfp4 24.7 / 23.1,
+// q4_0 26.3 / 26.3, q8_0 18.7 / 20.7 (34 MiB 22.4 / 22.4), mxfp8 20.9 / 22.4 (33 MiB 24.9 / 23.5); q6_K 20 / 22 rows, 46 MiB
+// 38.9 / 43.0 and 42.9 / 43.1, 92 MiB 66.4 / 71.8 and 72.3 / 71.9 (28 MiB cross at 27 rows, 184 MiB at 19).
+// SwiGLU pairs (bytes of both matrices), 9 and 16 rows, then 17 and 32 rows in 16-row passes:
+//   nvfp4   63 MiB  27.3 / 27.4, 28.8 / 26.6;  45.5 / 27.8, 55.1 / 27.5     100 MiB  34.9 / 35.4, 36.8 / 34.7
+//   mxfp4   68      30.6 / 34.5, 33.4 / 33.8                                119      50.2 / 46.7, 53.9 / 46.1
+//   mxfp8   74      30.4 / 34.3, 31.6 / 33.4                                116      44.9 / 45.3, 46.6 / 44.1
+//   q4_0   126      51.4 / 59.9, 52.3 / 59.0;  84.7 / 62.0, 102.9 / 61.8    252      86.8 / 101.4, 88.9 / 100.5
+//   q8_0   238      55.8 / 64.0, 62.2 / 63.6; 107.5 / 66.2, 129.4 / 68.8    476      97.9 / 111.7, 110.3 / 113.8
+//   q6_K   184      74.5 / 123, 91.6 / 123;    149 / 126, 182 / 127
+//   16 MiB, 17 and 32 rows: nvfp4 22.4 / 19.6, 28.1 / 19.0; q4_0 23.3 / 23.9, 28.7 / 24.7; q8_0 20.6 / 23.0, 23.6 / 22.4
+// Rows whose byte pitch the streaming kernel cannot take come here at every batch (the alternative is the scalar kernel: mxfp8
+// K = 1280, 15 rows, gate / up / down of 5888: 512 us).
 bool ts_preferred(const GemvArgs& a) {
   const int first = options().ts_min_rows;
   if (first > 0) return a.M >= first;
@@ -271,11 +286,15 @@ bool ts_preferred(const GemvArgs& a) {
   if (a.M > 32) return true;
   if (!stream_path_ok(a) && !stream_passes_ok(a)) return true;
   if (a.M > 16) return bytes >= (a.w1 ? (16 << 20) : (28 << 20)) && !(a.format == F_Q6_K && !a.w1 && a.M <= 20);
-  if (a.M <= 8 || a.format == F_Q6_K) return false;
-  const bool many = a.M >= 12 && !a.w1;
-  if (a.format == F_Q8_0 && !a.w1 && !many) return false;
-  if (a.format == F_MXFP4 || a.format == F_MXFP8) return bytes >= (a.format == F_MXFP4 && many ? (28 << 20) : (56 << 20));
-  return bytes >= (a.format == F_NVFP4 && many ? (64 << 20) : (100 << 20));
+  if (a.M <= 8) return false;
+  const bool many = a.M >= 12;
+  switch (a.format) {
+    case F_NVFP4: return bytes >= (many && !a.w1 ? (64 << 20) : (100 << 20));
+    case F_MXFP4: return bytes >= (a.w1 ? (100 << 20) : (many ? (28 << 20) : (56 << 20)));
+    case F_MXFP8: return bytes >= (a.w1 ? (100 << 20) : (56 << 20));
+    case F_Q8_0: return many && !a.w1 && bytes >= (200 << 20);
+    default: return false;
+  }
 }
 
 size_t ts_scratch_bytes(const GemvArgs& a) {

@@ -543,7 +543,7 @@ def test_top_k_merge(V, k, ties):
     check_ids(got, want, margin, 1e-4, "top-k")
 
 
-# Both sides of the lines in bytes and rows between the streaming kernel and the tensor-memory one
+# The same results on both sides of a line between the streaming kernel and the tensor-memory one
 @pytest.mark.parametrize("fmt,M,K,N", [("mxfp4", 11, 8192, 6784), ("mxfp4", 12, 8192, 6784), ("q6_K", 20, 8192, 4608), ("q6_K", 21, 8192, 4608)])
 def test_lines_between_the_kernels(fmt, M, K, N):
     x, W, _, _ = _linear(fmt, M, K, 64, "bf16", M)
@@ -552,3 +552,56 @@ def test_lines_between_the_kernels(fmt, M, K, N):
     ref = O.decode_linear_epilogue(x, W[:64], fmt, None, None, 0, "bf16")
     for n in range(0, N, 64):
         assert_close_dtype(got[:, n:n + 64], ref, "bf16")
+
+
+# Which kernel serves a call, on both sides of the lines in bytes and rows: its sums are those of the streaming kernel (and its
+# passes) or those of the tensor-memory one, which differ in their order.
+def _line(fmt, pair, M, mib, above):
+    from quixicore_metal_b200 import _lib
+    K = 8192
+    bk, bb = O.FORMATS[fmt]
+    N = -(-(mib << 20) // (K // bk * bb * (1 + pair))) - (not above)      # the first number of rows with that many bytes, the last below
+    x, W, _, _ = _linear(fmt, M, K, 64, "f16", M)
+    _, U, _, _ = _linear(fmt, M, K, 64, "f16", M + 1)
+    wide = lambda a, *one: dev(a).repeat(-(-N // 64), *one)[:N]
+    X, Wd, Ud = dev(x, "f16"), wide(W, 1, 1), wide(U, 1, 1) if pair else None
+    # up biases that leave the low bits of the first row's dot products: elsewhere rounding hides the order of the sums
+    gb, ub = np.zeros(64, np.float32), rounded(-(x[0].astype(np.float64) @ O.dequantize(fmt, U).astype(np.float64).T), "f16")
+    run = lambda: (tk.decode_swiglu(X, Wd, Ud, wide(gb).half(), wide(ub).half(), format=fmt) if pair
+                   else tk_torch.decode_linear_partial(X, Wd, fmt))
+    got, kinds = run(), {}
+    try:
+        for kind, rows in (("streaming", 1 << 20), ("tensor memory", 1)):
+            _lib.set_option("ts_min_rows", rows)
+            kinds[kind] = run()
+    finally:
+        _lib.set_option("ts_min_rows", 0)
+    of, x = np.arange(N) % 64, x.astype(np.float64)
+    dots = [x @ O.dequantize(fmt, w).astype(np.float64).T for w in (W, U)]
+    noise = [2e-5 * (np.abs(x) @ np.abs(O.dequantize(fmt, w)).astype(np.float64).T) for w in (W, U)]
+    want, tol = dots[0], noise[0]
+    if pair:                                                 # half an ulp of f16, half a step of its subnormals; |silu'| < 1.1, |silu(g)| <= |g|
+        up = dots[1] + ub
+        want = dots[0] / (1 + np.exp(-dots[0])) * up
+        tol = 2.0 ** -11 * np.abs(want) + 2.0 ** -25 + 1.1 * (noise[0] * np.abs(up) + noise[1] * np.abs(dots[0]))
+    assert (np.abs(host(got) - want[:, of]) <= tol[:, of]).all()
+    assert not torch.equal(kinds["streaming"], kinds["tensor memory"])
+    return [k for k, y in kinds.items() if torch.equal(y, got)]
+
+
+# (format, gate / up pair, rows, MiB of weights)
+@pytest.mark.parametrize("fmt,pair,M,mib", [("mxfp4", 0, 12, 28), ("mxfp4", 0, 9, 56), ("mxfp8", 0, 9, 56), ("nvfp4", 0, 12, 64),
+                                            ("nvfp4", 0, 9, 100), ("q8_0", 0, 12, 200), ("q6_K", 0, 21, 28), ("nvfp4", 1, 9, 100),
+                                            ("mxfp4", 1, 16, 100), ("mxfp8", 1, 9, 100)]
+                         + [(f, 0, 17, 28) for f in FMTS if f != "q6_K"] + [(f, 1, 17, 16) for f in FMTS])
+def test_kernel_at_the_lines(fmt, pair, M, mib):
+    assert _line(fmt, pair, M, mib, True) == ["tensor memory"]
+    assert _line(fmt, pair, M, mib, False) == ["streaming"]
+
+
+# one row fewer, or a format whose streaming kernel is the faster one up to 16 rows
+@pytest.mark.parametrize("fmt,pair,M,mib", [("mxfp4", 0, 11, 28), ("mxfp4", 0, 8, 56), ("mxfp8", 0, 8, 56), ("nvfp4", 0, 11, 64),
+                                            ("nvfp4", 1, 8, 100), ("q8_0", 0, 11, 200), ("q8_0", 1, 16, 200), ("q6_K", 0, 20, 28),
+                                            ("q4_0", 0, 16, 112), ("q4_0", 1, 16, 200), ("q6_K", 1, 16, 100)])
+def test_kernel_one_row_below_the_lines(fmt, pair, M, mib):
+    assert _line(fmt, pair, M, mib, True) == ["streaming"]

@@ -557,6 +557,8 @@ base_q_stream_kernel(const __grid_constant__ CUtensorMap map0, const __grid_cons
       while (*ep != tl) {
         if (++spins > (1 << 22)) { atomicExch(p.err, 1); dead = true; break; }
       }
+      // the lanes give up together: one may see the epoch on its last look and another not, and the waits below are votes
+      dead = __any_sync(0xffffffffu, dead);
       if (dead) break;
     }
     float* slotp = red + rs * 256 + mat * 128;

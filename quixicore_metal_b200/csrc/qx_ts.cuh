@@ -966,7 +966,9 @@ ts_kernel(const __grid_constant__ CUtensorMap map_a0, const __grid_constant__ CU
           e = __ldg(wrow);
         }
       }
-      wait(SEG_FULL(sb), (uint32_t)(nseg >> 1) & 1u);
+      // The helpers have not followed the phases of this barrier (a wait could pass one or two segments early): the output warps
+      // have, and the barrier that both meet at below is what lets the helpers read.
+      if (!helper) wait(SEG_FULL(sb), (uint32_t)(nseg >> 1) & 1u);
       __syncwarp();
       if constexpr (ts_shifts<FMT>())
         if (!helper) back[ot] = ts_pow2(-ts_row_shift<FMT>(e, wrow));

@@ -33,7 +33,7 @@ def test_linear_above_16_rows(fmt, M, K, N):
     assert_close_dtype(host(got), O.decode_linear_epilogue(x, W, fmt, bias, res, 2, dtype), dtype)
 
 
-# random bytes: scales outside the range that the decoded operand holds exactly, whose rows are computed apart
+# random bytes: scales outside the range that the decoded operand holds exactly, whose blocks are added apart
 @pytest.mark.parametrize("fmt,K", [("q4_0", 1024), ("q8_0", 1056), ("q6_K", 512), ("mxfp8", 4096), ("mxfp4", 1056)])
 def test_rows_with_extreme_scales(fmt, K):
     x, W, _, _ = _linear(fmt, 40, K, 136, "bf16", 5, pack="random")
@@ -256,8 +256,8 @@ def test_fresh_rows_as_weight_of_one_row(producer_rows, K, N):
     _rows_as_weight(producer_rows, 1, K, N)
 
 
-# Rows that hold a block whose scale leaves the range in which the decoded f16 operand is exact are made again in fp32, rows
-# that lie outside it as a whole are shifted.  Such blocks in the first and the last stage, in neighbouring rows and in a
+# Blocks whose scale leaves the range in which the decoded f16 operand is exact are added apart in fp32, rows that lie
+# outside it as a whole are shifted.  Such blocks in the first and the last stage, in neighbouring rows and in a
 # whole group of 32, above and below the range; K = 256 leaves items whole, the others are cut between CTAs; K = 256
 # and 768 of the mx formats have pitches that are no multiple of 16 bytes (rows interleaved in 2, 4 or 8 boxes).
 def _wild(fmt, W, n, big):
